@@ -178,9 +178,14 @@ __device__ __forceinline__ void kerr_accel(T x, T y, T z, T k0, T k1, T k2, T k3
     if constexpr (std::is_same<T, float>::value) {
         kerr_accel_f32(x, y, z, k0, k1, k2, k3, a, a0, a1, a2, a3, m);
     } else {
-        // the same contraction as kerr_accel_f32 (derivatives along k from
-        // k . grad r, F_i = l_i F0 + f (k.l)(d_i - D l_i) + f_i (k.l)^2/2),
-        // each operation in T
+        // The contraction of the header comment, reduced by what holds for
+        // this l: q = (r^4 + a^2 z^2) / (2 r^2) gives f = r / q, d_x r = f x / 2
+        // and f' = 3/q - 2 f^2; l.l = 1, l.grad r = 1 and l.grad l = 0 give l.F
+        // without forming the F_i; and F_0 - f (l.F) = -a^0.  With P = x k1 +
+        // y k2 and M = y k1 - x k2 every x-y component is x A + y B, y A - x B
+        // plus a turn of (k1, k2).  74 FP64-pipe instructions and the two
+        // roots and the reciprocal, against ~120 for the nine-derivative form
+        // it replaces (the FP64 kernels' time is that count); equal to rounding.
         const T aa = a * a;
         const T zz = z * z;
         const T kk = T(0.5f) * (x * x + y * y + zz - aa);
@@ -189,57 +194,42 @@ __device__ __forceinline__ void kerr_accel(T x, T y, T z, T k0, T k1, T k2, T k3
         const T rr = Q * iq + kk;                 // sqrt(kk^2 + a^2 z^2) + kk
         const T ir = inv_sqrt(rr);
         const T r = rr * ir;
-        const T i2rq = T(0.5f) * ir * iq;         // 1 / (2 r q)
-        const T den = rr * rr + aa * zz;
         const T rra = rr + aa;
-        // one division for the two reciprocals 1/den and 1/(rr + a^2)
-        const T inv2 = fdiv(T(1.0f), den * rra);
-        const T iden = rra * inv2;
-        const T ira = den * inv2;
-
-        const T c = rr * i2rq;
-        const T rx = c * x, ry = c * y;           // dr/dx, dr/dy
-        const T rz = rra * z * i2rq;
-        const T f = T(2.0f) * (rr * r * iden);
-        const T c1 = T(3.0f) * ir - T(2.0f) * f;
-
-        const T l1 = (r * x + a * y) * ira;
-        const T l2 = (r * y - a * x) * ira;
+        const T ira = fdiv(T(1.0f), rra);
         const T l3 = z * ir;
-        const T tr = T(2.0f) * r;
-        const T g1 = (x - tr * l1) * ira;
-        const T g2 = (y - tr * l2) * ira;
+        const T f = r * iq;
         const T rira = r * ira, aira = a * ira;
+
+        const T P = x * k1 + y * k2, M = y * k1 - x * k2;
+        const T c = T(0.5f) * f;                  // dr/dx = c x, dr/dy = c y
+        const T rz = T(0.5f) * l3 * (rra * iq);   // dr/dz
+        const T Dr = c * P + rz * k3;
+        const T L = rira * P + aira * M;          // l1 k1 + l2 k2
+        const T lv = k0 + (L + l3 * k3);
         const T h = l3 * ir;
-
-        const T Dr = k1 * rx + k2 * ry + k3 * rz;
-        const T fc = f * c1;
-        const T ft = f * (T(2.0f) * aa * z * iden);
-        const T fx = fc * rx, fy = fc * ry, fz = fc * rz - ft;
+        const T G = ira * P - T(2.0f) * rira * L - h * k3;  // k . dl/dr
+        const T Dlv = G * Dr + (rira * (k1 * k1 + k2 * k2) + ir * (k3 * k3));
+        const T fc = T(3.0f) * iq - T(2.0f) * f * f;
+        const T ft = aa * l3 * (iq * iq);
         const T Df = fc * Dr - ft * k3;
-        const T u1 = rira * k1, u2 = rira * k2, v1 = aira * k1, v2 = aira * k2;
-        const T Dl1 = g1 * Dr + (u1 + v2);
-        const T Dl2 = g2 * Dr + (u2 - v1);
-        const T Dl3 = ir * k3 - h * Dr;
-        const T G = g1 * k1 + g2 * k2 - h * k3;
-        const T dlx = rx * G + (u1 - v2);
-        const T dly = ry * G + (v1 + u2);
-        const T dlz = rz * G + ir * k3;
-
-        const T lv = k0 + l1 * k1 + l2 * k2 + l3 * k3;
-        const T Dlv = Dl1 * k1 + Dl2 * k2 + Dl3 * k3;
         const T flv = f * lv;
         const T hl = T(0.5f) * lv * lv;
-        const T F0 = -(Df * lv + f * Dlv);
-        const T F1 = l1 * F0 + flv * (dlx - Dl1) + fx * hl;
-        const T F2 = l2 * F0 + flv * (dly - Dl2) + fy * hl;
-        const T F3 = l3 * F0 + flv * (dlz - Dl3) + fz * hl;
-        const T lF = -F0 + l1 * F1 + l2 * F2 + l3 * F3;
-        const T flF = f * lF;
-        a0 = -F0 + flF;
-        a1 = F1 - l1 * flF;
-        a2 = F2 - l2 * flF;
-        a3 = F3 - l3 * flF;
+        const T mF0 = Df * lv + f * Dlv;          // -F_0
+        const T al = flv * G + fc * hl;
+        const T be = flv * Dr;
+        const T ga = T(2.0f) * flv * aira;
+        const T fth = ft * hl;
+        const T N = rira * M - aira * P;          // l2 k1 - l1 k2
+        const T lF = al + be * (rira + aa * ira * (h * l3)) + (ga * N - l3 * fth);
+        a0 = f * lF + mF0;
+        const T F2 = T(2.0f) * be * rira - a0;
+        const T A = rira * F2 + (al * c - be * ira);
+        const T B = aira * F2;
+        a1 = x * A + (y * B - ga * k2);
+        a2 = y * A + (ga * k1 - x * B);
+        a3 = l3 * (be * ir - a0) + (al * rz - fth);
+        const T l1 = (r * x + a * y) * ira;
+        const T l2 = (r * y - a * x) * ira;
         m.r = r;
         m.f = f;
         m.l1 = l1;
@@ -262,35 +252,44 @@ __device__ __forceinline__ void kerr_accel(T x, T y, T z, T k0, T k1, T k2, T k3
 // k_i = dt F_i, s + k/2 and (k1 + 2k2 + 2k3 + k4)/6 (geodesics.py:317-336)
 // with dt folded into the coefficients -- one fused multiply-add per
 // component and stage instead of a product and a sum (the FP64 form is
-// bound by its FP64 instruction count), equal to rounding.
+// bound by its FP64 instruction count), equal to rounding.  rk4_sum_k1 gives
+// F1 + 2 F2 + 2 F3 + F4 alone.
 template <typename T>
-__device__ __forceinline__ void rk4_step_k1(const T s[8], const T d1[4], T dt, T a, T out[8]) {
+__device__ __forceinline__ void rk4_sum_k1(const T s[8], const T d1[4], T dt, T a, T sum[8]) {
     const T h = T(0.5f) * dt;
-    T acc[8], tmp[8], d0, dd1, d2, d3;
+    T tmp[8], d0, dd1, d2, d3;
     {
         const T F[8] = {s[4], s[5], s[6], s[7], d1[0], d1[1], d1[2], d1[3]};
 #pragma unroll
-        for (int i = 0; i < 8; i++) { acc[i] = F[i]; tmp[i] = s[i] + h * F[i]; }
+        for (int i = 0; i < 8; i++) { sum[i] = F[i]; tmp[i] = s[i] + h * F[i]; }
     }
     kerr_accel(tmp[1], tmp[2], tmp[3], tmp[4], tmp[5], tmp[6], tmp[7], a, d0, dd1, d2, d3);
     {
         const T F[8] = {tmp[4], tmp[5], tmp[6], tmp[7], d0, dd1, d2, d3};
 #pragma unroll
-        for (int i = 0; i < 8; i++) { acc[i] = acc[i] + T(2.0f) * F[i]; tmp[i] = s[i] + h * F[i]; }
+        for (int i = 0; i < 8; i++) { sum[i] = sum[i] + T(2.0f) * F[i]; tmp[i] = s[i] + h * F[i]; }
     }
     kerr_accel(tmp[1], tmp[2], tmp[3], tmp[4], tmp[5], tmp[6], tmp[7], a, d0, dd1, d2, d3);
     {
         const T F[8] = {tmp[4], tmp[5], tmp[6], tmp[7], d0, dd1, d2, d3};
 #pragma unroll
-        for (int i = 0; i < 8; i++) { acc[i] = acc[i] + T(2.0f) * F[i]; tmp[i] = s[i] + dt * F[i]; }
+        for (int i = 0; i < 8; i++) { sum[i] = sum[i] + T(2.0f) * F[i]; tmp[i] = s[i] + dt * F[i]; }
     }
     kerr_accel(tmp[1], tmp[2], tmp[3], tmp[4], tmp[5], tmp[6], tmp[7], a, d0, dd1, d2, d3);
     {
         const T F[8] = {tmp[4], tmp[5], tmp[6], tmp[7], d0, dd1, d2, d3};
-        const T c = dt * sixth<T>();
 #pragma unroll
-        for (int i = 0; i < 8; i++) out[i] = s[i] + c * (acc[i] + F[i]);
+        for (int i = 0; i < 8; i++) sum[i] = sum[i] + F[i];
     }
+}
+
+template <typename T>
+__device__ __forceinline__ void rk4_step_k1(const T s[8], const T d1[4], T dt, T a, T out[8]) {
+    T sum[8];
+    rk4_sum_k1(s, d1, dt, a, sum);
+    const T c = dt * sixth<T>();
+#pragma unroll
+    for (int i = 0; i < 8; i++) out[i] = s[i] + c * sum[i];
 }
 
 // RK4_gen (geodesics.py:317-336) for one ray: out = s + 1/6 (k1+2k2+2k3+k4)
