@@ -2,6 +2,7 @@
 // shadow-bisection pass (geodesics.py), one thread per ray, FP64.
 #include "mk_common.cuh"
 #include "mk_kerr.cuh"
+#include "mk_tri.cuh"
 
 namespace mk {
 
@@ -26,41 +27,83 @@ __global__ void camera_points_kernel(const double *__restrict__ xs, const double
     for (int i = 0; i < 8; i++) s0[8 * p + i] = s[i];
 }
 
-// geodesic_integrator (geodesics.py:246-272) for one ray per thread.
-// rows (N, npx, 8) / dts (N, npx) optional.
-__global__ void __launch_bounds__(GEO_THREADS)
-integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a, int N, double div, double tol,
-                           double *__restrict__ rows, double *__restrict__ dts, int32_t *__restrict__ Kout,
-                           int32_t *__restrict__ why_out, double *__restrict__ state_out) {
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= npx) return;
-    double s[8], nw[8];
+// Ranges in which the triples (mk_tri.cuh) hold every intermediate with all
+// its words inside the float range; a ray outside them is integrated in
+// binary64 from its start (integrate_*_f64).
+constexpr float TRI_MAX_R = 1e6f, TRI_MAX_K = 1e12f, TRI_MIN_K = 1e-6f;
+// distance to the horizon below which a step's accelerations are binary64
+// (see mk_tri.cuh)
+constexpr float TRI_NEAR = 0.1f;
+
+__device__ __forceinline__ bool tri_range(const double s[8]) {
+    const double k = fmax(fmax(fabs(s[4]), fabs(s[5])), fmax(fabs(s[6]), fabs(s[7])));
+    const double x = fmax(fmax(fabs(s[1]), fabs(s[2])), fabs(s[3]));
+    return fabs(s[0]) <= TRI_MAX_R && x <= TRI_MAX_R && k <= TRI_MAX_K && k >= TRI_MIN_K;
+}
+// true out of range or at NaN: a step over the horizon toward r = 0 (the
+// fixed-fraction rule's) overflows floats before doubles
+__device__ __forceinline__ bool tri_left_range(const TriState &s, float r) {
+    const float k = (fabsf(s.K[0].h) + fabsf(s.K[1].h)) + (fabsf(s.K[2].h) + fabsf(s.K[3].h));
+    return !(r <= TRI_MAX_R && k <= TRI_MAX_K);
+}
+
+// one RK4 step of the triple state by its binary64 increment (s: the state)
+__device__ __noinline__ void rk4_step_near(TriState &st, const double s[8], double dt, double a) {
+    double d1[4], sum[8];
+    kerr_accel(s[1], s[2], s[3], s[4], s[5], s[6], s[7], a, d1[0], d1[1], d1[2], d1[3]);
+    rk4_sum_k1(s, d1, dt, a, sum);
+    const double c = dt * SIXTH;
 #pragma unroll
-    for (int i = 0; i < 8; i++) s[i] = s0[8 * p + i];
+    for (int i = 0; i < 4; i++) {
+        st.X[i] = t_add(st.X[i], t_from(c * sum[i]));
+        st.K[i] = t_add(st.K[i], t_from(c * sum[4 + i]));
+    }
+}
+
+// 16-byte stores where the caller's array allows them
+__device__ __forceinline__ void store_row(double *__restrict__ rows, int64_t at, const double s[8]) {
+    if (((uintptr_t)rows & 15) == 0) {
+        double2 *o = reinterpret_cast<double2 *>(rows + at * 8);
+#pragma unroll
+        for (int i = 0; i < 4; i++) o[i] = make_double2(s[2 * i], s[2 * i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) rows[at * 8 + i] = s[i];
+    }
+}
+
+// rows j .. N-1 of a stopped ray: its frozen state, dt = 0
+__device__ __forceinline__ void freeze_rows(double *rows, double *dts, int64_t p, int64_t npx, int j, int N,
+                                            const double s[8]) {
+    for (int r = j; r < N; r++) {
+        if (rows) store_row(rows, (int64_t)r * npx + p, s);
+        if (dts) dts[(int64_t)r * npx + p] = 0.0;
+    }
+}
+
+// geodesic_integrator (geodesics.py:246-272) for one ray, in binary64, from
+// its state s before step j0.  rows (N, npx, 8) / dts (N, npx) optional.
+__device__ __noinline__ void integrate_reference_f64(double s[8], int j0, int64_t p, int64_t npx, double a, int N,
+                                                     double div, double tol, double *rows, double *dts,
+                                                     int32_t *Kout, int32_t *why_out, double *state_out) {
+    double nw[8];
     const double reh = radius_eh(a);
     int K = N, why = MK_RAY_MAXSTEPS;
     // a step's dt is the previous step's dtn (the same radius_cal of the same
     // state), carried instead of recomputed
     int w0;
     double dt = reference_dt(radius_cal(s[1], s[2], s[3], a), reh, div, tol, w0);
-    for (int j = 0; j < N; j++) {
+    for (int j = j0; j < N; j++) {
         int w1;
         rk4_step(s, dt, a, nw);
         const double dtn = reference_dt(radius_cal(nw[1], nw[2], nw[3], a), reh, div, tol, w1);
         if (dtn == 0.0) {
             K = j;
             why = (w0 != MK_RAY_ACTIVE) ? w0 : w1;
-            if (rows)
-                for (int r = j; r < N; r++)
-#pragma unroll
-                    for (int i = 0; i < 8; i++) rows[((int64_t)r * npx + p) * 8 + i] = s[i];
-            if (dts)
-                for (int r = j; r < N; r++) dts[(int64_t)r * npx + p] = 0.0;
+            freeze_rows(rows, dts, p, npx, j, N, s);
             break;
         }
-        if (rows)
-#pragma unroll
-            for (int i = 0; i < 8; i++) rows[((int64_t)j * npx + p) * 8 + i] = s[i];
+        if (rows) store_row(rows, (int64_t)j * npx + p, s);
         if (dts) dts[(int64_t)j * npx + p] = dt;
 #pragma unroll
         for (int i = 0; i < 8; i++) s[i] = nw[i];
@@ -69,24 +112,87 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
     }
     Kout[p] = K;
     why_out[p] = why;
-#pragma unroll
-    for (int i = 0; i < 8; i++) state_out[8 * p + i] = s[i];
+    store_row(state_out, p, s);
 }
 
-// fixed-fraction vacuum policy: h = clamp(hfrac r, hmin, hmax), backwards
+// The same on triples (mk_tri.cuh).  rpw rays a warp: a ray's chain of steps
+// sets the time of a small launch, so its rays are spread over every SM
+// sub-partition before they share warps (lanes that near the horizon hold
+// the others of their warp).
 __global__ void __launch_bounds__(GEO_THREADS)
-integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int N, double hfrac, double hmin,
-                       double hmax, double capture, double r_escape, int32_t *__restrict__ Kout,
-                       int32_t *__restrict__ why_out, double *__restrict__ state_out) {
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= npx) return;
-    double s[8], nw[8];
+integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a, int N, double div, double tol,
+                           double *__restrict__ rows, double *__restrict__ dts, int32_t *__restrict__ Kout,
+                           int32_t *__restrict__ why_out, double *__restrict__ state_out, int rpw, int all_f64) {
+    const int lane = threadIdx.x & 31;
+    const int64_t p = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * rpw + lane;
+    if (lane >= rpw || p >= npx) return;
+    double s64[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) s[i] = s0[8 * p + i];
+    for (int i = 0; i < 8; i++) s64[i] = s0[8 * p + i];
+    bool out = all_f64 || !tri_range(s64);
+    int K = N, why = MK_RAY_MAXSTEPS, j = 0;
+    TriState s;
+    tri_state(s64, s);
+    const SpinTri sp = spin_tri(a);
+    const RuleTri R = rule_tri(a, div, tol);
+    if (!out) {
+        TriPoint q;
+        tri dt = {0.0f, 0.0f, 0.0f};
+        tri_step<true>(s, q, dt, sp.a, sp.aa, sp.aa3, true);
+        float d;
+        int w;
+        bool go = rule_dt(q.r, R, dt, d, w);
+        for (j = 0; j < N; j++) {
+            tri dtn = dt;
+            tri_doubles(s, s64);
+            if (go) {
+                const bool near = d < TRI_NEAR;
+                if (near) {  // through a copy: s itself stays in registers
+                    TriState n = s;
+                    double sc[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) sc[i] = s64[i];
+                    rk4_step_near(n, sc, t_to(dt), a);
+                    s = n;
+                }
+                tri_step<true>(s, q, dt, sp.a, sp.aa, sp.aa3, near);
+                if (tri_left_range(s, q.r.h)) { out = true; break; }
+                go = rule_dt(q.r, R, dtn, d, w);
+            }
+            if (!go) {
+                K = j;
+                why = w;
+                freeze_rows(rows, dts, p, npx, j, N, s64);
+                break;
+            }
+            if (rows) store_row(rows, (int64_t)j * npx + p, s64);
+            if (dts) dts[(int64_t)j * npx + p] = t_to(dt);
+            dt = dtn;
+        }
+    }
+    if (out) {
+        double sc[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) sc[i] = s64[i];
+        integrate_reference_f64(sc, j, p, npx, a, N, div, tol, rows, dts, Kout, why_out, state_out);
+        return;
+    }
+    if (K == N) tri_doubles(s, s64);  // else s64 is the state before the rejected step
+    Kout[p] = K;
+    why_out[p] = why;
+    store_row(state_out, p, s64);
+}
+
+// fixed-fraction vacuum policy: h = clamp(hfrac r, hmin, hmax), backwards, in
+// binary64 from the state before step j0
+__device__ __noinline__ void integrate_fixed_f64(double s[8], int j0, int64_t p, double a, int N, double hfrac,
+                                                 double hmin, double hmax, double capture, double r_escape,
+                                                 int32_t *Kout, int32_t *why_out, double *state_out) {
+    double nw[8];
     const double rcap = capture * radius_eh(a);
     double r = radius_cal(s[1], s[2], s[3], a);
     int st = MK_RAY_MAXSTEPS, j;
-    for (j = 0; j < N; j++) {
+    for (j = j0; j < N; j++) {
         double h = hfrac * r;
         h = h < hmin ? hmin : (h > hmax ? hmax : h);
         rk4_step(s, -h, a, nw);
@@ -100,8 +206,66 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
     }
     Kout[p] = j;
     why_out[p] = st;
+    store_row(state_out, p, s);
+}
+
+__global__ void __launch_bounds__(GEO_THREADS)
+integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int N, double hfrac, double hmin,
+                       double hmax, double capture, double r_escape, int32_t *__restrict__ Kout,
+                       int32_t *__restrict__ why_out, double *__restrict__ state_out, int rpw, int all_f64) {
+    const int lane = threadIdx.x & 31;
+    const int64_t p = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * rpw + lane;
+    if (lane >= rpw || p >= npx) return;
+    double s64[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) state_out[8 * p + i] = s[i];
+    for (int i = 0; i < 8; i++) s64[i] = s0[8 * p + i];
+    bool out = all_f64 || !tri_range(s64);
+    const double reh = radius_eh(a);
+    const tri rcap = t_from(capture * reh), resc = t_from(r_escape), hf = t_from(hfrac), h0 = t_from(hmin),
+              h1 = t_from(hmax);
+    const float near_r = (float)reh + TRI_NEAR;
+    TriState s, last;
+    tri_state(s64, s);
+    last = s;
+    const SpinTri sp = spin_tri(a);
+    int st = MK_RAY_MAXSTEPS, j = 0;
+    const bool started = !out;
+    if (!out) {
+        TriPoint q;
+        tri_step<true>(s, q, {0.0f, 0.0f, 0.0f}, sp.a, sp.aa, sp.aa3, true);
+        for (j = 0; j < N; j++) {
+            tri h = t_add(t_mul(hf, q.r), {0.0f, 0.0f, 0.0f});
+            h = t_less(h, h0) ? h0 : (t_less(h1, h) ? h1 : h);
+            h = t_neg(h);
+            const tri r = q.r;
+            const bool near = r.h < near_r;
+            last = s;
+            if (near) {  // through a copy: s itself stays in registers
+                TriState n = s;
+                double sc[8];
+                tri_doubles(s, sc);
+                rk4_step_near(n, sc, t_to(h), a);
+                s = n;
+            }
+            tri_step<true>(s, q, h, sp.a, sp.aa, sp.aa3, near);
+            if (tri_left_range(s, q.r.h)) { out = true; break; }
+            if (t_less(q.r, rcap)) { st = MK_RAY_CAPTURED; j++; break; }
+            if (t_less(resc, q.r) && t_less(r, q.r)) { st = MK_RAY_ESCAPED; j++; break; }
+        }
+    }
+    if (out) {
+        double sc[8];
+        tri_doubles(last, sc);
+        if (!started)
+#pragma unroll
+            for (int i = 0; i < 8; i++) sc[i] = s64[i];
+        integrate_fixed_f64(sc, j, p, a, N, hfrac, hmin, hmax, capture, r_escape, Kout, why_out, state_out);
+        return;
+    }
+    Kout[p] = j;
+    why_out[p] = st;
+    tri_doubles(s, s64);
+    store_row(state_out, p, s64);
 }
 
 __global__ void radius_kernel(const double *__restrict__ x, int64_t n, int64_t stride, double a,
@@ -115,15 +279,12 @@ __global__ void radius_kernel(const double *__restrict__ x, int64_t n, int64_t s
 // One bisection pass (select_photons_integrator, geodesics.py:354-378):
 // integrate each polar ray with div 40, tol 1e-2 and record what the host
 // needs to evaluate r[argmax(dt) - 1] on the trimmed trajectory.
-__global__ void __launch_bounds__(GEO_THREADS)
-shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa, const double *__restrict__ mid,
-                   int64_t n, double a, double ci, double si, double dist, int N, int32_t *__restrict__ Kout,
-                   int32_t *__restrict__ best_out, double *__restrict__ best_dt_out, double *__restrict__ r_km1,
-                   double *__restrict__ r_best, double *__restrict__ r_last) {
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= n) return;
+__device__ __noinline__ void shadow_ray_f64(const double start[8], int64_t p, double a, int N, int32_t *Kout,
+                                            int32_t *best_out, double *best_dt_out, double *r_km1, double *r_best,
+                                            double *r_last) {
     double s[8], nw[8];
-    camera_pixel(ca[p] * mid[p], sa[p] * mid[p], ci, si, dist, a, s);
+#pragma unroll
+    for (int i = 0; i < 8; i++) s[i] = start[i];
     const double reh = radius_eh(a);
     int K = N, best = -1;
     double best_dt = -INFINITY, r_prev = nan(""), rb = nan(""), rk = nan(""), rl = nan("");
@@ -155,6 +316,84 @@ shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa,
     r_km1[p] = rk;
     r_best[p] = rb;
     r_last[p] = rl;
+}
+
+// The pass on triples, all accelerations in pairs: it stops 1e-2 M from the
+// horizon and its result decides a side of the shadow's edge.
+__global__ void __launch_bounds__(GEO_THREADS)
+shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa, const double *__restrict__ mid,
+                   int64_t n, double a, double ci, double si, double dist, int N, int32_t *__restrict__ Kout,
+                   int32_t *__restrict__ best_out, double *__restrict__ best_dt_out, double *__restrict__ r_km1,
+                   double *__restrict__ r_best, double *__restrict__ r_last, int rpw) {
+    const int lane = threadIdx.x & 31;
+    const int64_t p = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * rpw + lane;
+    if (lane >= rpw || p >= n) return;
+    double s64[8];
+    camera_pixel(ca[p] * mid[p], sa[p] * mid[p], ci, si, dist, a, s64);
+    bool out = !tri_range(s64);
+    TriState s;
+    tri_state(s64, s);
+    const SpinTri sp = spin_tri(a);
+    const RuleTri R = rule_tri(a, 40.0, 1e-2);
+    const tri none = {NAN, NAN, NAN};
+    int K = N, best = -1;
+    tri best_dt = {-INFINITY, 0.0f, 0.0f}, r_prev = none, rb = none, rk = none, rl = none;
+    if (!out) {
+        TriPoint q;
+        tri dt = {0.0f, 0.0f, 0.0f};
+        tri_step<false>(s, q, dt, sp.a, sp.aa, sp.aa3, true);
+        tri r_here = q.r;
+        float d;
+        int w;
+        bool go = rule_dt(q.r, R, dt, d, w);
+        for (int j = 0; j < N; j++) {
+            tri dtn = dt;
+            if (go) {
+                tri_step<false>(s, q, dt, sp.a, sp.aa, sp.aa3, false);
+                if (tri_left_range(s, q.r.h)) { out = true; break; }
+                go = rule_dt(q.r, R, dtn, d, w);
+            }
+            if (!go) {
+                K = j;
+                rk = r_prev;   // row K-1
+                rl = r_here;   // frozen state = every later row
+                break;
+            }
+            if (t_less(best_dt, dt)) { best_dt = dt; best = j; rb = r_prev; }
+            r_prev = r_here;
+            if (j == N - 1) rl = r_here;  // row N-1 = state before step N-1
+            r_here = q.r;
+            dt = dtn;
+        }
+    }
+    if (out) {
+        shadow_ray_f64(s64, p, a, N, Kout, best_out, best_dt_out, r_km1, r_best, r_last);
+        return;
+    }
+    Kout[p] = K;
+    best_out[p] = best;
+    best_dt_out[p] = t_to(best_dt);
+    r_km1[p] = t_to(rk);
+    r_best[p] = t_to(rb);
+    r_last[p] = t_to(rl);
+}
+
+// rays a warp: the fewest (a power of two) with which the launch's warps
+// still fit one to an SM sub-partition, 32 at most
+static int rays_per_warp(int64_t n) {
+    const int64_t slots = (int64_t)device_sm_count() * 4;
+    int w = 1;
+    while (w < 32 && n > slots * w) w *= 2;
+    return w;
+}
+static unsigned ray_grid(int64_t n, int rpw) {
+    const int64_t warps = (n + rpw - 1) / rpw;
+    return (unsigned)((warps + GEO_THREADS / 32 - 1) / (GEO_THREADS / 32));
+}
+// step rules the triples' range covers
+static bool tri_policy(const mk_step_policy &p) {
+    if (p.kind == MK_POLICY_REFERENCE) return p.div >= 1e-2 && p.div <= 1e6 && p.tol >= 1e-12;
+    return p.hfrac >= 1e-6 && p.hfrac <= 1e3 && p.hmin >= 1e-9 && p.hmax >= 1e-9 && p.hmin <= 1e6;
 }
 
 }  // namespace mk
@@ -190,15 +429,17 @@ extern "C" int mk_integrate(const double *s0_dev, int64_t npx, double bhspin, co
     MK_REQUIRE(npx >= 0 && policy->nmax >= 0, MK_ERR_ARG, "mk_integrate: negative size");
     if (npx == 0) return MK_OK;
     cudaStream_t st = as_stream(stream);
+    const int rpw = rays_per_warp(npx);
     if (policy->kind == MK_POLICY_REFERENCE) {
-        integrate_reference_kernel<<<grid_for(npx, GEO_THREADS), GEO_THREADS, 0, st>>>(
-            s0_dev, npx, bhspin, policy->nmax, policy->div, policy->tol, rows_dev, dt_dev, K_dev, why_dev, state_dev);
+        integrate_reference_kernel<<<ray_grid(npx, rpw), GEO_THREADS, 0, st>>>(
+            s0_dev, npx, bhspin, policy->nmax, policy->div, policy->tol, rows_dev, dt_dev, K_dev, why_dev, state_dev,
+            rpw, !tri_policy(*policy));
         MK_LAUNCHED("integrate_reference_kernel");
     } else if (policy->kind == MK_POLICY_FIXED) {
         MK_REQUIRE(!rows_dev && !dt_dev, MK_ERR_UNSUPPORTED, "mk_integrate: rows only for the reference policy");
-        integrate_fixed_kernel<<<grid_for(npx, GEO_THREADS), GEO_THREADS, 0, st>>>(
+        integrate_fixed_kernel<<<ray_grid(npx, rpw), GEO_THREADS, 0, st>>>(
             s0_dev, npx, bhspin, policy->nmax, policy->hfrac, policy->hmin, policy->hmax, policy->capture,
-            policy->r_escape, K_dev, why_dev, state_dev);
+            policy->r_escape, K_dev, why_dev, state_dev, rpw, !tri_policy(*policy));
         MK_LAUNCHED("integrate_fixed_kernel");
     } else {
         MK_REQUIRE(false, MK_ERR_ARG, "mk_integrate: unknown policy %d", (int)policy->kind);
@@ -225,9 +466,10 @@ extern "C" int mk_shadow_pass(const double *cos_dev, const double *sin_dev, cons
                MK_ERR_ARG, "mk_shadow_pass: null pointer");
     MK_REQUIRE(n >= 0 && max_steps >= 1, MK_ERR_ARG, "mk_shadow_pass: bad sizes");
     if (n == 0) return MK_OK;
-    shadow_pass_kernel<<<grid_for(n, GEO_THREADS), GEO_THREADS, 0, as_stream(stream)>>>(
+    const int rpw = rays_per_warp(n);
+    shadow_pass_kernel<<<ray_grid(n, rpw), GEO_THREADS, 0, as_stream(stream)>>>(
         cos_dev, sin_dev, mid_dev, n, bhspin, cos_inc, sin_inc, distance, max_steps, K_dev, best_dev, best_dt_dev,
-        r_km1_dev, r_best_dev, r_last_dev);
+        r_km1_dev, r_best_dev, r_last_dev, rpw);
     MK_LAUNCHED("shadow_pass_kernel");
     return MK_OK;
 }
