@@ -723,6 +723,52 @@ __device__ __forceinline__ void camera_ray(const mk_camera &c, int64_t p, double
                  c.cos_inc, c.sin_inc, c.distance, c.bhspin, s);
 }
 
+// camera_ray for the fused FP64 render: a grid pixel's position and direction
+// rounded as camera_pixel rounds them (the direction's rounding moves a ray
+// by ~1e-10 M at the hole), its null rescaling to rounding of the factor only
+// (_Nullify's quadratic from l.v, its roots and quotients by rsqrt64 and
+// rcp64): ~90 FP64-pipe instructions instead of ~300, which a warp's other
+// lanes wait for at each refill.
+__device__ __forceinline__ void camera_ray_fast(const mk_camera &c, int64_t p, double s[8]) {
+    if (c.kind == MK_CAMERA_EQUATOR) {
+        camera_ray(c, p, s);
+        return;
+    }
+    const int n = c.pixels, ix = (int)(p / n), iy = (int)(p % n);
+    const double x = grid_coord(ix, n, c.fov_lower, c.fov_upper), y = grid_coord(iy, n, c.fov_lower, c.fov_upper);
+    const double ci = c.cos_inc, si = c.sin_inc, dsi = __dmul_rn(c.distance, si), dci = __dmul_rn(c.distance, ci);
+    const double px = __dadd_rn(x, y), py = __dsub_rn(y, x);
+    const double i0 = __dadd_rn(__dmul_rn(-y, ci), dsi), i2 = __dadd_rn(__dmul_rn(y, si), dci);
+    const double p0 = __dadd_rn(__dmul_rn(-py, ci), dsi), p2 = __dadd_rn(__dmul_rn(py, si), dci);
+    const double u0 = __dadd_rn(-i0, dsi), u1 = -x, u2 = __dadd_rn(-i2, dci);
+    const double w0 = __dsub_rn(p0, i0), w1 = __dsub_rn(px, x), w2 = __dsub_rn(p2, i2);
+    const double v1 = __dsub_rn(__dmul_rn(u1, w2), __dmul_rn(u2, w1));
+    const double v2 = __dsub_rn(__dmul_rn(u2, w0), __dmul_rn(u0, w2));
+    const double v3 = __dsub_rn(__dmul_rn(u0, w1), __dmul_rn(u1, w0));
+    // metric data at (i0, x, i2)
+    const double a = c.bhspin, aa = a * a, zz = i2 * i2;
+    const double kk = 0.5 * (i0 * i0 + x * x + zz - aa);
+    const double Q = kk * kk + aa * zz;
+    const double iq = rsqrt64(Q), rr = Q * iq + kk, ir = rsqrt64(rr), r = rr * ir, f = r * iq, ira = rcp64(rr + aa);
+    const double lv = ((r * i0 + a * x) * v1 + (r * x - a * i0) * v2) * ira + i2 * ir * v3;
+    const double A = f - 1.0, b = f * lv, C = v1 * v1 + v2 * v2 + v3 * v3 + b * lv;
+    const double bb = b * b, AC = A * C;
+    const double root = fabs(bb - AC) <= 1e-8 + 1e-5 * fabs(AC) ? 0.0 : sqrt64(bb - AC);
+    const double D = -(b < 0.0 ? b : b + root);
+    const double x1 = D * rcp64(A), x2 = C * rcp64(D);
+    const bool none = isnan(x1) || isnan(x2);
+    const double d1 = fmin(x1, x2), d2 = fmax(x1, x2);
+    const double iS = none ? nan("") : rcp64(d1 > 0.0 ? d1 : (d2 > 0.0 ? d2 : nan("")));
+    s[0] = 0.0;
+    s[1] = i0;
+    s[2] = x;
+    s[3] = i2;
+    s[4] = 1.0;
+    s[5] = v1 * iS;
+    s[6] = v2 * iS;
+    s[7] = v3 * iS;
+}
+
 // initial state of pixel p as float pairs, for the mixed forms: grid
 // cameras in double-float (camera_ray_pair), equator cameras in binary64
 __device__ __forceinline__ void camera_pair(const mk_camera &c, int64_t p, f2 X[4], f2 K[4]) {

@@ -48,10 +48,13 @@
 #include "mk_common.cuh"
 #include "mk_dd.cuh"
 #include "mk_fluid.cuh"
+#include "mk_sample_pair.cuh"
 
 namespace mk {
 
 constexpr int RENDER_THREADS = 128;
+// resident blocks an SM of the FP64 form's kernel
+constexpr int TRI_BLOCKS = 4;
 constexpr double R_FP64 = 3.0;
 constexpr double R_TURN = 6.0;
 // F32_RENULL (the FP32 queue): renormalise each resumed ray to null in
@@ -172,6 +175,7 @@ struct RenderWorkspace {
     unsigned long long steps_c;       // steps the FP32 continuation over the FP32 queue took
     unsigned long long samples_c;     // samples it took
     unsigned long long zone_error;    // bounded waits of the near-hole phase that ran out (images invalid)
+    unsigned long long odd_rays;      // MK_FP64 rays of requests left to the binary64 kernel
 };
 constexpr size_t WS_HEADER = 256;
 static_assert(sizeof(RenderWorkspace) <= WS_HEADER, "workspace header");
@@ -300,40 +304,53 @@ __device__ __forceinline__ void finish_ray(const mk_request &R, int64_t pix, con
 // j = alpha = 0 exactly.
 // row >= 0: also store em and ab at that trajectory row of the request's
 // per-step diagnostic arrays (row < R.rows).
-__device__ __forceinline__ void sample_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
-                                            const KerrPoint<double> &m, double dt_used, double I[MK_MAX_NU],
-                                            double P[MK_MAX_NU], int &nsamples, double &max_tau, int64_t pix,
-                                            int64_t row) {
+// emission_fp64: the coefficients alone, false outside the snapshot.
+__device__ __forceinline__ bool emission_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
+                                              const KerrPoint<double> &m, double em[MK_MAX_NU],
+                                              double ab[MK_MAX_NU]) {
     CellPos c;
-    if (!locate_fast(sv, s[1], s[2], s[3], c)) return;
-    ++nsamples;
+    if (!locate_fast(sv, s[1], s[2], s[3], c)) return false;
     double prim[8];
     trilinear8_fast(sv, c, prim);
     const FluidFrame fs = fluid_frame_m(prim, m, s + 4, R.cos_fallback_pitch);
     // derived quantities (images.py:87-102)
     // quotients as products with rcp64 reciprocals (within a few ulp of the
-    // reference's divisions; the FP64 pipe is this kernel's bound)
+    // reference's divisions; the FP64 pipe is this form's bound)
     const double bsq = fs.b * fs.b;
     const double beta = fs.u * (R.fluid_gamma - 1.) * 2.0 * rcp64(bsq);
     const double sigma = bsq * rcp64(fs.dens);
     const double Th = rlow_rhigh_fast(fs.dens, fs.u, beta, R.r_low, R.r_high, R.electron_gamma_m1, R.ion_gamma_m1);
     const SynchroPre sp = synchro_pre_sin(R.Ne_unit * fs.dens, Th, R.B_unit * fs.b, sin_from_cos(fs.cos_pitch));
-    const double w = -dt_used * R.L_unit;
     const bool cut = sigma > R.sigma_cut;  // images.py:116-118
 #pragma unroll
     for (int ch = 0; ch < MK_MAX_NU; ch++) {
         if (ch < R.nnu) {
             const double nu_obs = R.nu[ch];
-            double em, ab;
-            synchro_eval(sp, -fs.kdotu * nu_obs, true, rcp64(nu_obs), em, ab);
-            if (cut) { em = 0.0; ab = 0.0; }
+            synchro_eval(sp, -fs.kdotu * nu_obs, true, rcp64(nu_obs), em[ch], ab[ch]);
+            if (cut) { em[ch] = 0.0; ab[ch] = 0.0; }
+        }
+    }
+    return true;
+}
+
+__device__ __forceinline__ void sample_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
+                                            const KerrPoint<double> &m, double dt_used, double I[MK_MAX_NU],
+                                            double P[MK_MAX_NU], int &nsamples, double &max_tau, int64_t pix,
+                                            int64_t row) {
+    double em[MK_MAX_NU], ab[MK_MAX_NU];
+    if (!emission_fp64(R, sv, s, m, em, ab)) return;
+    ++nsamples;
+    const double w = -dt_used * R.L_unit;
+#pragma unroll
+    for (int ch = 0; ch < MK_MAX_NU; ch++) {
+        if (ch < R.nnu) {
             if (row >= 0) {
                 const int64_t at = (ch * R.rows + row) * request_pixels(R.camera) + pix;
-                R.rows_em[at] = em;
-                R.rows_ab[at] = ab;
+                R.rows_em[at] = em[ch];
+                R.rows_ab[at] = ab[ch];
             }
-            const double tau = w * ab;
-            I[ch] += (w * em) * P[ch];
+            const double tau = w * ab[ch];
+            I[ch] += (w * em[ch]) * P[ch];
             P[ch] *= (1.0 - tau);
             max_tau = fmax(max_tau, tau);
         }
@@ -546,8 +563,9 @@ __device__ __forceinline__ void fill_req_f32(const mk_request &R, const mk_snaps
 
 
 
-// FP64 render.  SRC_CAMERA: every ray of the job, start to end (MK_FP64).
-// SRC_QUEUE: mixed-form phase B over the FP64 queue; rays leaving R_TURN
+// Binary64 render.  SRC_CAMERA: the rays, start to end, of MK_FP64 requests
+// outside the triples' range (pair_request; render_tri_kernel takes the
+// others).  SRC_QUEUE: mixed-form phase B over the FP64 queue; rays leaving R_TURN
 // outward go to the FP32 queue.  T is the geodesic arithmetic: double, or
 // dd (double-float pairs) for the MK_MIXED_DF variant of phase B.
 template <int SRC, typename T = double>
@@ -559,7 +577,9 @@ render_fp64_kernel(const mk_request *__restrict__ reqs, int nreq, long long tota
         nreq = job->nreq;
         total_camera = job->total_rays;
     }
-    unsigned long long *counter = SRC == SRC_CAMERA ? &ws->counter : &ws->q64_next;
+    // SRC_CAMERA: the rays render_tri_kernel left, usually none
+    if (SRC == SRC_CAMERA && *(volatile unsigned long long *)&ws->odd_rays == 0) return;
+    unsigned long long *counter = &ws->q64_next;
     // lanes not on the stride never take work and stay masked off
     const bool lane_works = ((threadIdx.x & 31) % lane_stride) == 0;
     const long long total =
@@ -578,7 +598,8 @@ render_fp64_kernel(const mk_request *__restrict__ reqs, int nreq, long long tota
         const long long idx = fetch(lane_works && !active && !exhausted, counter, total);
         if (idx == -1) exhausted = true;
         if (!lane_works) exhausted = true;
-        if (idx >= 0 && (SRC != SRC_CAMERA || ray_in_request(reqs, nreq, idx))) {
+        if (idx >= 0 && (SRC != SRC_CAMERA || (ray_in_request(reqs, nreq, idx) &&
+                                               !pair_request(reqs[find_request(reqs, nreq, idx)])))) {
             if (SRC == SRC_CAMERA) {
                 rq = find_request(reqs, nreq, idx);
                 pix = fetch_pixel(reqs[rq].camera, idx - reqs[rq].ray_offset);
@@ -632,7 +653,10 @@ render_fp64_kernel(const mk_request *__restrict__ reqs, int nreq, long long tota
                 active = true;
             }
         }
-        if (!__any_sync(0xffffffffu, active)) break;
+        if (!__any_sync(0xffffffffu, active)) {
+            if (__all_sync(0xffffffffu, exhausted)) break;
+            continue;  // every fetched ray ended at once or was not this kernel's
+        }
         if (active) {
             const mk_request &R = reqs[rq];
             const T a = T(R.camera.bhspin);
@@ -702,6 +726,151 @@ render_fp64_kernel(const mk_request *__restrict__ reqs, int nreq, long long tota
     }
     if (SRC == SRC_QUEUE && fp64_steps) atomicAdd(&ws->steps_fp64, (unsigned long long)fp64_steps);
     if (SRC == SRC_QUEUE && fp64_samples) atomicAdd(&ws->samples_fp64, (unsigned long long)fp64_samples);
+}
+
+// A sample in binary64 for render_tri_kernel: blocks kept in binary64 (ghosts
+// averaged from finer cells) and primitives outside the pairs' range.
+__device__ __noinline__ void coefficients_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
+                                               double em[MK_MAX_NU], double ab[MK_MAX_NU]) {
+    for (int ch = 0; ch < MK_MAX_NU; ch++) em[ch] = ab[ch] = 0.0;
+    emission_fp64(R, sv, s, kerr_point(s[1], s[2], s[3], R.camera.bhspin), em, ab);
+}
+
+// MK_FP64: every ray of the job, start to end, state in 72 bits, geodesic and
+// sampling in float pairs, transfer sums in binary64 (mk_tri.cuh,
+// mk_sample_pair.cuh say why and to what accuracy).  Bound by FP32 issue and
+// latency: ~4.4 k instructions a step and ~1.9 k a sample, against ~50 k
+// cycles of the FP64 pipe for the same step in binary64.
+// A ray's constants and its sums sit in shared memory, one column a thread.
+// lane_stride: lanes that take rays (a small job's rays are spread over every
+// SM sub-partition, where each then runs at its own chain's speed).
+__global__ void __launch_bounds__(RENDER_THREADS, TRI_BLOCKS)
+render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total_camera,
+                  const mk_snapshot_view *__restrict__ snaps, RenderWorkspace *ws, const mk_job *job,
+                  int lane_stride) {
+    __shared__ float s_const[PC_COUNT * RENDER_THREADS];
+    __shared__ double s_I[MK_MAX_NU][RENDER_THREADS], s_P[MK_MAX_NU][RENDER_THREADS];
+    __shared__ float2 s_exp[EXP_STEPS];
+    if (job) {  // request count and ray total from the device (graph replays)
+        nreq = job->nreq;
+        total_camera = job->total_rays;
+    }
+    const int tid = threadIdx.x;
+    if (tid < EXP_STEPS) {
+        const tri t = t_from(exp2(-(double)tid / EXP_STEPS));
+        s_exp[tid] = make_float2(t.h, t.m);
+    }
+    __syncthreads();
+    const PairConsts<RENDER_THREADS> C = {s_const + tid};
+    const bool lane_works = ((tid & 31) % lane_stride) == 0;
+    bool active = false, exhausted = !lane_works;
+    int rq = 0, steps = 0, nsamples = 0;
+    int64_t pix = 0;
+    long long max_tau = 0;  // bits of a double >= 0: they order as integers
+    TriState s;
+    TriPoint q;
+    tri dt = {0.0f, 0.0f, 0.0f};
+
+    for (;;) {
+        const long long idx = fetch(!active && !exhausted, &ws->counter, total_camera);
+        if (idx == -1) exhausted = true;
+        if (idx >= 0 && ray_in_request(reqs, nreq, idx)) {
+            rq = find_request(reqs, nreq, idx);
+            const mk_request &R = reqs[rq];
+            if (!pair_request(R)) {
+                atomicAdd(&ws->odd_rays, 1ull);  // left to render_fp64_kernel
+            } else {
+                pix = fetch_pixel(R.camera, idx - R.ray_offset);
+                double s64[8];
+                camera_ray_fast(R.camera, pix, s64);
+                tri_state(s64, s);
+                pair_consts(R, snaps[R.snapshot], C);
+                steps = nsamples = 0;
+                max_tau = 0;
+#pragma unroll
+                for (int ch = 0; ch < MK_MAX_NU; ch++) { s_I[ch][tid] = 0.0; s_P[ch][tid] = 1.0; }
+                // the first RK4 stage at s also yields r for the step rule
+                tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), true);
+                float d;
+                int why;
+                const RuleTri rule = {C.t(PC_REH), C.t(PC_NINV), C.p(PC_TOL)};
+                const bool go = rule_dt(q.r, rule, dt, d, why);
+                if (!go || R.policy.nmax < 2) {
+                    // stopped before its next step (reference K = steps), or N < 2
+                    // leaves no row pair for the transfer solve
+                    double I[MK_MAX_NU] = {0.0, 0.0, 0.0, 0.0};
+                    finish_ray(R, pix, I, 0, go ? MK_RAY_MAXSTEPS : why, 0, 0.0, ws);
+                } else {
+                    active = true;
+                }
+            }
+        }
+        if (!__any_sync(0xffffffffu, active)) {
+            if (__all_sync(0xffffffffu, exhausted)) break;
+            continue;  // every fetched ray ended at once; more may be left
+        }
+        if (active) {
+            const mk_request &R = reqs[rq];
+            // next step's first stage, evaluated with the step: gives r and the
+            // metric at the new point for the rule and the sample
+            tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), false);
+            float d;
+            int why;
+            tri dtn;
+            const RuleTri rule = {C.t(PC_REH), C.t(PC_NINV), C.p(PC_TOL)};
+            bool done = !rule_dt(q.r, rule, dtn, d, why);
+            if (!done) {  // else the step is rejected and the ray stays frozen (geodesics.py:263-267)
+                ++steps;
+                const bool row = steps < R.rows;
+                if (R.rows_dt && row)  // per-step diagnostics: row `steps` = this state
+                    R.rows_dt[(int64_t)(steps - 1) * request_pixels(R.camera) + pix] = t_to(dt);
+                const mk_snapshot_view &sv = snaps[R.snapshot];
+                const tri x[3] = {s.X[1], s.X[2], s.X[3]};
+                const pr k[4] = {t_pair(s.K[0]), t_pair(s.K[1]), t_pair(s.K[2]), t_pair(s.K[3])};
+                double em[MK_MAX_NU], ab[MK_MAX_NU];
+                int got = sample_pair(sv, C, R.nnu, x, k, q.m, s_exp, em, ab);
+                if (got == PS_BINARY64) {
+                    double s64[8], e64[MK_MAX_NU], a64[MK_MAX_NU];  // copies: em and ab stay in registers
+                    tri_doubles(s, s64);
+                    coefficients_fp64(R, sv, s64, e64, a64);
+#pragma unroll
+                    for (int ch = 0; ch < MK_MAX_NU; ch++) { em[ch] = e64[ch]; ab[ch] = a64[ch]; }
+                }
+                if (got != PS_OUTSIDE) {
+                    ++nsamples;
+                    const double w = -t_to(dt) * R.L_unit;
+#pragma unroll
+                    for (int ch = 0; ch < MK_MAX_NU; ch++) {
+                        if (ch < R.nnu) {
+                            if (R.rows_em && R.rows_dt && row) {
+                                const int64_t at = (ch * R.rows + steps) * request_pixels(R.camera) + pix;
+                                R.rows_em[at] = em[ch];
+                                R.rows_ab[at] = ab[ch];
+                            }
+                            const double tau = w * ab[ch], P = s_P[ch][tid];
+                            s_I[ch][tid] += (w * em[ch]) * P;
+                            s_P[ch][tid] = P * (1.0 - tau);
+                            const long long bits = __double_as_longlong(tau);
+                            max_tau = bits > max_tau ? bits : max_tau;
+                        }
+                    }
+                }
+                dt = dtn;
+                // trajectory rows stop at N-1: step N-1 never reaches the solve
+                if (steps >= R.policy.nmax - 1) {
+                    done = true;
+                    why = MK_RAY_MAXSTEPS;
+                }
+            }
+            if (done) {
+                double I[MK_MAX_NU];
+#pragma unroll
+                for (int ch = 0; ch < MK_MAX_NU; ch++) I[ch] = s_I[ch][tid];
+                finish_ray(R, pix, I, steps, why, nsamples, __longlong_as_double(max_tau), ws);
+                active = false;
+            }
+        }
+    }
 }
 
 __device__ __forceinline__ void finish_ray_f32(const mk_request &R, int64_t pix, const float I[MK_MAX_NU],
@@ -1510,10 +1679,17 @@ static int launch_render(const mk_request *reqs_dev, int32_t nreq, int64_t total
     int rc = phase_mark(st, 0);
     if (rc != MK_OK) return rc;
     if (precision == MK_FP64) {
-        const unsigned grid = persistent_grid(blocks_per_sm(render_fp64_kernel<SRC_CAMERA>, 0), max_rays);
-        render_fp64_kernel<SRC_CAMERA><<<grid, RENDER_THREADS, 0, st>>>(reqs_dev, nreq, (long long)total_rays,
-                                                                        snaps_dev, ws, nullptr, nullptr, 0, 1,
-                                                                        job_dev);
+        // the fewest rays a warp (a power of two) with which every ray has a
+        // lane while one warp runs on each SM sub-partition
+        int stride = 32;
+        while (stride > 1 && max_rays > (int64_t)device_sm_count() * 4 * (32 / stride)) stride /= 2;
+        const unsigned grid = persistent_grid(TRI_BLOCKS, max_rays * stride);
+        render_tri_kernel<<<grid, RENDER_THREADS, 0, st>>>(reqs_dev, nreq, (long long)total_rays, snaps_dev, ws,
+                                                            job_dev, stride);
+        MK_LAUNCHED("render_tri_kernel");
+        render_fp64_kernel<SRC_CAMERA>
+            <<<persistent_grid(blocks_per_sm(render_fp64_kernel<SRC_CAMERA>, 0), max_rays), RENDER_THREADS, 0, st>>>(
+                reqs_dev, nreq, (long long)total_rays, snaps_dev, ws, nullptr, nullptr, 0, 1, job_dev);
         MK_LAUNCHED("render_fp64_kernel");
         return phase_mark(st, 1);
     }

@@ -1,0 +1,365 @@
+// mk_sample_pair.cuh -- the fused FP64 render's sampling and emission on the
+// FP32 pipe, in float pairs (mk_tri.cuh).
+//
+// In binary64 a sample is ~510 FP64-pipe instructions (64-76 cycles of a warp
+// each on GB300, conversions between float and double included): ~35 k
+// cycles, eight times an RK4 step on pairs.  Here it is ~1.9 k FP32
+// instructions to ~2^-47 of each quantity; the emission's exponential keeps
+// its exponent apart, so faint pixels keep their digits, and the transfer
+// sums stay binary64.  A sample's error (~1e-14, times x^(1/3) through the
+// exponential) stays below what the geodesic's rounding leaves in the image
+// (1e-13 to 1e-11): images are no further from plain 64-bit arithmetic than
+// with the binary64 sampler.
+//
+// Identities used (g = eta + f l l, l null): u_i = U_i + f (l.U) l_i, l_mu
+// u^mu = gamma alpha + l.U, b^2 = (B.B + f (l.B)^2 + (B.u)^2) / (u^t)^2, so
+// the frame needs eight dot products and no vector of its own; with Z =
+// nu_s / nu and Y = Z^(1/3) = x^(-1/3) the synchrotron fit (transfer.py:30-86)
+// is Ne const (1 + 2^(11/12) Y)^2 exp(-1/Y) / (2 Theta_e^2 nu), without roots.
+#pragma once
+
+#include "mk_fluid.cuh"
+#include "mk_tri.cuh"
+
+namespace mk {
+
+// A ray's constants, one column of shared memory per thread (registers hold
+// the ray itself).
+enum PairConst {
+    PC_A = 0, PC_AA = 2, PC_AA_L = 4, PC_REH = 5, PC_NINV = 8, PC_TOL = 11, PC_BOX = 13, PC_INVW = 19,
+    PC_GAM2 = 22, PC_RHIGH = 24, PC_RLOW = 26, PC_GEM1 = 28, PC_GIM1 = 30, PC_KTH = 32, PC_SIGMA = 34,
+    PC_NU = 36,  // per frequency: emissivity, nu_s, bx and 1/B_nu factors, 8 floats
+    PC_COUNT = PC_NU + 8 * MK_MAX_NU
+};
+constexpr int EXP_STEPS = 32;  // table of 2^(-j/32)
+
+template <int STRIDE>
+struct PairConsts {
+    float *c;  // this thread's column
+    __device__ __forceinline__ pr p(int i) const { return {c[i * STRIDE], c[(i + 1) * STRIDE]}; }
+    __device__ __forceinline__ tri t(int i) const { return {c[i * STRIDE], c[(i + 1) * STRIDE], c[(i + 2) * STRIDE]}; }
+    __device__ __forceinline__ float f(int i) const { return c[i * STRIDE]; }
+    __device__ __forceinline__ void set(int i, double v, int words) {
+        const tri t = t_from(v);
+        c[i * STRIDE] = t.h;
+        c[(i + 1) * STRIDE] = t.m;
+        if (words > 2) c[(i + 2) * STRIDE] = t.l;
+    }
+};
+
+// the folded constants of the emission at one frequency
+struct EmissionFold {
+    double kem, knus, kbx, kib;
+};
+__device__ __forceinline__ EmissionFold emission_fold(const mk_request &R, double nu) {
+    EmissionFold e;
+    e.kem = (0.5 * SQRT2 * PI * EE2 / THREE_CL) * nu * R.Ne_unit;
+    e.knus = (TWO_NINTHS * EE / TWO_PI_ME_CL) * R.B_unit / nu;
+    e.kbx = HPL * nu / ME_CL_CL;
+    e.kib = CL2 / (TWO_HPL * nu * nu * nu);
+    return e;
+}
+
+// Requests whose constants and step rule leave every pair's low word inside
+// the float range.  Any other request is rendered by the binary64 kernel.
+__device__ __forceinline__ bool pair_request(const mk_request &R) {
+    auto in = [](double v, double lo, double hi) { return fabs(v) >= lo && fabs(v) <= hi; };
+    bool ok = R.policy.div >= 1e-2 && R.policy.div <= 1e6 && R.policy.tol >= 1e-8 && fabs(R.camera.bhspin) <= 1.0 &&
+              fabs(R.camera.distance) <= 1e6 && fabs(R.camera.fov_lower) <= 1e6 && fabs(R.camera.fov_upper) <= 1e6;
+    ok = ok && in(R.fluid_gamma - 1.0, 1e-6, 1e6) && R.r_low >= 0.0 && R.r_low <= 1e6 && R.r_high >= 0.0 &&
+         R.r_high <= 1e6 && R.r_low + R.r_high >= 1e-6 && in(R.electron_gamma_m1, 1e-6, 1e6) &&
+         in(R.ion_gamma_m1, 1e-6, 1e6) && in(R.sigma_cut, 1e-12, 1e12);
+    for (int ch = 0; ch < MK_MAX_NU; ch++)
+        if (ch < R.nnu) {
+            const EmissionFold e = emission_fold(R, R.nu[ch]);
+            ok = ok && in(e.kem, 1e-22, 1e20) && in(e.knus, 1e-20, 1e20) && in(e.kbx, 1e-16, 1e10) &&
+                 in(e.kib, 1e-10, 1e25);
+        }
+    return ok;
+}
+
+template <int STRIDE>
+__device__ __forceinline__ void pair_consts(const mk_request &R, const mk_snapshot_view &sv, PairConsts<STRIDE> C) {
+    const double a = R.camera.bhspin;
+    C.set(PC_A, a, 2);
+    C.set(PC_AA, a * a, 3);  // the third word is PC_AA_L
+    C.set(PC_REH, radius_eh(a), 3);
+    C.set(PC_NINV, -1.0 / R.policy.div, 3);
+    C.set(PC_TOL, R.policy.tol, 2);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        // the block grid's box, widened by more than the float's rounding
+        const double lo = sv.lo[i], hi = sv.lo[i] + sv.nb[i] * sv.width[i], m = 1e-5 * (fabs(lo) + fabs(hi));
+        C.c[(PC_BOX + i) * STRIDE] = (float)(lo - m);
+        C.c[(PC_BOX + 3 + i) * STRIDE] = (float)(hi + m);
+        C.c[(PC_INVW + i) * STRIDE] = (float)(1.0 / sv.width[i]);
+    }
+    C.set(PC_GAM2, 2.0 * (R.fluid_gamma - 1.0), 2);
+    C.set(PC_RHIGH, R.r_high, 2);
+    C.set(PC_RLOW, R.r_low, 2);
+    C.set(PC_GEM1, R.electron_gamma_m1, 2);
+    C.set(PC_GIM1, R.ion_gamma_m1, 2);
+    C.set(PC_KTH, (MP * CL2 / ME_CL_CL) * R.electron_gamma_m1 * R.ion_gamma_m1, 2);
+    C.set(PC_SIGMA, R.sigma_cut, 2);
+#pragma unroll
+    for (int ch = 0; ch < MK_MAX_NU; ch++)
+        if (ch < R.nnu) {
+            const EmissionFold e = emission_fold(R, R.nu[ch]);
+            C.set(PC_NU + 8 * ch, e.kem, 2);
+            C.set(PC_NU + 8 * ch + 2, e.knus, 2);
+            C.set(PC_NU + 8 * ch + 4, e.kbx, 2);
+            C.set(PC_NU + 8 * ch + 6, e.kib, 2);
+        }
+}
+
+// The cell of x: the block whose faces enclose it (left < x <= right, to 48
+// bits) and the ghost-shifted index and offset in it (locate_fast).  The
+// candidate comes from the float coordinate; its own cell coordinate t, faces
+// at 1/2 and n + 1/2, decides and moves it across a face it lies beyond.
+template <int STRIDE>
+__device__ __forceinline__ int locate_pair(const mk_snapshot_view &sv, const PairConsts<STRIDE> &C, const tri x[3],
+                                           int idx[3], pr del[3]) {
+    int c[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const float lo = C.f(PC_BOX + a);
+        if (!(x[a].h >= lo && x[a].h <= C.f(PC_BOX + 3 + a))) return -1;
+        c[a] = max(0, min((int)((x[a].h - lo) * C.f(PC_INVW + a)), sv.nb[a] - 1));
+    }
+    const float n = (float)sv.n;
+    for (int it = 0; it < 4; ++it) {
+        const int mb = table_at(sv, c);
+        if (mb < 0) return -1;
+        const double *g = sv.geom + 6 * (int64_t)mb;
+        bool moved = false;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const tri left = t_from(__ldg(g + a)), d = t_from(__ldg(g + 3 + a));
+            const tri s = t_add(x[a], t_neg(left));
+            const pr w = {d.h, d.m}, iw = p_rcp(w), t = p_mulr({s.h, s.m}, iw);
+            // t + 1 in (1/2, n + 1/2]
+            if (t.h < -0.5f || (t.h == -0.5f && t.l <= 0.0f)) { --c[a]; moved = true; }
+            else if (t.h > n - 0.5f || (t.h == n - 0.5f && t.l > 0.0f)) { ++c[a]; moved = true; }
+            float fl = floorf(t.h);
+            if (fl == t.h && t.l < 0.0f) fl -= 1.0f;
+            fl = fminf(fmaxf(fl, -1.0f), n - 1.0f);
+            idx[a] = (int)fl + 1;
+            // offset from the cell's own centre, so that it keeps its digits
+            const float p = f_mul(fl, d.h), e = fmaf(fl, d.h, -p);
+            float uh, ul;
+            two_sum_f(s.h, -p, uh, ul);
+            const pr u = p_norm({uh, f_add(f_add(ul, fmaf(-fl, d.m, s.m)), -e)});
+            del[a] = p_mulr(u, iw);
+        }
+        if (!moved) return mb;
+    }
+    return -1;
+}
+
+// Z^(-1/3): the float unit's estimate, one Newton step in float, a third-order
+// correction from the pair residual 1 - Z x^3
+__device__ __forceinline__ pr p_rcbrt(pr z) {
+    float l, x;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(z.h));
+    l *= -0.333333343f;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(l));
+    x = fmaf(f_mul(x, 0.333333343f), fmaf(-f_mul(f_mul(z.h, x), x), x, 1.0f), x);
+    const pr x2 = {f_mul(x, x), fmaf(x, x, -f_mul(x, x))};
+    const pr x3 = p_mulr(x2, {x, 0.0f});
+    const float p = f_mul(z.h, x3.h);
+    float e = fmaf(z.h, x3.h, -p);
+    e = fmaf(z.h, x3.l, e);
+    e = fmaf(z.l, x3.h, e);
+    const float d = f_sub(f_sub(1.0f, p), e);
+    return p_norm({x, f_mul(f_mul(x, d), fmaf(0.222222222f, d, 0.333333343f))});
+}
+
+// exp(-x) for x >= 0 as m 2^-e, m in [1/2, 1]: x = (32 e + j) ln2/32 - r, the
+// table's 2^(-j/32), and the series of exp(r), |r| < 0.011
+__device__ __forceinline__ pr p_exp_neg(pr x, const float2 *tab, int &e) {
+    const float n = rintf(x.h * (float)(EXP_STEPS * 1.4426950408889634));
+    constexpr double STEP = 0.693147180559945309417 / EXP_STEPS;
+    constexpr float c1 = (float)STEP, c2 = (float)(STEP - (double)c1);
+    const float p = f_mul(n, c1), pe = fmaf(n, c1, -p);
+    float rh, re;
+    two_sum_f(p, -x.h, rh, re);
+    pr r;
+    fast_sum_f(rh, f_add(re, fmaf(n, c2, f_sub(pe, x.l))), r.h, r.l);
+    const pr s = p_two(p_sqr(r), 0.5f);
+    const float t = f_mul(f_mul(f_mul(r.h, r.h), r.h), fmaf(r.h, fmaf(r.h, 1.0f / 120.0f, 1.0f / 24.0f), 1.0f / 6.0f));
+    pr q = p_add(r, {s.h, f_add(s.l, t)});
+    float h, l;
+    fast_sum_f(1.0f, q.h, h, l);
+    const int k = (int)n, j = k & (EXP_STEPS - 1);
+    e = k / EXP_STEPS;
+    const float2 T = tab[j];
+    return p_mulr({T.x, T.y}, {h, f_add(l, q.l)});
+}
+
+// m 2^-e as a double
+__device__ __forceinline__ double p_scaled(pr m, int e) {
+    if (e > 1000) return 0.0;
+    return (d_from(m.h) + d_from(m.l)) * __hiloint2double((1023 - e) << 20, 0);
+}
+
+enum { PS_OUTSIDE = 0, PS_SAMPLED = 1, PS_BINARY64 = 2 };
+
+// One sample at x (triples) for the photon k.  PS_SAMPLED: em, ab hold the
+// invariant coefficients of every frequency; PS_BINARY64: the point lies in
+// the snapshot, in a block kept in binary64 or at primitives outside the
+// pairs' range, and the caller samples it in binary64.
+template <int STRIDE>
+__device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const PairConsts<STRIDE> &C, int nnu,
+                                           const tri x[3], const pr k[4], const PairPoint &m, const float2 *tab,
+                                           double em[MK_MAX_NU], double ab[MK_MAX_NU]) {
+    int idx[3];
+    pr del[3];
+    const int mb = locate_pair(sv, C, x, idx, del);
+    if (mb < 0) return PS_OUTSIDE;
+    if (sv.blocks64 && __ldg(sv.block64 + mb) >= 0) return PS_BINARY64;
+    // each primitive as the sum of eight weights times cells; one copy of the
+    // code for the four (z, y) neighbours (see tri_step), the cells on their
+    // way to L1 meanwhile
+    const int n2 = sv.n + 2;
+    const int64_t sj = (int64_t)n2 * 8, sk = (int64_t)n2 * n2 * 8;
+    const float *base = sv.blocks + ((((int64_t)mb * n2 + idx[2]) * n2 + idx[1]) * n2 + idx[0]) * 8;
+#pragma unroll
+    for (int q = 1; q < 4; q++) {
+        const float *p = base + (q >> 1) * sk + (q & 1) * sj;
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 8));
+    }
+    const pr one = {1.0f, 0.0f};
+    const pr u0 = p_subr(one, del[0]), u1 = p_subr(one, del[1]), u2 = p_subr(one, del[2]);
+    pr prim[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) prim[i] = {0.0f, 0.0f};
+#pragma unroll 1
+    for (int q = 0; q < 4; q++) {
+        const float *p = base + (q >> 1) * sk + (q & 1) * sj;
+        const float4 c[4] = {ldg4(p), ldg4(p + 4), ldg4(p + 8), ldg4(p + 12)};
+        const pr zy = p_mulr((q & 2) ? del[2] : u2, (q & 1) ? del[1] : u1);
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            const pr w = p_mulr(zy, x ? del[0] : u0);
+            const float4 lo = c[2 * x], hi = c[2 * x + 1];
+            const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float t = f_mul(w.h, v[i]);
+                const float e = fmaf(w.l, v[i], fmaf(w.h, v[i], -t));
+                float s, r;
+                two_sum_f(prim[i].h, t, s, r);
+                prim[i] = {s, f_add(prim[i].l, f_add(e, r))};
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) prim[i] = p_norm(prim[i]);
+#pragma unroll
+    for (int ch = 0; ch < MK_MAX_NU; ch++) em[ch] = ab[ch] = 0.0;
+    if (prim[0].h == 0.0f) return PS_SAMPLED;  // excised cells: sigma or Theta_e is not a number
+    const float Bm = fmaxf(fmaxf(fabsf(prim[5].h), fabsf(prim[6].h)), fabsf(prim[7].h));
+    const float Um = fmaxf(fmaxf(fabsf(prim[1].h), fabsf(prim[2].h)), fabsf(prim[3].h));
+    if (!(Bm >= 1e-25f && Bm <= 1e25f && Um <= 1e6f && prim[0].h >= 1e-25f && prim[0].h <= 1e25f &&
+          prim[4].h >= 1e-12f * prim[0].h && prim[4].h <= 1e12f * prim[0].h))
+        return PS_BINARY64;
+    // density and energy, and the field, scaled to order one by powers of two
+    // (along the poles of a torus they fall by tens of decades)
+    const int ed = ((int)(__float_as_uint(prim[0].h) >> 23) & 255) - 127;
+    const int eB = ((int)(__float_as_uint(Bm) >> 23) & 255) - 127;
+    const int ex = ed - 2 * eB;  // of dens / B^2
+    if (ex < -100 || ex > 100) return PS_BINARY64;
+    const float sd = __uint_as_float((unsigned)(127 - ed) << 23), sB = __uint_as_float((unsigned)(127 - eB) << 23);
+    const pr dens = p_two(prim[0], sd), ue = p_two(prim[4], sd);
+    const pr *U = prim + 1;
+    const pr B[3] = {p_two(prim[5], sB), p_two(prim[6], sB), p_two(prim[7], sB)};
+    const float ratio = __uint_as_float((unsigned)(127 + ex) << 23);  // (dens / B^2) over the scaled one
+    // the frame
+    const pr f = m.f, l3 = m.l3;
+    const pr a = C.p(PC_A);
+    const pr X = {x[0].h, x[0].m}, Y = {x[1].h, x[1].m};
+    const pr l1 = p_mulr(p_addr(p_mul(m.r, X), p_mul(a, Y)), m.ira);
+    const pr l2 = p_mulr(p_subr(p_mul(m.r, Y), p_mul(a, X)), m.ira);
+    auto dot = [](pr x1, pr y1, pr x2, pr y2, pr x3, pr y3) {
+        return p_addr(p_add(p_mul(x1, y1), p_mul(x2, y2)), p_mul(x3, y3));
+    };
+    const pr lU = dot(l1, U[0], l2, U[1], l3, U[2]), lB = dot(l1, B[0], l2, B[1], l3, B[2]);
+    const pr UU = dot(U[0], U[0], U[1], U[1], U[2], U[2]), BB = dot(B[0], B[0], B[1], B[1], B[2], B[2]);
+    const pr BU = dot(B[0], U[0], B[1], U[1], B[2], U[2]);
+    const pr kU = dot(k[1], U[0], k[2], U[1], k[3], U[2]), kB = dot(k[1], B[0], k[2], B[1], k[3], B[2]);
+    const pr flU = p_mulr(f, lU), flB = p_mulr(f, lB);
+    const pr G = p_addr(p_add(UU, p_mul(flU, lU)), one);
+    const pr alpha = p_rsqrt(p_addr(f, one)), rG = p_rsqrt(G);
+    const pr ga = p_mulr(p_mulr(G, rG), alpha);           // gamma alpha
+    const pr iut = p_mulr(alpha, rG);                     // 1/u^t
+    const pr Bu = p_addr(BU, p_mul(flU, lB));             // b^t = B^i u_i
+    const pr b2 = p_mulr(p_addr(p_add(BB, p_mul(flB, lB)), p_sqr(Bu)), p_mulr(iut, iut));
+    if (!(b2.h > 0.0f)) return PS_SAMPLED;
+    const pr ku = p_subr(p_add(kU, p_mul(flU, m.lv)), p_mul(k[0], ga));  // k.u
+    const pr lk = p_subr(m.lv, k[0]);
+    const pr gaf = p_mulr(ga, f);
+    // l_mu b^mu = b^t + (l.B + (l.U - gamma alpha f) b^t) / u^t, and k.b
+    const pr lb = p_addr(Bu, p_mul(p_addr(lB, p_mul(p_subr(lU, gaf), Bu)), iut));
+    const pr kb3 = p_mulr(p_addr(kB, p_mul(p_subr(kU, p_mul(gaf, lk)), Bu)), iut);
+    const pr kb = p_addr(p_subr(kb3, p_mul(k[0], Bu)), p_mul(p_mulr(f, lb), m.lv));
+    const pr ib = p_rsqrt(b2);
+    const pr b = p_mulr(b2, ib);
+    const pr nup = p_neg(ku);                             // nu'
+    if (!(nup.h > 0.0f)) return PS_SAMPLED;               // the fit's roots are not numbers
+    const pr inup = p_rcp(nup);
+    const pr cp = p_mulr(p_mul(kb, ib), inup);
+    const pr s2 = p_mulr(p_subr(one, cp), p_addr(one, cp));
+    if (!(s2.h > 0.0f)) return PS_SAMPLED;                // nu_s = 0
+    const pr sp = p_mulr(s2, p_rsqrt(s2));
+    // sigma cut, electron temperature
+    if (p_sub(b2, p_mul(C.p(PC_SIGMA), p_two(dens, ratio))).h > 0.0f) return PS_SAMPLED;
+    pr beta = p_mulr(p_mulr(p_two(ue, ratio), C.p(PC_GAM2)), p_mulr(ib, ib));
+    if (beta.h > 1e15f) beta = {1e15f, 0.0f};             // T_ratio is r_high to 2^-99
+    const pr be2 = p_mulr(beta, beta), ope = p_addr(be2, one);
+    const pr gi = C.p(PC_GIM1), ge = C.p(PC_GEM1);
+    // Theta_e = K u (1 + beta^2) / (dens (g_i (1 + beta^2) + g_e (R_high beta^2 + R_low)))
+    const pr D = p_mulr(dens, p_addr(p_mul(gi, ope), p_mul(ge, p_addr(p_mul(C.p(PC_RHIGH), be2), C.p(PC_RLOW)))));
+    const pr th = p_mulr(p_mulr(C.p(PC_KTH), ue), p_mulr(ope, p_rcp(D)));
+    if (!(p_sub(th, {0.3f, (float)(0.3 - (double)0.3f)}).h >= 0.0f)) return PS_SAMPLED;
+    if (!(th.h < 1e8f)) return PS_BINARY64;
+    const pr ith = p_rcp(th);
+    const pr base_nus = p_mulr(p_mulr(p_mulr(b, sp), p_mulr(th, th)), inup);
+    const pr base_em = p_mulr(p_mulr(dens, inup), p_mulr(ith, ith));
+    const pr base_bx = p_mulr(nup, ith);
+    const float iB = __uint_as_float((unsigned)(127 + eB) << 23);
+    if (!(base_nus.h >= 1e-26f && base_nus.h <= 1e26f && base_em.h >= 1e-26f && base_em.h <= 1e26f))
+        return PS_BINARY64;
+#pragma unroll
+    for (int ch = 0; ch < MK_MAX_NU; ch++) {
+        if (ch >= nnu) break;
+        const int at = PC_NU + 8 * ch;
+        const pr Z = p_mulr(C.p(at + 2), p_two(base_nus, iB));  // nu_s / nu'
+        if (!(Z.h >= 1e-12f)) continue;                   // X > 1e12: no emission
+        const pr x3 = p_rcbrt(Z);
+        const pr Yc = p_mulr(p_mulr(x3, x3), Z);
+        constexpr pr C211 = {(float)C2_11_12, (float)(C2_11_12 - (double)(float)C2_11_12)};
+        const pr t = p_addr(one, p_mul(C211, Yc));
+        int e;
+        const pr E = p_exp_neg(x3, tab, e);
+        e -= ed;
+        const pr em_m = p_mulr(p_mulr(C.p(at), base_em), p_mulr(p_mulr(t, t), E));
+        if (!(em_m.h >= 1e-28f && em_m.h <= 1e28f)) return PS_BINARY64;
+        em[ch] = p_scaled(em_m, e);
+        const pr bx = p_mulr(C.p(at + 4), base_bx);
+        if (bx.h < 2.e-3f) {
+            // bx (1 + bx/2 (1 + bx/3 (1 + bx/4))), as the reference cuts it
+            const pr q = p_sqr(bx);
+            const float c3 = f_mul(f_mul(f_mul(bx.h, bx.h), bx.h), fmaf(bx.h, 1.0f / 24.0f, 1.0f / 6.0f));
+            const pr den = p_addr(bx, {f_mul(0.5f, q.h), fmaf(0.5f, q.l, c3)});
+            ab[ch] = p_scaled(p_mulr(em_m, p_mulr(den, C.p(at + 6))), e);
+        } else {
+            const double den = exp((double)bx.h + (double)bx.l) - 1.0;
+            const pr ki = C.p(at + 6);
+            ab[ch] = em[ch] * den * ((double)ki.h + (double)ki.l);
+        }
+    }
+    return PS_SAMPLED;
+}
+
+}  // namespace mk
