@@ -728,151 +728,6 @@ render_fp64_kernel(const mk_request *__restrict__ reqs, int nreq, long long tota
     if (SRC == SRC_QUEUE && fp64_samples) atomicAdd(&ws->samples_fp64, (unsigned long long)fp64_samples);
 }
 
-// A sample in binary64 for render_tri_kernel: blocks kept in binary64 (ghosts
-// averaged from finer cells) and primitives outside the pairs' range.
-__device__ __noinline__ void coefficients_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
-                                               double em[MK_MAX_NU], double ab[MK_MAX_NU]) {
-    for (int ch = 0; ch < MK_MAX_NU; ch++) em[ch] = ab[ch] = 0.0;
-    emission_fp64(R, sv, s, kerr_point(s[1], s[2], s[3], R.camera.bhspin), em, ab);
-}
-
-// MK_FP64: every ray of the job, start to end, state in 72 bits, geodesic and
-// sampling in float pairs, transfer sums in binary64 (mk_tri.cuh,
-// mk_sample_pair.cuh say why and to what accuracy).  Bound by FP32 issue and
-// latency: ~4.4 k instructions a step and ~1.9 k a sample, against ~50 k
-// cycles of the FP64 pipe for the same step in binary64.
-// A ray's constants and its sums sit in shared memory, one column a thread.
-// lane_stride: lanes that take rays (a small job's rays are spread over every
-// SM sub-partition, where each then runs at its own chain's speed).
-__global__ void __launch_bounds__(RENDER_THREADS, TRI_BLOCKS)
-render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total_camera,
-                  const mk_snapshot_view *__restrict__ snaps, RenderWorkspace *ws, const mk_job *job,
-                  int lane_stride) {
-    __shared__ float s_const[PC_COUNT * RENDER_THREADS];
-    __shared__ double s_I[MK_MAX_NU][RENDER_THREADS], s_P[MK_MAX_NU][RENDER_THREADS];
-    __shared__ float2 s_exp[EXP_STEPS];
-    if (job) {  // request count and ray total from the device (graph replays)
-        nreq = job->nreq;
-        total_camera = job->total_rays;
-    }
-    const int tid = threadIdx.x;
-    if (tid < EXP_STEPS) {
-        const tri t = t_from(exp2(-(double)tid / EXP_STEPS));
-        s_exp[tid] = make_float2(t.h, t.m);
-    }
-    __syncthreads();
-    const PairConsts<RENDER_THREADS> C = {s_const + tid};
-    const bool lane_works = ((tid & 31) % lane_stride) == 0;
-    bool active = false, exhausted = !lane_works;
-    int rq = 0, steps = 0, nsamples = 0;
-    int64_t pix = 0;
-    long long max_tau = 0;  // bits of a double >= 0: they order as integers
-    TriState s;
-    TriPoint q;
-    tri dt = {0.0f, 0.0f, 0.0f};
-
-    for (;;) {
-        const long long idx = fetch(!active && !exhausted, &ws->counter, total_camera);
-        if (idx == -1) exhausted = true;
-        if (idx >= 0 && ray_in_request(reqs, nreq, idx)) {
-            rq = find_request(reqs, nreq, idx);
-            const mk_request &R = reqs[rq];
-            if (!pair_request(R)) {
-                atomicAdd(&ws->odd_rays, 1ull);  // left to render_fp64_kernel
-            } else {
-                pix = fetch_pixel(R.camera, idx - R.ray_offset);
-                double s64[8];
-                camera_ray_fast(R.camera, pix, s64);
-                tri_state(s64, s);
-                pair_consts(R, snaps[R.snapshot], C);
-                steps = nsamples = 0;
-                max_tau = 0;
-#pragma unroll
-                for (int ch = 0; ch < MK_MAX_NU; ch++) { s_I[ch][tid] = 0.0; s_P[ch][tid] = 1.0; }
-                // the first RK4 stage at s also yields r for the step rule
-                tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), true);
-                float d;
-                int why;
-                const RuleTri rule = {C.t(PC_REH), C.t(PC_NINV), C.p(PC_TOL)};
-                const bool go = rule_dt(q.r, rule, dt, d, why);
-                if (!go || R.policy.nmax < 2) {
-                    // stopped before its next step (reference K = steps), or N < 2
-                    // leaves no row pair for the transfer solve
-                    double I[MK_MAX_NU] = {0.0, 0.0, 0.0, 0.0};
-                    finish_ray(R, pix, I, 0, go ? MK_RAY_MAXSTEPS : why, 0, 0.0, ws);
-                } else {
-                    active = true;
-                }
-            }
-        }
-        if (!__any_sync(0xffffffffu, active)) {
-            if (__all_sync(0xffffffffu, exhausted)) break;
-            continue;  // every fetched ray ended at once; more may be left
-        }
-        if (active) {
-            const mk_request &R = reqs[rq];
-            // next step's first stage, evaluated with the step: gives r and the
-            // metric at the new point for the rule and the sample
-            tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), false);
-            float d;
-            int why;
-            tri dtn;
-            const RuleTri rule = {C.t(PC_REH), C.t(PC_NINV), C.p(PC_TOL)};
-            bool done = !rule_dt(q.r, rule, dtn, d, why);
-            if (!done) {  // else the step is rejected and the ray stays frozen (geodesics.py:263-267)
-                ++steps;
-                const bool row = steps < R.rows;
-                if (R.rows_dt && row)  // per-step diagnostics: row `steps` = this state
-                    R.rows_dt[(int64_t)(steps - 1) * request_pixels(R.camera) + pix] = t_to(dt);
-                const mk_snapshot_view &sv = snaps[R.snapshot];
-                const tri x[3] = {s.X[1], s.X[2], s.X[3]};
-                const pr k[4] = {t_pair(s.K[0]), t_pair(s.K[1]), t_pair(s.K[2]), t_pair(s.K[3])};
-                double em[MK_MAX_NU], ab[MK_MAX_NU];
-                int got = sample_pair(sv, C, R.nnu, x, k, q.m, s_exp, em, ab);
-                if (got == PS_BINARY64) {
-                    double s64[8], e64[MK_MAX_NU], a64[MK_MAX_NU];  // copies: em and ab stay in registers
-                    tri_doubles(s, s64);
-                    coefficients_fp64(R, sv, s64, e64, a64);
-#pragma unroll
-                    for (int ch = 0; ch < MK_MAX_NU; ch++) { em[ch] = e64[ch]; ab[ch] = a64[ch]; }
-                }
-                if (got != PS_OUTSIDE) {
-                    ++nsamples;
-                    const double w = -t_to(dt) * R.L_unit;
-#pragma unroll
-                    for (int ch = 0; ch < MK_MAX_NU; ch++) {
-                        if (ch < R.nnu) {
-                            if (R.rows_em && R.rows_dt && row) {
-                                const int64_t at = (ch * R.rows + steps) * request_pixels(R.camera) + pix;
-                                R.rows_em[at] = em[ch];
-                                R.rows_ab[at] = ab[ch];
-                            }
-                            const double tau = w * ab[ch], P = s_P[ch][tid];
-                            s_I[ch][tid] += (w * em[ch]) * P;
-                            s_P[ch][tid] = P * (1.0 - tau);
-                            const long long bits = __double_as_longlong(tau);
-                            max_tau = bits > max_tau ? bits : max_tau;
-                        }
-                    }
-                }
-                dt = dtn;
-                // trajectory rows stop at N-1: step N-1 never reaches the solve
-                if (steps >= R.policy.nmax - 1) {
-                    done = true;
-                    why = MK_RAY_MAXSTEPS;
-                }
-            }
-            if (done) {
-                double I[MK_MAX_NU];
-#pragma unroll
-                for (int ch = 0; ch < MK_MAX_NU; ch++) I[ch] = s_I[ch][tid];
-                finish_ray(R, pix, I, steps, why, nsamples, __longlong_as_double(max_tau), ws);
-                active = false;
-            }
-        }
-    }
-}
-
 __device__ __forceinline__ void finish_ray_f32(const mk_request &R, int64_t pix, const float I[MK_MAX_NU],
                                                const float Ic[MK_MAX_NU], int steps, int why, int nsamples,
                                                float max_tau, RenderWorkspace *ws) {
@@ -976,7 +831,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Bounded wait of a whole warp (every lane calls it and gets the same
 // answer) for the phase of parity `parity` of mbarrier b: false when
 // limit_ns ran out or the block aborted.
-__device__ __forceinline__ bool zone_wait(unsigned long long *b, unsigned parity, const ZoneShared &zs,
+template <typename Shared>
+__device__ __forceinline__ bool zone_wait(unsigned long long *b, unsigned parity, const Shared &zs,
                                           unsigned long long limit_ns) {
     const unsigned FULL = 0xffffffffu;
     // the common case, a phase already complete, reads no timer
@@ -1012,7 +868,8 @@ __device__ __forceinline__ bool zone_wait_fold(const ZoneShared &zs, int j, unsi
 }
 
 // a wait ran out: stop the block's other warps and count it once per warp
-__device__ __forceinline__ void zone_fail(ZoneShared &zs, RenderWorkspace *ws) {
+template <typename Shared>
+__device__ __forceinline__ void zone_fail(Shared &zs, RenderWorkspace *ws) {
     *(volatile int *)&zs.abort = 1;
     if ((threadIdx.x & 31) == 0) atomicAdd(&ws->zone_error, 1ull);
 }
@@ -1363,6 +1220,281 @@ render_zone_kernel(const mk_request *__restrict__ reqs, const mk_snapshot_view *
         zone_sample(w - 1, reqs, snaps, ws, q64, zs, wait_ns);
 }
 
+// A sample in binary64 for render_tri_kernel: blocks kept in binary64 (ghosts
+// averaged from finer cells) and primitives outside the pairs' range.
+__device__ __noinline__ void coefficients_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
+                                               double em[MK_MAX_NU], double ab[MK_MAX_NU]) {
+    for (int ch = 0; ch < MK_MAX_NU; ch++) em[ch] = ab[ch] = 0.0;
+    emission_fp64(R, sv, s, kerr_point(s[1], s[2], s[3], R.camera.bhspin), em, ab);
+}
+
+// MK_FP64: every ray of the job, start to end, state in 72 bits, geodesic and
+// sampling in float pairs, transfer sums in binary64 (mk_tri.cuh,
+// mk_sample_pair.cuh say why and to what accuracy).
+//
+// An image's time is the chain of its longest rays (a captured ray around a
+// spinning hole takes 1000 to 3500 steps, the mean ray ~450), so a step and
+// its sample, ~7.3 k and ~6.4 k cycles of a lone warp, are taken by two warps:
+// one integrates 32 rays and posts a message per step, the other samples the
+// snapshot there and folds the sample into the rays' transfer sums, up to
+// TRI_SLOTS steps behind.  A block holds two such couples; in every other
+// block the roles change sides, since an integrating warp issues more than
+// twice what a sampling one does and the SM's four sub-partitions should
+// share both.
+//
+// Messages pass through slots in shared memory with two mbarriers each, waits
+// are bounded and abort the block, all as in the near-hole phase
+// (render_zone_kernel).  A ray's constants sit in shared memory, one column a
+// thread, each role's loaded by itself when the ray starts.
+// lane_stride: lanes that take rays (a small job's rays are spread over every
+// couple before they share warps).
+enum : unsigned { TM_START = 1u, TM_SAMPLE = 2u, TM_END = 4u, TM_DONE = 8u };
+constexpr int TRI_COUPLES = 2;
+constexpr int TRI_LANES = 32 * TRI_COUPLES;
+constexpr int TRI_SLOTS = 3;
+static_assert(RENDER_THREADS == 2 * TRI_LANES, "two warps a couple");
+
+struct TriSlot {
+    unsigned flags[32];
+    int why[32];         // TM_END
+    long long ray[32];   // TM_START
+    float v[28][32];     // x^1..x^3 (h m l), k^0..k^3 (h l), r f l3 ira lv... see tri_post
+};
+// message words
+enum { TV_X = 0, TV_K = 9, TV_M = 17, TV_DT = 25, TV_COUNT = 28 };
+
+struct TriShared {
+    TriSlot slot[TRI_COUPLES][TRI_SLOTS];
+    float c_int[13 * TRI_LANES];              // PC_A .. PC_TOL
+    float c_smp[(PC_COUNT - PC_BOX) * TRI_LANES];
+    double I[MK_MAX_NU][TRI_LANES], P[MK_MAX_NU][TRI_LANES];
+    float2 exptab[EXP_STEPS];
+    unsigned long long full[TRI_COUPLES][TRI_SLOTS], empty[TRI_COUPLES][TRI_SLOTS];
+    int abort;
+};
+
+__device__ __forceinline__ void tri_integrate(int couple, const mk_request *__restrict__ reqs, int nreq,
+                                              long long total, RenderWorkspace *ws, int lane_stride, TriShared &sh,
+                                              unsigned long long limit_ns) {
+    const int lane = threadIdx.x & 31;
+    const PairConsts<TRI_LANES> C = {sh.c_int + 32 * couple + lane};
+    bool active = false, exhausted = lane % lane_stride != 0;
+    int steps = 0, nmax = 0;
+    TriState s;
+    TriPoint q;
+    tri dt = {0.0f, 0.0f, 0.0f};
+    for (int it = 0;; ++it) {
+        const int sl = it % TRI_SLOTS;
+        TriSlot &msg = sh.slot[couple][sl];
+        unsigned flags = 0;
+        const long long idx = fetch(!active && !exhausted, &ws->counter, total);
+        if (idx == -1) exhausted = true;
+        bool start = false;
+        if (idx >= 0 && ray_in_request(reqs, nreq, idx)) {
+            const mk_request &R = reqs[find_request(reqs, nreq, idx)];
+            if (!pair_request(R)) {
+                atomicAdd(&ws->odd_rays, 1ull);  // left to render_fp64_kernel
+            } else {
+                double s64[8];
+                camera_ray_fast(R.camera, fetch_pixel(R.camera, idx - R.ray_offset), s64);
+                tri_state(s64, s);
+                pair_consts_geodesic(R, C);
+                nmax = R.policy.nmax;
+                steps = 0;
+                start = true;
+            }
+        }
+        const bool step = active;
+        const tri used = dt;
+        float d;
+        int why = MK_RAY_ACTIVE;
+        if (start || step) {
+            // the new state, and with it the next step's first stage, which
+            // gives r and the metric there for the rule and the sample
+            tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), start);
+            const RuleTri rule = {C.t(PC_REH), C.t(PC_NINV), C.p(PC_TOL)};
+            const bool go = rule_dt(q.r, rule, dt, d, why);
+            if (start) {
+                flags = TM_START;
+                // stopped before its first step (reference K = 0), or N < 2
+                // leaves no row pair for the transfer solve
+                active = go && nmax >= 2;
+            } else if (!go) {
+                active = false;  // the step is rejected and the ray stays frozen (geodesics.py:263-267)
+            } else {
+                flags = TM_SAMPLE;
+                // trajectory rows stop at N-1: step N-1 never reaches the solve
+                active = ++steps < nmax - 1;
+            }
+            if (!active) {
+                flags |= TM_END;
+                if (go) why = MK_RAY_MAXSTEPS;
+            }
+        }
+        const bool last = __all_sync(0xffffffffu, !active && exhausted);
+        if (it >= TRI_SLOTS && !zone_wait(&sh.empty[couple][sl], (unsigned)((it / TRI_SLOTS) - 1) & 1u, sh, limit_ns)) {
+            zone_fail(sh, ws);
+            return;
+        }
+        msg.flags[lane] = flags | (last ? TM_DONE : 0u);
+        if (flags & TM_START) msg.ray[lane] = idx;
+        if (flags & TM_END) msg.why[lane] = why;
+        if (flags & TM_SAMPLE) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                msg.v[TV_X + 3 * i][lane] = s.X[1 + i].h;
+                msg.v[TV_X + 3 * i + 1][lane] = s.X[1 + i].m;
+                msg.v[TV_X + 3 * i + 2][lane] = s.X[1 + i].l;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                msg.v[TV_K + 2 * i][lane] = s.K[i].h;
+                msg.v[TV_K + 2 * i + 1][lane] = s.K[i].m;
+            }
+            const pr m[4] = {q.m.r, q.m.f, q.m.l3, q.m.ira};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                msg.v[TV_M + 2 * i][lane] = m[i].h;
+                msg.v[TV_M + 2 * i + 1][lane] = m[i].l;
+            }
+            msg.v[TV_DT][lane] = used.h;
+            msg.v[TV_DT + 1][lane] = used.m;
+            msg.v[TV_DT + 2][lane] = used.l;
+        }
+        __syncwarp();
+        mbar_arrive(&sh.full[couple][sl]);
+        if (last) return;
+    }
+}
+
+__device__ __forceinline__ void tri_sample(int couple, const mk_request *__restrict__ reqs, int nreq,
+                                           const mk_snapshot_view *__restrict__ snaps, RenderWorkspace *ws,
+                                           TriShared &sh, unsigned long long limit_ns) {
+    const int lane = threadIdx.x & 31, col = 32 * couple + lane;
+    // the sampler's constants start at PC_BOX
+    const PairConsts<TRI_LANES> C = {sh.c_smp + col - PC_BOX * TRI_LANES};
+    int rq = 0, steps = 0, nsamples = 0;
+    int64_t pix = 0;
+    pr a = {0.0f, 0.0f};
+    long long max_tau = 0;  // bits of a double >= 0: they order as integers
+    for (int j = 0;; ++j) {
+        const int sl = j % TRI_SLOTS;
+        const TriSlot &msg = sh.slot[couple][sl];
+        if (!zone_wait(&sh.full[couple][sl], (unsigned)(j / TRI_SLOTS) & 1u, sh, limit_ns)) {
+            zone_fail(sh, ws);
+            return;
+        }
+        const unsigned flags = msg.flags[lane];
+        const long long ray = msg.ray[lane];
+        const int why = msg.why[lane];
+        tri x[3] = {}, dt = {0.0f, 0.0f, 0.0f};
+        pr k[4] = {}, m[4] = {};
+        if (flags & TM_SAMPLE) {
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+                x[i] = {msg.v[TV_X + 3 * i][lane], msg.v[TV_X + 3 * i + 1][lane], msg.v[TV_X + 3 * i + 2][lane]};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                k[i] = {msg.v[TV_K + 2 * i][lane], msg.v[TV_K + 2 * i + 1][lane]};
+                m[i] = {msg.v[TV_M + 2 * i][lane], msg.v[TV_M + 2 * i + 1][lane]};
+            }
+            dt = {msg.v[TV_DT][lane], msg.v[TV_DT + 1][lane], msg.v[TV_DT + 2][lane]};
+        }
+        __syncwarp();
+        mbar_arrive(&sh.empty[couple][sl]);  // the slot is free for message j + TRI_SLOTS
+        if (flags & TM_START) {
+            rq = find_request(reqs, nreq, ray);
+            const mk_request &R = reqs[rq];
+            pix = fetch_pixel(R.camera, ray - R.ray_offset);
+            const tri a3 = t_from(R.camera.bhspin);
+            a = {a3.h, a3.m};
+            pair_consts_sample(R, snaps[R.snapshot], C);
+            steps = nsamples = 0;
+            max_tau = 0;
+#pragma unroll
+            for (int ch = 0; ch < MK_MAX_NU; ch++) { sh.I[ch][col] = 0.0; sh.P[ch][col] = 1.0; }
+        }
+        if (flags & TM_SAMPLE) {
+            const mk_request &R = reqs[rq];
+            ++steps;
+            const bool row = steps < R.rows;
+            if (R.rows_dt && row)  // per-step diagnostics: row `steps` = this state
+                R.rows_dt[(int64_t)(steps - 1) * request_pixels(R.camera) + pix] = t_to(dt);
+            const mk_snapshot_view &sv = snaps[R.snapshot];
+            double em[MK_MAX_NU], ab[MK_MAX_NU];
+            const int got = sample_pair(sv, C, R.nnu, x, k, a, m, sh.exptab, em, ab);
+            if (got == PS_BINARY64) {
+                // through copies: em and ab stay in registers
+                double s64[8], e64[MK_MAX_NU], a64[MK_MAX_NU];
+                s64[0] = 0.0;  // x^0 is not read
+#pragma unroll
+                for (int i = 0; i < 3; i++) s64[1 + i] = t_to(x[i]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) s64[4 + i] = d_from(k[i].h) + d_from(k[i].l);
+                coefficients_fp64(R, sv, s64, e64, a64);
+#pragma unroll
+                for (int ch = 0; ch < MK_MAX_NU; ch++) { em[ch] = e64[ch]; ab[ch] = a64[ch]; }
+            }
+            if (got != PS_OUTSIDE) {
+                ++nsamples;
+                const double w = -t_to(dt) * R.L_unit;
+#pragma unroll
+                for (int ch = 0; ch < MK_MAX_NU; ch++) {
+                    if (ch < R.nnu) {
+                        if (R.rows_em && R.rows_dt && row) {
+                            const int64_t at = (ch * R.rows + steps) * request_pixels(R.camera) + pix;
+                            R.rows_em[at] = em[ch];
+                            R.rows_ab[at] = ab[ch];
+                        }
+                        const double tau = w * ab[ch], P = sh.P[ch][col];
+                        sh.I[ch][col] += (w * em[ch]) * P;
+                        sh.P[ch][col] = P * (1.0 - tau);
+                        const long long bits = __double_as_longlong(tau);
+                        max_tau = bits > max_tau ? bits : max_tau;
+                    }
+                }
+            }
+        }
+        if (flags & TM_END) {
+            double I[MK_MAX_NU];
+#pragma unroll
+            for (int ch = 0; ch < MK_MAX_NU; ch++) I[ch] = sh.I[ch][col];
+            finish_ray(reqs[rq], pix, I, steps, why, nsamples, __longlong_as_double(max_tau), ws);
+        }
+        if (__any_sync(0xffffffffu, (flags & TM_DONE) != 0u)) return;
+    }
+}
+
+__global__ void __launch_bounds__(RENDER_THREADS, TRI_BLOCKS)
+render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total_camera,
+                  const mk_snapshot_view *__restrict__ snaps, RenderWorkspace *ws, const mk_job *job,
+                  int lane_stride, unsigned flip, unsigned long long wait_ns) {
+    __shared__ TriShared sh;
+    if (job) {  // request count and ray total from the device (graph replays)
+        nreq = job->nreq;
+        total_camera = job->total_rays;
+    }
+    if (threadIdx.x == 0) {
+        for (int c = 0; c < TRI_COUPLES; c++)
+            for (int i = 0; i < TRI_SLOTS; i++) {
+                mbar_init(&sh.full[c][i], 32);
+                mbar_init(&sh.empty[c][i], 32);
+            }
+        sh.abort = 0;
+    }
+    if (threadIdx.x < EXP_STEPS) {
+        const tri t = t_from(exp2(-(double)threadIdx.x / EXP_STEPS));
+        sh.exptab[threadIdx.x] = make_float2(t.h, t.m);
+    }
+    __syncthreads();
+    const int w = threadIdx.x >> 5;
+    const unsigned odd = (blockIdx.x / flip) & 1u;
+    if (((unsigned)w / TRI_COUPLES) == odd)
+        tri_integrate(w % TRI_COUPLES, reqs, nreq, total_camera, ws, lane_stride, sh, wait_ns);
+    else
+        tri_sample(w % TRI_COUPLES, reqs, nreq, snaps, ws, sh, wait_ns);
+}
+
 // Initial states of every camera ray of a launch as float pairs (x^mu
 // then k^mu, hi and lo words: 64 B a ray), for mixed-form launches larger
 // than one wave of phase A: there each thread of phase A takes a new ray
@@ -1680,12 +1812,16 @@ static int launch_render(const mk_request *reqs_dev, int32_t nreq, int64_t total
     if (rc != MK_OK) return rc;
     if (precision == MK_FP64) {
         // the fewest rays a warp (a power of two) with which every ray has a
-        // lane while one warp runs on each SM sub-partition
+        // lane among the integrating warps of one block an SM
+        const int sms = device_sm_count();
         int stride = 32;
-        while (stride > 1 && max_rays > (int64_t)device_sm_count() * 4 * (32 / stride)) stride /= 2;
-        const unsigned grid = persistent_grid(TRI_BLOCKS, max_rays * stride);
-        render_tri_kernel<<<grid, RENDER_THREADS, 0, st>>>(reqs_dev, nreq, (long long)total_rays, snaps_dev, ws,
-                                                            job_dev, stride);
+        while (stride > 1 && max_rays > (int64_t)sms * TRI_COUPLES * (32 / stride)) stride /= 2;
+        const int64_t rays_per_block = TRI_COUPLES * (32 / stride);
+        const int64_t blocks = std::min<int64_t>((max_rays + rays_per_block - 1) / rays_per_block,
+                                                 (int64_t)sms * TRI_BLOCKS);
+        render_tri_kernel<<<(unsigned)blocks, RENDER_THREADS, 0, st>>>(reqs_dev, nreq, (long long)total_rays,
+                                                                        snaps_dev, ws, job_dev, stride,
+                                                                        (unsigned)sms, g_zone_wait_ns);
         MK_LAUNCHED("render_tri_kernel");
         render_fp64_kernel<SRC_CAMERA>
             <<<persistent_grid(blocks_per_sm(render_fp64_kernel<SRC_CAMERA>, 0), max_rays), RENDER_THREADS, 0, st>>>(

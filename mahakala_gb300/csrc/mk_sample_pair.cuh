@@ -78,14 +78,20 @@ __device__ __forceinline__ bool pair_request(const mk_request &R) {
     return ok;
 }
 
+// the integrating warp's part (to PC_TOL) and the sampling warp's (from PC_BOX)
 template <int STRIDE>
-__device__ __forceinline__ void pair_consts(const mk_request &R, const mk_snapshot_view &sv, PairConsts<STRIDE> C) {
+__device__ __forceinline__ void pair_consts_geodesic(const mk_request &R, PairConsts<STRIDE> C) {
     const double a = R.camera.bhspin;
     C.set(PC_A, a, 2);
     C.set(PC_AA, a * a, 3);  // the third word is PC_AA_L
     C.set(PC_REH, radius_eh(a), 3);
     C.set(PC_NINV, -1.0 / R.policy.div, 3);
     C.set(PC_TOL, R.policy.tol, 2);
+}
+
+template <int STRIDE>
+__device__ __forceinline__ void pair_consts_sample(const mk_request &R, const mk_snapshot_view &sv,
+                                                   PairConsts<STRIDE> C) {
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         // the block grid's box, widened by more than the float's rounding
@@ -204,13 +210,14 @@ __device__ __forceinline__ double p_scaled(pr m, int e) {
 
 enum { PS_OUTSIDE = 0, PS_SAMPLED = 1, PS_BINARY64 = 2 };
 
-// One sample at x (triples) for the photon k.  PS_SAMPLED: em, ab hold the
+// One sample at x (triples) for the photon k; a: the spin, m: r, f, l3 and
+// 1/(r^2 + a^2) there.  PS_SAMPLED: em, ab hold the
 // invariant coefficients of every frequency; PS_BINARY64: the point lies in
 // the snapshot, in a block kept in binary64 or at primitives outside the
 // pairs' range, and the caller samples it in binary64.
 template <int STRIDE>
 __device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const PairConsts<STRIDE> &C, int nnu,
-                                           const tri x[3], const pr k[4], const PairPoint &m, const float2 *tab,
+                                           const tri x[3], const pr k[4], pr a, const pr m[4], const float2 *tab,
                                            double em[MK_MAX_NU], double ab[MK_MAX_NU]) {
     int idx[3];
     pr del[3];
@@ -276,11 +283,10 @@ __device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const Pai
     const pr B[3] = {p_two(prim[5], sB), p_two(prim[6], sB), p_two(prim[7], sB)};
     const float ratio = __uint_as_float((unsigned)(127 + ex) << 23);  // (dens / B^2) over the scaled one
     // the frame
-    const pr f = m.f, l3 = m.l3;
-    const pr a = C.p(PC_A);
+    const pr r = m[0], f = m[1], l3 = m[2], ira = m[3];
     const pr X = {x[0].h, x[0].m}, Y = {x[1].h, x[1].m};
-    const pr l1 = p_mulr(p_addr(p_mul(m.r, X), p_mul(a, Y)), m.ira);
-    const pr l2 = p_mulr(p_subr(p_mul(m.r, Y), p_mul(a, X)), m.ira);
+    const pr l1 = p_mulr(p_addr(p_mul(r, X), p_mul(a, Y)), ira);
+    const pr l2 = p_mulr(p_subr(p_mul(r, Y), p_mul(a, X)), ira);
     auto dot = [](pr x1, pr y1, pr x2, pr y2, pr x3, pr y3) {
         return p_addr(p_add(p_mul(x1, y1), p_mul(x2, y2)), p_mul(x3, y3));
     };
@@ -288,6 +294,7 @@ __device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const Pai
     const pr UU = dot(U[0], U[0], U[1], U[1], U[2], U[2]), BB = dot(B[0], B[0], B[1], B[1], B[2], B[2]);
     const pr BU = dot(B[0], U[0], B[1], U[1], B[2], U[2]);
     const pr kU = dot(k[1], U[0], k[2], U[1], k[3], U[2]), kB = dot(k[1], B[0], k[2], B[1], k[3], B[2]);
+    const pr lk = dot(l1, k[1], l2, k[2], l3, k[3]), lv = p_addr(k[0], lk);  // l.k, l_mu k^mu
     const pr flU = p_mulr(f, lU), flB = p_mulr(f, lB);
     const pr G = p_addr(p_add(UU, p_mul(flU, lU)), one);
     const pr alpha = p_rsqrt(p_addr(f, one)), rG = p_rsqrt(G);
@@ -296,13 +303,12 @@ __device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const Pai
     const pr Bu = p_addr(BU, p_mul(flU, lB));             // b^t = B^i u_i
     const pr b2 = p_mulr(p_addr(p_add(BB, p_mul(flB, lB)), p_sqr(Bu)), p_mulr(iut, iut));
     if (!(b2.h > 0.0f)) return PS_SAMPLED;
-    const pr ku = p_subr(p_add(kU, p_mul(flU, m.lv)), p_mul(k[0], ga));  // k.u
-    const pr lk = p_subr(m.lv, k[0]);
+    const pr ku = p_subr(p_add(kU, p_mul(flU, lv)), p_mul(k[0], ga));  // k.u
     const pr gaf = p_mulr(ga, f);
     // l_mu b^mu = b^t + (l.B + (l.U - gamma alpha f) b^t) / u^t, and k.b
     const pr lb = p_addr(Bu, p_mul(p_addr(lB, p_mul(p_subr(lU, gaf), Bu)), iut));
     const pr kb3 = p_mulr(p_addr(kB, p_mul(p_subr(kU, p_mul(gaf, lk)), Bu)), iut);
-    const pr kb = p_addr(p_subr(kb3, p_mul(k[0], Bu)), p_mul(p_mulr(f, lb), m.lv));
+    const pr kb = p_addr(p_subr(kb3, p_mul(k[0], Bu)), p_mul(p_mulr(f, lb), lv));
     const pr ib = p_rsqrt(b2);
     const pr b = p_mulr(b2, ib);
     const pr nup = p_neg(ku);                             // nu'

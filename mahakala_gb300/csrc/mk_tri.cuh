@@ -228,9 +228,9 @@ MK_HD SpinTri spin_tri(double a) {
 }
 
 // What accel_pair meets on its way and the radius, step rule and sampler use:
-// r, f, l3, 1/(r^2 + a^2), l_mu k^mu, and 1/q, 1/r to float.
+// r, f, l3, 1/(r^2 + a^2), and 1/q, 1/r to float.
 struct PairPoint {
-    pr r, f, l3, ira, lv;
+    pr r, f, l3, ira;
     float iq, ir;
 };
 
@@ -275,7 +275,6 @@ MK_HD void accel_pair(pr x, pr y, pr z, pr k0, pr k1, pr k2, pr k3, pr a, pr aa,
     o.f = f;
     o.l3 = l3;
     o.ira = ira;
-    o.lv = lv;
     o.iq = iq.h;
     o.ir = ir.h;
 }
