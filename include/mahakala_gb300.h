@@ -203,6 +203,18 @@ int mk_integrate(const double *s0_dev, int64_t npx, double bhspin, const mk_step
                  double *rows_dev, double *dt_dev, int32_t *K_dev, int32_t *why_dev,
                  double *state_dev, void *stream);
 
+/* mk_integrate with rows that leaves each ray's rows from its stopping step
+   K on unwritten, and the filling of them apart: rows j of 0 .. nrows - 1
+   with j >= K_dev[p] get the ray's state and dt 0 (rows_dev (nrows, npx, 8),
+   dt_dev (nrows, npx), either may be NULL).  A caller that keeps only the
+   rows up to its longest ray (geodesic_integrator trims to max K + 2) fills
+   only those. */
+int mk_integrate_moving(const double *s0_dev, int64_t npx, double bhspin, const mk_step_policy *policy,
+                        double *rows_dev, double *dt_dev, int32_t *K_dev, int32_t *why_dev,
+                        double *state_dev, void *stream);
+int mk_freeze_rows(const double *state_dev, const int32_t *K_dev, int64_t npx, int32_t nrows,
+                   double *rows_dev, double *dt_dev, void *stream);
+
 /* radius_cal (geodesics.py:284-291) on npts points of stride `stride` doubles */
 int mk_radius_cal(const double *x_dev, int64_t npts, int64_t stride, double bhspin,
                   double *r_dev, void *stream);

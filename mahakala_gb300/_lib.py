@@ -95,6 +95,8 @@ SIGNATURES = {
     "mk_camera_init": (_c.c_int, [_c.POINTER(Camera), _VP, _VP]),
     "mk_camera_points": (_c.c_int, [_VP, _VP, _I64, _D, _D, _D, _D, _VP, _VP]),
     "mk_integrate": (_c.c_int, [_VP, _I64, _D, _c.POINTER(StepPolicy), _VP, _VP, _VP, _VP, _VP, _VP]),
+    "mk_integrate_moving": (_c.c_int, [_VP, _I64, _D, _c.POINTER(StepPolicy), _VP, _VP, _VP, _VP, _VP, _VP]),
+    "mk_freeze_rows": (_c.c_int, [_VP, _VP, _I64, _I32, _VP, _VP, _VP]),
     "mk_radius_cal": (_c.c_int, [_VP, _I64, _I64, _D, _VP, _VP]),
     "mk_shadow_pass": (_c.c_int, [_VP, _VP, _VP, _I64, _D, _D, _D, _D, _I32, _VP, _VP, _VP, _VP, _VP, _VP,
                                   _VP]),

@@ -1,5 +1,7 @@
 // mk_geodesic.cu -- camera initialisation, geodesic integration and the
 // shadow-bisection pass (geodesics.py), one thread per ray, FP64.
+#include <algorithm>
+
 #include "mk_common.cuh"
 #include "mk_kerr.cuh"
 #include "mk_tri.cuh"
@@ -72,12 +74,23 @@ __device__ __forceinline__ void store_row(double *__restrict__ rows, int64_t at,
     }
 }
 
-// rows j .. N-1 of a stopped ray: its frozen state, dt = 0
-__device__ __forceinline__ void freeze_rows(double *rows, double *dts, int64_t p, int64_t npx, int j, int N,
-                                            const double s[8]) {
-    for (int r = j; r < N; r++) {
-        if (rows) store_row(rows, (int64_t)r * npx + p, s);
-        if (dts) dts[(int64_t)r * npx + p] = 0.0;
+// Rows j >= K[p] of stopped rays: the frozen state, dt = 0.  A pass of its
+// own over (row, ray), 16 bytes a thread: written by the thread of the ray
+// that stopped, a row at a time, they were two thirds of the time of 1600
+// trajectories with 10000 rows.  V: double2, or double where the arrays are
+// not 16-byte aligned.
+template <typename V>
+__global__ void freeze_rows_kernel(const double *__restrict__ state, const int32_t *__restrict__ K, int64_t npx,
+                                   int nrows, double *__restrict__ rows, double *__restrict__ dts) {
+    constexpr int PARTS = 8 * sizeof(double) / sizeof(V);
+    const int64_t row = npx * PARTS;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < row; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = e / PARTS;
+        const V v = reinterpret_cast<const V *>(state)[e];
+        for (int j = max(0, K[p]) + blockIdx.y; j < nrows; j += gridDim.y) {
+            if (rows) reinterpret_cast<V *>(rows)[j * row + e] = v;
+            if (dts && e % PARTS == 0) dts[j * npx + p] = 0.0;
+        }
     }
 }
 
@@ -100,7 +113,6 @@ __device__ __noinline__ void integrate_reference_f64(double s[8], int j0, int64_
         if (dtn == 0.0) {
             K = j;
             why = (w0 != MK_RAY_ACTIVE) ? w0 : w1;
-            freeze_rows(rows, dts, p, npx, j, N, s);
             break;
         }
         if (rows) store_row(rows, (int64_t)j * npx + p, s);
@@ -162,7 +174,6 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
             if (!go) {
                 K = j;
                 why = w;
-                freeze_rows(rows, dts, p, npx, j, N, s64);
                 break;
             }
             if (rows) store_row(rows, (int64_t)j * npx + p, s64);
@@ -422,9 +433,8 @@ extern "C" int mk_camera_points(const double *x_dev, const double *y_dev, int64_
     return MK_OK;
 }
 
-extern "C" int mk_integrate(const double *s0_dev, int64_t npx, double bhspin, const mk_step_policy *policy,
-                            double *rows_dev, double *dt_dev, int32_t *K_dev, int32_t *why_dev, double *state_dev,
-                            void *stream) {
+static int integrate(const double *s0_dev, int64_t npx, double bhspin, const mk_step_policy *policy, double *rows_dev,
+                     double *dt_dev, int32_t *K_dev, int32_t *why_dev, double *state_dev, void *stream) {
     MK_REQUIRE(s0_dev && policy && K_dev && why_dev && state_dev, MK_ERR_ARG, "mk_integrate: null pointer");
     MK_REQUIRE(npx >= 0 && policy->nmax >= 0, MK_ERR_ARG, "mk_integrate: negative size");
     if (npx == 0) return MK_OK;
@@ -445,6 +455,38 @@ extern "C" int mk_integrate(const double *s0_dev, int64_t npx, double bhspin, co
         MK_REQUIRE(false, MK_ERR_ARG, "mk_integrate: unknown policy %d", (int)policy->kind);
     }
     return MK_OK;
+}
+
+extern "C" int mk_freeze_rows(const double *state_dev, const int32_t *K_dev, int64_t npx, int32_t nrows,
+                              double *rows_dev, double *dt_dev, void *stream) {
+    MK_REQUIRE(state_dev && K_dev, MK_ERR_ARG, "mk_freeze_rows: null pointer");
+    MK_REQUIRE(npx >= 0 && nrows >= 0, MK_ERR_ARG, "mk_freeze_rows: negative size");
+    if (npx == 0 || nrows == 0 || (!rows_dev && !dt_dev)) return MK_OK;
+    // about 16 blocks an SM over (ray, row)
+    const bool wide = (((uintptr_t)state_dev | (uintptr_t)rows_dev) & 15) == 0;
+    const int64_t bx = std::min<int64_t>((npx * (wide ? 4 : 8) + 255) / 256, 65535);
+    const int64_t by = std::max<int64_t>(1, std::min<int64_t>(nrows, (int64_t)device_sm_count() * 16 / bx));
+    const dim3 grid((unsigned)bx, (unsigned)by);
+    if (wide)
+        freeze_rows_kernel<double2><<<grid, 256, 0, as_stream(stream)>>>(state_dev, K_dev, npx, nrows, rows_dev, dt_dev);
+    else
+        freeze_rows_kernel<double><<<grid, 256, 0, as_stream(stream)>>>(state_dev, K_dev, npx, nrows, rows_dev, dt_dev);
+    MK_LAUNCHED("freeze_rows_kernel");
+    return MK_OK;
+}
+
+extern "C" int mk_integrate_moving(const double *s0_dev, int64_t npx, double bhspin, const mk_step_policy *policy,
+                                   double *rows_dev, double *dt_dev, int32_t *K_dev, int32_t *why_dev,
+                                   double *state_dev, void *stream) {
+    return integrate(s0_dev, npx, bhspin, policy, rows_dev, dt_dev, K_dev, why_dev, state_dev, stream);
+}
+
+extern "C" int mk_integrate(const double *s0_dev, int64_t npx, double bhspin, const mk_step_policy *policy,
+                            double *rows_dev, double *dt_dev, int32_t *K_dev, int32_t *why_dev, double *state_dev,
+                            void *stream) {
+    const int rc = integrate(s0_dev, npx, bhspin, policy, rows_dev, dt_dev, K_dev, why_dev, state_dev, stream);
+    if (rc != MK_OK || (!rows_dev && !dt_dev)) return rc;
+    return mk_freeze_rows(state_dev, K_dev, npx, policy->nmax, rows_dev, dt_dev, stream);
 }
 
 extern "C" int mk_radius_cal(const double *x_dev, int64_t npts, int64_t stride, double bhspin, double *r_dev,

@@ -66,11 +66,12 @@ def step_policy(N, div=40.0, tol=1e-4, kind="reference", hfrac=0.05, hmin=0.01, 
     return pol
 
 
-def trace(s0, bhspin, policy, rows=False):
+def trace(s0, bhspin, policy, rows=False, freeze=True):
     """Integrate every ray to its stop; returns dict(K, why, state[, S, dt]).
 
     Reference policy: K = first stopped step (N if none), state = state after
-    K steps; with rows=True also the full (N, npx, 8) rows and (N, npx) dt.
+    K steps; with rows=True also the full (N, npx, 8) rows and (N, npx) dt
+    (freeze=False leaves each ray's rows from K on unwritten).
     Fixed policy: K = steps taken, state = final state."""
     s0 = f64(s0)
     if s0.ndim != 2 or s0.shape[1] != 8:
@@ -84,8 +85,8 @@ def trace(s0, bhspin, policy, rows=False):
     if rows:
         S = torch.empty((policy.nmax, npx, 8), dtype=torch.float64, device=dev)
         dt = torch.empty((policy.nmax, npx), dtype=torch.float64, device=dev)
-    _lib.call("mk_integrate", ptr(s0), npx, float(bhspin), _lib.ctypes.byref(policy), ptr(S), ptr(dt), ptr(K),
-              ptr(why), ptr(state), stream_ptr())
+    _lib.call("mk_integrate" if freeze else "mk_integrate_moving", ptr(s0), npx, float(bhspin),
+              _lib.ctypes.byref(policy), ptr(S), ptr(dt), ptr(K), ptr(why), ptr(state), stream_ptr())
     out = dict(K=K, why=why, state=state)
     if rows:
         out["S"], out["dt"] = S, dt
@@ -104,10 +105,14 @@ def trimmed_rows(K, N):
 
 
 def geodesic_integrator(N, s0, div, tol, bhspin):
-    """geodesics.py:233-281 -> (S[N_t, npx, 8], dt[N_t, npx]) CUDA tensors."""
-    r = trace(s0, bhspin, step_policy(N, div, tol), rows=True)
+    """geodesics.py:233-281 -> (S[N_t, npx, 8], dt[N_t, npx]) CUDA tensors.
+
+    Only the kept rows of stopped rays are filled with their last state."""
+    r = trace(s0, bhspin, step_policy(N, div, tol), rows=True, freeze=False)
     nt = trimmed_rows(r["K"], N)
-    return r["S"][:nt], r["dt"][:nt]
+    S, dt = r["S"][:nt], r["dt"][:nt]
+    _lib.call("mk_freeze_rows", ptr(r["state"]), ptr(r["K"]), S.shape[1], nt, ptr(S), ptr(dt), stream_ptr())
+    return S, dt
 
 
 def radius_cal(x, bhspin):
@@ -133,37 +138,36 @@ def _shadow_pass(inc, ca, sa, mid, bhspin, distance, max_steps):
     n = len(mid)
     ci, si = _cos_sin(inc)
     cat, sat, midt = f64(ca, dev), f64(sa, dev), f64(mid, dev)
-    K = torch.empty(n, dtype=torch.int32, device=dev)
-    best = torch.empty(n, dtype=torch.int32, device=dev)
-    best_dt, r_km1, r_best, r_last = (torch.empty(n, dtype=torch.float64, device=dev) for _ in range(4))
+    ints = torch.empty((2, n), dtype=torch.int32, device=dev)
+    vals = torch.empty((4, n), dtype=torch.float64, device=dev)
     _lib.call("mk_shadow_pass", ptr(cat), ptr(sat), ptr(midt), n, float(bhspin), ci, si, float(distance),
-              int(max_steps), ptr(K), ptr(best), ptr(best_dt), ptr(r_km1), ptr(r_best), ptr(r_last),
+              int(max_steps), ptr(ints[0]), ptr(ints[1]), ptr(vals[0]), ptr(vals[1]), ptr(vals[2]), ptr(vals[3]),
               stream_ptr())
-    K, best = K.cpu().numpy(), best.cpu().numpy()
-    best_dt, r_km1, r_best, r_last = (t.cpu().numpy() for t in (best_dt, r_km1, r_best, r_last))
-    N = int(max_steps)
+    K, best = ints.cpu().numpy()
+    best_dt, r_km1, r_best, r_last = vals.cpu().numpy()
     # argmax(dt) over the trimmed rows: a stopped ray's rows from K on hold
     # dt == 0, and K always lies inside the trimmed range, so argmax is K
     # unless an accepted step had dt > 0; a ray that never stopped keeps all
     # N rows and argmax is its largest dt.
-    out = np.empty(n)
-    for p in range(n):
-        if K[p] < N:
-            am = best[p] if (best[p] >= 0 and best_dt[p] > 0) else K[p]
-        else:
-            am = best[p]
-        row = am - 1
-        if row < 0:
-            out[p] = r_last[p]          # row -1 wraps to the last kept row
-        elif am == K[p]:
-            out[p] = r_km1[p]
-        else:
-            out[p] = r_best[p]
-    return out
+    am = np.where((K < int(max_steps)) & ~((best >= 0) & (best_dt > 0)), K, best)
+    # row am - 1; row -1 wraps to the last kept row
+    return np.where(am < 1, r_last, np.where(am == K, r_km1, r_best))
+
+
+# Rays a bisection pass may take: one a lane of one warp on each of the 608 SM
+# sub-partitions, up to where a pass costs its longest ray's chain of steps
+# whatever their number.
+SHADOW_RAYS = 608 * 32
 
 
 def find_shadow_bisection_angles(bhspin, inc, angles, max_steps=2000, error_allowed=0.001, max_it=40):
-    """geodesics.py:405-435: bisection on 'fell in' (r < 100) per angle."""
+    """geodesics.py:405-435: bisection on 'fell in' (r < 100) per angle.
+
+    Each pass integrates the midpoints of the next few bisections at once,
+    every one that the results of those before it can lead to (2^L - 1 for L
+    of them), then follows each angle's branch: the same midpoints, decisions
+    and radii as one bisection a pass, in fewer of the passes whose length is
+    a ray's chain of steps."""
     angles = np.asarray(angles, dtype=np.float64)
     ca, sa = np.cos(angles), np.sin(angles)
     inner = np.zeros_like(angles) + 0.5
@@ -171,14 +175,40 @@ def find_shadow_bisection_angles(bhspin, inc, angles, max_steps=2000, error_allo
     error = outer - inner
     counter = 0
     while np.max(error) > error_allowed and counter < max_it:
-        mid = (outer - inner) / 2 + inner
-        final_mid = _shadow_pass(inc, ca, sa, mid, bhspin, 1000, max_steps)
-        fell = np.where(final_mid < 100)
-        got_away = np.where(final_mid >= 100)
-        inner[fell] = (outer[fell] - inner[fell]) / 2 + inner[fell]
-        outer[got_away] = (outer[got_away] - inner[got_away]) / 2 + inner[got_away]
-        error = outer - inner
-        counter += 1
+        left = int(min(np.ceil(np.log2(max(np.max(error) / error_allowed, 2.0))) if error_allowed > 0 else max_it,
+                       max_it - counter))
+        most = max(1, int(np.log2(SHADOW_RAYS / max(angles.size, 1) + 1.0)) if angles.size < SHADOW_RAYS else 1)
+        passes = -(-left // most)
+        depth = -(-left // passes)
+        # node i of level l: its interval's ends; children 2i (got away: the
+        # outer end moves) and 2i + 1 (fell in: the inner end moves)
+        lo, hi, mids = [inner[None]], [outer[None]], []
+        for _ in range(depth):
+            a, b = lo[-1], hi[-1]
+            mid = (b - a) / 2 + a
+            mids.append(mid)
+            lo.append(np.stack([a, mid], 1).reshape((-1,) + angles.shape))
+            hi.append(np.stack([mid, b], 1).reshape((-1,) + angles.shape))
+        flat = np.concatenate(mids).reshape(-1, angles.size)
+        shape = (len(flat), angles.size)
+        r = _shadow_pass(inc, np.broadcast_to(ca.reshape(-1), shape).reshape(-1),
+                         np.broadcast_to(sa.reshape(-1), shape).reshape(-1), flat.reshape(-1), bhspin, 1000,
+                         max_steps).reshape(shape)
+        node = np.zeros(angles.size, dtype=np.int64)
+        stuck = np.zeros(angles.size, dtype=bool)     # a ray with no radius moves neither end
+        cols = np.arange(angles.size)
+        for level in range(depth):
+            if not (np.max(error) > error_allowed and counter < max_it):
+                break
+            at = r[2 ** level - 1 + node, cols]
+            mid = mids[level].reshape(-1, angles.size)[node, cols]
+            fell, away = (at < 100) & ~stuck, (at >= 100) & ~stuck
+            stuck |= ~(fell | away)
+            inner.reshape(-1)[fell] = mid[fell]
+            outer.reshape(-1)[away] = mid[away]
+            node = 2 * node + fell
+            error = outer - inner
+            counter += 1
     return inner
 
 
