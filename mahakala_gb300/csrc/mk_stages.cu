@@ -5,6 +5,7 @@
 // stage-by-stage call sequence available on the device.
 #include "mk_common.cuh"
 #include "mk_fluid.cuh"
+#include "mk_stage_tri.cuh"
 
 namespace mk {
 
@@ -141,24 +142,40 @@ __global__ void geom_f32_kernel(const double *__restrict__ geom, int nmb, float 
     o[1] = make_float4((float)(1.0 / g[4]), (float)(1.0 / g[5]), 0.0f, 0.0f);
 }
 
-__global__ void fluid_scalars_kernel(mk_snapshot_view sv, double a, const double *__restrict__ S, int64_t npts,
-                                     double cos_fallback, double *__restrict__ out) {
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= npts) return;
-    const double *s = S + 8 * p;
+__device__ __noinline__ void fluid_point_f64(const mk_snapshot_view &sv, double a, const double s[8],
+                                             double cos_fallback, double out[5]) {
     double prim[8];
     CellPos c;
     if (locate(sv, s[1], s[2], s[3], c)) trilinear8(sv, c, prim);
     else
 #pragma unroll
         for (int q = 0; q < 8; q++) prim[q] = 0.0;
-    const double k[4] = {s[4], s[5], s[6], s[7]};
-    const FluidScalars fs = fluid_frame(prim, s[1], s[2], s[3], k, a, cos_fallback);
-    out[5 * p + 0] = fs.dens;
-    out[5 * p + 1] = fs.u;
-    out[5 * p + 2] = fs.pitch;
-    out[5 * p + 3] = fs.kdotu;
-    out[5 * p + 4] = fs.b;
+    const FluidScalars fs = fluid_frame(prim, s[1], s[2], s[3], s + 4, a, cos_fallback);
+    out[0] = fs.dens;
+    out[1] = fs.u;
+    out[2] = fs.pitch;
+    out[3] = fs.kdotu;
+    out[4] = fs.b;
+}
+
+__global__ void __launch_bounds__(128, 4)
+fluid_scalars_kernel(mk_snapshot_view sv, double a, FluidTri c, const double *__restrict__ S, int64_t npts,
+                     double cos_fallback, double *__restrict__ out) {
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p >= npts) return;
+    double s[8], o[5];
+#pragma unroll
+    for (int i = 0; i < 8; i++) s[i] = S[8 * p + i];
+    if (!fluid_point_tri(sv, c, s, o)) {
+        double s64[8], o64[5];  // through copies: s and o stay in registers
+#pragma unroll
+        for (int i = 0; i < 8; i++) s64[i] = s[i];
+        fluid_point_f64(sv, a, s64, cos_fallback, o64);
+#pragma unroll
+        for (int i = 0; i < 5; i++) o[i] = o64[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 5; i++) out[5 * p + i] = o[i];
 }
 
 __global__ void fluid_prims_kernel(mk_snapshot_view sv, const double *__restrict__ S, int64_t npts,
@@ -181,25 +198,43 @@ __global__ void fluid_prims_kernel(mk_snapshot_view sv, const double *__restrict
     if (block) block[p] = mb;
 }
 
+// the binary64 forms, for inputs outside the triples' range
+__device__ __noinline__ double rlow_rhigh_f64(double dens, double u, double beta, double r_low, double r_high,
+                                              double gem1, double gim1) {
+    return rlow_rhigh(dens, u, beta, r_low, r_high, gem1, gim1);
+}
+__device__ __noinline__ void synchrotron_f64(double Ne, double Th, double B, double pitch, double nu, bool invariant,
+                                             double rescale_nu, double *em, double *ab) {
+    synchro_eval(synchro_pre(Ne, Th, B, pitch), nu, invariant, rescale_nu, *em, *ab);
+}
+
 __global__ void rlow_rhigh_kernel(const double *__restrict__ dens, const double *__restrict__ u,
                                   const double *__restrict__ beta, int64_t n, double r_low, double r_high,
-                                  double gem1, double gim1, double *__restrict__ out) {
+                                  double gem1, double gim1, RlowTri k, double *__restrict__ out) {
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= n) return;
-    out[p] = rlow_rhigh(dens[p], u[p], beta[p], r_low, r_high, gem1, gim1);
+    const double d = dens[p], e = u[p], b = beta[p];
+    double v;
+    if (!rlow_tri(k, d, e, b, v)) v = rlow_rhigh_f64(d, e, b, r_low, r_high, gem1, gim1);
+    out[p] = v;
 }
 
 __global__ void synchrotron_kernel(const double *__restrict__ Ne, const double *__restrict__ Th,
                                    const double *__restrict__ B, const double *__restrict__ pitch,
                                    const double *__restrict__ nu, int64_t n, int invariant, double rescale_nu,
-                                   double *__restrict__ em, double *__restrict__ ab) {
+                                   SynchroTri c, double *__restrict__ em, double *__restrict__ ab) {
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= n) return;
-    const SynchroPre sp = synchro_pre(Ne[p], Th[p], B[p], pitch[p]);
-    double e, b;
-    synchro_eval(sp, nu[p], invariant != 0, rescale_nu, e, b);
+    const double ne = Ne[p], th = Th[p], b = B[p], pa = pitch[p], v = nu[p];
+    double e, a;
+    if (!synchro_tri(c, ne, th, b, pa, v, invariant != 0, e, a)) {
+        double e64, a64;  // through copies: e and a stay in registers
+        synchrotron_f64(ne, th, b, pa, v, invariant != 0, rescale_nu, &e64, &a64);
+        e = e64;
+        a = a64;
+    }
     em[p] = e;
-    ab[p] = b;
+    ab[p] = a;
 }
 
 // backward explicit Euler (transfer.py:106-119), one thread per pixel
@@ -295,8 +330,8 @@ extern "C" int mk_fluid_scalars(const mk_snapshot_view *view, double bhspin, con
     MK_REQUIRE(view && S_dev && out_dev, MK_ERR_ARG, "mk_fluid_scalars: null pointer");
     MK_REQUIRE(npts >= 0, MK_ERR_ARG, "mk_fluid_scalars: negative size");
     if (npts == 0) return MK_OK;
-    fluid_scalars_kernel<<<grid_for(npts, 128), 128, 0, as_stream(stream)>>>(*view, bhspin, S_dev, npts,
-                                                                           cos_fallback, out_dev);
+    fluid_scalars_kernel<<<grid_for(npts, 128), 128, 0, as_stream(stream)>>>(
+        *view, bhspin, fluid_tri_consts(*view, bhspin, cos_fallback), S_dev, npts, cos_fallback, out_dev);
     MK_LAUNCHED("fluid_scalars_kernel");
     return MK_OK;
 }
@@ -318,7 +353,10 @@ extern "C" int mk_rlow_rhigh(const double *dens_dev, const double *u_dev, const 
     MK_REQUIRE(n >= 0, MK_ERR_ARG, "mk_rlow_rhigh: negative size");
     if (n == 0) return MK_OK;
     rlow_rhigh_kernel<<<grid_for(n, 256), 256, 0, as_stream(stream)>>>(dens_dev, u_dev, beta_dev, n, r_low, r_high,
-                                                                     electron_gamma_m1, ion_gamma_m1, theta_dev);
+                                                                     electron_gamma_m1, ion_gamma_m1,
+                                                                     rlow_tri_consts(r_low, r_high, electron_gamma_m1,
+                                                                                     ion_gamma_m1),
+                                                                     theta_dev);
     MK_LAUNCHED("rlow_rhigh_kernel");
     return MK_OK;
 }
@@ -331,7 +369,9 @@ extern "C" int mk_synchrotron(const double *Ne_dev, const double *theta_dev, con
     MK_REQUIRE(n >= 0, MK_ERR_ARG, "mk_synchrotron: negative size");
     if (n == 0) return MK_OK;
     synchrotron_kernel<<<grid_for(n, 128), 128, 0, as_stream(stream)>>>(Ne_dev, theta_dev, B_dev, pitch_dev, nu_dev,
-                                                                      n, invariant, rescale_nu, em_dev, ab_dev);
+                                                                      n, invariant, rescale_nu,
+                                                                      synchro_tri_consts(invariant != 0, rescale_nu),
+                                                                      em_dev, ab_dev);
     MK_LAUNCHED("synchrotron_kernel");
     return MK_OK;
 }

@@ -135,6 +135,24 @@ MK_HD pr p_rcp(pr x) {
     return p_norm({y, f_mul(y, fmaf(d, d, d))});
 }
 
+// Z^(-1/3): the float unit's estimate, one Newton step in float, a third-order
+// correction from the pair residual 1 - Z x^3
+__device__ __forceinline__ pr p_rcbrt(pr z) {
+    float l, x;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(z.h));
+    l *= -0.333333343f;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(l));
+    x = fmaf(f_mul(x, 0.333333343f), fmaf(-f_mul(f_mul(z.h, x), x), x, 1.0f), x);
+    const pr x2 = {f_mul(x, x), fmaf(x, x, -f_mul(x, x))};
+    const pr x3 = p_mulr(x2, {x, 0.0f});
+    const float p = f_mul(z.h, x3.h);
+    float e = fmaf(z.h, x3.h, -p);
+    e = fmaf(z.h, x3.l, e);
+    e = fmaf(z.l, x3.h, e);
+    const float d = f_sub(f_sub(1.0f, p), e);
+    return p_norm({x, f_mul(f_mul(x, d), fmaf(0.222222222f, d, 0.333333343f))});
+}
+
 // ---------------------------------------------------------------- triples
 // On the device both conversions keep off the FP64 pipe, where each F2F costs
 // as much as an addition (64 cycles a warp instruction): the words are moved
