@@ -143,7 +143,48 @@ __device__ __forceinline__ tri t_acos(tri c) {
     return t_add(t0, t_add(x, t_norm({r.h, r.l, 0.0f})));
 }
 
-__device__ __forceinline__ bool within(double v, double lo, double hi) { return v >= lo && v <= hi; }
+// Tests and scalings by the bits: a comparison costs the FP64 pipe as much as
+// an addition.  Positive doubles order as integers; NaN lies above infinity.
+__device__ __forceinline__ bool within(double v, double lo, double hi) {
+    const long long b = __double_as_longlong(v);
+    return b >= __double_as_longlong(lo) && b <= __double_as_longlong(hi);
+}
+__device__ __forceinline__ bool is_zero(double v) { return (__double_as_longlong(v) << 1) == 0; }
+// v 2^e, v a positive normal number and the result too, or v = 0
+__device__ __forceinline__ double scaled(double v, int e) {
+    return is_zero(v) ? 0.0 : __hiloint2double(__double2hiint(v) + (int)((unsigned)e << 20), __double2loint(v));
+}
+
+// doubles in order as integers (-0 = 0)
+__device__ __forceinline__ long long ordered(double v) {
+    const long long b = __double_as_longlong(v);
+    return (b << 1) == 0 ? 0 : b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+
+// sin(x) for 0 <= x <= 100: x = n pi/64 + r, the table's sine and cosine and
+// the series of r, |r| < 0.025
+__device__ __forceinline__ tri t_sin(tri x) {
+    const float n = rintf(x.h * 20.371832f);
+    const float c1 = 0x1.921fb6p-5f, c2 = -0x1.777a5cp-30f, c3 = -0x1.ee59dap-55f;
+    const float p = f_mul(n, c1), pe = fmaf(n, c1, -p), q = f_mul(n, c2), qe = fmaf(n, c3, fmaf(n, c2, -q));
+    const tri r = t_sub(x, t_add({p, pe, 0.0f}, {q, qe, 0.0f}));
+    const int k = (int)n & 127, m = k & 63, i = m <= 32 ? m : 64 - m;  // sin and cos of k pi/64 from the first octant pair
+    const float *T = COSSIN64[i];
+    const float g = k < 64 ? 1.0f : -1.0f, gc = m <= 32 ? g : -g;
+    const tri s0 = {g * __ldg(T + 3), g * __ldg(T + 4), g * __ldg(T + 5)};
+    const tri c0 = {gc * __ldg(T), gc * __ldg(T + 1), gc * __ldg(T + 2)};
+    const pr r1 = {r.h, r.m}, r2 = p_mulr(r1, r1), r3 = p_mulr(r2, r1), r4 = p_mulr(r2, r2);
+    const float z = r2.h;
+    // sin r - r and cos r - 1
+    pr a = p_mul(r3, {-0x1.555556p-3f, 0x1.555556p-28f});
+    const pr a5 = p_mul(p_mulr(r4, r1), {0x1.111112p-7f, -0x1.dddddep-32f});
+    a = p_add(a, {a5.h, fmaf(f_mul(f_mul(r4.h, r3.h), 1.0f), fmaf(z, 1.0f / 362880.0f, -1.0f / 5040.0f), a5.l)});
+    pr b = p_two(r2, -0.5f);
+    const pr b4 = p_mul(r4, {0x1.555556p-5f, -0x1.555556p-30f});
+    b = p_add(b, {b4.h, fmaf(f_mul(r4.h, z), fmaf(z, 1.0f / 40320.0f, -1.0f / 720.0f), b4.l)});
+    const tri sr = t_add(r, t_norm({a.h, a.l, 0.0f})), cr = t_norm({b.h, b.l, 0.0f});
+    return t_add(t_add(s0, t_mul(s0, cr)), t_mul(c0, sr));
+}
 
 // synchrotron_coefficients (transfer.py:30-86): with Z = nu_s / nu and Y =
 // Z^(1/3) the emissivity is K Ne nu (1 + 2^(11/12) Y)^2 exp(-1/Y) / Theta_e^2
@@ -171,16 +212,17 @@ __device__ __forceinline__ bool synchro_tri(const SynchroTri &c, double Ne, doub
                                             double nu, bool invariant, double &em_out, double &ab_out) {
     em_out = ab_out = 0.0;
     // no emission: Theta_e below 0.3 or NaN, no electrons, no field
-    if (!(Th >= 0.3) || Ne == 0.0 || B == 0.0) return true;
+    if (!within(Th, 0.3, __longlong_as_double(0x7ff0000000000000LL)) || is_zero(Ne) || is_zero(B)) return true;
     // the density's exponent goes to the result (it falls by tens of decades
     // along a torus' poles)
     const unsigned hn = (unsigned)__double2hiint(Ne);
     const int en = (int)(hn >> 20) - 1023;  // of a positive normal number
-    if (!(c.ok && en > -500 && en < 500 && Th <= 1e6 && within(B, 1e-20, 1e10) && within(nu, 1e3, 1e16)))
+    if (!(c.ok && en > -400 && en < 400 && within(Th, 0.3, 1e6) && within(B, 1e-20, 1e10) && within(nu, 1e3, 1e16) &&
+          within(pitch, 0.0, 100.0)))
         return false;
     const tri ne = t_from(__hiloint2double((int)(hn - ((unsigned)en << 20)), __double2loint(Ne)));
-    const tri th = t_from(Th), v = t_from(nu * 0x1p-37), rv = t_rcp(v), rth = t_rcp(th);
-    const tri nus = t_mulr(t_mulr(c.knus, t_from(B)), t_mulr(t_mulr(th, th), t_from(sin(pitch))));
+    const tri th = t_from(Th), v = t_from(scaled(nu, -37)), rv = t_rcp(v), rth = t_rcp(th);
+    const tri nus = t_mulr(t_mulr(c.knus, t_from(B)), t_mulr(t_mulr(th, th), t_sin(t_from(pitch))));
     const tri Z = t_mulr(nus, rv);
     if (!(Z.h >= 1e-12f)) return true;  // X > 1e12, or a sine that is not positive (X < 0: not a number)
     const pr y0 = p_rcbrt({Z.h, Z.m});
@@ -212,10 +254,14 @@ __device__ __forceinline__ bool synchro_tri(const SynchroTri &c, double Ne, doub
     } else {
         em = t_mulr(em, v);
     }
-    const int x = en - 60 - e;
-    const double s = x > -1000 ? __hiloint2double((1023 + x) << 20, 0) : 0.0;
-    em_out = t_to(em) * s;
-    ab_out = t_to(ab) * s;
+    if (e > 400) {  // faint to the end of the doubles' range
+        const double s = e < 900 ? __hiloint2double((1023 - e) << 20, 0) : 0.0;
+        em_out = scaled(t_to(em), en - 60) * s;
+        ab_out = scaled(t_to(ab), en - 60) * s;
+    } else {
+        em_out = scaled(t_to(em), en - 60 - e);
+        ab_out = scaled(t_to(ab), en - 60 - e);
+    }
     return true;
 }
 
@@ -239,20 +285,23 @@ inline RlowTri rlow_tri_consts(double r_low, double r_high, double gem1, double 
 }
 
 __device__ __forceinline__ bool rlow_tri(const RlowTri &k, double dens, double u, double beta, double &out) {
-    if (dens == 0.0 && u == 0.0) {  // outside the snapshot: 0 / 0
+    if (is_zero(dens) && is_zero(u)) {  // outside the snapshot: 0 / 0
         out = nan("");
         return true;
     }
     const unsigned hd = (unsigned)__double2hiint(dens), hu = (unsigned)__double2hiint(u);
     const int ed = (int)(hd >> 20) - 1023, eu = (int)(hu >> 20) - 1023;  // of positive normal numbers
-    if (!(k.ok && ed > -500 && ed < 500 && eu > -500 && eu < 500 && fabs(beta) <= 1e9)) return false;
+    if (!(k.ok && ed > -400 && ed < 400 && eu > -400 && eu < 400 &&
+          ((unsigned)__double2hiint(beta) & 0x7fffffffu) <= 0x41cdcd65u))  // |beta| <= 1e9
+        return false;
     // significands in [1, 2); the exponents go to the result
     const tri d = t_from(__hiloint2double((int)(hd - ((unsigned)ed << 20)), __double2loint(dens)));
     const tri s = t_from(__hiloint2double((int)(hu - ((unsigned)eu << 20)), __double2loint(u)));
     const tri b = t_from(beta), b2 = t_mulr(b, b), ob = t_add({1.0f, 0.0f, 0.0f}, b2);
     const tri D = t_add(t_mulr(k.gi, ob), t_mulr(k.ge, t_add(t_mulr(k.rh, b2), k.rl)));
     const tri th = t_mulr(t_mulr(k.c, s), t_mulr(ob, t_rcp(t_mulr(d, D))));
-    out = t_to(th) * __hiloint2double((1023 + eu - ed) << 20, 0);
+    if (k.rh.h > 0.0f && !(th.h > 1e-30f)) return false;
+    out = scaled(t_to(th), eu - ed);
     return true;
 }
 
@@ -262,9 +311,8 @@ __device__ __forceinline__ bool rlow_tri(const RlowTri &k, double dens, double u
 // operations), the angle by t_acos.  In binary64 the point was ~500 FP64-pipe
 // instructions, also outside the snapshot, where only k.u = -k^t / sqrt(1 + f)
 // is needed.  false: the point is left to the binary64 code (not finite or
-// beyond 1e6, a wavevector beyond 1e12, next to the ring or within 1e-9 of a
-// block's face, whose rule left < x <= right is decided exactly there;
-// primitives beyond the floats' range).
+// beyond 1e6, a wavevector beyond 1e12, next to the ring, or at a face two
+// blocks do not share to the bit; velocities beyond 1e6).
 struct FluidTri {
     tri a, aa;                // spin and its square
     float lo[3], inv_w[3];    // the block grid
@@ -295,7 +343,7 @@ __device__ __forceinline__ bool fluid_point_tri(const mk_snapshot_view &sv, cons
     if (!(xm <= 1e6f && ks >= 1e-6f && ks <= 1e12f && x[0].h == x[0].h && x[1].h == x[1].h && x[2].h == x[2].h))
         return false;
     // the block and cell
-    int c[3], idx[3], mb = -1;
+    int c[3], idx[3], near[3], mb = -1;
     tri del[3];
     bool inside = true;
 #pragma unroll
@@ -317,19 +365,45 @@ __device__ __forceinline__ bool fluid_point_tri(const mk_snapshot_view &sv, cons
                 const tri left = t_from(__ldg(g + i)), d = t_from(__ldg(g + 3 + i));
                 const tri v = t_sub(x[i], left), id = t_rcp(d);
                 const pr t = p_mulr({v.h, v.m}, {id.h, id.m});
-                // faces at t = -1/2 and n - 1/2
-                const float e0 = f_add(t.h, 0.5f) + t.l, e1 = f_sub(t.h, n - 0.5f) + t.l;
-                if (!(fabsf(e0) > 1e-6f && fabsf(e1) > 1e-6f)) return false;
+                // faces at t = -1/2 and n - 1/2; next to one, the block's own
+                // face decides (left < x <= right)
+                float e0 = f_add(t.h, 0.5f) + t.l, e1 = f_sub(t.h, n - 0.5f) + t.l;
+                const bool n0 = !(fabsf(e0) > 1e-6f), n1 = !(fabsf(e1) > 1e-6f);
+                if (n0 || n1) {
+                    const double *fc = sv.faces + 6 * (int64_t)mb + 2 * i;
+                    if (n0) e0 = ordered(s[1 + i]) <= ordered(__ldg(fc)) ? -1.0f : 1.0f;
+                    if (n1) e1 = ordered(s[1 + i]) > ordered(__ldg(fc + 1)) ? 1.0f : -1.0f;
+                }
+                near[i] = n0 ? -1 : (n1 ? 1 : 0);
                 if (e0 < 0.0f) { --c[i]; moved = true; }
                 else if (e1 > 0.0f) { ++c[i]; moved = true; }
                 float fl = floorf(t.h);
-                if (fl == t.h && t.l < 0.0f) fl -= 1.0f;
+                tri u = t_sub(v, t_mul({fl, 0.0f, 0.0f}, d));
+                // the quotient may have rounded across a cell's edge: the rest
+                // lies in [0, d), and is 0 at a cell centre
+                if (u.h < 0.0f) { fl -= 1.0f; u = t_add(u, d); }
+                else if (!t_less(u, d)) { fl += 1.0f; u = t_sub(u, d); }
                 fl = fminf(fmaxf(fl, -1.0f), n - 1.0f);
                 idx[i] = (int)fl + 1;
-                del[i] = t_mulr(t_sub(v, t_mul({fl, 0.0f, 0.0f}, d)), id);
+                del[i] = t_mulr(u, id);
             }
-            if (!moved) break;
-            if (it == 3) { mb = -1; break; }
+            if (!moved) {
+                // two blocks can both hold a point next to a face they do not
+                // share to the bit: the binary64 code takes the later one
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+                    if (near[i]) {
+                        int o[3] = {c[0], c[1], c[2]};
+                        o[i] += near[i];
+                        const int nb = table_at(sv, o);
+                        const int mine = 2 * i + (near[i] > 0), theirs = 2 * i + (near[i] < 0);
+                        if (nb >= 0 && ordered(__ldg(sv.faces + 6 * (int64_t)mb + mine)) !=
+                                           ordered(__ldg(sv.faces + 6 * (int64_t)nb + theirs)))
+                            return false;
+                    }
+                break;
+            }
+            if (it == 3) return false;
         }
     }
     // metric data
@@ -377,21 +451,21 @@ __device__ __forceinline__ bool fluid_point_tri(const mk_snapshot_view &sv, cons
             for (int i = 0; i < 8; i++) prim[i] = q == 0 ? w * v[i] : fma(w, v[i], prim[i]);
         }
     }
+    // the field scaled to order one by a power of two: along the poles of a
+    // torus it falls by tens of decades
+    const unsigned hB = max(max((unsigned)__double2hiint(prim[5]) & 0x7fffffffu, (unsigned)__double2hiint(prim[6]) & 0x7fffffffu),
+                            (unsigned)__double2hiint(prim[7]) & 0x7fffffffu);
+    const bool noB = hB == 0u;
+    const int eB = noB ? 0 : (int)(hB >> 20) - 1023;
+    const double sB = __hiloint2double((1023 - eB) << 20, 0);
     tri U[3], B[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         U[i] = t_from(prim[1 + i]);
-        B[i] = t_from(prim[5 + i]);
+        B[i] = t_from(prim[5 + i] * sB);
     }
-    const float Bm = fmaxf(fmaxf(fabsf(B[0].h), fabsf(B[1].h)), fabsf(B[2].h));
     const float Um = fmaxf(fmaxf(fabsf(U[0].h), fabsf(U[1].h)), fabsf(U[2].h));
-    const bool noB = prim[5] == 0.0 && prim[6] == 0.0 && prim[7] == 0.0;
-    if (!(Bm <= 1e15f && Um <= 1e6f && (Bm >= 1e-20f || noB))) return false;
-    // the field scaled to order one by a power of two
-    const int eB = noB ? 0 : ((int)(__float_as_uint(Bm) >> 23) & 255) - 127;
-    const float sB = __uint_as_float((unsigned)(127 - eB) << 23);
-#pragma unroll
-    for (int i = 0; i < 3; i++) B[i] = {B[i].h * sB, B[i].m * sB, B[i].l * sB};
+    if (!(eB > -500 && eB < 500 && Um <= 1e6f)) return false;
     const tri ira = t_rcp(t_add(rr, aa));
     const tri l1 = t_mulr(t_add(t_mul(r, x[0]), t_mul(a, x[1])), ira);
     const tri l2 = t_mulr(t_sub(t_mul(r, x[1]), t_mul(a, x[0])), ira);

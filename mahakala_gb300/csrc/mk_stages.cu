@@ -237,18 +237,39 @@ __global__ void synchrotron_kernel(const double *__restrict__ Ne, const double *
     ab[p] = a;
 }
 
-// backward explicit Euler (transfer.py:106-119), one thread per pixel
-__global__ void solve_intensity_kernel(const double *__restrict__ em, const double *__restrict__ ab,
-                                       const double *__restrict__ dt, int64_t nsteps, int64_t npx, double L,
-                                       double *__restrict__ I, double *__restrict__ dIs) {
+// backward explicit Euler (transfer.py:106-119), one thread per pixel.  The
+// recurrence is serial but its inputs are not: TRANSFER_AHEAD rows are loaded
+// before the first is used, so that a few warps an SM (an image's pixels are
+// no more) keep the memory busy; small blocks spread them evenly.
+constexpr int TRANSFER_AHEAD = 16, TRANSFER_THREADS = 64;
+template <bool DIS>
+__global__ void __launch_bounds__(TRANSFER_THREADS)
+solve_intensity_kernel(const double *__restrict__ em, const double *__restrict__ ab, const double *__restrict__ dt,
+                       int64_t nsteps, int64_t npx, double L, double *__restrict__ I, double *__restrict__ dIs) {
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= npx) return;
     double Iv = 0.0;
-    for (int64_t i = nsteps - 1, r = 0; i >= 1; i--, r++) {
-        const double dI = (-dt[(i - 1) * npx + p]) * L * (em[i * npx + p] - (ab[i * npx + p] * Iv));
-        Iv += dI;
-        if (dIs) dIs[r * npx + p] = dI;
+    int64_t i = nsteps - 1, r = 0;
+    auto fold = [&](double e, double a, double d) {
+        const double w = (-d) * L, t = e - a * Iv;
+        if (DIS) {
+            dIs[r * npx + p] = w * t;
+            ++r;
+        }
+        Iv += w * t;
+    };
+    for (; i >= TRANSFER_AHEAD; i -= TRANSFER_AHEAD) {
+        double e[TRANSFER_AHEAD], a[TRANSFER_AHEAD], d[TRANSFER_AHEAD];
+#pragma unroll
+        for (int q = 0; q < TRANSFER_AHEAD; q++) {
+            e[q] = em[(i - q) * npx + p];
+            a[q] = ab[(i - q) * npx + p];
+            d[q] = dt[(i - q - 1) * npx + p];
+        }
+#pragma unroll
+        for (int q = 0; q < TRANSFER_AHEAD; q++) fold(e[q], a[q], d[q]);
     }
+    for (; i >= 1; i--) fold(em[i * npx + p], ab[i * npx + p], dt[(i - 1) * npx + p]);
     I[p] = Iv;
 }
 
@@ -381,8 +402,13 @@ extern "C" int mk_solve_intensity(const double *em_dev, const double *ab_dev, co
     MK_REQUIRE(em_dev && ab_dev && dt_dev && I_dev, MK_ERR_ARG, "mk_solve_intensity: null pointer");
     MK_REQUIRE(nsteps >= 0 && npx >= 0, MK_ERR_ARG, "mk_solve_intensity: negative size");
     if (npx == 0) return MK_OK;
-    solve_intensity_kernel<<<grid_for(npx, 128), 128, 0, as_stream(stream)>>>(em_dev, ab_dev, dt_dev, nsteps, npx,
-                                                                            L_unit, I_dev, dIs_dev);
+    const unsigned grid = grid_for(npx, TRANSFER_THREADS);
+    if (dIs_dev)
+        solve_intensity_kernel<true><<<grid, TRANSFER_THREADS, 0, as_stream(stream)>>>(em_dev, ab_dev, dt_dev, nsteps,
+                                                                                       npx, L_unit, I_dev, dIs_dev);
+    else
+        solve_intensity_kernel<false><<<grid, TRANSFER_THREADS, 0, as_stream(stream)>>>(em_dev, ab_dev, dt_dev, nsteps,
+                                                                                        npx, L_unit, I_dev, nullptr);
     MK_LAUNCHED("solve_intensity_kernel");
     return MK_OK;
 }
