@@ -24,7 +24,8 @@ __device__ __forceinline__ bool in_block(const double *__restrict__ f, double x,
            z <= __ldg(f + 5);
 }
 
-__device__ __forceinline__ int table_at(const mk_snapshot_view &s, const int c[3]) {
+template <typename View>
+__device__ __forceinline__ int table_at(const View &s, const int c[3]) {
     if (c[0] < 0 || c[1] < 0 || c[2] < 0 || c[0] >= s.nb[0] || c[1] >= s.nb[1] || c[2] >= s.nb[2]) return -1;
     return __ldg(s.table + ((int64_t)c[2] * s.nb[1] + c[1]) * s.nb[0] + c[0]);
 }

@@ -1258,9 +1258,9 @@ struct TriSlot {
     unsigned flags[32];
     int why[32];         // TM_END
     long long ray[32];   // TM_START
-    float v[28][32];     // x^1..x^3 (h m l), k^0..k^3 (h l), r f l3 ira lv... see tri_post
+    float v[28][32];
 };
-// message words
+// message words (TM_SAMPLE): x^1..x^3 (h m l), k^0..k^3 (h l), r f l3 1/(r^2+a^2) (h l), dt (h m l)
 enum { TV_X = 0, TV_K = 9, TV_M = 17, TV_DT = 25, TV_COUNT = 28 };
 
 struct TriShared {
@@ -1279,7 +1279,7 @@ __device__ __forceinline__ void tri_integrate(int couple, const mk_request *__re
     const int lane = threadIdx.x & 31;
     const PairConsts<TRI_LANES> C = {sh.c_int + 32 * couple + lane};
     bool active = false, exhausted = lane % lane_stride != 0;
-    int steps = 0, nmax = 0;
+    int steps = 0, nmax = 0, last_rq = -1;  // the request whose constants are loaded
     TriState s;
     TriPoint q;
     tri dt = {0.0f, 0.0f, 0.0f};
@@ -1291,14 +1291,16 @@ __device__ __forceinline__ void tri_integrate(int couple, const mk_request *__re
         if (idx == -1) exhausted = true;
         bool start = false;
         if (idx >= 0 && ray_in_request(reqs, nreq, idx)) {
-            const mk_request &R = reqs[find_request(reqs, nreq, idx)];
-            if (!pair_request(R)) {
+            const int rq = find_request(reqs, nreq, idx);
+            const mk_request &R = reqs[rq];
+            if (rq != last_rq && !pair_request(R)) {
                 atomicAdd(&ws->odd_rays, 1ull);  // left to render_fp64_kernel
             } else {
                 double s64[8];
                 camera_ray_fast(R.camera, fetch_pixel(R.camera, idx - R.ray_offset), s64);
                 tri_state(s64, s);
-                pair_consts_geodesic(R, C);
+                if (rq != last_rq) pair_consts_geodesic(R, C);
+                last_rq = rq;
                 nmax = R.policy.nmax;
                 steps = 0;
                 start = true;
@@ -1376,6 +1378,9 @@ __device__ __forceinline__ void tri_sample(int couple, const mk_request *__restr
     int rq = 0, steps = 0, nsamples = 0;
     int64_t pix = 0;
     pr a = {0.0f, 0.0f};
+    SampleView view = {};
+    int nnu = 0, last_rq = -1;  // the request whose constants are loaded
+    int64_t rows = 0;           // per-step diagnostic rows
     long long max_tau = 0;  // bits of a double >= 0: they order as integers
     for (int j = 0;; ++j) {
         const int sl = j % TRI_SLOTS;
@@ -1406,49 +1411,64 @@ __device__ __forceinline__ void tri_sample(int couple, const mk_request *__restr
             rq = find_request(reqs, nreq, ray);
             const mk_request &R = reqs[rq];
             pix = fetch_pixel(R.camera, ray - R.ray_offset);
-            const tri a3 = t_from(R.camera.bhspin);
-            a = {a3.h, a3.m};
-            pair_consts_sample(R, snaps[R.snapshot], C);
+            if (rq != last_rq) {
+                const tri a3 = t_from(R.camera.bhspin);
+                a = {a3.h, a3.m};
+                view = sample_view(snaps[R.snapshot]);
+                nnu = R.nnu;
+                rows = R.rows_dt ? R.rows : 0;
+                pair_consts_sample(R, snaps[R.snapshot], C);
+                last_rq = rq;
+            }
             steps = nsamples = 0;
             max_tau = 0;
 #pragma unroll
             for (int ch = 0; ch < MK_MAX_NU; ch++) { sh.I[ch][col] = 0.0; sh.P[ch][col] = 1.0; }
         }
         if (flags & TM_SAMPLE) {
-            const mk_request &R = reqs[rq];
             ++steps;
-            const bool row = steps < R.rows;
-            if (R.rows_dt && row)  // per-step diagnostics: row `steps` = this state
+            const bool row = steps < rows;
+            if (row) {  // per-step diagnostics: row `steps` = this state
+                const mk_request &R = reqs[rq];
                 R.rows_dt[(int64_t)(steps - 1) * request_pixels(R.camera) + pix] = t_to(dt);
-            const mk_snapshot_view &sv = snaps[R.snapshot];
-            double em[MK_MAX_NU], ab[MK_MAX_NU];
-            const int got = sample_pair(sv, C, R.nnu, x, k, a, m, sh.exptab, em, ab);
-            if (got == PS_BINARY64) {
-                // through copies: em and ab stay in registers
-                double s64[8], e64[MK_MAX_NU], a64[MK_MAX_NU];
-                s64[0] = 0.0;  // x^0 is not read
-#pragma unroll
-                for (int i = 0; i < 3; i++) s64[1 + i] = t_to(x[i]);
-#pragma unroll
-                for (int i = 0; i < 4; i++) s64[4 + i] = d_from(k[i].h) + d_from(k[i].l);
-                coefficients_fp64(R, sv, s64, e64, a64);
-#pragma unroll
-                for (int ch = 0; ch < MK_MAX_NU; ch++) { em[ch] = e64[ch]; ab[ch] = a64[ch]; }
             }
+            PairCoeff co[MK_MAX_NU];
+            const int got = sample_pair(view, C, nnu, x, k, a, m, sh.exptab, co);
             if (got != PS_OUTSIDE) {
                 ++nsamples;
-                const double w = -t_to(dt) * R.L_unit;
+                const pr w = p_neg(p_mulr({dt.h, dt.m}, C.p(PC_LUNIT)));
+                double e64[MK_MAX_NU], a64[MK_MAX_NU];
+                if (got == PS_BINARY64) {
+                    const mk_request &R = reqs[rq];
+                    double s64[8];
+                    s64[0] = 0.0;  // x^0 is not read
+#pragma unroll
+                    for (int i = 0; i < 3; i++) s64[1 + i] = t_to(x[i]);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) s64[4 + i] = d_from(k[i].h) + d_from(k[i].l);
+                    coefficients_fp64(R, snaps[R.snapshot], s64, e64, a64);
+                }
 #pragma unroll
                 for (int ch = 0; ch < MK_MAX_NU; ch++) {
-                    if (ch < R.nnu) {
-                        if (R.rows_em && R.rows_dt && row) {
-                            const int64_t at = (ch * R.rows + steps) * request_pixels(R.camera) + pix;
-                            R.rows_em[at] = em[ch];
-                            R.rows_ab[at] = ab[ch];
+                    if (ch < nnu) {
+                        double wem, tau;
+                        if (got == PS_BINARY64) {
+                            const double wd = d_from(w.h) + d_from(w.l);
+                            wem = wd * e64[ch];
+                            tau = wd * a64[ch];
+                        } else {
+                            wem = p_scaled(p_mulr(w, co[ch].em), co[ch].e);
+                            tau = p_scaled(p_mulr(w, co[ch].ab), co[ch].e);
                         }
-                        const double tau = w * ab[ch], P = sh.P[ch][col];
-                        sh.I[ch][col] += (w * em[ch]) * P;
-                        sh.P[ch][col] = P * (1.0 - tau);
+                        if (row && reqs[rq].rows_em) {
+                            const mk_request &R = reqs[rq];
+                            const int64_t at = (ch * R.rows + steps) * request_pixels(R.camera) + pix;
+                            R.rows_em[at] = got == PS_BINARY64 ? e64[ch] : p_scaled(co[ch].em, co[ch].e);
+                            R.rows_ab[at] = got == PS_BINARY64 ? a64[ch] : p_scaled(co[ch].ab, co[ch].e);
+                        }
+                        const double P = sh.P[ch][col];
+                        sh.I[ch][col] += wem * P;
+                        sh.P[ch][col] = P - tau * P;
                         const long long bits = __double_as_longlong(tau);
                         max_tau = bits > max_tau ? bits : max_tau;
                     }

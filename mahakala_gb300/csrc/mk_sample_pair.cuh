@@ -28,7 +28,7 @@ namespace mk {
 enum PairConst {
     PC_A = 0, PC_AA = 2, PC_AA_L = 4, PC_REH = 5, PC_NINV = 8, PC_TOL = 11, PC_BOX = 13, PC_INVW = 19,
     PC_GAM2 = 22, PC_RHIGH = 24, PC_RLOW = 26, PC_GEM1 = 28, PC_GIM1 = 30, PC_KTH = 32, PC_SIGMA = 34,
-    PC_NU = 36,  // per frequency: emissivity, nu_s, bx and 1/B_nu factors, 8 floats
+    PC_LUNIT = 36, PC_NU = 38,  // per frequency: emissivity, nu_s, bx and 1/B_nu factors, 8 floats
     PC_COUNT = PC_NU + 8 * MK_MAX_NU
 };
 constexpr int EXP_STEPS = 32;  // table of 2^(-j/32)
@@ -68,7 +68,7 @@ __device__ __forceinline__ bool pair_request(const mk_request &R) {
               fabs(R.camera.distance) <= 1e6 && fabs(R.camera.fov_lower) <= 1e6 && fabs(R.camera.fov_upper) <= 1e6;
     ok = ok && in(R.fluid_gamma - 1.0, 1e-6, 1e6) && R.r_low >= 0.0 && R.r_low <= 1e6 && R.r_high >= 0.0 &&
          R.r_high <= 1e6 && R.r_low + R.r_high >= 1e-6 && in(R.electron_gamma_m1, 1e-6, 1e6) &&
-         in(R.ion_gamma_m1, 1e-6, 1e6) && in(R.sigma_cut, 1e-12, 1e12);
+         in(R.ion_gamma_m1, 1e-6, 1e6) && in(R.sigma_cut, 1e-12, 1e12) && in(R.L_unit, 1e5, 1e20);
     for (int ch = 0; ch < MK_MAX_NU; ch++)
         if (ch < R.nnu) {
             const EmissionFold e = emission_fold(R, R.nu[ch]);
@@ -107,6 +107,7 @@ __device__ __forceinline__ void pair_consts_sample(const mk_request &R, const mk
     C.set(PC_GIM1, R.ion_gamma_m1, 2);
     C.set(PC_KTH, (MP * CL2 / ME_CL_CL) * R.electron_gamma_m1 * R.ion_gamma_m1, 2);
     C.set(PC_SIGMA, R.sigma_cut, 2);
+    C.set(PC_LUNIT, R.L_unit, 2);
 #pragma unroll
     for (int ch = 0; ch < MK_MAX_NU; ch++)
         if (ch < R.nnu) {
@@ -118,12 +119,23 @@ __device__ __forceinline__ void pair_consts_sample(const mk_request &R, const mk
         }
 }
 
+// The snapshot's fields a sample reads, held in registers by the sampling warp.
+struct SampleView {
+    const float *blocks;
+    const double *geom;
+    const int32_t *table, *block64;  // block64: null if no block is kept in binary64
+    int nb[3], n;
+};
+__device__ __forceinline__ SampleView sample_view(const mk_snapshot_view &sv) {
+    return {sv.blocks, sv.geom, sv.table, sv.blocks64 ? sv.block64 : nullptr, {sv.nb[0], sv.nb[1], sv.nb[2]}, sv.n};
+}
+
 // The cell of x: the block whose faces enclose it (left < x <= right, to 48
 // bits) and the ghost-shifted index and offset in it (locate_fast).  The
 // candidate comes from the float coordinate; its own cell coordinate t, faces
 // at 1/2 and n + 1/2, decides and moves it across a face it lies beyond.
 template <int STRIDE>
-__device__ __forceinline__ int locate_pair(const mk_snapshot_view &sv, const PairConsts<STRIDE> &C, const tri x[3],
+__device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConsts<STRIDE> &C, const tri x[3],
                                            int idx[3], pr del[3]) {
     int c[3];
 #pragma unroll
@@ -184,80 +196,99 @@ __device__ __forceinline__ pr p_exp_neg(pr x, const float2 *tab, int &e) {
     return p_mulr({T.x, T.y}, {h, f_add(l, q.l)});
 }
 
-// m 2^-e as a double
+// m 2^-e as a double, |m| a normal float or 0, by the exponent's bits
 __device__ __forceinline__ double p_scaled(pr m, int e) {
-    if (e > 1000) return 0.0;
-    return (d_from(m.h) + d_from(m.l)) * __hiloint2double((1023 - e) << 20, 0);
+    if (e > 850 || m.h == 0.0f) return 0.0;
+    const double v = d_from(m.h) + d_from(m.l);
+    return __hiloint2double(__double2hiint(v) - (int)((unsigned)e << 20), __double2loint(v));
 }
+// A sample's coefficients at one frequency: em 2^-e and ab 2^-e.
+struct PairCoeff {
+    pr em, ab;
+    int e;
+};
 
 enum { PS_OUTSIDE = 0, PS_SAMPLED = 1, PS_BINARY64 = 2 };
 
 // One sample at x (triples) for the photon k; a: the spin, m: r, f, l3 and
-// 1/(r^2 + a^2) there.  PS_SAMPLED: em, ab hold the
+// 1/(r^2 + a^2) there.  PS_SAMPLED: co holds the
 // invariant coefficients of every frequency; PS_BINARY64: the point lies in
 // the snapshot, in a block kept in binary64 or at primitives outside the
 // pairs' range, and the caller samples it in binary64.
 template <int STRIDE>
-__device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const PairConsts<STRIDE> &C, int nnu,
+__device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConsts<STRIDE> &C, int nnu,
                                            const tri x[3], const pr k[4], pr a, const pr m[4], const float2 *tab,
-                                           double em[MK_MAX_NU], double ab[MK_MAX_NU]) {
+                                           PairCoeff co[MK_MAX_NU]) {
     int idx[3];
     pr del[3];
     const int mb = locate_pair(sv, C, x, idx, del);
     if (mb < 0) return PS_OUTSIDE;
-    if (sv.blocks64 && __ldg(sv.block64 + mb) >= 0) return PS_BINARY64;
-    // each primitive as the sum of eight weights times cells; one copy of the
-    // code for the four (z, y) neighbours (see tri_step), the cells on their
-    // way to L1 meanwhile
+    if (sv.block64 && __ldg(sv.block64 + mb) >= 0) return PS_BINARY64;
+    // Each primitive as the sum of eight weights times cells; one copy of the
+    // code for the four (z, y) neighbours (see tri_step), a neighbour's cells
+    // loaded while the one before it is summed.  Density, energy and field can
+    // fall by tens of decades (along a torus' poles): where they leave the
+    // floats' comfortable range the sums are taken again with those weights
+    // scaled by 2^100.
     const int n2 = sv.n + 2;
     const int64_t sj = (int64_t)n2 * 8, sk = (int64_t)n2 * n2 * 8;
     const float *base = sv.blocks + ((((int64_t)mb * n2 + idx[2]) * n2 + idx[1]) * n2 + idx[0]) * 8;
-#pragma unroll
-    for (int q = 1; q < 4; q++) {
-        const float *p = base + (q >> 1) * sk + (q & 1) * sj;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 8));
-    }
     const pr one = {1.0f, 0.0f};
     const pr u0 = p_subr(one, del[0]), u1 = p_subr(one, del[1]), u2 = p_subr(one, del[2]);
     pr prim[8];
+    float Bm, up = 1.0f;
+    for (;;) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) prim[i] = {0.0f, 0.0f};
+        for (int i = 0; i < 8; i++) prim[i] = {0.0f, 0.0f};
+        float4 next[4] = {ldg4(base), ldg4(base + 4), ldg4(base + 8), ldg4(base + 12)};
 #pragma unroll 1
-    for (int q = 0; q < 4; q++) {
-        const float *p = base + (q >> 1) * sk + (q & 1) * sj;
-        const float4 c[4] = {ldg4(p), ldg4(p + 4), ldg4(p + 8), ldg4(p + 12)};
-        const pr zy = p_mulr((q & 2) ? del[2] : u2, (q & 1) ? del[1] : u1);
+        for (int q = 0; q < 4; q++) {
+            const float4 c[4] = {next[0], next[1], next[2], next[3]};
+            if (q < 3) {
+                const float *p = base + ((q + 1) >> 1) * sk + ((q + 1) & 1) * sj;
+                next[0] = ldg4(p);
+                next[1] = ldg4(p + 4);
+                next[2] = ldg4(p + 8);
+                next[3] = ldg4(p + 12);
+            }
+            const pr zy = p_mulr((q & 2) ? del[2] : u2, (q & 1) ? del[1] : u1);
 #pragma unroll
-        for (int x = 0; x < 2; x++) {
-            const pr w = p_mulr(zy, x ? del[0] : u0);
-            const float4 lo = c[2 * x], hi = c[2 * x + 1];
-            const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            for (int x = 0; x < 2; x++) {
+                const pr w = p_mulr(zy, x ? del[0] : u0), ws = p_two(w, up);
+                const float4 lo = c[2 * x], hi = c[2 * x + 1];
+                const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const float t = f_mul(w.h, v[i]);
-                const float e = fmaf(w.l, v[i], fmaf(w.h, v[i], -t));
-                float s, r;
-                two_sum_f(prim[i].h, t, s, r);
-                prim[i] = {s, f_add(prim[i].l, f_add(e, r))};
+                for (int i = 0; i < 8; i++) {
+                    const pr g = i >= 1 && i <= 3 ? w : ws;
+                    const float t = f_mul(g.h, v[i]);
+                    const float e = fmaf(g.l, v[i], fmaf(g.h, v[i], -t));
+                    float s, r;
+                    two_sum_f(prim[i].h, t, s, r);
+                    prim[i] = {s, f_add(prim[i].l, f_add(e, r))};
+                }
             }
         }
+#pragma unroll
+        for (int i = 0; i < 8; i++) prim[i] = p_norm(prim[i]);
+        Bm = fmaxf(fmaxf(fabsf(prim[5].h), fabsf(prim[6].h)), fabsf(prim[7].h));
+        if ((prim[0].h >= 1e-22f && prim[4].h >= 1e-22f && Bm >= 1e-22f) || up != 1.0f) break;
+        // excised cells: nothing emits (sigma or Theta_e is not a number)
+        if (prim[0].h == 0.0f) break;
+        up = 0x1p100f;
     }
 #pragma unroll
-    for (int i = 0; i < 8; i++) prim[i] = p_norm(prim[i]);
-#pragma unroll
-    for (int ch = 0; ch < MK_MAX_NU; ch++) em[ch] = ab[ch] = 0.0;
-    if (prim[0].h == 0.0f) return PS_SAMPLED;  // excised cells: sigma or Theta_e is not a number
-    const float Bm = fmaxf(fmaxf(fabsf(prim[5].h), fabsf(prim[6].h)), fabsf(prim[7].h));
+    for (int ch = 0; ch < MK_MAX_NU; ch++) co[ch] = {{0.0f, 0.0f}, {0.0f, 0.0f}, 0};
+    // no energy: Theta_e = 0; no field: beta is infinite and Theta_e not a number
+    if (prim[0].h == 0.0f || prim[4].h == 0.0f || Bm == 0.0f) return PS_SAMPLED;
     const float Um = fmaxf(fmaxf(fabsf(prim[1].h), fabsf(prim[2].h)), fabsf(prim[3].h));
-    if (!(Bm >= 1e-25f && Bm <= 1e25f && Um <= 1e6f && prim[0].h >= 1e-25f && prim[0].h <= 1e25f &&
-          prim[4].h >= 1e-12f * prim[0].h && prim[4].h <= 1e12f * prim[0].h))
+    if (!(Bm >= 1e-22f && Bm <= 1e25f && Um <= 1e6f && prim[0].h >= 1e-22f && prim[0].h <= 1e25f &&
+          prim[4].h <= 1e12f * prim[0].h && prim[4].h >= 0.0f))
         return PS_BINARY64;
     // density and energy, and the field, scaled to order one by powers of two
-    // (along the poles of a torus they fall by tens of decades)
+    const int shift = up == 1.0f ? 0 : 100;
     const int ed = ((int)(__float_as_uint(prim[0].h) >> 23) & 255) - 127;
     const int eB = ((int)(__float_as_uint(Bm) >> 23) & 255) - 127;
-    const int ex = ed - 2 * eB;  // of dens / B^2
+    const int ex = (ed - shift) - 2 * (eB - shift);  // of dens / B^2
     if (ex < -100 || ex > 100) return PS_BINARY64;
     const float sd = __uint_as_float((unsigned)(127 - ed) << 23), sB = __uint_as_float((unsigned)(127 - eB) << 23);
     const pr dens = p_two(prim[0], sd), ue = p_two(prim[4], sd);
@@ -315,7 +346,8 @@ __device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const Pai
     const pr base_nus = p_mulr(p_mulr(p_mulr(b, sp), p_mulr(th, th)), inup);
     const pr base_em = p_mulr(p_mulr(dens, inup), p_mulr(ith, ith));
     const pr base_bx = p_mulr(nup, ith);
-    const float iB = __uint_as_float((unsigned)(127 + eB) << 23);
+    if (eB - shift < -120) return PS_SAMPLED;              // X > 1e12 at any temperature
+    const float iB = __uint_as_float((unsigned)(127 + eB - shift) << 23);
     if (!(base_nus.h >= 1e-26f && base_nus.h <= 1e26f && base_em.h >= 1e-26f && base_em.h <= 1e26f))
         return PS_BINARY64;
 #pragma unroll
@@ -330,22 +362,24 @@ __device__ __forceinline__ int sample_pair(const mk_snapshot_view &sv, const Pai
         const pr t = p_addr(one, p_mul(C211, Yc));
         int e;
         const pr E = p_exp_neg(x3, tab, e);
-        e -= ed;
+        e -= ed - shift;
         const pr em_m = p_mulr(p_mulr(C.p(at), base_em), p_mulr(p_mulr(t, t), E));
-        if (!(em_m.h >= 1e-28f && em_m.h <= 1e28f)) return PS_BINARY64;
-        em[ch] = p_scaled(em_m, e);
+        if (!(em_m.h >= 1e-28f && em_m.h <= 1e15f)) return PS_BINARY64;
         const pr bx = p_mulr(C.p(at + 4), base_bx);
+        pr den;
         if (bx.h < 2.e-3f) {
             // bx (1 + bx/2 (1 + bx/3 (1 + bx/4))), as the reference cuts it
             const pr q = p_sqr(bx);
             const float c3 = f_mul(f_mul(f_mul(bx.h, bx.h), bx.h), fmaf(bx.h, 1.0f / 24.0f, 1.0f / 6.0f));
-            const pr den = p_addr(bx, {f_mul(0.5f, q.h), fmaf(0.5f, q.l, c3)});
-            ab[ch] = p_scaled(p_mulr(em_m, p_mulr(den, C.p(at + 6))), e);
+            den = p_addr(bx, {f_mul(0.5f, q.h), fmaf(0.5f, q.l, c3)});
         } else {
-            const double den = exp((double)bx.h + (double)bx.l) - 1.0;
-            const pr ki = C.p(at + 6);
-            ab[ch] = em[ch] * den * ((double)ki.h + (double)ki.l);
+            if (!(bx.h < 60.0f)) return PS_BINARY64;
+            const tri v = t_from(exp((double)bx.h + (double)bx.l) - 1.0);
+            den = {v.h, v.m};
         }
+        const pr ab_m = p_mulr(em_m, p_mulr(den, C.p(at + 6)));
+        if (!(ab_m.h >= 1e-30f && ab_m.h <= 1e15f)) return PS_BINARY64;
+        co[ch] = {em_m, ab_m, e};
     }
     return PS_SAMPLED;
 }
