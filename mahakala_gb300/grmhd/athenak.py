@@ -66,9 +66,10 @@ def mesh_tables(arrs, max_table_cells=1 << 28):
     if np.any(locs < 0) or np.any(levels < 0) or np.any(locs >= 1 << 18) or np.any(levels >= 512):
         raise ValueError("logical locations must lie in [0, 2^18) and levels in [0, 512)")
     keys = _lib.mesh_key(levels, locs[:, 0], locs[:, 1], locs[:, 2])
-    if len(np.unique(keys)) != nmb:
-        raise ValueError("duplicate (level, logical location) blocks")
     order = np.argsort(keys, kind="stable")
+    sorted_keys = np.ascontiguousarray(keys[order])
+    if np.any(sorted_keys[1:] == sorted_keys[:-1]):
+        raise ValueError("duplicate (level, logical location) blocks")
     faces = np.stack([arrs.x1f[:, 0], arrs.x1f[:, -1], arrs.x2f[:, 0], arrs.x2f[:, -1],
                       arrs.x3f[:, 0], arrs.x3f[:, -1]], axis=1).astype(np.float64)
     left, right = faces[:, 0::2], faces[:, 1::2]
@@ -83,29 +84,38 @@ def mesh_tables(arrs, max_table_cells=1 << 28):
     table = -np.ones((nb[2], nb[1], nb[0]), np.int32)
     start = np.rint((left - lo) / wf).astype(np.int64)
     span = np.rint(widths / wf).astype(np.int64)
-    for m in range(nmb):
-        sl = tuple(slice(start[m, a], start[m, a] + span[m, a]) for a in (2, 1, 0))
-        if np.any(table[sl] >= 0):
-            raise ValueError("overlapping blocks")
-        table[sl] = m
-    keyset = set(keys.tolist())
+    taken = 0
+    kinds, kind = np.unique(span @ np.array([1, 1 << 20, 1 << 40]), return_inverse=True)
+    for s in range(len(kinds)):                   # one span a level
+        m = np.flatnonzero(kind == s)
+        sx, sy, sz = span[m[0]]
+        # the table cells of these blocks, cut at the table's edge as a slice is
+        i, j, k = (start[m, a, None, None, None] + np.arange(n).reshape(sh) for a, n, sh in
+                   ((0, sx, (1, 1, 1, -1)), (1, sy, (1, 1, -1, 1)), (2, sz, (1, -1, 1, 1))))
+        ok = (i < nb[0]) & (j < nb[1]) & (k < nb[2])
+        flat = ((k * nb[1] + j) * nb[0] + i)[ok]
+        taken += flat.size
+        table.reshape(-1)[flat] = np.broadcast_to(m[:, None, None, None], ok.shape)[ok]
+    if np.count_nonzero(table >= 0) != taken:     # a cell taken twice
+        raise ValueError("overlapping blocks")
     fine_ghosts = np.zeros(nmb, bool)
     if np.any(levels != levels[0]):
-        for m in range(nmb):
-            lv, t = int(levels[m]), [int(v) for v in locs[m]]
-            for d in ((di, dj, dk) for di in (-1, 0, 1) for dj in (-1, 0, 1) for dk in (-1, 0, 1)):
-                if d == (0, 0, 0):
-                    continue
-                u = [t[a] + d[a] for a in range(3)]
-                if min(u) >= 0 and int(_lib.mesh_key(lv, *u)) in keyset:
-                    continue
-                if lv > 0 and int(_lib.mesh_key(lv - 1, *[v // 2 for v in u])) in keyset:
-                    continue
-                if min(u) >= 0 and int(_lib.mesh_key(lv + 1, *[2 * v for v in u])) in keyset:
-                    fine_ghosts[m] = True
-                    break
+        def there(lv, u):
+            """Whether a block sits at level lv, location u, row by row."""
+            ok = (lv >= 0) & (u >= 0).all(axis=1)
+            want = _lib.mesh_key(np.where(ok, lv, 0), *np.where(ok[:, None], u, 0).T)
+            at = np.minimum(np.searchsorted(sorted_keys, want), nmb - 1)
+            return ok & (sorted_keys[at] == want)
+
+        lv, t = levels.astype(np.int64), locs.astype(np.int64)
+        for d in np.ndindex(3, 3, 3):
+            d = np.array(d) - 1
+            if not d.any():
+                continue
+            u = t + d
+            fine_ghosts |= ~there(lv, u) & ~there(lv - 1, u // 2) & there(lv + 1, 2 * u)
     block64 = np.where(fine_ghosts, np.cumsum(fine_ghosts) - 1, -1).astype(np.int32)
-    return dict(locs=locs, levels=levels, keys=np.ascontiguousarray(keys[order]),
+    return dict(locs=locs, levels=levels, keys=sorted_keys,
                 key_block=np.ascontiguousarray(order.astype(np.int32)), faces=faces, table=table, nb=nb,
                 lo=lo, width=wf, block64=block64, n64=int(fine_ghosts.sum()))
 
