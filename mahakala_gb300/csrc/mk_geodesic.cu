@@ -131,6 +131,9 @@ __device__ __noinline__ void integrate_reference_f64(double s[8], int j0, int64_
 // sets the time of a small launch, so its rays are spread over every SM
 // sub-partition before they share warps (lanes that near the horizon hold
 // the others of their warp).
+// ROWS: rows or dts wanted; the state is then converted to binary64 at every
+// step, and the state before a rejected step is that row.
+template <bool ROWS>
 __global__ void __launch_bounds__(GEO_THREADS)
 integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a, int N, double div, double tol,
                            double *__restrict__ rows, double *__restrict__ dts, int32_t *__restrict__ Kout,
@@ -143,8 +146,10 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
     for (int i = 0; i < 8; i++) s64[i] = s0[8 * p + i];
     bool out = all_f64 || !tri_range(s64);
     int K = N, why = MK_RAY_MAXSTEPS, j = 0;
-    TriState s;
+    const bool started = !out;
+    TriState s, last;
     tri_state(s64, s);
+    last = s;
     const SpinTri sp = spin_tri(a);
     const RuleTri R = rule_tri(a, div, tol);
     if (!out) {
@@ -156,12 +161,14 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
         bool go = rule_dt(q.r, R, dt, d, w);
         for (j = 0; j < N; j++) {
             tri dtn = dt;
-            tri_doubles(s, s64);
+            if (ROWS) tri_doubles(s, s64);
+            else last = s;
             if (go) {
                 const bool near = d < TRI_NEAR;
                 if (near) {  // through a copy: s itself stays in registers
                     TriState n = s;
                     double sc[8];
+                    if (!ROWS) tri_doubles(s, s64);
 #pragma unroll
                     for (int i = 0; i < 8; i++) sc[i] = s64[i];
                     rk4_step_near(n, sc, t_to(dt), a);
@@ -176,21 +183,23 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
                 why = w;
                 break;
             }
-            if (rows) store_row(rows, (int64_t)j * npx + p, s64);
-            if (dts) dts[(int64_t)j * npx + p] = t_to(dt);
+            if (ROWS && rows) store_row(rows, (int64_t)j * npx + p, s64);
+            if (ROWS && dts) dts[(int64_t)j * npx + p] = t_to(dt);
             dt = dtn;
         }
     }
     if (out) {
+        if (!ROWS && started) tri_doubles(last, s64);
         double sc[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) sc[i] = s64[i];
         integrate_reference_f64(sc, j, p, npx, a, N, div, tol, rows, dts, Kout, why_out, state_out);
         return;
     }
-    if (K == N) tri_doubles(s, s64);  // else s64 is the state before the rejected step
     Kout[p] = K;
     why_out[p] = why;
+    if (K == N) tri_doubles(s, s64);
+    else if (!ROWS) tri_doubles(last, s64);  // a rejected step leaves the state before it
     store_row(state_out, p, s64);
 }
 
@@ -441,7 +450,8 @@ static int integrate(const double *s0_dev, int64_t npx, double bhspin, const mk_
     cudaStream_t st = as_stream(stream);
     const int rpw = rays_per_warp(npx);
     if (policy->kind == MK_POLICY_REFERENCE) {
-        integrate_reference_kernel<<<ray_grid(npx, rpw), GEO_THREADS, 0, st>>>(
+        const auto kernel = rows_dev || dt_dev ? integrate_reference_kernel<true> : integrate_reference_kernel<false>;
+        kernel<<<ray_grid(npx, rpw), GEO_THREADS, 0, st>>>(
             s0_dev, npx, bhspin, policy->nmax, policy->div, policy->tol, rows_dev, dt_dev, K_dev, why_dev, state_dev,
             rpw, !tri_policy(*policy));
         MK_LAUNCHED("integrate_reference_kernel");

@@ -15,35 +15,6 @@
 
 namespace mk {
 
-MK_HD tri t_norm(tri x) {
-    float h, t;
-    tri o;
-    fast_sum_f(x.h, x.m, h, t);
-    fast_sum_f(t, x.l, o.m, o.l);
-    fast_sum_f(h, o.m, o.h, o.m);
-    return o;
-}
-MK_HD tri t_mulr(tri x, tri y) { return t_norm(t_mul(x, y)); }
-
-// 1/x: the pair reciprocal and a Newton step from the triple residual
-__device__ __forceinline__ tri t_rcp(tri x) {
-    const pr y = p_rcp({x.h, x.m});
-    const tri p = t_mul(x, {y.h, y.l, 0.0f});
-    const float d = f_sub(f_sub(f_sub(1.0f, p.h), p.m), p.l);
-    return t_norm({y.h, y.l, f_mul(y.h, d)});
-}
-
-static __device__ __noinline__ tri t_rsqrt(tri x) {
-    const pr y = p_rsqrt({x.h, x.m});
-    const tri y3 = {y.h, y.l, 0.0f}, p = t_mul(t_norm(t_sqr(y3)), x);
-    const float d = f_sub(f_sub(f_sub(1.0f, p.h), p.m), p.l);
-    return t_norm({y.h, y.l, f_mul(f_mul(0.5f, y.h), d)});
-}
-static __device__ __noinline__ tri t_dot(tri x1, tri y1, tri x2, tri y2, tri x3, tri y3) {
-    return t_add(t_add(t_mul(x1, y1), t_mul(x2, y2)), t_mul(x3, y3));
-}
-__device__ __forceinline__ tri t_sub(tri x, tri y) { return t_add(x, t_neg(y)); }
-
 // 2^(-j/32), three words each
 __device__ const float EXP32[32][3] = {
     {0x1.0000000000000p+0f, 0x0.0p+0f, 0x0.0p+0f}, {0x1.f507660000000p-1f, -0x1.246eb00000000p-27f, 0x1.9d3e120000000p-55f},

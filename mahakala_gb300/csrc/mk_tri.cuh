@@ -16,7 +16,8 @@
 // Against a 113-bit integration of 400 random rays each at spin 0, 0.5 and
 // 0.94 (camera at 1000 M), end states are 0.17-0.24 times as far off as
 // those of the binary64 integrator (geometric mean), captured and escaping
-// rays alike, if the last approach to the horizon is taken in binary64:
+// rays alike, if the last approach to the horizon is taken in binary64 (in
+// triples it took longer, ~38 k cycles a step against ~31 k):
 // there k grows as 1 / (r - r_EH), and E and L, which steer the ray, are
 // small differences of its components.  TRI_NEAR is where: 0.1 M keeps
 // captured rays at 0.10-0.33 times the binary64 form's error, 0.03 M at
@@ -228,13 +229,42 @@ MK_HD tri t_sqr(tri x) {
     two_sum_f(e, c, s, t);
     return {p, s, fmaf(x.m, x.m, fmaf(g, x.l, f_add(ce, t)))};
 }
+MK_HD tri t_norm(tri x) {
+    float h, t;
+    tri o;
+    fast_sum_f(x.h, x.m, h, t);
+    fast_sum_f(t, x.l, o.m, o.l);
+    fast_sum_f(h, o.m, o.h, o.m);
+    return o;
+}
+MK_HD tri t_mulr(tri x, tri y) { return t_norm(t_mul(x, y)); }
+
+// 1/x: the pair reciprocal and a Newton step from the triple residual
+__device__ __forceinline__ tri t_rcp(tri x) {
+    const pr y = p_rcp({x.h, x.m});
+    const tri p = t_mul(x, {y.h, y.l, 0.0f});
+    const float d = f_sub(f_sub(f_sub(1.0f, p.h), p.m), p.l);
+    return t_norm({y.h, y.l, f_mul(y.h, d)});
+}
+
+__device__ __forceinline__ tri t_rsqrt(tri x) {
+    const pr y = p_rsqrt({x.h, x.m});
+    const tri y3 = {y.h, y.l, 0.0f}, p = t_mul(t_norm(t_sqr(y3)), x);
+    const float d = f_sub(f_sub(f_sub(1.0f, p.h), p.m), p.l);
+    return t_norm({y.h, y.l, f_mul(f_mul(0.5f, y.h), d)});
+}
+static __device__ __noinline__ tri t_dot(tri x1, tri y1, tri x2, tri y2, tri x3, tri y3) {
+    return t_add(t_add(t_mul(x1, y1), t_mul(x2, y2)), t_mul(x3, y3));
+}
+__device__ __forceinline__ tri t_sub(tri x, tri y) { return t_add(x, t_neg(y)); }
+
 // x < y on the two leading words (x and y normalised)
 MK_HD bool t_less(tri x, tri y) { return x.h < y.h || (x.h == y.h && x.m < y.m); }
 
 // ----------------------------------------------------------- acceleration
 struct SpinTri {
-    pr a, aa;  // spin and its square as pairs
-    tri aa3;   // the square to 72 bits
+    pr a, aa;     // spin and its square as pairs
+    tri aa3;      // the square to 72 bits
 };
 MK_HD SpinTri spin_tri(double a) {
     SpinTri s;
