@@ -895,6 +895,8 @@ __device__ __forceinline__ void zone_integrate(const mk_request *__restrict__ re
     float xf[8];  // the state rounded to float
     float d1[4], dt = 0.0f, r_cur = 0.0f, dr_prev = 0.0f, reh = 0.0f, a = 0.0f, div = 0.0f, tol = 0.0f;
     float r_out = 0.0f;
+    unsigned moving = 0u;   // lanes with a ray after the last step
+    bool drained = false;   // no lane will find another ray
 
     for (int it = 0;; ++it) {
         const int sl = it % ZONE_SLOTS;
@@ -904,8 +906,13 @@ __device__ __forceinline__ void zone_integrate(const mk_request *__restrict__ re
             return;
         }
         unsigned flags = 0;
-        const long long idx = fetch(!active && !exhausted, counter, total);
-        if (idx == -1) exhausted = true;
+        // votes sit on the chain: one a step (at its end) tells whether lanes
+        // want a ray and whether any still moves
+        long long idx = -2;
+        if (moving != 0xffffffffu && !drained) {
+            idx = fetch(!active && !exhausted, counter, total);
+            if (idx == -1) exhausted = true;
+        }
         if (idx >= 0) {
             const RayRecord &q = q64[idx];
             double s[8];
@@ -947,7 +954,11 @@ __device__ __forceinline__ void zone_integrate(const mk_request *__restrict__ re
                 active = true;
             }
         }
-        const bool any = __any_sync(0xffffffffu, active);
+        bool any = moving != 0u;
+        if (moving != 0xffffffffu && !drained) {
+            any = __any_sync(0xffffffffu, active);
+            drained = __any_sync(0xffffffffu, exhausted) != 0;  // the queue only shrinks
+        }
         if (active) {
             float xa[4], dK[4];
             rk4_increment_f32(xf, xf + 4, d1, dt, a, xa, dK);
@@ -968,49 +979,53 @@ __device__ __forceinline__ void zone_integrate(const mk_request *__restrict__ re
             int w1;
             const float r_new = m.r;
             const float dtn = reference_dt(r_new, reh, div, tol, w1);
-            if (dtn == 0.0f) {
+            // Every message is written whole (a rejected step's is not read),
+            // and the ray's events are told apart only when there is one: the
+            // common step takes one branch.
+#pragma unroll
+            for (int i = 0; i < 4; i++) { X[i] = Xn[i]; K[i] = Kn[i]; }
+#pragma unroll
+            for (int i = 0; i < 8; i++) xf[i] = xn[i];
+#pragma unroll
+            for (int i = 0; i < 4; i++) d1[i] = dn[i];
+#pragma unroll
+            for (int i = 0; i < 7; i++) msg.s[i][lane] = xn[1 + i];
+            msg.m[0][lane] = m.r;
+            msg.m[1][lane] = m.f;
+            msg.m[2][lane] = m.l1;
+            msg.m[3][lane] = m.l2;
+            msg.m[4][lane] = m.l3;
+            msg.dt[lane] = dt;
+            const bool moved = dtn != 0.0f;
+            flags |= moved ? ZM_SAMPLE | (inzone ? ZM_ZONE : 0u) : ZM_END;
+            dt = dtn;
+            steps += moved;
+            b_steps += moved;
+            zone_steps += moved && inzone;
+            run += moved && inzone;
+            run_max = max(run_max, run);
+            const float dr = r_new - r_cur;
+            const bool last = steps >= nmax - 1, turn = (dr_prev < 0.0f && dr > 0.0f) || (dr_prev > 0.0f && dr < 0.0f);
+            const bool away = dr > 0.0f && (inzone ? r_new >= (float)R_TURN : escape && r_new > r_out);
+            if (!moved) {
                 // the step is rejected and the ray stays frozen (geodesics.py:263-267)
-                flags |= ZM_END;
                 msg.why[lane] = w1;
                 msg.steps[lane] = steps;
                 active = false;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; i++) { X[i] = Xn[i]; K[i] = Kn[i]; }
-#pragma unroll
-                for (int i = 0; i < 8; i++) xf[i] = xn[i];
-#pragma unroll
-                for (int i = 0; i < 4; i++) d1[i] = dn[i];
-                flags |= ZM_SAMPLE | (inzone ? ZM_ZONE : 0u);
-#pragma unroll
-                for (int i = 0; i < 7; i++) msg.s[i][lane] = xn[1 + i];
-                msg.m[0][lane] = m.r;
-                msg.m[1][lane] = m.f;
-                msg.m[2][lane] = m.l1;
-                msg.m[3][lane] = m.l2;
-                msg.m[4][lane] = m.l3;
-                msg.dt[lane] = dt;
-                dt = dtn;
-                ++steps;
-                ++b_steps;
-                if (inzone) {
-                    ++zone_steps;
-                    run_max = max(run_max, ++run);
-                }
-                const float dr = r_new - r_cur;
-                if (steps >= nmax - 1) {
+            } else if (last || away || (inzone && turn)) {
+                if (last) {
                     // trajectory rows stop at N-1: step N-1 never reaches the solve
                     flags |= ZM_END;
                     msg.why[lane] = MK_RAY_MAXSTEPS;
                     msg.steps[lane] = steps;
                     active = false;
-                } else if (escape && !inzone && r_new > r_out && dr > 0.0f) {
+                } else if (away && !inzone) {
                     // outbound beyond every snapshot cell: no sample follows
                     flags |= ZM_END;
                     msg.why[lane] = MK_RAY_ESCAPED;
                     msg.steps[lane] = steps;
                     active = false;
-                } else if (inzone && r_new >= (float)R_TURN && dr > 0.0f) {
+                } else if (away) {
                     // outbound past the photon-ring region: on to the ray's end
                     // in float pairs, as phase C continues its parked rays,
                     // with no renormalisation (one here changed no pixel by
@@ -1018,7 +1033,7 @@ __device__ __forceinline__ void zone_integrate(const mk_request *__restrict__ re
                     // chain ~6 k cycles per ray)
                     inzone = false;
                     atomicAdd(&ws->zone_exits, 1ull);
-                } else if (inzone && ((dr_prev < 0.0f && dr > 0.0f) || (dr_prev > 0.0f && dr < 0.0f))) {
+                } else {
                     // a radial turning point: renormalise to null in
                     // double-float arithmetic and re-evaluate the first stage
                     // of the next step there (in binary64 its ~100 FP64-pipe
@@ -1031,10 +1046,11 @@ __device__ __forceinline__ void zone_integrate(const mk_request *__restrict__ re
                     xf[4] = K[0].hi;
                     kerr_accel(xf[1], xf[2], xf[3], xf[4], xf[5], xf[6], xf[7], a, d1[0], d1[1], d1[2], d1[3]);
                 }
-                r_cur = r_new;
-                dr_prev = dr;
             }
+            r_cur = r_new;
+            dr_prev = dr;
         }
+        moving = __ballot_sync(0xffffffffu, active);
         msg.idx[lane] = ray;
         msg.flags[lane] = flags | (any ? 0u : ZM_DONE);
         __syncwarp();
