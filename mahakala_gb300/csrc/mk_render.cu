@@ -1594,9 +1594,17 @@ render_f32_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
     float I[MK_MAX_NU], Ic[MK_MAX_NU], P[MK_MAX_NU];
     int queue_steps = 0, queue_samples = 0;  // SRC_QUEUE: this thread's share of the launch's work
 
+    unsigned moving = 0u;   // lanes with a ray after the last step
+    bool drained = false;   // no lane will find another ray
     for (;;) {
-        const long long idx = fetch(!active && !exhausted, counter, total);
-        if (idx == -1) exhausted = true;
+        // one vote a step, at its end, tells whether lanes want a ray and
+        // whether any still moves
+        const bool refill = moving != 0xffffffffu && !drained;
+        long long idx = -2;
+        if (refill) {
+            idx = fetch(!active && !exhausted, counter, total);
+            if (idx == -1) exhausted = true;
+        }
         if (idx >= 0 && (SRC != SRC_CAMERA || ray_in_request(reqs, nreq, idx))) {
             double s64[8];  // a queue record's state
             if (SRC == SRC_CAMERA) {
@@ -1665,7 +1673,13 @@ render_f32_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                 }
             }
         }
-        if (!__any_sync(0xffffffffu, active)) {
+        bool any = moving != 0u;
+        if (refill) {
+            any = __any_sync(0xffffffffu, active);
+            drained = __any_sync(0xffffffffu, exhausted) != 0;  // the work only shrinks
+        }
+        if (!any) {
+            if (!drained) continue;  // every fetched ray ended at once; more may be left
             if (SRC == SRC_QUEUE && queue_steps) {
                 atomicAdd(&ws->steps_c, (unsigned long long)queue_steps);
                 atomicAdd(&ws->samples_c, (unsigned long long)queue_samples);
@@ -1703,22 +1717,22 @@ render_f32_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                     ++queue_steps;
                     queue_samples += inside;
                 }
-                if (steps >= R.policy.nmax - 1) {
-                    finish_ray_f32(R, pix, I, Ic, steps, MK_RAY_MAXSTEPS, nsamples, max_tau, ws);
-                    active = false;
-                } else if ((mode & F32_ESCAPE) && r_new > Q.sf.r_out && r_new > r_cur) {
-                    // outbound beyond every snapshot cell: no sample follows
-                    finish_ray_f32(R, pix, I, Ic, steps, MK_RAY_ESCAPED, nsamples, max_tau, ws);
-                    active = false;
-                } else if (SRC == SRC_CAMERA && (mode & (F32_HANDOFF | F32_PARK))) {
-                    // near the horizon or inbound in the photon-ring region: to
-                    // the near-hole queue; outbound past it (F32_PARK): to the
-                    // FP32 continuation queue, whose kernel runs beside the
-                    // near-hole one
-                    const bool to64 = (mode & F32_HANDOFF) &&
-                                      (r_new < (float)R_FP64 || (r_new < (float)R_TURN && r_new < r_cur));
-                    const bool park = !to64 && (mode & F32_PARK) && r_new >= (float)R_TURN && r_new > r_cur;
-                    if (to64 || park) {
+                const bool last = steps >= R.policy.nmax - 1, out = r_new > r_cur;
+                const bool away = (mode & F32_ESCAPE) && r_new > Q.sf.r_out && out;
+                // near the horizon or inbound in the photon-ring region: to
+                // the near-hole queue; outbound past it (F32_PARK): to the
+                // FP32 continuation queue, whose kernel runs beside the
+                // near-hole one
+                const bool to64 = SRC == SRC_CAMERA && (mode & F32_HANDOFF) &&
+                                  (r_new < (float)R_FP64 || (r_new < (float)R_TURN && r_new < r_cur));
+                const bool park = SRC == SRC_CAMERA && !to64 && (mode & F32_PARK) && r_new >= (float)R_TURN && out;
+                if (last || away || to64 || park) {
+                    if (last || away) {
+                        // away: outbound beyond every snapshot cell, no sample follows
+                        finish_ray_f32(R, pix, I, Ic, steps, last ? MK_RAY_MAXSTEPS : MK_RAY_ESCAPED, nsamples, max_tau,
+                                       ws);
+                        active = false;
+                    } else {
                         const unsigned long long slot = atomicAdd(to64 ? &ws->q64_count : &ws->q32_count, 1ull);
                         if ((long long)slot < capacity) {
                             RayRecord &q = (to64 ? q64 : q32)[slot];
@@ -1743,6 +1757,7 @@ render_f32_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                 r_cur = r_new;
             }
         }
+        moving = __ballot_sync(0xffffffffu, active);
     }
 }
 
