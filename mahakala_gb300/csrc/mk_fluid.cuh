@@ -409,7 +409,8 @@ __device__ __forceinline__ SnapF32 snap_f32(const mk_snapshot_view &s) {
 }
 
 // index of the lookup-table cell holding (x, y, z), or -1 outside the grid
-__device__ __forceinline__ int64_t table_cell_f32(const mk_snapshot_view &s, const SnapF32 &sf, const float xs[3]) {
+template <typename View>
+__device__ __forceinline__ int64_t table_cell_f32(const View &s, const SnapF32 &sf, const float xs[3]) {
     int b[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -422,7 +423,8 @@ __device__ __forceinline__ int64_t table_cell_f32(const mk_snapshot_view &s, con
 
 // cell and offsets of (x, y, z) in a block with first cell centre `left`
 // and reciprocal cell widths inv_dx
-__device__ __forceinline__ void cell_in_block_f32(const mk_snapshot_view &s, const float xs[3], const float left[3],
+template <typename View>
+__device__ __forceinline__ void cell_in_block_f32(const View &s, const float xs[3], const float left[3],
                                                   const float inv_dx[3], CellPosF &c) {
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -437,7 +439,8 @@ __device__ __forceinline__ void cell_in_block_f32(const mk_snapshot_view &s, con
     }
 }
 
-__device__ __forceinline__ bool locate_f32(const mk_snapshot_view &s, const SnapF32 &sf, float x, float y, float z,
+template <typename View>
+__device__ __forceinline__ bool locate_f32(const View &s, const SnapF32 &sf, float x, float y, float z,
                                            CellPosF &c) {
     const float xs[3] = {x, y, z};
     const int64_t cell = table_cell_f32(s, sf, xs);
@@ -464,7 +467,8 @@ struct BlockCacheF {
     float left[3], inv_dx[3];
 };
 
-__device__ __forceinline__ bool locate_f32_cached(const mk_snapshot_view &s, const SnapF32 &sf, float x, float y,
+template <typename View>
+__device__ __forceinline__ bool locate_f32_cached(const View &s, const SnapF32 &sf, float x, float y,
                                                   float z, CellPosF &c, BlockCacheF &bc) {
     const float xs[3] = {x, y, z};
     const int64_t cell = table_cell_f32(s, sf, xs);
@@ -494,7 +498,8 @@ __device__ __forceinline__ bool locate_f32_cached(const mk_snapshot_view &s, con
 // taken after the next acceleration finds them there: the phases that run
 // one warp per sub-partition are latency-bound, not bandwidth-bound.  c comes
 // from a successful locate_f32, so every address lies in the block array.
-__device__ __forceinline__ void prefetch_cells_f32(const mk_snapshot_view &s, const CellPosF &c) {
+template <typename View>
+__device__ __forceinline__ void prefetch_cells_f32(const View &s, const CellPosF &c) {
     const int n2 = s.n + 2;
     const int64_t sj = (int64_t)n2 * 8, sk = (int64_t)n2 * n2 * 8;
     const float *base = s.blocks + ((((int64_t)c.mb * n2 + c.idx[2]) * n2 + c.idx[1]) * n2 + c.idx[0]) * 8;
@@ -508,7 +513,8 @@ __device__ __forceinline__ void prefetch_cells_f32(const mk_snapshot_view &s, co
         }
 }
 
-__device__ __forceinline__ void trilinear8_f32(const mk_snapshot_view &s, const CellPosF &c, float prim[8]) {
+template <typename View>
+__device__ __forceinline__ void trilinear8_f32(const View &s, const CellPosF &c, float prim[8]) {
     const int n2 = s.n + 2;
     const int64_t sj = (int64_t)n2 * 8, sk = (int64_t)n2 * n2 * 8;
     const float *base = s.blocks + ((((int64_t)c.mb * n2 + c.idx[2]) * n2 + c.idx[1]) * n2 + c.idx[0]) * 8;

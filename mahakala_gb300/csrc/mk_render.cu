@@ -419,7 +419,8 @@ __device__ __forceinline__ RayF32 ray_f32(const mk_request &R) {
 
 // emission coefficients of one sample in float (mixed forms) at the located
 // cell c: em, ab per frequency (invariant, rescaled as in the FP64 path)
-__device__ __forceinline__ void emission_f32_at(const mk_snapshot_view &sv, const CellPosF &c, const RayF32 &rc,
+template <typename View>
+__device__ __forceinline__ void emission_f32_at(const View &sv, const CellPosF &c, const RayF32 &rc,
                                                 const float s[8], const KerrPoint<float> &m,
                                                 const SynchroF32 sc[MK_MAX_NU], float em_out[MK_MAX_NU],
                                                 float ab_out[MK_MAX_NU]) {
@@ -471,7 +472,8 @@ __device__ __forceinline__ void emission_f32_at(const mk_snapshot_view &sv, cons
 
 // one FP32 sample at the located cell folded into a compensated (Kahan)
 // float intensity sum; w = -dt L
-__device__ __forceinline__ void sample_f32(const mk_snapshot_view &sv, const CellPosF &c, const RayF32 &rc,
+template <typename View>
+__device__ __forceinline__ void sample_f32(const View &sv, const CellPosF &c, const RayF32 &rc,
                                            const float s[8], const KerrPoint<float> &m, float dt_used,
                                            float I[MK_MAX_NU], float Ic[MK_MAX_NU], float P[MK_MAX_NU],
                                            const SynchroF32 sc[MK_MAX_NU], int &nsamples, float &max_tau) {
@@ -539,7 +541,16 @@ enum { SRC_CAMERA = 0, SRC_QUEUE = 1 };
 // A request's float constants, one shared-memory entry per request of the
 // launch: read where used instead of held in ~37 registers per ray, which
 // lets the FP32 phases keep more warps resident.
+// The snapshot's fields and the step limit sit there too: from the request and
+// the view in global memory they were three loads in a row on every step.
+struct ViewF32 {
+    const float *blocks, *geom_f32;
+    const int32_t *table;
+    int nb[3], n;
+};
 struct ReqF32 {
+    ViewF32 sv;
+    int nmax;
     RayF32 rc;
     SynchroF32 sc[MK_MAX_NU];
     SnapF32 sf;
@@ -550,6 +561,9 @@ struct ReqF32 {
 
 __device__ __forceinline__ void fill_req_f32(const mk_request &R, const mk_snapshot_view *snaps, ReqF32 &o) {
     o.rc = ray_f32(R);
+    const mk_snapshot_view &sv = snaps[R.snapshot];
+    o.sv = {sv.blocks, sv.geom_f32, sv.table, {sv.nb[0], sv.nb[1], sv.nb[2]}, sv.n};
+    o.nmax = R.policy.nmax;
 #pragma unroll
     for (int ch = 0; ch < MK_MAX_NU; ch++)
         if (ch < R.nnu) o.sc[ch] = synchro_consts(R.nu[ch]);
@@ -1692,7 +1706,7 @@ render_f32_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
             f2 Xn[4], Kn[4];
             float dn[4];
             rk4_step_pair(X, K, d1, dt, Q.a, Xn, Kn);
-            const mk_snapshot_view &sv = snaps[R.snapshot];
+            const ViewF32 &sv = Q.sv;
             CellPosF cell;
             const bool inside = locate_f32(sv, Q.sf, Xn[1].hi, Xn[2].hi, Xn[3].hi, cell);
             if (inside) prefetch_cells_f32(sv, cell);
@@ -1717,7 +1731,7 @@ render_f32_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                     ++queue_steps;
                     queue_samples += inside;
                 }
-                const bool last = steps >= R.policy.nmax - 1, out = r_new > r_cur;
+                const bool last = steps >= Q.nmax - 1, out = r_new > r_cur;
                 const bool away = (mode & F32_ESCAPE) && r_new > Q.sf.r_out && out;
                 // near the horizon or inbound in the photon-ring region: to
                 // the near-hole queue; outbound past it (F32_PARK): to the
