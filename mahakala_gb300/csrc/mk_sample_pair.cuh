@@ -238,8 +238,10 @@ __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConst
     pr prim[8];
     float Bm, up = 1.0f;
     for (;;) {
+        // primitives two by two (0-1, 2-3, 4-5, 6-7) on paired instructions
+        float2 sh[4], sl[4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) prim[i] = {0.0f, 0.0f};
+        for (int i = 0; i < 4; i++) sh[i] = sl[i] = make_float2(0.0f, 0.0f);
         float4 next[4] = {ldg4(base), ldg4(base + 4), ldg4(base + 8), ldg4(base + 12)};
 #pragma unroll 1
         for (int q = 0; q < 4; q++) {
@@ -256,20 +258,26 @@ __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConst
             for (int x = 0; x < 2; x++) {
                 const pr w = p_mulr(zy, x ? del[0] : u0), ws = p_two(w, up);
                 const float4 lo = c[2 * x], hi = c[2 * x + 1];
-                const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                const float2 v[4] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y),
+                                     make_float2(hi.z, hi.w)};
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const pr g = i >= 1 && i <= 3 ? w : ws;
-                    const float t = f_mul(g.h, v[i]);
-                    const float e = fmaf(g.l, v[i], fmaf(g.h, v[i], -t));
-                    float s, r;
-                    two_sum_f(prim[i].h, t, s, r);
-                    prim[i] = {s, f_add(prim[i].l, f_add(e, r))};
+                for (int i = 0; i < 4; i++) {
+                    // velocities (1, 2, 3) are not scaled
+                    const float2 gh = i == 0 ? make_float2(ws.h, w.h) : (i == 1 ? make_float2(w.h, w.h) : make_float2(ws.h, ws.h));
+                    const float2 gl = i == 0 ? make_float2(ws.l, w.l) : (i == 1 ? make_float2(w.l, w.l) : make_float2(ws.l, ws.l));
+                    const float2 t = __fmul2_rn(gh, v[i]);
+                    const float2 e = __ffma2_rn(gl, v[i], __ffma2_rn(gh, v[i], make_float2(-t.x, -t.y)));
+                    float2 r;
+                    sh[i] = v_two_sum(sh[i], t, r);
+                    sl[i] = __fadd2_rn(sl[i], __fadd2_rn(e, r));
                 }
             }
         }
 #pragma unroll
-        for (int i = 0; i < 8; i++) prim[i] = p_norm(prim[i]);
+        for (int i = 0; i < 4; i++) {
+            prim[2 * i] = p_norm({sh[i].x, sl[i].x});
+            prim[2 * i + 1] = p_norm({sh[i].y, sl[i].y});
+        }
         Bm = fmaxf(fmaxf(fabsf(prim[5].h), fabsf(prim[6].h)), fabsf(prim[7].h));
         if ((prim[0].h >= 1e-22f && prim[4].h >= 1e-22f && Bm >= 1e-22f) || up != 1.0f) break;
         // excised cells: nothing emits (sigma or Theta_e is not a number)

@@ -136,6 +136,14 @@ MK_HD pr p_rcp(pr x) {
     return p_norm({y, f_mul(y, fmaf(d, d, d))});
 }
 
+// Paired FP32 instructions (each lane rounds as its scalar twin): the pipe
+// takes two cycles for one, but half as many are fetched and issued.
+__device__ __forceinline__ float2 v_two_sum(float2 a, float2 b, float2 &e) {
+    const float2 m1 = make_float2(-1.0f, -1.0f), s = __fadd2_rn(a, b), v = __ffma2_rn(a, m1, s);
+    e = __fadd2_rn(__ffma2_rn(__ffma2_rn(v, m1, s), m1, a), __ffma2_rn(v, m1, b));
+    return s;
+}
+
 // Z^(-1/3): the float unit's estimate, one Newton step in float, a third-order
 // correction from the pair residual 1 - Z x^3
 __device__ __forceinline__ pr p_rcbrt(pr z) {
