@@ -198,8 +198,10 @@ __device__ __forceinline__ pr p_exp_neg(pr x, const float2 *tab, int &e) {
 
 // m 2^-e as a double, |m| a normal float or 0, by the exponent's bits
 __device__ __forceinline__ double p_scaled(pr m, int e) {
-    if (e > 850 || m.h == 0.0f) return 0.0;
+    if (e > 1201 || m.h == 0.0f) return 0.0;  // |m| < 2^128: below every double
     const double v = d_from(m.h) + d_from(m.l);
+    if (e > 850)  // 2^-e in two normal factors, one rounding
+        return v * __hiloint2double((1023 - e / 2) << 20, 0) * __hiloint2double((1023 - (e - e / 2)) << 20, 0);
     return __hiloint2double(__double2hiint(v) - (int)((unsigned)e << 20), __double2loint(v));
 }
 // A sample's coefficients at one frequency: em 2^-e and ab 2^-e.

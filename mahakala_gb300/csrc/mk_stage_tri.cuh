@@ -200,7 +200,7 @@ __device__ __forceinline__ bool synchro_tri(const SynchroTri &c, double Ne, doub
     const tri y = {y0.h, y0.l, 0.0f}, p3 = t_mul(t_mulr(t_mulr(y, y), y), Z);
     const float d = f_sub(f_sub(f_sub(1.0f, p3.h), p3.m), p3.l);
     const tri x3 = t_norm({y0.h, y0.l, f_mul(f_mul(y0.h, d), 0.333333343f)});  // X^(1/3)
-    if (!(x3.h < 740.0f)) return true;  // exp(-x3) = 0
+    if (!(x3.h < 745.13f)) return true;  // exp(-x3) = 0
     const tri Y = t_mulr(t_mulr(x3, x3), Z);
     const tri t = t_add({1.0f, 0.0f, 0.0f}, t_mulr({0x1.e3437ep+0f, 0x1.c404dp-26f, 0x1.dbca56p-51f}, Y));
     int e;
@@ -226,9 +226,10 @@ __device__ __forceinline__ bool synchro_tri(const SynchroTri &c, double Ne, doub
         em = t_mulr(em, v);
     }
     if (e > 400) {  // faint to the end of the doubles' range
-        const double s = e < 900 ? __hiloint2double((1023 - e) << 20, 0) : 0.0;
-        em_out = scaled(t_to(em), en - 60) * s;
-        ab_out = scaled(t_to(ab), en - 60) * s;
+        // 2^-e in two normal factors, one rounding
+        const double s1 = __hiloint2double((1023 - e / 2) << 20, 0), s2 = __hiloint2double((1023 - (e - e / 2)) << 20, 0);
+        em_out = scaled(t_to(em), en - 60) * s1 * s2;
+        ab_out = scaled(t_to(ab), en - 60) * s1 * s2;
     } else {
         em_out = scaled(t_to(em), en - 60 - e);
         ab_out = scaled(t_to(ab), en - 60 - e);
