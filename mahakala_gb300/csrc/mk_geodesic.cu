@@ -146,7 +146,6 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
     for (int i = 0; i < 8; i++) s64[i] = s0[8 * p + i];
     bool out = all_f64 || !tri_range(s64);
     int K = N, why = MK_RAY_MAXSTEPS, j = 0;
-    const bool started = !out;
     TriState s, last;
     tri_state(s64, s);
     last = s;
@@ -161,16 +160,14 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
         bool go = rule_dt(q.r, R, dt, d, w);
         for (j = 0; j < N; j++) {
             tri dtn = dt;
-            if (ROWS) tri_doubles(s, s64);
-            else last = s;
+            if (!ROWS) last = s;
+            else if (j) tri_doubles(s, s64);  // the first state is the caller's, bit for bit
             if (go) {
                 const bool near = d < TRI_NEAR;
                 if (near) {  // through a copy: s itself stays in registers
                     TriState n = s;
                     double sc[8];
-                    if (!ROWS) tri_doubles(s, s64);
-#pragma unroll
-                    for (int i = 0; i < 8; i++) sc[i] = s64[i];
+                    tri_doubles(s, sc);
                     rk4_step_near(n, sc, t_to(dt), a);
                     s = n;
                 }
@@ -189,7 +186,7 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
         }
     }
     if (out) {
-        if (!ROWS && started) tri_doubles(last, s64);
+        if (!ROWS && j) tri_doubles(last, s64);
         double sc[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) sc[i] = s64[i];
@@ -198,8 +195,8 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
     }
     Kout[p] = K;
     why_out[p] = why;
-    if (K == N) tri_doubles(s, s64);
-    else if (!ROWS) tri_doubles(last, s64);  // a rejected step leaves the state before it
+    if (K == N && N) tri_doubles(s, s64);
+    else if (!ROWS && K) tri_doubles(last, s64);  // a rejected step leaves the state before it
     store_row(state_out, p, s64);
 }
 
@@ -249,7 +246,6 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
     last = s;
     const SpinTri sp = spin_tri(a);
     int st = MK_RAY_MAXSTEPS, j = 0;
-    const bool started = !out;
     if (!out) {
         TriPoint q;
         tri_step<true>(s, q, {0.0f, 0.0f, 0.0f}, sp.a, sp.aa, sp.aa3, true);
@@ -276,7 +272,7 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
     if (out) {
         double sc[8];
         tri_doubles(last, sc);
-        if (!started)
+        if (!j)
 #pragma unroll
             for (int i = 0; i < 8; i++) sc[i] = s64[i];
         integrate_fixed_f64(sc, j, p, a, N, hfrac, hmin, hmax, capture, r_escape, Kout, why_out, state_out);
@@ -284,7 +280,7 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
     }
     Kout[p] = j;
     why_out[p] = st;
-    tri_doubles(s, s64);
+    if (j) tri_doubles(s, s64);
     store_row(state_out, p, s64);
 }
 

@@ -191,9 +191,8 @@ def find_shadow_bisection_angles(bhspin, inc, angles, max_steps=2000, error_allo
             hi.append(np.stack([mid, b], 1).reshape((-1,) + angles.shape))
         flat = np.concatenate(mids).reshape(-1, angles.size)
         shape = (len(flat), angles.size)
-        r = _shadow_pass(inc, np.broadcast_to(ca.reshape(-1), shape).reshape(-1),
-                         np.broadcast_to(sa.reshape(-1), shape).reshape(-1), flat.reshape(-1), bhspin, 1000,
-                         max_steps).reshape(shape)
+        r = _shadow_pass(inc, np.tile(ca.reshape(-1), len(flat)), np.tile(sa.reshape(-1), len(flat)),
+                         flat.reshape(-1), bhspin, 1000, max_steps).reshape(shape)
         node = np.zeros(angles.size, dtype=np.int64)
         stuck = np.zeros(angles.size, dtype=bool)     # a ray with no radius moves neither end
         cols = np.arange(angles.size)
