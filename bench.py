@@ -8,7 +8,7 @@ One "step" is one full render of the workload's image through the fused
 persistent kernels: every ray of the image traced, sampled and solved.
 Default workload (``render256``): render of the seeded 256^3-cell synthetic
 snapshot at 256x256 pixels (a=0.94, 17 deg, 230 GHz, <= 8192 steps), timed
-in every form -- plain FP64 and the mixed FP32/FP64 forms (mixed,
+in every form -- FP64 and the mixed FP32/FP64 forms (mixed,
 mixed_strict, mixed_df) -- with each mixed form's flux and per-pixel error
 against the FP64 image of the same run.  The headline value is the mixed
 form's rays/s.  The default run also prints: the FP64 image checked
@@ -42,7 +42,8 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 # algorithmic FLOPs (add/sub/mul/div/sqrt = 1, FMA = 2, transcendental = 1),
-# counted from the FP64 device code: one accepted RK4 step (4 closed-form
+# counted from a binary64 evaluation (the FP64 form's own pairs and triples
+# take ~11 FP32 instructions for each): one accepted RK4 step (4 closed-form
 # accelerations of 184 + RK4 combine 136 + radius_cal 18 + step rule 3) and
 # one in-snapshot sample at one frequency (lookup 34, trilinear 168, metric
 # 20, fluid frame 92, electrons/units 24, synchrotron 36, transfer 5)
@@ -68,10 +69,9 @@ CHAIN_FLOOR_CYCLES = 1270
 # `python bench.py --precision mixed --steps 2 --warmup 3 --quick --serving 0 --sampling-rays 0`
 NCU_TRAFFIC_RENDER256 = {"A": 106.92e6 + 3.01e6, "B": 76.74e6 + 1.58e6, "C": 113.40e6 + 0.16e6}
 
-# FP64 FLOP (DFMA = 2) per point of the standalone sampling stage, from ncu's
-# DADD/DMUL/DFMA thread-instruction counters on fluid_scalars_kernel (64x64
-# camera over the 256^3-cell snapshot, 19 % of points inside it)
-SAMPLING_FP64_FLOP_PER_POINT = 399
+# operations (FMA = 2) per point of the standalone sampling stage in a binary64
+# evaluation (64x64 camera over the 256^3-cell snapshot, 19 % of points inside it)
+SAMPLING_FLOP_PER_POINT = 399
 
 
 def parse():
@@ -496,7 +496,7 @@ def hbm_peak():
         return 6800.0, "fallback (6.8 TB/s, one earlier GB300 copy measurement)"
 
 
-def sampling_stage(torch, model, spec, flush, stream, fp64_peak, rays_per_side=128, reps=3):
+def sampling_stage(torch, model, spec, flush, stream, fp32_peak, rays_per_side=128, reps=3):
     """The sampling stage alone (get_fluid_scalars_from_geodesics as the
     standalone mk_fluid_scalars kernel) over the reference's trajectory rows
     of a rays_per_side^2 camera with the workload's view: every row of every
@@ -538,20 +538,20 @@ def sampling_stage(torch, model, spec, flush, stream, fp64_peak, rays_per_side=1
         ts.append(e0.elapsed_time(e1) * 1e-3)
     t = statistics.mean(ts)
     nbytes = n * (64 + 40) + inside * 256
-    flops = SAMPLING_FP64_FLOP_PER_POINT * n
+    flops = SAMPLING_FLOP_PER_POINT * n
     peak, src = hbm_peak()
     del S, pts, out
     torch.cuda.empty_cache()
-    return {"kernel": "fluid_scalars_kernel", "bound": "fp64", "rays": rays_per_side ** 2, "rows": nt,
+    return {"kernel": "fluid_scalars_kernel", "bound": "fp32", "rays": rays_per_side ** 2, "rows": nt,
             "points": n, "in_snapshot": inside, "ms": 1e3 * t, "algorithmic_bytes": nbytes,
             "hbm": {"achieved": nbytes / t / 1e9, "peak": peak, "unit": "GB/s", "frac": nbytes / t / 1e9 / peak,
                     "peak_source": src},
-            "fp64": {"achieved": flops / t / 1e12, "peak": fp64_peak / 1e12, "unit": "TFLOP/s",
-                     "frac": flops / t / fp64_peak, "flop_per_point": SAMPLING_FP64_FLOP_PER_POINT},
+            "fp32": {"achieved": flops / t / 1e12, "peak": fp32_peak / 1e12, "unit": "TFLOP/s",
+                     "frac": flops / t / fp32_peak, "flop_per_point": SAMPLING_FLOP_PER_POINT},
             "traffic": None,
-            "note": "every point needs the metric, fluid frame and arccos in binary64 to return the reference's "
-                    "values, so the stage is FP64-pipe bound (ncu on the 64x64 case: 87.5 % FP64 pipe, 2.6 % DRAM); "
-                    "FLOP per point from ncu's FP64 instruction counters on the same case"}
+            "note": "every point needs the metric, fluid frame and arccos to binary64's precision, evaluated in "
+                    "float triples (about a dozen FP32 instructions an operation): bound by instruction issue; FLOP "
+                    "per point are those of a binary64 evaluation"}
 
 
 def stress_record(torch, stream, flush, peaks):
@@ -559,7 +559,7 @@ def stress_record(torch, stream, flush, peaks):
     86/230/345 GHz in one ray pass, <= 16384 steps) in the mixed form and in
     FP64, each CUDA-event timed with per-kernel times, with each mixed
     channel's flux and pixel error against the FP64 image.  Mixed: 3
-    warm-up and 3 timed renders; FP64 (1.3 s a render): 1 and 1."""
+    warm-up and 3 timed renders; FP64: 1 and 1."""
     from mahakala_gb300 import configs, metrics
     from mahakala_gb300.grmhd.athenak import AthenakFluidModel
     from mahakala_gb300.images import PreparedRender
@@ -578,7 +578,7 @@ def stress_record(torch, stream, flush, peaks):
         t = statistics.mean(times)
         steps, samples = prep.work_totals()
         flops = steps * FLOP_PER_STEP + samples * per_sample
-        pk = peaks["fp64"] if form == "fp64" else peaks["fp32"]
+        pk = peaks["fp32"]  # the FP64 form's arithmetic is float pairs and triples
         out[form] = {"rays_per_s": rays / t, "ms": 1e3 * t, "images_per_s": nnu / t,
                      "phase_ms": [1e3 * statistics.mean(p[i] for p in phases) for i in range(len(phases[0]))],
                      "accepted_steps": steps, "samples": samples, "ray_steps_per_s": steps / t,
@@ -621,7 +621,7 @@ def run_vacuum(args):
                                  capture=c["capture"], r_escape=c["r_escape"])}
     stream = torch.cuda.current_stream()
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
-    peak64 = measure_fma_peak(torch, _lib.MK_FP64)
+    peak32 = probe_peaks(torch, local)["fp32"]
     proc, fh, cpath = clocks_sampler() if rank == 0 else (None, None, None)
     lines = {}
     for name, pol in pols.items():
@@ -652,8 +652,8 @@ def run_vacuum(args):
             e2e.append(time.perf_counter() - t0)
         lines[name] = {"rays_per_s": n / t, "ms_per_step": 1e3 * t, "ray_steps": steps,
                        "ray_steps_per_s": steps / t, "e2e_rays_per_s": n / statistics.mean(e2e),
-                       "roofline": {"bound": "fp64", "achieved": flops / t / 1e12, "peak": peak64 / 1e12,
-                                    "unit": "TFLOP/s", "frac": flops / t / peak64, "traffic": None,
+                       "roofline": {"bound": "fp32", "achieved": flops / t / 1e12, "peak": peak32 / 1e12,
+                                    "unit": "TFLOP/s", "frac": flops / t / peak32, "traffic": None,
                                     "kernel": "integrate_%s_kernel" % ("reference" if name == "reference"
                                                                         else "fixed")}}
     clocks = clocks_summary(proc, fh, cpath, local) if rank == 0 else None
@@ -753,7 +753,7 @@ def main():
     sampling = None
     srays = args.sampling_rays if args.sampling_rays >= 0 else 128
     if srays:
-        sampling = sampling_stage(torch, model, spec, flush, stream, peak64 if not args.quick else float("nan"),
+        sampling = sampling_stage(torch, model, spec, flush, stream, peak32 if not args.quick else float("nan"),
                                   rays_per_side=srays)
 
     serving = None
@@ -818,8 +818,8 @@ def main():
                "probe, the paired-FP32 FMA probe and the issue limit SMs x 128 x 2 FLOP x the maximum SM clock; "
                "the measured-peak file holds no FP64/FP32 ALU figure")
         if form == "fp64":
-            kernels = [("render_fp64_kernel", "fp64", r["steps"] * FLOP_PER_STEP + r["samples"] * per_sample,
-                        r["t_phase"][0], peak64, None)]
+            kernels = [("render_tri_kernel", "fp32", r["steps"] * FLOP_PER_STEP + r["samples"] * per_sample,
+                        r["t_phase"][0], peak32, None)]
         else:
             to64, back32, steps64 = r["split"]
             stb, smb = r["work_b"] if r["work_b"] else (steps64, r["samples64"])
@@ -853,8 +853,9 @@ def main():
                                      "kernel on this workload (bytes per launch); the kernels are ALU- and "
                                      "latency-bound, the gathers hit L1/L2")
         if form == "fp64":
-            out["traffic_note"] = ("ncu on the 192x192 case: 242 MB DRAM read per launch; the kernel is "
-                                   "FP64-pipe bound (71 % FP64 pipe, 0.04 % DRAM)")
+            out["note"] = ("binary64 precision in float pairs and triples on the FP32 pipe, about a dozen FP32 "
+                           "instructions for each counted operation; achieved over the FP64 FMA probe: %.2f"
+                           % (top["achieved"] * 1e12 / peak64))
         else:
             out["note"] = ("phase B runs the serial chain of its longest ray (zone_run_max steps): one integrating "
                            "warp per block, three sampling warps beside it on the other sub-partitions; "
@@ -954,9 +955,10 @@ def main():
         "sampling_stage": sampling,
         "stress1024": stress,
         "sweep512": sweep,
-        # per render: FP64 one kernel; mixed forms A, B, C, plus the camera-state
+        # per render: FP64 the render and the launch that takes what it leaves to
+        # binary64; mixed forms A, B, C, plus the camera-state
         # kernel when the launch exceeds one wave of phase A at 4 blocks per SM
-        "gpu_launches": args.steps * (1 if head == "fp64" else
+        "gpu_launches": args.steps * (2 if head == "fp64" else
                                       3 + int(rays > _lib.load().mk_device_sm_count() * 4 * 128)),
         "phase_ms": {f: [1e3 * t for t in res[f]["t_phase"]] for f in forms},
         "clocks": clocks,

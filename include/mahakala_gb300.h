@@ -47,7 +47,12 @@ typedef enum {
     MK_RAY_NAN = 4
 } mk_ray_status;
 
-/* MK_FP64: every operation in binary64.
+/* MK_FP64: binary64 results.  The ray state is carried in 72 bits (three
+   floats), the accelerations and the sampling in float pairs (~48 bits)
+   whose errors enter the result scaled down, the transfer sums in binary64;
+   against a 140-bit evaluation the images are no further off than binary64
+   throughout.  Requests and samples whose values the pairs cannot hold are
+   taken in binary64.
    MK_MIXED: FP32 arithmetic (ray state as float pairs, Kahan-compensated
    intensity); near the hole (r < 3 M, or inbound inside 6 M where
    photon-ring rays turn) the wavevector is renormalised to null on entry
@@ -306,8 +311,8 @@ int mk_attenuated_emissivity(const double *em_dev, const double *ab_dev, const d
    MK_WS_SAMPLES_B the steps and samples MK_MIXED's near-hole kernel took
    (near the hole and after), MK_WS_STEPS_C / MK_WS_SAMPLES_C those the
    FP32 continuation kernel took (mixed forms), MK_WS_ERROR the waits of
-   MK_MIXED's near-hole pipeline that ran out (each bounded by the
-   "zone_wait_ns" tuning): nonzero means the launch's images are invalid,
+   MK_MIXED's near-hole pipeline and of MK_FP64's integrating and sampling
+   warps that ran out (each bounded by the "zone_wait_ns" tuning): nonzero means the launch's images are invalid,
    and a host reads it as status MK_ERR_TIMEOUT once the stream has passed
    the launch. */
 #define MK_WS_STEPS 1
@@ -378,7 +383,7 @@ int mk_render_job(const mk_job *job_dev, const mk_request *reqs_dev, const mk_sn
    CUDA context current on that device (after a reset) looks it up again.
    All calls share the array: calls that overlap on the GPU race.  The
    workspace header, MK_WS_ERROR included, stays inside the library: a
-   near-hole wait that ran out (never expected) is not reported here. */
+   wait that ran out (never expected) is not reported here. */
 #define MK_NOALLOC_WORKSPACE_BYTES (16u << 20)
 #define MK_NOALLOC_MAX_MIXED_RAYS ((MK_NOALLOC_WORKSPACE_BYTES - 256u) / 320u)
 int mk_render_noalloc(const mk_request *reqs_dev, int32_t nreq, int64_t total_rays,
@@ -400,7 +405,7 @@ int mk_render_noalloc(const mk_request *reqs_dev, int32_t nreq, int64_t total_ra
    stream around each kernel for mk_render_phase_ms; not for renders that
    are captured into a CUDA graph.
    "zone_wait_ns" (1 .. 6e10; default 1e9): the limit of each wait between
-   the warps of MK_MIXED's near-hole pipeline; a wait that runs out ends
+   the warps of MK_MIXED's near-hole pipeline and of MK_FP64's couples; a wait that runs out ends
    its block and counts in the workspace word MK_WS_ERROR.
    "zone_wait_test" (0 or 1; default 0): test switch -- the near-hole
    pipeline's integrating warps withhold their first message, so the

@@ -2,9 +2,10 @@
 
 Drop-in for the reference package ``mahakala``: the same public names
 (mahakala/__init__.py:25-45), with every compute step in hand-written CUDA
-kernels behind a C ABI (``include/mahakala_gb300.h``).  FP64 throughout, as
-the reference enables ``jax_enable_x64``.  Arrays come back as float64 CUDA
-tensors; ``make_image`` returns a NumPy image like the reference.
+kernels behind a C ABI (``include/mahakala_gb300.h``).  Results have
+binary64 precision, as the reference enables ``jax_enable_x64``.  Arrays
+come back as float64 CUDA tensors; ``make_image`` returns a NumPy image like
+the reference.
 
 Importing this package does not need a GPU; calling any compute function
 does, and fails loudly without one (there is no CPU fallback).

@@ -19,7 +19,12 @@
 // search over the requests' ray offsets.
 //
 // Precision forms:
-//   MK_FP64  one launch, every operation in FP64 (the reference's x64).
+//   MK_FP64  binary64 results from the FP32 pipe (render_tri_kernel): ray
+//   states in 72 bits, geodesic and sampling in float pairs, transfer sums
+//   in binary64, at most as far from a 140-bit evaluation as binary64
+//   throughout (mk_tri.cuh, mk_sample_pair.cuh).  Requests whose constants
+//   the pairs cannot hold are left to a second launch, binary64 throughout
+//   (render_fp64_kernel<camera>; it returns at once when there are none).
 //   MK_MIXED three launches, A on the caller's stream, then B on it and C
 //   on a side stream forked after A and joined back after C:
 //     A  FP32 from the camera (camera rays in double-float).  A ray whose
