@@ -167,7 +167,9 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
                 if (near) {  // through a copy: s itself stays in registers
                     TriState n = s;
                     double sc[8];
-                    tri_doubles(s, sc);
+                    if (!ROWS) tri_doubles(s, s64);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) sc[i] = s64[i];
                     rk4_step_near(n, sc, t_to(dt), a);
                     s = n;
                 }
