@@ -311,8 +311,8 @@ int mk_attenuated_emissivity(const double *em_dev, const double *ab_dev, const d
    MK_WS_SAMPLES_B the steps and samples MK_MIXED's near-hole kernel took
    (near the hole and after), MK_WS_STEPS_C / MK_WS_SAMPLES_C those the
    FP32 continuation kernel took (mixed forms), MK_WS_ERROR the waits of
-   MK_MIXED's near-hole pipeline and of MK_FP64's integrating and sampling
-   warps that ran out (each bounded by the "zone_wait_ns" tuning): nonzero means the launch's images are invalid,
+   MK_MIXED's near-hole pipeline that ran out (each bounded by the
+   "zone_wait_ns" tuning): nonzero means the launch's images are invalid,
    and a host reads it as status MK_ERR_TIMEOUT once the stream has passed
    the launch. */
 #define MK_WS_STEPS 1
@@ -405,7 +405,7 @@ int mk_render_noalloc(const mk_request *reqs_dev, int32_t nreq, int64_t total_ra
    stream around each kernel for mk_render_phase_ms; not for renders that
    are captured into a CUDA graph.
    "zone_wait_ns" (1 .. 6e10; default 1e9): the limit of each wait between
-   the warps of MK_MIXED's near-hole pipeline and of MK_FP64's couples; a wait that runs out ends
+   the warps of MK_MIXED's near-hole pipeline; a wait that runs out ends
    its block and counts in the workspace word MK_WS_ERROR.
    "zone_wait_test" (0 or 1; default 0): test switch -- the near-hole
    pipeline's integrating warps withhold their first message, so the

@@ -58,8 +58,6 @@
 namespace mk {
 
 constexpr int RENDER_THREADS = 128;
-// resident blocks an SM of the FP64 form's kernel
-constexpr int TRI_BLOCKS = 4;
 constexpr double R_FP64 = 3.0;
 constexpr double R_TURN = 6.0;
 // F32_RENULL (the FP32 queue): renormalise each resumed ray to null in
@@ -1267,287 +1265,445 @@ __device__ __noinline__ void coefficients_fp64(const mk_request &R, const mk_sna
 // sampling in float pairs, transfer sums in binary64 (mk_tri.cuh,
 // mk_sample_pair.cuh say why and to what accuracy).
 //
-// An image's time is the chain of its longest rays (a captured ray around a
-// spinning hole takes 1000 to 3500 steps, the mean ray ~450), so a step and
-// its sample, ~7.3 k and ~6.4 k cycles of a lone warp, are taken by two warps:
-// one integrates 32 rays and posts a message per step, the other samples the
-// snapshot there and folds the sample into the rays' transfer sums, up to
-// TRI_SLOTS steps behind.  A block holds two such couples; in every other
-// block the roles change sides, since an integrating warp issues more than
-// twice what a sampling one does and the SM's four sub-partitions should
-// share both.
+// One block an SM takes rays through phases: its warps integrate their rays a
+// few steps, leaving a message in shared memory for each step inside the
+// snapshot's box; then they sample the messages, 32 at a time whichever rays
+// they come from; then each lane folds its samples into its ray's transfer
+// sums, in step order.  Why phases: the loops of an integrating and of a
+// sampling warp are ~22 and ~30 KB of code, and an SM's instruction cache
+// holds 32 KB (a loop of independent FFMAs issues one a cycle up to there and
+// one in three beyond).  Couples of warps, one integrating and one sampling
+// side by side, waited for instructions half of their time: 7.7, 19.2 and 52
+// ms for 24^2, 256^2 and 512^2 rays around a hole of spin 0.94, against 6.2,
+// 14.9 and 29.8 ms.
 //
-// Messages pass through slots in shared memory with two mbarriers each, waits
-// are bounded and abort the block, all as in the near-hole phase
-// (render_zone_kernel).  A ray's constants sit in shared memory, one column a
-// thread, each role's loaded by itself when the ray starts.
-// lane_stride: lanes that take rays (a small job's rays are spread over every
-// couple before they share warps).
-enum : unsigned { TM_START = 1u, TM_SAMPLE = 2u, TM_END = 4u, TM_DONE = 8u };
-constexpr int TRI_COUPLES = 2;
-constexpr int TRI_LANES = 32 * TRI_COUPLES;
-constexpr int TRI_SLOTS = 3;
-static_assert(RENDER_THREADS == 2 * TRI_LANES, "two warps a couple");
-
-struct TriSlot {
-    unsigned flags[32];
-    int why[32];         // TM_END
-    long long ray[32];   // TM_START
-    float v[28][32];
-};
-// message words (TM_SAMPLE): x^1..x^3 (h m l), k^0..k^3 (h l), r f l3 1/(r^2+a^2) (h l), dt (h m l)
-enum { TV_X = 0, TV_K = 9, TV_M = 17, TV_DT = 25, TV_COUNT = 28 };
+// Eight warps, two a sub-partition: a step of a warp alone is 7.5 k cycles
+// and of two 12.0 k (issue 70 % busy); twelve and sixteen, at 168 and 128
+// registers, spill (10 k cycles for a warp alone; 24^2 6.9 and 8.1 ms).  The
+// messages fill the shared memory: a phase is as many steps as that allows
+// (6, or 12 with four warps) since its other parts cost ~25 k and ~10 k cycles.
+//
+// When the job's rays run out, the block moves those it still has into four
+// warps once they fit there: an image's time ends with the chain of its
+// longest rays (a captured ray around a spinning hole takes 1000 to 3500
+// steps, the mean ray ~450), whose steps a warp takes fastest alone on its
+// sub-partition.
+constexpr int TRI_WARPS = 8, TRI_THREADS = 32 * TRI_WARPS;
+constexpr int TRI_MSGS = 1536;  // messages of a phase; its steps are as many as fill them
+constexpr int TRI_STEPS = TRI_MSGS / 128;  // with the fewest warps, four
+constexpr int TRI_REQS = 32;    // requests a block has rays of at a time
+constexpr int TRI_REFILL = 4;   // idle lanes of a warp that take new rays together
+// message words: x^1..x^3 (h m l), k^0..k^3 (h l), r f l3 1/(r^2+a^2) (h l),
+// dt (h l), thread of the ray, its step; the sample's reply lies over the first:
+// per frequency w j and w alpha as doubles
+enum { TV_X = 0, TV_K = 9, TV_M = 17, TV_DT = 25, TV_COL = 27, TV_STEP = 28, TV_COUNT = 29 };
 
 struct TriShared {
-    TriSlot slot[TRI_COUPLES][TRI_SLOTS];
-    float c_int[13 * TRI_LANES];              // PC_A .. PC_TOL
-    float c_smp[(PC_COUNT - PC_BOX) * TRI_LANES];
-    double I[MK_MAX_NU][TRI_LANES], P[MK_MAX_NU][TRI_LANES];
+    float v[TV_COUNT][TRI_MSGS];
+    double I[MK_MAX_NU][TRI_THREADS], P[MK_MAX_NU][TRI_THREADS];
+    float c[PC_COUNT][TRI_REQS];  // requests' constants, one column each
+    SampleView view[TRI_REQS];
+    int rq[TRI_REQS], users[TRI_REQS], nnu[TRI_REQS], nmax[TRI_REQS], rows[TRI_REQS], odd[TRI_REQS];
+    // by thread, out of the registers that the geodesic needs: its ray, the ray
+    // to start next (nxt: taken, with a column if nslot >= 0), samples so far,
+    // the largest optical depth of one (bits of a double >= 0: they order as
+    // integers), why the ray ended
+    long long ray[TRI_THREADS], nxt[TRI_THREADS], tau[TRI_THREADS];
+    int slot[TRI_THREADS], nslot[TRI_THREADS], samples[TRI_THREADS], why[TRI_THREADS];
+    unsigned mask[TRI_WARPS][TRI_STEPS];  // lanes that left a message, by step
+    int count[TRI_WARPS], alive[TRI_WARPS];
     float2 exptab[EXP_STEPS];
-    unsigned long long full[TRI_COUPLES][TRI_SLOTS], empty[TRI_COUPLES][TRI_SLOTS];
-    int abort;
+    long long total, rest;  // rays, and those of them handed out by the counter
+    int chunk, drained;
 };
+// words of a ray moved to another thread
+constexpr int TRI_MOVE = 39 + 4 * MK_MAX_NU;
+static_assert(TRI_MOVE * (TRI_THREADS - 128) <= TV_COUNT * TRI_MSGS, "moved rays lie over the messages");
+static_assert(sizeof(TriShared) <= 227 * 1024, "shared memory of a block");
 
-__device__ __forceinline__ void tri_integrate(int couple, const mk_request *__restrict__ reqs, int nreq,
-                                              long long total, RenderWorkspace *ws, int lane_stride, TriShared &sh,
-                                              unsigned long long limit_ns) {
-    const int lane = threadIdx.x & 31;
-    const PairConsts<TRI_LANES> C = {sh.c_int + 32 * couple + lane};
-    bool active = false, exhausted = lane % lane_stride != 0;
-    int steps = 0, nmax = 0, last_rq = -1;  // the request whose constants are loaded
-    TriState s;
-    TriPoint q;
-    tri dt = {0.0f, 0.0f, 0.0f};
-    for (int it = 0;; ++it) {
-        const int sl = it % TRI_SLOTS;
-        TriSlot &msg = sh.slot[couple][sl];
-        unsigned flags = 0;
-        const long long idx = fetch(!active && !exhausted, &ws->counter, total);
-        if (idx == -1) exhausted = true;
-        bool start = false;
-        if (idx >= 0 && ray_in_request(reqs, nreq, idx)) {
-            const int rq = find_request(reqs, nreq, idx);
+// A column for request rq: its own, or a free one, which is filled here and
+// read after the block's next barrier; -1: none free.  Columns are given back
+// between other barriers than they are taken between.
+__device__ __noinline__ int tri_acquire(TriShared &sh, int rq, const mk_request *__restrict__ reqs,
+                                        const mk_snapshot_view *__restrict__ snaps) {
+    for (int j = 0; j < TRI_REQS; j++) {
+        const int i = (rq + j) % TRI_REQS;
+        const int was = atomicCAS(&sh.rq[i], -1, rq);
+        if (was != -1 && was != rq) continue;
+        atomicAdd(&sh.users[i], 1);
+        if (was == -1) {
             const mk_request &R = reqs[rq];
-            if (rq != last_rq && !pair_request(R)) {
-                atomicAdd(&ws->odd_rays, 1ull);  // left to render_fp64_kernel
-            } else {
-                double s64[8];
-                camera_ray_fast(R.camera, fetch_pixel(R.camera, idx - R.ray_offset), s64);
-                tri_state(s64, s);
-                if (rq != last_rq) pair_consts_geodesic(R, C);
-                last_rq = rq;
-                nmax = R.policy.nmax;
-                steps = 0;
-                start = true;
-            }
+            const PairConsts<TRI_REQS> C = {&sh.c[0][i]};
+            sh.nnu[i] = R.nnu;
+            sh.nmax[i] = R.policy.nmax;
+            sh.rows[i] = R.rows_dt ? (int)min((long long)R.rows, 0x7fffffffll) : 0;
+            sh.view[i] = sample_view(snaps[R.snapshot]);
+            sh.odd[i] = !pair_request(R);
+            pair_consts_geodesic(R, C);
+            pair_consts_sample(R, snaps[R.snapshot], C);
         }
-        const bool step = active;
-        const tri used = dt;
-        float d;
-        int why = MK_RAY_ACTIVE;
-        if (start || step) {
-            // the new state, and with it the next step's first stage, which
-            // gives r and the metric there for the rule and the sample
-            tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), start);
-            const RuleTri rule = {C.t(PC_REH), C.t(PC_NINV), C.p(PC_TOL)};
-            const bool go = rule_dt(q.r, rule, dt, d, why);
-            if (start) {
-                flags = TM_START;
-                // stopped before its first step (reference K = 0), or N < 2
-                // leaves no row pair for the transfer solve
-                active = go && nmax >= 2;
-            } else if (!go) {
-                active = false;  // the step is rejected and the ray stays frozen (geodesics.py:263-267)
-            } else {
-                flags = TM_SAMPLE;
-                // trajectory rows stop at N-1: step N-1 never reaches the solve
-                active = ++steps < nmax - 1;
-            }
-            if (!active) {
-                flags |= TM_END;
-                if (go) why = MK_RAY_MAXSTEPS;
-            }
-        }
-        const bool last = __all_sync(0xffffffffu, !active && exhausted);
-        if (it >= TRI_SLOTS && !zone_wait(&sh.empty[couple][sl], (unsigned)((it / TRI_SLOTS) - 1) & 1u, sh, limit_ns)) {
-            zone_fail(sh, ws);
-            return;
-        }
-        msg.flags[lane] = flags | (last ? TM_DONE : 0u);
-        if (flags & TM_START) msg.ray[lane] = idx;
-        if (flags & TM_END) msg.why[lane] = why;
-        if (flags & TM_SAMPLE) {
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                msg.v[TV_X + 3 * i][lane] = s.X[1 + i].h;
-                msg.v[TV_X + 3 * i + 1][lane] = s.X[1 + i].m;
-                msg.v[TV_X + 3 * i + 2][lane] = s.X[1 + i].l;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                msg.v[TV_K + 2 * i][lane] = s.K[i].h;
-                msg.v[TV_K + 2 * i + 1][lane] = s.K[i].m;
-            }
-            const pr m[4] = {q.m.r, q.m.f, q.m.l3, q.m.ira};
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                msg.v[TV_M + 2 * i][lane] = m[i].h;
-                msg.v[TV_M + 2 * i + 1][lane] = m[i].l;
-            }
-            msg.v[TV_DT][lane] = used.h;
-            msg.v[TV_DT + 1][lane] = used.m;
-            msg.v[TV_DT + 2][lane] = used.l;
-        }
-        __syncwarp();
-        mbar_arrive(&sh.full[couple][sl]);
-        if (last) return;
+        return i;
     }
+    return -1;
+}
+__device__ __forceinline__ void tri_release(TriShared &sh, int slot) {
+    if (atomicSub(&sh.users[slot], 1) == 1) sh.rq[slot] = -1;
 }
 
-__device__ __forceinline__ void tri_sample(int couple, const mk_request *__restrict__ reqs, int nreq,
-                                           const mk_snapshot_view *__restrict__ snaps, RenderWorkspace *ws,
-                                           TriShared &sh, unsigned long long limit_ns) {
-    const int lane = threadIdx.x & 31, col = 32 * couple + lane;
-    // the sampler's constants start at PC_BOX
-    const PairConsts<TRI_LANES> C = {sh.c_smp + col - PC_BOX * TRI_LANES};
-    int rq = 0, steps = 0, nsamples = 0;
-    int64_t pix = 0;
-    pr a = {0.0f, 0.0f};
-    SampleView view = {};
-    int nnu = 0, last_rq = -1;  // the request whose constants are loaded
-    int64_t rows = 0;           // per-step diagnostic rows
-    long long max_tau = 0;  // bits of a double >= 0: they order as integers
-    for (int j = 0;; ++j) {
-        const int sl = j % TRI_SLOTS;
-        const TriSlot &msg = sh.slot[couple][sl];
-        if (!zone_wait(&sh.full[couple][sl], (unsigned)(j / TRI_SLOTS) & 1u, sh, limit_ns)) {
-            zone_fail(sh, ws);
-            return;
-        }
-        const unsigned flags = msg.flags[lane];
-        const long long ray = msg.ray[lane];
-        const int why = msg.why[lane];
-        tri x[3] = {}, dt = {0.0f, 0.0f, 0.0f};
-        pr k[4] = {}, m[4] = {};
-        if (flags & TM_SAMPLE) {
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-                x[i] = {msg.v[TV_X + 3 * i][lane], msg.v[TV_X + 3 * i + 1][lane], msg.v[TV_X + 3 * i + 2][lane]};
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                k[i] = {msg.v[TV_K + 2 * i][lane], msg.v[TV_K + 2 * i + 1][lane]};
-                m[i] = {msg.v[TV_M + 2 * i][lane], msg.v[TV_M + 2 * i + 1][lane]};
-            }
-            dt = {msg.v[TV_DT][lane], msg.v[TV_DT + 1][lane], msg.v[TV_DT + 2][lane]};
-        }
-        __syncwarp();
-        mbar_arrive(&sh.empty[couple][sl]);  // the slot is free for message j + TRI_SLOTS
-        if (flags & TM_START) {
-            rq = find_request(reqs, nreq, ray);
-            const mk_request &R = reqs[rq];
-            pix = fetch_pixel(R.camera, ray - R.ray_offset);
-            if (rq != last_rq) {
-                const tri a3 = t_from(R.camera.bhspin);
-                a = {a3.h, a3.m};
-                view = sample_view(snaps[R.snapshot]);
-                nnu = R.nnu;
-                rows = R.rows_dt ? R.rows : 0;
-                pair_consts_sample(R, snaps[R.snapshot], C);
-                last_rq = rq;
-            }
-            steps = nsamples = 0;
-            max_tau = 0;
-#pragma unroll
-            for (int ch = 0; ch < MK_MAX_NU; ch++) { sh.I[ch][col] = 0.0; sh.P[ch][col] = 1.0; }
-        }
-        if (flags & TM_SAMPLE) {
-            ++steps;
-            const bool row = steps < rows;
-            if (row) {  // per-step diagnostics: row `steps` = this state
-                const mk_request &R = reqs[rq];
-                R.rows_dt[(int64_t)(steps - 1) * request_pixels(R.camera) + pix] = t_to(dt);
-            }
-            PairCoeff co[MK_MAX_NU];
-            const int got = sample_pair(view, C, nnu, x, k, a, m, sh.exptab, co);
-            if (got != PS_OUTSIDE) {
-                ++nsamples;
-                const pr w = p_neg(p_mulr({dt.h, dt.m}, C.p(PC_LUNIT)));
-                double e64[MK_MAX_NU], a64[MK_MAX_NU];
-                if (got == PS_BINARY64) {
-                    const mk_request &R = reqs[rq];
-                    double s64[8];
-                    s64[0] = 0.0;  // x^0 is not read
-#pragma unroll
-                    for (int i = 0; i < 3; i++) s64[1 + i] = t_to(x[i]);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) s64[4 + i] = d_from(k[i].h) + d_from(k[i].l);
-                    coefficients_fp64(R, snaps[R.snapshot], s64, e64, a64);
-                }
-#pragma unroll
-                for (int ch = 0; ch < MK_MAX_NU; ch++) {
-                    if (ch < nnu) {
-                        double wem, tau;
-                        if (got == PS_BINARY64) {
-                            const double wd = d_from(w.h) + d_from(w.l);
-                            wem = wd * e64[ch];
-                            tau = wd * a64[ch];
-                        } else {
-                            wem = p_scaled(p_mulr(w, co[ch].em), co[ch].e);
-                            tau = p_scaled(p_mulr(w, co[ch].ab), co[ch].e);
-                        }
-                        if (row && reqs[rq].rows_em) {
-                            const mk_request &R = reqs[rq];
-                            const int64_t at = (ch * R.rows + steps) * request_pixels(R.camera) + pix;
-                            R.rows_em[at] = got == PS_BINARY64 ? e64[ch] : p_scaled(co[ch].em, co[ch].e);
-                            R.rows_ab[at] = got == PS_BINARY64 ? a64[ch] : p_scaled(co[ch].ab, co[ch].e);
-                        }
-                        const double P = sh.P[ch][col];
-                        sh.I[ch][col] += wem * P;
-                        sh.P[ch][col] = P - tau * P;
-                        const long long bits = __double_as_longlong(tau);
-                        max_tau = bits > max_tau ? bits : max_tau;
-                    }
-                }
-            }
-        }
-        if (flags & TM_END) {
-            double I[MK_MAX_NU];
-#pragma unroll
-            for (int ch = 0; ch < MK_MAX_NU; ch++) I[ch] = sh.I[ch][col];
-            finish_ray(reqs[rq], pix, I, steps, why, nsamples, __longlong_as_double(max_tau), ws);
-        }
-        if (__any_sync(0xffffffffu, (flags & TM_DONE) != 0u)) return;
-    }
+__device__ __noinline__ void tri_camera(const mk_request &R, long long ray, TriState &s) {
+    double s64[8];
+    camera_ray_fast(R.camera, fetch_pixel(R.camera, ray - R.ray_offset), s64);
+    tri_state(s64, s);
 }
 
-__global__ void __launch_bounds__(RENDER_THREADS, TRI_BLOCKS)
+// the sample of message e, its reply written over it
+__device__ __noinline__ void tri_sample(TriShared &sh, int e, const mk_request *__restrict__ reqs,
+                                           const mk_snapshot_view *__restrict__ snaps) {
+    const int col = __float_as_int(sh.v[TV_COL][e]), slot = sh.slot[col];
+    const PairConsts<TRI_REQS> C = {&sh.c[0][slot]};
+    tri x[3];
+    pr k[4], m[4];
+#pragma unroll
+    for (int i = 0; i < 3; i++) x[i] = {sh.v[TV_X + 3 * i][e], sh.v[TV_X + 3 * i + 1][e], sh.v[TV_X + 3 * i + 2][e]};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        k[i] = {sh.v[TV_K + 2 * i][e], sh.v[TV_K + 2 * i + 1][e]};
+        m[i] = {sh.v[TV_M + 2 * i][e], sh.v[TV_M + 2 * i + 1][e]};
+    }
+    const int nnu = sh.nnu[slot];
+    PairCoeff co[MK_MAX_NU];
+    const int got = sample_pair(sh.view[slot], C, nnu, x, k, C.p(PC_A), m, sh.exptab, co);
+    if (got != PS_OUTSIDE) {
+        const pr w = p_neg(p_mulr({sh.v[TV_DT][e], sh.v[TV_DT + 1][e]}, C.p(PC_LUNIT)));
+        double e64[MK_MAX_NU], a64[MK_MAX_NU];
+        if (got == PS_BINARY64) {
+            const mk_request &R = reqs[sh.rq[slot]];
+            double s64[8];
+            s64[0] = 0.0;  // x^0 is not read
+#pragma unroll
+            for (int i = 0; i < 3; i++) s64[1 + i] = t_to(x[i]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) s64[4 + i] = d_from(k[i].h) + d_from(k[i].l);
+            coefficients_fp64(R, snaps[R.snapshot], s64, e64, a64);
+        }
+        const int step = __float_as_int(sh.v[TV_STEP][e]);
+#pragma unroll
+        for (int ch = 0; ch < MK_MAX_NU; ch++) {
+            if (ch >= nnu) break;
+            double wem, tau;
+            if (got == PS_BINARY64) {
+                const double wd = d_from(w.h) + d_from(w.l);
+                wem = wd * e64[ch];
+                tau = wd * a64[ch];
+            } else {
+                wem = p_scaled(p_mulr(w, co[ch].em), co[ch].e);
+                tau = p_scaled(p_mulr(w, co[ch].ab), co[ch].e);
+            }
+            if (step < sh.rows[slot]) {  // per-step diagnostics: row `step` = this state
+                const mk_request &R = reqs[sh.rq[slot]];
+                if (R.rows_em) {
+                    const int64_t at = (ch * R.rows + step) * request_pixels(R.camera) +
+                                       fetch_pixel(R.camera, sh.ray[col] - R.ray_offset);
+                    R.rows_em[at] = got == PS_BINARY64 ? e64[ch] : p_scaled(co[ch].em, co[ch].e);
+                    R.rows_ab[at] = got == PS_BINARY64 ? a64[ch] : p_scaled(co[ch].ab, co[ch].e);
+                }
+            }
+            sh.v[4 * ch][e] = __int_as_float(__double2loint(wem));
+            sh.v[4 * ch + 1][e] = __int_as_float(__double2hiint(wem));
+            sh.v[4 * ch + 2][e] = __int_as_float(__double2loint(tau));
+            sh.v[4 * ch + 3][e] = __int_as_float(__double2hiint(tau));
+        }
+    }
+    sh.v[TV_STEP][e] = __int_as_float(got != PS_OUTSIDE);
+}
+
+__global__ void __launch_bounds__(TRI_THREADS, 1)
 render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total_camera,
-                  const mk_snapshot_view *__restrict__ snaps, RenderWorkspace *ws, const mk_job *job,
-                  int lane_stride, unsigned flip, unsigned long long wait_ns) {
-    __shared__ TriShared sh;
+                  const mk_snapshot_view *__restrict__ snaps, RenderWorkspace *ws, const mk_job *job) {
+    extern __shared__ __align__(16) unsigned char s_tri_raw[];
+    TriShared &sh = *reinterpret_cast<TriShared *>(s_tri_raw);
     if (job) {  // request count and ray total from the device (graph replays)
         nreq = job->nreq;
         total_camera = job->total_rays;
     }
-    if (threadIdx.x == 0) {
-        for (int c = 0; c < TRI_COUPLES; c++)
-            for (int i = 0; i < TRI_SLOTS; i++) {
-                mbar_init(&sh.full[c][i], 32);
-                mbar_init(&sh.empty[c][i], 32);
-            }
-        sh.abort = 0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned FULL = 0xffffffffu, below = (1u << lane) - 1u;
+    if (tid < TRI_REQS) {
+        sh.rq[tid] = -1;
+        sh.users[tid] = 0;
     }
-    if (threadIdx.x < EXP_STEPS) {
-        const tri t = t_from(exp2(-(double)threadIdx.x / EXP_STEPS));
-        sh.exptab[threadIdx.x] = make_float2(t.h, t.m);
+    if (tid < EXP_STEPS) {
+        const tri t = t_from(exp2(-(double)tid / EXP_STEPS));
+        sh.exptab[tid] = make_float2(t.h, t.m);
     }
+    if (tid == 0) sh.drained = 0;
+    // The first rays, dealt over the blocks (by eights, so that a warp's rays
+    // stay neighbours), since the first are the longest; the rest by the
+    // counter.  A block's rays are spread over its sub-partitions before they
+    // share warps, and fill warps before more are used.
+    const long long share = (total_camera + gridDim.x - 1) / gridDim.x;
+    const int group = share >= 64 ? 8 : 1;
+    const int mine = share >= TRI_THREADS ? TRI_THREADS : (int)((share + group - 1) / group) * group;
+    int warps = min(TRI_WARPS, 4 * max(1, (mine + 127) / 128));
+    const int lanes = (mine + warps - 1) / warps, at = warp * lanes + lane;
+    const bool usable = warp < warps && lane < lanes && at < mine;
+    const long long dealt = (long long)mine * gridDim.x;
+    bool exhausted = !usable, waiting = false;  // waiting: nxt is a ray
+    sh.nslot[tid] = -1;
+    if (usable) {
+        sh.nxt[tid] = ((long long)(at / group) * gridDim.x + blockIdx.x) * group + at % group;
+        waiting = sh.nxt[tid] < total_camera;
+    }
+    if (tid == 0) {
+        sh.total = total_camera;
+        sh.rest = total_camera - dealt;
+    }
+
+    bool active = false, fresh = false, ended = false;
+    int slot = 0, steps = 0;
+    TriState s;
+    TriPoint q;
+    tri dt = {0.0f, 0.0f, 0.0f};
     __syncthreads();
-    const int w = threadIdx.x >> 5;
-    const unsigned odd = (blockIdx.x / flip) & 1u;
-    if (((unsigned)w / TRI_COUPLES) == odd)
-        tri_integrate(w % TRI_COUPLES, reqs, nreq, total_camera, ws, lane_stride, sh, wait_ns);
-    else
-        tri_sample(w % TRI_COUPLES, reqs, nreq, snaps, ws, sh, wait_ns);
+    for (;;) {
+        // ---- integrate
+        const int room = TRI_MSGS / warps, base = warp * room, most = room / 32;
+        int count = 0, its = 0;
+        for (; its < most; ++its) {
+            if (!__any_sync(FULL, active || fresh)) break;
+            const tri used = dt;
+            bool sample = false;
+            if (active || fresh) {
+                const PairConsts<TRI_REQS> C = {&sh.c[0][slot]};
+                // the new state, and with it the next step's first stage,
+                // which gives r and the metric there for the rule and the sample
+                tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), fresh);
+                const RuleTri rule = {C.t(PC_REH), C.t(PC_NINV), C.p(PC_TOL)};
+                float d;
+                int why;
+                const bool go = rule_dt(q.r, rule, dt, d, why);
+                if (fresh) {
+                    fresh = false;
+                    // stopped before its first step (reference K = 0), or N < 2
+                    // leaves no row pair for the transfer solve
+                    active = go && sh.nmax[slot] >= 2;
+                } else if (!go) {
+                    active = false;  // the step is rejected and the ray stays frozen (geodesics.py:263-267)
+                } else {
+                    // trajectory rows stop at N-1: step N-1 never reaches the solve
+                    active = ++steps < sh.nmax[slot] - 1;
+                    sample = true;
+#pragma unroll
+                    for (int i = 0; i < 3; i++)
+                        sample = sample && s.X[1 + i].h >= C.f(PC_BOX + i) && s.X[1 + i].h <= C.f(PC_BOX + 3 + i);
+                    if (steps < sh.rows[slot]) {
+                        const mk_request &R = reqs[sh.rq[slot]];
+                        R.rows_dt[(int64_t)(steps - 1) * request_pixels(R.camera) +
+                                  fetch_pixel(R.camera, sh.ray[tid] - R.ray_offset)] = t_to(used);
+                    }
+                }
+                if (!active) {
+                    ended = true;
+                    sh.why[tid] = go ? MK_RAY_MAXSTEPS : why;
+                }
+            }
+            const unsigned mask = __ballot_sync(FULL, sample);
+            if (lane == 0) sh.mask[warp][its] = mask;
+            if (sample) {
+                const int e = base + count + __popc(mask & below);
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    sh.v[TV_X + 3 * i][e] = s.X[1 + i].h;
+                    sh.v[TV_X + 3 * i + 1][e] = s.X[1 + i].m;
+                    sh.v[TV_X + 3 * i + 2][e] = s.X[1 + i].l;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    sh.v[TV_K + 2 * i][e] = s.K[i].h;
+                    sh.v[TV_K + 2 * i + 1][e] = s.K[i].m;
+                }
+                const pr m[4] = {q.m.r, q.m.f, q.m.l3, q.m.ira};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    sh.v[TV_M + 2 * i][e] = m[i].h;
+                    sh.v[TV_M + 2 * i + 1][e] = m[i].l;
+                }
+                sh.v[TV_DT][e] = used.h;
+                sh.v[TV_DT + 1][e] = used.m;
+                sh.v[TV_COL][e] = __int_as_float(tid);
+                sh.v[TV_STEP][e] = __int_as_float(steps);
+            }
+            count += __popc(mask);
+        }
+        if (lane == 0) sh.count[warp] = count;
+        if (tid == 0) sh.chunk = 0;
+        if (!__syncthreads_or(active || fresh || ended || waiting || !exhausted)) return;
+
+        // ---- new rays for idle lanes, a few at a time (a camera ray is ~20 k
+        // cycles of the warp, in binary64), while other warps sample
+        const unsigned idle = __ballot_sync(FULL, usable && !active && !exhausted && !waiting);
+        const unsigned busy = __ballot_sync(FULL, active);
+        if (__popc(idle) >= TRI_REFILL || (idle && !busy)) {
+            const long long idx = fetch((idle >> lane) & 1u, &ws->counter, sh.rest);
+            if (idx == -1) sh.drained = 1;
+            if (idx >= 0) {
+                waiting = true;
+                sh.nxt[tid] = sh.total - sh.rest + idx;
+            }
+        }
+        if (waiting && !active) {
+            const long long nxt = sh.nxt[tid];
+            if (!ray_in_request(reqs, nreq, nxt)) waiting = false;
+            else {
+                const int rq = find_request(reqs, nreq, nxt), nslot = tri_acquire(sh, rq, reqs, snaps);
+                if (nslot >= 0) {
+                    sh.nslot[tid] = nslot;
+                    TriState n;  // a copy: s itself stays in registers
+                    tri_camera(reqs[rq], nxt, n);
+                    s = n;
+                }
+            }
+        }
+
+        // ---- sample
+        int total = 0;
+#pragma unroll 1
+        for (int w = 0; w < TRI_WARPS; w++) total += sh.count[w];
+        for (;;) {
+            int first = 0;
+            if (lane == 0) first = atomicAdd(&sh.chunk, 32);
+            first = __shfl_sync(FULL, first, 0);
+            if (first >= total) break;
+            int g = first + lane;
+            if (g < total) {
+                int w = 0;
+                while (g >= sh.count[w]) g -= sh.count[w++];
+                tri_sample(sh, w * room + g, reqs, snaps);
+            }
+        }
+        bool left = __syncthreads_or(waiting);
+        exhausted = exhausted || sh.drained;  // the counter passed the job's end
+        left = left || !sh.drained;
+
+        // ---- fold, finish, start
+        {
+            const int nnu = sh.nnu[slot];
+            int e = base;
+            for (int i = 0; i < its; i++) {
+                const unsigned mask = sh.mask[warp][i];
+                const int at_e = e + __popc(mask & below);
+                e += __popc(mask);
+                if (!((mask >> lane) & 1u) || !__float_as_int(sh.v[TV_STEP][at_e])) continue;
+                ++sh.samples[tid];
+                for (int ch = 0; ch < nnu; ch++) {
+                    const double wem = __hiloint2double(__float_as_int(sh.v[4 * ch + 1][at_e]),
+                                                        __float_as_int(sh.v[4 * ch][at_e]));
+                    const double tau = __hiloint2double(__float_as_int(sh.v[4 * ch + 3][at_e]),
+                                                        __float_as_int(sh.v[4 * ch + 2][at_e]));
+                    const double P = sh.P[ch][tid];
+                    sh.I[ch][tid] += wem * P;
+                    sh.P[ch][tid] = P - tau * P;
+                    const long long bits = __double_as_longlong(tau);
+                    if (bits > sh.tau[tid]) sh.tau[tid] = bits;
+                }
+            }
+        }
+        if (ended) {
+            ended = false;
+            const mk_request &R = reqs[sh.rq[slot]];
+            double I[MK_MAX_NU];
+#pragma unroll
+            for (int ch = 0; ch < MK_MAX_NU; ch++) I[ch] = sh.I[ch][tid];
+            finish_ray(R, fetch_pixel(R.camera, sh.ray[tid] - R.ray_offset), I, steps, sh.why[tid],
+                       sh.samples[tid], __longlong_as_double(sh.tau[tid]), ws);
+            tri_release(sh, slot);
+        }
+        if (const int nslot = sh.nslot[tid]; nslot >= 0) {
+            if (sh.odd[nslot]) {
+                atomicAdd(&ws->odd_rays, 1ull);  // left to render_fp64_kernel
+                tri_release(sh, nslot);
+            } else {
+                slot = nslot;
+                sh.slot[tid] = slot;
+                sh.ray[tid] = sh.nxt[tid];
+                steps = sh.samples[tid] = 0;
+                sh.tau[tid] = 0;
+                fresh = true;
+#pragma unroll
+                for (int ch = 0; ch < MK_MAX_NU; ch++) {
+                    sh.I[ch][tid] = 0.0;
+                    sh.P[ch][tid] = 1.0;
+                }
+            }
+            waiting = false;
+            sh.nslot[tid] = -1;
+        }
+
+        // ---- the last rays into fewer warps
+        if (!left) {
+            const unsigned live = __ballot_sync(FULL, active);
+            if (lane == 0) sh.alive[warp] = __popc(live);
+            __syncthreads();
+            int rank = __popc(live & below), rays = 0;
+#pragma unroll 1
+            for (int w = 0; w < TRI_WARPS; w++) {
+                if (w < warp) rank += sh.alive[w];
+                rays += sh.alive[w];
+            }
+            const int need = 4 * ((rays + 127) / 128);
+            if (need < warps) {
+                warps = need;
+                float *mv = &sh.v[0][0];
+                constexpr int N = TRI_THREADS - 128;  // rays at most
+                int j = rank;
+                auto put = [&](float f) { mv[j] = f; j += N; };
+                auto get = [&]() { const float f = mv[j]; j += N; return f; };
+                auto put64 = [&](long long v) { put(__int_as_float((int)v)); put(__int_as_float((int)(v >> 32))); };
+                auto get64 = [&]() {
+                    const unsigned lo = __float_as_uint(get());
+                    return (long long)(((unsigned long long)__float_as_uint(get()) << 32) | lo);
+                };
+                if (active) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        if (i) { put(s.X[i].h); put(s.X[i].m); put(s.X[i].l); }
+                        put(s.K[i].h); put(s.K[i].m); put(s.K[i].l);
+                        put(q.a1[i].h); put(q.a1[i].l);
+                    }
+                    put(dt.h); put(dt.m); put(dt.l);
+                    put(__int_as_float(slot)); put(__int_as_float(steps)); put(__int_as_float(sh.samples[tid]));
+                    put64(sh.tau[tid]);
+                    put64(sh.ray[tid]);
+                    for (int ch = 0; ch < sh.nnu[slot]; ch++) {
+                        put64(__double_as_longlong(sh.I[ch][tid]));
+                        put64(__double_as_longlong(sh.P[ch][tid]));
+                    }
+                }
+                __syncthreads();
+                active = warp < need && lane * need + warp < rays;
+                j = lane * need + warp;
+                if (active) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        if (i) { s.X[i].h = get(); s.X[i].m = get(); s.X[i].l = get(); }
+                        s.K[i].h = get(); s.K[i].m = get(); s.K[i].l = get();
+                        q.a1[i].h = get(); q.a1[i].l = get();
+                    }
+                    dt.h = get(); dt.m = get(); dt.l = get();
+                    slot = __float_as_int(get()); steps = __float_as_int(get());
+                    sh.samples[tid] = __float_as_int(get());
+                    sh.tau[tid] = get64();
+                    sh.ray[tid] = get64();
+                    sh.slot[tid] = slot;
+                    for (int ch = 0; ch < sh.nnu[slot]; ch++) {
+                        sh.I[ch][tid] = __longlong_as_double(get64());
+                        sh.P[ch][tid] = __longlong_as_double(get64());
+                    }
+                }
+                __syncthreads();
+            }
+        }
+    }
 }
 
 // Initial states of every camera ray of a launch as float pairs (x^mu
@@ -1881,17 +2037,12 @@ static int launch_render(const mk_request *reqs_dev, int32_t nreq, int64_t total
     int rc = phase_mark(st, 0);
     if (rc != MK_OK) return rc;
     if (precision == MK_FP64) {
-        // the fewest rays a warp (a power of two) with which every ray has a
-        // lane among the integrating warps of one block an SM
-        const int sms = device_sm_count();
-        int stride = 32;
-        while (stride > 1 && max_rays > (int64_t)sms * TRI_COUPLES * (32 / stride)) stride /= 2;
-        const int64_t rays_per_block = TRI_COUPLES * (32 / stride);
-        const int64_t blocks = std::min<int64_t>((max_rays + rays_per_block - 1) / rays_per_block,
-                                                 (int64_t)sms * TRI_BLOCKS);
-        render_tri_kernel<<<(unsigned)blocks, RENDER_THREADS, 0, st>>>(reqs_dev, nreq, (long long)total_rays,
-                                                                        snaps_dev, ws, job_dev, stride,
-                                                                        (unsigned)sms, g_zone_wait_ns);
+        MK_CUDA(cudaFuncSetAttribute(render_tri_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(TriShared)));
+        // one block an SM, at least one ray for each of a block's sub-partitions
+        const int64_t blocks = std::min<int64_t>((max_rays + 3) / 4, (int64_t)device_sm_count());
+        render_tri_kernel<<<(unsigned)blocks, TRI_THREADS, sizeof(TriShared), st>>>(
+            reqs_dev, nreq, (long long)total_rays, snaps_dev, ws, job_dev);
         MK_LAUNCHED("render_tri_kernel");
         render_fp64_kernel<SRC_CAMERA>
             <<<persistent_grid(blocks_per_sm(render_fp64_kernel<SRC_CAMERA>, 0), max_rays), RENDER_THREADS, 0, st>>>(

@@ -149,13 +149,13 @@ class PreparedRender:
 
     def check(self):
         """Raise MKError (MK_ERR_TIMEOUT) if a bounded wait of the last
-        launch's pipelined warps ran out, which leaves its images invalid
+        launch's near-hole pipeline ran out, which leaves its images invalid
         (syncs).  Never expected; the limit only keeps a fault from hanging
         the GPU."""
         n = int(self.ws[_lib.MK_WS_ERROR].item())
         if n:
             raise _lib.MKError(_lib.MK_ERR_TIMEOUT,
-                               f"mk_render: {n} waits between the render's warps ran out; the images are invalid")
+                               f"mk_render: {n} waits of the near-hole pipeline ran out; the images are invalid")
 
     def work_totals(self):
         """(accepted steps, in-snapshot samples) of the last launch (syncs)."""
@@ -202,7 +202,7 @@ def render_requests(requests, precision="fp64", stream=None, with_steps=False):
 
     Each request's ``out`` dict receives ``image`` ((nnu, res, res) float64
     CUDA tensor), ``check`` (PreparedRender.check of the launch: raises if
-    a wait between the render's pipelined warps ran out; syncs) and, with
+    a wait of the mixed form's near-hole pipeline ran out; syncs) and, with
     ``with_steps``, ``nsteps`` and ``status``.  Returns the list of image
     tensors.  The launch is asynchronous on ``stream`` (default: the current
     stream)."""
@@ -239,7 +239,7 @@ def make_image(fluid_model, camera_inclination=60, camera_distance=1000, mass_sc
         err.copy_(prep.ws[_lib.MK_WS_ERROR:_lib.MK_WS_ERROR + 1], non_blocking=True)
     s.synchronize()
     if int(err[0]):
-        raise _lib.MKError(_lib.MK_ERR_TIMEOUT, f"mk_render: {int(err[0])} waits between the render's warps ran out; "
+        raise _lib.MKError(_lib.MK_ERR_TIMEOUT, f"mk_render: {int(err[0])} waits of the near-hole pipeline ran out; "
                                                 "the image is invalid")
     out = out_host.numpy()
     if np.ndim(observing_frequency) == 0:
@@ -266,9 +266,7 @@ def step_diagnostics(fluid_model, camera_inclination=60, camera_distance=1000, m
     from .transfer import solve_attenuated_emissivity, solve_specific_intensity
     req = RenderRequest(fluid_model, camera_inclination, camera_distance, mass_scale, M_bh, r_high,
                         observing_frequency, fov, resolution, max_nsteps, r_low, rows=max_nsteps)
-    prep = PreparedRender([req], precision="fp64")
-    prep.launch()
-    prep.check()
+    PreparedRender([req], precision="fp64").launch()
     K = req.out["nsteps"].reshape(-1)
     nt = trimmed_rows(K, max_nsteps)
     em, ab, dt = req.out["rows_em"][:, :nt], req.out["rows_ab"][:, :nt], req.out["rows_dt"][:nt]
