@@ -898,7 +898,13 @@ __device__ __forceinline__ void zone_integrate(const mk_request *__restrict__ re
     const int lane = threadIdx.x & 31;
     unsigned long long *counter = &ws->q64_next;
     const long long total = min((long long)*(volatile unsigned long long *)&ws->q64_count, capacity);
-    bool active = false, exhausted = false;
+    // A short queue is spread over the blocks, at least 12 rays a warp: lanes
+    // meet fewer of each other's turning points and ends.  Phase B of 32^2 and
+    // 63^2 rays 1.11 -> 1.08 and 1.75 -> 1.72 ms; with one ray a warp 1.69 at
+    // 63^2, but its many blocks then slow phase C beside it (0.30 -> 0.47, at
+    // 64^2 0.32 -> 0.75 ms), and so do longer queues spread (256^2 2.6 -> 3.0 ms).
+    const bool spread = total <= 4 * (long long)gridDim.x;
+    bool active = false, exhausted = spread && lane >= max(12, (int)((total + gridDim.x - 1) / gridDim.x));
     int steps = 0, nmax = 0, zone_steps = 0, run = 0, run_max = 0, b_steps = 0, ray = -1;
     // float-pair state (X, K) throughout, as in the FP32 phases; near the
     // hole the wavevector is renormalised to null on entry (binary64) and
@@ -1760,7 +1766,10 @@ render_f32_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
     const long long total =
         SRC == SRC_CAMERA ? total_camera
                           : min((long long)*(volatile unsigned long long *)&ws->q32_count, capacity);
-    bool active = false, exhausted = false;
+    // lanes that take rays: a camera launch of fewer rays than lanes spreads
+    // them over its warps (a warp's step costs what its lanes do between them)
+    const long long warps = (long long)gridDim.x * (blockDim.x / 32);
+    bool active = false, exhausted = SRC == SRC_CAMERA && (threadIdx.x & 31) * warps >= total;
     int rq = 0, steps = 0, nsamples = 0, why = MK_RAY_ACTIVE;
     long long ray = 0;
     int64_t pix = 0;
@@ -2073,14 +2082,28 @@ static int launch_render(const mk_request *reqs_dev, int32_t nreq, int64_t total
     // dynamic shared memory of the FP32 kernels: their request table
     const size_t req_smem =
         (size_t)(job_dev ? MK_MAX_REQUESTS_MIXED : std::min<int32_t>(nreq, MK_MAX_REQUESTS_MIXED)) * sizeof(ReqF32);
+    // One wave of rays, a few requests (each block holds a table of them):
+    // smaller blocks, whose warps spread evenly over the SMs, and one warp a
+    // sub-partition before rays share warps.  63^2 and 64^2 rays: phase A 0.41
+    // -> 0.35 and 0.42 -> 0.36 ms, C 0.36 -> 0.30 and 0.32; 256^2 (13.5 warps
+    // an SM) 0.71 -> 0.65 ms with two warps a block (0.70 with one).
+    int small = 0;
+    int64_t small_warps = (max_rays + 31) / 32;
+    if (!job_dev && nreq <= 16 && small_warps <= (int64_t)device_sm_count() * 16) {
+        const int64_t spread = (int64_t)device_sm_count() * 4;
+        small = small_warps < spread ? 32 : 64;
+        small_warps = std::max<int64_t>(small_warps, std::min<int64_t>(max_rays, spread));
+        small_warps = (small_warps + small / 32 - 1) / (small / 32) * (small / 32);
+    }
     if (f32_blocks == 5)
         render_f32_kernel<SRC_CAMERA, 5>
             <<<persistent_grid(blocks_per_sm(render_f32_kernel<SRC_CAMERA, 5>, 5), max_rays), RENDER_THREADS, req_smem,
                st>>>(reqs_dev, nreq, (long long)total_rays, snaps_dev, ws, q64, q32, cap, job_dev, mode, cam);
     else if (f32_blocks == 4)
         render_f32_kernel<SRC_CAMERA, 4>
-            <<<persistent_grid(blocks_per_sm(render_f32_kernel<SRC_CAMERA, 4>, 1), max_rays), RENDER_THREADS, req_smem,
-               st>>>(reqs_dev, nreq, (long long)total_rays, snaps_dev, ws, q64, q32, cap, job_dev, mode, cam);
+            <<<small ? (unsigned)(small_warps * 32 / small) :
+                       persistent_grid(blocks_per_sm(render_f32_kernel<SRC_CAMERA, 4>, 1), max_rays),
+               small ? small : RENDER_THREADS, req_smem, st>>>(reqs_dev, nreq, (long long)total_rays, snaps_dev, ws, q64, q32, cap, job_dev, mode, cam);
     else
         render_f32_kernel<SRC_CAMERA, 3>
             <<<persistent_grid(blocks_per_sm(render_f32_kernel<SRC_CAMERA, 3>, 2), max_rays), RENDER_THREADS, req_smem,
