@@ -238,11 +238,11 @@ __global__ void synchrotron_kernel(const double *__restrict__ Ne, const double *
 }
 
 // backward explicit Euler (transfer.py:106-119), one thread per pixel.  The
-// recurrence is serial but its inputs are not: TRANSFER_AHEAD rows are loaded
-// before the first is used, so that a few warps an SM (an image's pixels are
-// no more) keep the memory busy; small blocks spread them evenly.
-constexpr int TRANSFER_AHEAD = 16, TRANSFER_THREADS = 64;
-template <bool DIS>
+// recurrence is serial but its inputs are not: AHEAD rows are loaded while the
+// AHEAD before them are folded, so that a few warps an SM (an image's pixels
+// are no more) keep the memory busy; small blocks spread them evenly.
+constexpr int TRANSFER_THREADS = 64;
+template <bool DIS, int AHEAD>
 __global__ void __launch_bounds__(TRANSFER_THREADS)
 solve_intensity_kernel(const double *__restrict__ em, const double *__restrict__ ab, const double *__restrict__ dt,
                        int64_t nsteps, int64_t npx, double L, double *__restrict__ I, double *__restrict__ dIs) {
@@ -258,16 +258,30 @@ solve_intensity_kernel(const double *__restrict__ em, const double *__restrict__
         }
         Iv += w * t;
     };
-    for (; i >= TRANSFER_AHEAD; i -= TRANSFER_AHEAD) {
-        double e[TRANSFER_AHEAD], a[TRANSFER_AHEAD], d[TRANSFER_AHEAD];
+    double e[AHEAD], a[AHEAD], d[AHEAD];
+    auto load = [&](int64_t j, double (&x)[AHEAD], double (&y)[AHEAD], double (&z)[AHEAD]) {
 #pragma unroll
-        for (int q = 0; q < TRANSFER_AHEAD; q++) {
-            e[q] = em[(i - q) * npx + p];
-            a[q] = ab[(i - q) * npx + p];
-            d[q] = dt[(i - q - 1) * npx + p];
+        for (int q = 0; q < AHEAD; q++) {
+            x[q] = em[(j - q) * npx + p];
+            y[q] = ab[(j - q) * npx + p];
+            z[q] = dt[(j - q - 1) * npx + p];
         }
+    };
+    if (i >= AHEAD) load(i, e, a, d);
+    for (; i >= AHEAD; i -= AHEAD) {
+        double e1[AHEAD], a1[AHEAD], d1[AHEAD];
+        const bool more = i >= 2 * AHEAD;
+        if (more) load(i - AHEAD, e1, a1, d1);
 #pragma unroll
-        for (int q = 0; q < TRANSFER_AHEAD; q++) fold(e[q], a[q], d[q]);
+        for (int q = 0; q < AHEAD; q++) fold(e[q], a[q], d[q]);
+        if (more) {
+#pragma unroll
+            for (int q = 0; q < AHEAD; q++) {
+                e[q] = e1[q];
+                a[q] = a1[q];
+                d[q] = d1[q];
+            }
+        }
     }
     for (; i >= 1; i--) fold(em[i * npx + p], ab[i * npx + p], dt[(i - 1) * npx + p]);
     I[p] = Iv;
@@ -403,12 +417,15 @@ extern "C" int mk_solve_intensity(const double *em_dev, const double *ab_dev, co
     MK_REQUIRE(nsteps >= 0 && npx >= 0, MK_ERR_ARG, "mk_solve_intensity: negative size");
     if (npx == 0) return MK_OK;
     const unsigned grid = grid_for(npx, TRANSFER_THREADS);
-    if (dIs_dev)
-        solve_intensity_kernel<true><<<grid, TRANSFER_THREADS, 0, as_stream(stream)>>>(em_dev, ab_dev, dt_dev, nsteps,
-                                                                                       npx, L_unit, I_dev, dIs_dev);
-    else
-        solve_intensity_kernel<false><<<grid, TRANSFER_THREADS, 0, as_stream(stream)>>>(em_dev, ab_dev, dt_dev, nsteps,
-                                                                                        npx, L_unit, I_dev, nullptr);
+    // 16 rows take ~200 registers a thread, two warps a sub-partition; more
+    // pixels than those hold take six rows.  500 x 1600 rows and pixels 68 ->
+    // 66 us, 1000 x 4096 210 -> 156, 500 x 25600 135 -> 104; 800 x 40000 267
+    // -> 243 (314 with 16), 60 x 65536 30 -> 27 (33) against one row at a time.
+    const bool few = npx <= (int64_t)device_sm_count() * 4 * 2 * 32;
+    const auto kernel = dIs_dev ? (few ? solve_intensity_kernel<true, 16> : solve_intensity_kernel<true, 6>)
+                                : (few ? solve_intensity_kernel<false, 16> : solve_intensity_kernel<false, 6>);
+    kernel<<<grid, TRANSFER_THREADS, 0, as_stream(stream)>>>(em_dev, ab_dev, dt_dev, nsteps, npx, L_unit, I_dev,
+                                                             dIs_dev);
     MK_LAUNCHED("solve_intensity_kernel");
     return MK_OK;
 }

@@ -257,9 +257,11 @@ def test_fluid_at_faces_and_edges(cuda, orc, refined):
     assert np.nanmax(np.abs(x - ref["kdotu"]) / np.maximum(np.abs(ref["kdotu"]), kn)) < 1e-12
 
 
-@pytest.mark.parametrize("nsteps,npx", [(2, 1), (16, 65), (17, 64), (18, 63), (34, 1), (150, 129)])
+@pytest.mark.parametrize("nsteps,npx", [(2, 1), (16, 65), (17, 64), (18, 63), (34, 1), (150, 129), (6, 40000),
+                                        (14, 40001), (20, 38912)])
 def test_transfer_read_ahead(cuda, orc, nsteps, npx):
-    """Steps read 16 ahead, 64 rays a block: each side of both."""
+    """Rows read 16 ahead, or 6 for many pixels, 64 pixels a block: each side
+    of each."""
     import mahakala_gb300 as mk
     rng = np.random.default_rng(nsteps)
     em, ab = rng.uniform(0, 1e-3, (2, nsteps, npx))
