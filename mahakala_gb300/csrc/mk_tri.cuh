@@ -20,8 +20,8 @@
 // triples it took longer, ~38 k cycles a step against ~31 k):
 // there k grows as 1 / (r - r_EH), and E and L, which steer the ray, are
 // small differences of its components.  TRI_NEAR is where: 0.1 M keeps
-// captured rays at 0.10-0.33 times the binary64 form's error, 0.03 M at
-// 0.28-1.6, 0.01 M at 0.57-5.5.  The fused render needs no such switch: what
+// captured rays at 0.09-0.33 times the binary64 form's error, 0.05 M at
+// 0.23-0.81, 0.03 M at 0.28-1.6, 0.01 M at 0.57-5.5.  The fused render needs no such switch: what
 // a ray emits there is redshifted away (its images are measured instead).
 //
 // Error-free steps: TwoSum (Knuth, TAOCP vol. 2, 4.2.2), FastTwoSum (Dekker
