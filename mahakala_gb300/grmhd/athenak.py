@@ -85,9 +85,15 @@ def mesh_tables(arrs, max_table_cells=1 << 28):
     start = np.rint((left - lo) / wf).astype(np.int64)
     span = np.rint(widths / wf).astype(np.int64)
     taken = 0
-    kinds, kind = np.unique(span @ np.array([1, 1 << 20, 1 << 40]), return_inverse=True)
-    for s in range(len(kinds)):                   # one span a level
-        m = np.flatnonzero(kind == s)
+    if (span == 1).all():                         # one level: a cell a block
+        flat = (start[:, 2] * nb[1] + start[:, 1]) * nb[0] + start[:, 0]
+        m = np.flatnonzero((start < nb).all(axis=1))
+        table.reshape(-1)[flat[m]] = m
+        taken, sets = m.size, []
+    else:                                         # one span a level
+        kinds, kind = np.unique(span @ np.array([1, 1 << 20, 1 << 40]), return_inverse=True)
+        sets = [np.flatnonzero(kind == s) for s in range(len(kinds))]
+    for m in sets:
         sx, sy, sz = span[m[0]]
         # the table cells of these blocks, cut at the table's edge as a slice is
         i, j, k = (start[m, a, None, None, None] + np.arange(n).reshape(sh) for a, n, sh in
@@ -107,13 +113,13 @@ def mesh_tables(arrs, max_table_cells=1 << 28):
             at = np.minimum(np.searchsorted(sorted_keys, want), nmb - 1)
             return ok & (sorted_keys[at] == want)
 
-        lv, t = levels.astype(np.int64), locs.astype(np.int64)
-        for d in np.ndindex(3, 3, 3):
-            d = np.array(d) - 1
-            if not d.any():
-                continue
-            u = t + d
-            fine_ghosts |= ~there(lv, u) & ~there(lv - 1, u // 2) & there(lv + 1, 2 * u)
+        d = np.stack(np.meshgrid(*3 * ([-1, 0, 1],), indexing="ij"), axis=-1).reshape(-1, 1, 3)
+        d = d[d.any(axis=-1)[:, 0]]
+        for m in range(0, nmb, 4096):             # the 26 directions of some blocks at a time
+            u = (locs[m:m + 4096].astype(np.int64) + d).reshape(-1, 3)
+            lv = np.tile(levels[m:m + 4096].astype(np.int64), len(d))
+            fine = ~there(lv, u) & ~there(lv - 1, u // 2) & there(lv + 1, 2 * u)
+            fine_ghosts[m:m + 4096] = fine.reshape(len(d), -1).any(axis=0)
     block64 = np.where(fine_ghosts, np.cumsum(fine_ghosts) - 1, -1).astype(np.int32)
     return dict(locs=locs, levels=levels, keys=sorted_keys,
                 key_block=np.ascontiguousarray(order.astype(np.int32)), faces=faces, table=table, nb=nb,
