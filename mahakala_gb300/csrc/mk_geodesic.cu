@@ -127,14 +127,13 @@ __device__ __noinline__ void integrate_reference_f64(double s[8], int j0, int64_
     store_row(state_out, p, s);
 }
 
-// The same on triples (mk_tri.cuh).  A warp's lanes near the horizon wait until
-// none of the others moves (NEAR_LAST): a binary64 step holds the warp ~31 k
+// The same on triples (mk_tri.cuh).  rpw rays a warp: a ray's chain of steps
+// sets the time of a small launch, so its rays are spread over every SM
+// sub-partition before they share warps.  A warp's lanes near the horizon
+// wait until none of the others moves: a binary64 step holds the warp ~31 k
 // cycles whatever number of lanes takes it, so the lanes take them together,
 // after as many steps on triples as the longest ray has (40^2 rays, spin 0.1:
-// 12.3 -> 9.9 ms).  rpw rays a warp: a ray's chain of steps
-// sets the time of a small launch, so its rays are spread over every SM
-// sub-partition before they share warps (lanes that near the horizon hold
-// the others of their warp).
+// 12.3 -> 9.9 ms).
 // ROWS: rows or dts wanted; the state is then converted to binary64 at every
 // step, and the state before a rejected step is that row.
 template <bool ROWS>
@@ -168,7 +167,7 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
         }
         while (__any_sync(team, moving)) {
             const bool near = go && d < TRI_NEAR;
-            if (__any_sync(team, moving && !near) && near) continue;  // see NEAR_LAST
+            if (__any_sync(team, moving && !near) && near) continue;
             if (!moving) continue;
             tri dtn = dt;
             if (!ROWS) last = s;
@@ -244,13 +243,14 @@ __device__ __noinline__ void integrate_fixed_f64(double s[8], int j0, int64_t p,
     store_row(state_out, p, s);
 }
 
+// Lanes near the horizon do not wait here: the fixed-fraction rule takes few
+// steps there (128^2 rays 1.80 ms, 1.82 with the wait).
 __global__ void __launch_bounds__(GEO_THREADS)
 integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int N, double hfrac, double hmin,
                        double hmax, double capture, double r_escape, int32_t *__restrict__ Kout,
                        int32_t *__restrict__ why_out, double *__restrict__ state_out, int rpw, int all_f64) {
     const int lane = threadIdx.x & 31;
     const int64_t p = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * rpw + lane;
-    const unsigned team = __ballot_sync(0xffffffffu, lane < rpw && p < npx);
     if (lane >= rpw || p >= npx) return;
     double s64[8];
 #pragma unroll
@@ -265,19 +265,15 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
     last = s;
     const SpinTri sp = spin_tri(a);
     int st = MK_RAY_MAXSTEPS, j = 0;
-    {
+    if (!out) {
         TriPoint q;
-        bool moving = !out && N > 0;
-        q.r = {0.0f, 0.0f, 0.0f};
-        if (moving) tri_step<true>(s, q, {0.0f, 0.0f, 0.0f}, sp.a, sp.aa, sp.aa3, true);
-        while (__any_sync(team, moving)) {
-            const bool near = q.r.h < near_r;
-            if (__any_sync(team, moving && !near) && near) continue;  // see NEAR_LAST
-            if (!moving) continue;
+        tri_step<true>(s, q, {0.0f, 0.0f, 0.0f}, sp.a, sp.aa, sp.aa3, true);
+        for (j = 0; j < N; j++) {
             tri h = t_add(t_mul(hf, q.r), {0.0f, 0.0f, 0.0f});
             h = t_less(h, h0) ? h0 : (t_less(h1, h) ? h1 : h);
             h = t_neg(h);
             const tri r = q.r;
+            const bool near = r.h < near_r;
             last = s;
             if (near) {  // through a copy: s itself stays in registers
                 TriState n = s;
@@ -287,16 +283,9 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
                 s = n;
             }
             tri_step<true>(s, q, h, sp.a, sp.aa, sp.aa3, near);
-            if (tri_left_range(s, q.r.h)) {
-                out = true;
-                moving = false;
-                continue;
-            }
-            ++j;
-            moving = false;
-            if (t_less(q.r, rcap)) st = MK_RAY_CAPTURED;
-            else if (t_less(resc, q.r) && t_less(r, q.r)) st = MK_RAY_ESCAPED;
-            else moving = j < N;
+            if (tri_left_range(s, q.r.h)) { out = true; break; }
+            if (t_less(q.r, rcap)) { st = MK_RAY_CAPTURED; j++; break; }
+            if (t_less(resc, q.r) && t_less(r, q.r)) { st = MK_RAY_ESCAPED; j++; break; }
         }
     }
     if (out) {
