@@ -23,8 +23,8 @@
 
 namespace mk {
 
-// A ray's constants, one column of shared memory per thread (registers hold
-// the ray itself).
+// A request's constants, one column of shared memory each (registers hold the
+// ray itself).
 enum PairConst {
     PC_A = 0, PC_AA = 2, PC_AA_L = 4, PC_REH = 5, PC_NINV = 8, PC_TOL = 11, PC_BOX = 13, PC_INVW = 19,
     PC_GAM2 = 22, PC_RHIGH = 24, PC_RLOW = 26, PC_GEM1 = 28, PC_GIM1 = 30, PC_KTH = 32, PC_SIGMA = 34,
@@ -35,7 +35,7 @@ constexpr int EXP_STEPS = 32;  // table of 2^(-j/32)
 
 template <int STRIDE>
 struct PairConsts {
-    float *c;  // this thread's column
+    float *c;  // the request's column
     __device__ __forceinline__ pr p(int i) const { return {c[i * STRIDE], c[(i + 1) * STRIDE]}; }
     __device__ __forceinline__ tri t(int i) const { return {c[i * STRIDE], c[(i + 1) * STRIDE], c[(i + 2) * STRIDE]}; }
     __device__ __forceinline__ float f(int i) const { return c[i * STRIDE]; }
@@ -78,7 +78,7 @@ __device__ __forceinline__ bool pair_request(const mk_request &R) {
     return ok;
 }
 
-// the integrating warp's part (to PC_TOL) and the sampling warp's (from PC_BOX)
+// the geodesic's part (to PC_TOL) and the sampler's (from PC_BOX)
 template <int STRIDE>
 __device__ __forceinline__ void pair_consts_geodesic(const mk_request &R, PairConsts<STRIDE> C) {
     const double a = R.camera.bhspin;
@@ -119,7 +119,7 @@ __device__ __forceinline__ void pair_consts_sample(const mk_request &R, const mk
         }
 }
 
-// The snapshot's fields a sample reads, held in registers by the sampling warp.
+// The snapshot's fields a sample reads.
 struct SampleView {
     const float *blocks;
     const double *geom;
