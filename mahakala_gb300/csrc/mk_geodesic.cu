@@ -1,5 +1,7 @@
 // mk_geodesic.cu -- camera initialisation, geodesic integration and the
-// shadow-bisection pass (geodesics.py), one thread per ray, FP64.
+// shadow-bisection pass (geodesics.py), one thread per ray: cameras in
+// binary64, geodesics in float triples (mk_tri.cuh) with binary64 where those
+// do not hold.
 #include <algorithm>
 
 #include "mk_common.cuh"
