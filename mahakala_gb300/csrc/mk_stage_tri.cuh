@@ -126,6 +126,14 @@ __device__ __forceinline__ double scaled(double v, int e) {
     return is_zero(v) ? 0.0 : __hiloint2double(__double2hiint(v) + (int)((unsigned)e << 20), __double2loint(v));
 }
 
+// v 2^e for 2^-140 <= v < 2^128, or v = 0: faint to the end of the doubles'
+// range, where 2^e is taken in two normal factors with one rounding
+__device__ __forceinline__ double pow2_scaled(double v, int e) {
+    if (e < -850)
+        return v * __hiloint2double((1023 + e / 2) << 20, 0) * __hiloint2double((1023 + (e - e / 2)) << 20, 0);
+    return scaled(v, e);
+}
+
 // doubles in order as integers (-0 = 0)
 __device__ __forceinline__ long long ordered(double v) {
     const long long b = __double_as_longlong(v);
@@ -218,22 +226,21 @@ __device__ __forceinline__ bool synchro_tri(const SynchroTri &c, double Ne, doub
     }
     // alpha = em_raw / B_nu, B_nu = 2 h nu^3 / (c^2 den)
     tri ab = t_mulr(t_mulr(em, t_mulr(rv, rv)), t_mulr(den, c.kab));
+    int ex = en - 60 - e;  // the result's power of two
     if (invariant) {
-        const tri w = t_mulr(v, c.resc), rw = t_rcp(w);
+        // 1/w^2 by w's significand: at rescale_nu = 1 it is 1e-23 at 230 GHz,
+        // whose low words no float holds
+        const tri w = t_mulr(v, c.resc);
+        const int ew = ((int)(__float_as_uint(w.h) >> 23) & 255) - 127;
+        const float sw = __uint_as_float((unsigned)(127 - ew) << 23);
+        const tri rw = t_rcp({sw * w.h, sw * w.m, sw * w.l});
         em = t_mulr(t_mulr(em, v), t_mulr(rw, rw));
+        em_out = pow2_scaled(t_to(em), ex - 2 * ew);
         ab = t_mulr(ab, w);
     } else {
-        em = t_mulr(em, v);
+        em_out = pow2_scaled(t_to(t_mulr(em, v)), ex);
     }
-    if (e > 400) {  // faint to the end of the doubles' range
-        // 2^-e in two normal factors, one rounding
-        const double s1 = __hiloint2double((1023 - e / 2) << 20, 0), s2 = __hiloint2double((1023 - (e - e / 2)) << 20, 0);
-        em_out = scaled(t_to(em), en - 60) * s1 * s2;
-        ab_out = scaled(t_to(ab), en - 60) * s1 * s2;
-    } else {
-        em_out = scaled(t_to(em), en - 60 - e);
-        ab_out = scaled(t_to(ab), en - 60 - e);
-    }
+    ab_out = pow2_scaled(t_to(ab), ex);
     return true;
 }
 
