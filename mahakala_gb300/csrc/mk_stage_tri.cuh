@@ -430,6 +430,12 @@ __device__ __forceinline__ bool fluid_point_tri(const mk_snapshot_view &sv, cons
             for (int i = 0; i < 8; i++) prim[i] = q == 0 ? w * v[i] : fma(w, v[i], prim[i]);
         }
     }
+    // cells that are not finite: which sums are infinite and which not a number
+    // follows from the order of the binary64 code's
+    unsigned top = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) top = max(top, (unsigned)__double2hiint(prim[i]) & 0x7fffffffu);
+    if (top >= 0x7ff00000u) return false;
     // the field scaled to order one by a power of two: along the poles of a
     // torus it falls by tens of decades
     const unsigned hB = max(max((unsigned)__double2hiint(prim[5]) & 0x7fffffffu, (unsigned)__double2hiint(prim[6]) & 0x7fffffffu),

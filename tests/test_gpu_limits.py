@@ -50,3 +50,29 @@ def test_synchrotron_default_rescaling_golden(cuda):
     d = golden("synchrotron")
     em, ab = mk.synchrotron_coefficients(*(d[k] for k in ("Ne", "Theta", "B", "pitch", "nu")))
     assert np.max(rel_err(_np(em), d["em_inv1"])) < 1e-11 and np.max(rel_err(_np(ab), d["ab_inv1"])) < 1e-11
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("which", [(0,), (1,), (2,), (3,), (4,), (1, 3), (1, 2, 3), (5,), (5, 6, 7)])
+def test_fluid_with_cells_that_are_not_finite(cuda, orc, which, value):
+    """What such a cell reaches is not a number, as the reference has it."""
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    arrs = make_synthetic_snapshot(nblocks=2, cells_per_block=8, extent=20., bhspin=0.94)
+    rng = np.random.default_rng(6)
+    bad = rng.random(arrs.uov.shape[1:]) < 0.02
+    for i in which:
+        (arrs.uov[i] if i < 5 else arrs.B[i - 5])[bad] = value
+    X = rng.uniform(-19, 19, (3000, 3))
+    X = X[(X ** 2).sum(axis=1) > 4.0]
+    S = np.concatenate([np.zeros((len(X), 1)), X, rng.normal(size=(len(X), 4))], 1)
+    with np.errstate(all="ignore"):
+        ref = orc.OracleSnapshot(arrs).get_fluid_scalars_from_geodesics(S)
+    assert sum(np.isnan(v).sum() for v in ref.values()) > 100
+    g = _model(arrs).get_fluid_scalars_from_geodesics(S)
+    for k, x in g.items():
+        x = _np(x)
+        assert np.array_equal(np.isnan(x), np.isnan(ref[k])), k
+        if k in ("dens", "u", "b"):
+            assert np.array_equal(np.isinf(x), np.isinf(ref[k])), k
+            ok = np.isfinite(ref[k])
+            assert np.max(rel_err(x[ok], ref[k][ok])) < 1e-12, k
