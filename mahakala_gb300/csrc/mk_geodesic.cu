@@ -259,8 +259,8 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
     for (int i = 0; i < 8; i++) s64[i] = s0[8 * p + i];
     bool out = all_f64 || !tri_range(s64);
     const double reh = radius_eh(a);
-    const tri rcap = t_from(capture * reh), resc = t_from(r_escape), hf = t_from(hfrac), h0 = t_from(hmin),
-              h1 = t_from(hmax);
+    const tri rcap = t_near(capture * reh), resc = t_near(r_escape), hf = t_from(hfrac), h0 = t_near(hmin),
+              h1 = t_near(hmax);
     const float near_r = (float)reh + TRI_NEAR;
     TriState s, last;
     tri_state(s64, s);

@@ -1439,8 +1439,8 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
         sh.users[tid] = 0;
     }
     if (tid < EXP_STEPS) {
-        const tri t = t_from(exp2(-(double)tid / EXP_STEPS));
-        sh.exptab[tid] = make_float2(t.h, t.m);
+        const pr t = p_near(exp2(-(double)tid / EXP_STEPS));
+        sh.exptab[tid] = make_float2(t.h, t.l);
     }
     if (tid == 0) sh.drained = 0;
     // The first rays, dealt over the blocks (by eights, so that a warp's rays

@@ -40,7 +40,7 @@ struct PairConsts {
     __device__ __forceinline__ tri t(int i) const { return {c[i * STRIDE], c[(i + 1) * STRIDE], c[(i + 2) * STRIDE]}; }
     __device__ __forceinline__ float f(int i) const { return c[i * STRIDE]; }
     __device__ __forceinline__ void set(int i, double v, int words) {
-        const tri t = t_from(v);
+        const tri t = t_near(v);
         c[i * STRIDE] = t.h;
         c[(i + 1) * STRIDE] = t.m;
         if (words > 2) c[(i + 2) * STRIDE] = t.l;
@@ -152,7 +152,7 @@ __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConst
         bool moved = false;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            const tri left = t_from(__ldg(g + a)), d = t_from(__ldg(g + 3 + a));
+            const tri left = t_from(__ldg(g + a)), d = t_near(__ldg(g + 3 + a));
             const tri s = t_add(x[a], t_neg(left));
             const pr w = {d.h, d.m}, iw = p_rcp(w), t = p_mulr({s.h, s.m}, iw);
             // t + 1 in (1/2, n + 1/2]
@@ -384,8 +384,7 @@ __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConst
             den = p_addr(bx, {f_mul(0.5f, q.h), fmaf(0.5f, q.l, c3)});
         } else {
             if (!(bx.h < 60.0f)) return PS_BINARY64;
-            const tri v = t_from(exp((double)bx.h + (double)bx.l) - 1.0);
-            den = {v.h, v.m};
+            den = p_near(exp((double)bx.h + (double)bx.l) - 1.0);
         }
         const pr ab_m = p_mulr(em_m, p_mulr(den, C.p(at + 6)));
         if (!(ab_m.h >= 1e-30f && ab_m.h <= 1e15f)) return PS_BINARY64;

@@ -341,7 +341,7 @@ __device__ __forceinline__ bool fluid_point_tri(const mk_snapshot_view &sv, cons
             bool moved = false;
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                const tri left = t_from(__ldg(g + i)), d = t_from(__ldg(g + 3 + i));
+                const tri left = t_from(__ldg(g + i)), d = t_near(__ldg(g + 3 + i));
                 const tri v = t_sub(x[i], left), id = t_rcp(d);
                 const pr t = p_mulr({v.h, v.m}, {id.h, id.m});
                 // faces at t = -1/2 and n - 1/2; next to one, the block's own

@@ -193,6 +193,23 @@ MK_HD tri t_from(double v) {
 #endif
     return t_from_cvt(v);
 }
+MK_HD tri t_norm(tri x) {
+    float h, t;
+    tri o;
+    fast_sum_f(x.h, x.m, h, t);
+    fast_sum_f(t, x.l, o.m, o.l);
+    fast_sum_f(h, o.m, o.h, o.m);
+    return o;
+}
+// t_from cuts its words off; these are rounded to the nearest, as the sums
+// below leave theirs: for words that t_less compares, and for constants of
+// which a pair is kept (cut off they were up to 2^-48 too small, the spin of
+// every step among them)
+MK_HD tri t_near(double v) { return t_norm(t_from(v)); }
+MK_HD pr p_near(double v) {
+    const tri t = t_near(v);
+    return {t.h, t.m};
+}
 MK_HD double d_from(float x) {
 #ifdef __CUDA_ARCH__
     const unsigned u = __float_as_uint(x), a = u & 0x7fffffffu;
@@ -237,14 +254,6 @@ MK_HD tri t_sqr(tri x) {
     two_sum_f(e, c, s, t);
     return {p, s, fmaf(x.m, x.m, fmaf(g, x.l, f_add(ce, t)))};
 }
-MK_HD tri t_norm(tri x) {
-    float h, t;
-    tri o;
-    fast_sum_f(x.h, x.m, h, t);
-    fast_sum_f(t, x.l, o.m, o.l);
-    fast_sum_f(h, o.m, o.h, o.m);
-    return o;
-}
 MK_HD tri t_mulr(tri x, tri y) { return t_norm(t_mul(x, y)); }
 
 // 1/x: the pair reciprocal and a Newton step from the triple residual
@@ -276,9 +285,8 @@ struct SpinTri {
 };
 MK_HD SpinTri spin_tri(double a) {
     SpinTri s;
-    const tri t = t_from(a);
-    s.a = {t.h, t.m};
-    s.aa3 = t_from(a * a);
+    s.a = p_near(a);
+    s.aa3 = t_near(a * a);
     s.aa = {s.aa3.h, s.aa3.m};
     return s;
 }
@@ -443,8 +451,7 @@ MK_HD RuleTri rule_tri(double a, double div, double tol) {
     RuleTri o;
     o.reh = t_from(radius_eh(a));
     o.ninv = t_from(-1.0 / div);
-    const tri t = t_from(tol);
-    o.tol = {t.h, t.m};
+    o.tol = p_near(tol);
     return o;
 }
 MK_HD bool rule_dt(tri r, const RuleTri &R, tri &dt, float &d_out, int &why) {

@@ -76,3 +76,63 @@ def test_fluid_with_cells_that_are_not_finite(cuda, orc, which, value):
             assert np.array_equal(np.isinf(x), np.isinf(ref[k])), k
             ok = np.isfinite(ref[k])
             assert np.max(rel_err(x[ok], ref[k][ok])) < 1e-12, k
+
+
+@pytest.mark.parametrize("extent", [20.0, 21.7, 30.1, 47.3])
+def test_fluid_beside_cell_centres(cuda, orc, extent):
+    """Points within float rounding of a cell's centre, either side; cells of
+    like size, so that the oracle's 1e-15 of a weight is 1e-15 of the sum."""
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    arrs = make_synthetic_snapshot(nblocks=4, cells_per_block=8, extent=extent, bhspin=0.94)
+    rng = np.random.default_rng(8)
+    arrs.uov[:] = rng.uniform(1, 2, arrs.uov.shape)
+    arrs.B[:] = rng.uniform(1, 2, arrs.B.shape)
+    d = 2 * extent / 32
+    X = (rng.integers(0, 32, (40000, 3)) + 0.5) * d - extent
+    X += d * rng.uniform(-1.5e-7, 1.5e-7, X.shape)
+    X = X[(X ** 2).sum(axis=1) > 4.0]
+    S = np.concatenate([np.zeros((len(X), 1)), X, rng.normal(size=(len(X), 4))], 1)
+    ref = orc.OracleSnapshot(arrs).get_fluid_scalars_from_geodesics(S)
+    g = _model(arrs).get_fluid_scalars_from_geodesics(S)
+    for k in ("dens", "u", "b"):
+        assert np.nanmax(rel_err(_np(g[k]), ref[k])) < 1e-12, k
+
+
+# thresholds whose first 24 bits, cut, leave more than half a unit behind, and
+# some that do not: the distance decides to its last bits
+@pytest.mark.parametrize("tol", [1e-3, 1e-4, 3e-3, 7.3e-4, 0.011])
+def test_capture_radius_to_the_last_bits(cuda, orc, tol):
+    from mahakala_gb300.geodesics import step_policy, trace
+    eps = np.array([-1e-6, -1e-7, -3e-8, -1e-8, -1e-9, 1e-9, 1e-8, 3e-8, 1e-7, 1e-6])
+    s0 = np.zeros((len(eps), 8))
+    s0[:, 1] = 2.0 + tol * (1.0 + eps)
+    s0[:, 4:6] = (1.0, -0.4)     # outward, traced back
+    o = orc.integrate(s0, 4, 40.0, tol, 0.0)
+    g = trace(s0, 0.0, step_policy(4, 40.0, tol))
+    assert np.array_equal(o["K"] > 0, eps > 0)
+    assert np.array_equal(_np(g["K"]), o["K"]) and np.array_equal(_np(g["why"]), o["why"])
+
+
+@pytest.mark.parametrize("key", ["capture", "r_escape", "hmin", "hmax"])
+def test_fixed_rule_to_the_last_bits(cuda, orc, key):
+    """The fixed-fraction rule's thresholds at 1 +- 1e-8 of the value that
+    decides: stops, and step sizes, on the right side."""
+    from mahakala_gb300.geodesics import step_policy, trace
+    rng = np.random.default_rng(12)
+    for r0 in rng.uniform(20.0, 60.0, 24):
+        s0 = np.zeros((1, 8))
+        s0[:, 1] = r0
+        s0[:, 4:6] = (1.0, 0.9) if key == "capture" else (1.0, -0.9)
+        if key in ("capture", "r_escape"):
+            r1 = orc.trace_fixed(s0, 1, 0.0)["state"][0, 1]
+            value = r1 / 2.0 if key == "capture" else r1
+        else:
+            value = 0.05 * r0
+        for e in (-1e-8, 1e-8):
+            kw = {key: value * (1.0 + e)}
+            if key == "hmin":
+                kw["hmax"] = 100.0
+            o = orc.trace_fixed(s0, 1, 0.0, **kw)
+            g = trace(s0, 0.0, step_policy(1, kind="fixed", **kw))
+            assert _np(g["why"])[0] == o["why"][0], (r0, e)
+            assert np.max(rel_err(_np(g["state"]), o["state"], floor=1e-3)) < 1e-12, (r0, e)
