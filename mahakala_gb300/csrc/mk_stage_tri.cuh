@@ -324,19 +324,25 @@ __device__ __forceinline__ bool fluid_point_tri(const mk_snapshot_view &sv, cons
     // the block and cell
     int c[3], idx[3], near[3], mb = -1;
     tri del[3];
-    bool inside = true;
+    bool inside = true, beside = false;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         const float lo = cst.lo[i], u = (x[i].h - lo) * cst.inv_w[i];
         const float tol = 1e-5f * ((fabsf(lo) + xm) * cst.inv_w[i] + 1.0f);  // of u
         if (u < -tol || u > (float)sv.nb[i] + tol) inside = false;
+        if (fabsf(u - rintf(u)) <= tol) beside = true;
         c[i] = max(0, min((int)u, sv.nb[i] - 1));
     }
     if (inside) {
         const float n = (float)sv.n;
         for (int it = 0;; ++it) {
             mb = table_at(sv, c);
-            if (mb < 0) break;
+            if (mb < 0) {
+                // a place without a block: beside a face of the table the
+                // point may lie across it, in one that is there
+                if (it == 0 && beside) return false;
+                break;
+            }
             const double *g = sv.geom + 6 * (int64_t)mb;
             bool moved = false;
 #pragma unroll

@@ -136,3 +136,32 @@ def test_fixed_rule_to_the_last_bits(cuda, orc, key):
             g = trace(s0, 0.0, step_policy(1, kind="fixed", **kw))
             assert _np(g["why"])[0] == o["why"][0], (r0, e)
             assert np.max(rel_err(_np(g["state"]), o["state"], floor=1e-3)) < 1e-12, (r0, e)
+
+
+def _without_block(arrs, m):
+    import copy
+    out, keep = copy.copy(arrs), np.arange(len(arrs.Levels)) != m
+    out.uov, out.B = arrs.uov[:, keep], arrs.B[:, keep]
+    for k in ("x1v", "x2v", "x3v", "x1f", "x2f", "x3f", "LogicalLocations", "Levels"):
+        setattr(out, k, np.asarray(getattr(arrs, k))[keep])
+    return out
+
+
+def test_fluid_beside_a_missing_block(cuda, orc):
+    """Points within float rounding of a block that the snapshot lacks."""
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    arrs = make_synthetic_snapshot(nblocks=4, cells_per_block=8, extent=20., bhspin=0.94)
+    m = int(np.flatnonzero((np.asarray(arrs.LogicalLocations) == (0, 1, 2)).all(axis=1))[0])
+    arrs = _without_block(arrs, m)      # x in (-20, -10], y in (-10, 0], z in (0, 10]
+    rng = np.random.default_rng(9)
+    X = rng.uniform((-20, -10, 0), (-10, 0, 10), (4000, 3))
+    off = rng.choice([-1, 1], 4000) * 10.0 ** rng.uniform(-9, -6, 4000)
+    side, axis = rng.integers(0, 2, 4000), rng.integers(0, 3, 4000)
+    face = np.array([[-20, -10], [-10, 0], [0, 10]], float)
+    X[np.arange(4000), axis] = face[axis, side] + off
+    X = X[X[:, 0] > -20]
+    S = np.concatenate([np.zeros((len(X), 1)), X, rng.normal(size=(len(X), 4))], 1)
+    ref = orc.OracleSnapshot(arrs).get_fluid_scalars_from_geodesics(S)
+    g = _model(arrs).get_fluid_scalars_from_geodesics(S)
+    for k in ("dens", "u", "b"):
+        assert np.nanmax(rel_err(_np(g[k]), ref[k])) < 1e-12, k
