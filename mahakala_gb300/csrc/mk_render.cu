@@ -1260,11 +1260,11 @@ render_zone_kernel(const mk_request *__restrict__ reqs, const mk_snapshot_view *
 }
 
 // A sample in binary64 for render_tri_kernel: blocks kept in binary64 (ghosts
-// averaged from finer cells) and primitives outside the pairs' range.
-__device__ __noinline__ void coefficients_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
+// averaged from finer cells), primitives outside the pairs' range, and places
+// that only the binary64 lookup tells apart.  false: outside the snapshot
+__device__ __noinline__ bool coefficients_fp64(const mk_request &R, const mk_snapshot_view &sv, const double s[8],
                                                double em[MK_MAX_NU], double ab[MK_MAX_NU]) {
-    for (int ch = 0; ch < MK_MAX_NU; ch++) em[ch] = ab[ch] = 0.0;
-    emission_fp64(R, sv, s, kerr_point(s[1], s[2], s[3], R.camera.bhspin), em, ab);
+    return emission_fp64(R, sv, s, kerr_point(s[1], s[2], s[3], R.camera.bhspin), em, ab);
 }
 
 // MK_FP64: every ray of the job, start to end, state in 72 bits, geodesic and
@@ -1378,7 +1378,7 @@ __device__ __noinline__ void tri_sample(TriShared &sh, int e, const mk_request *
     }
     const int nnu = sh.nnu[slot];
     PairCoeff co[MK_MAX_NU];
-    const int got = sample_pair(sh.view[slot], C, nnu, x, k, C.p(PC_A), m, sh.exptab, co);
+    int got = sample_pair(sh.view[slot], C, nnu, x, k, C.p(PC_A), m, sh.exptab, co);
     if (got != PS_OUTSIDE) {
         const pr w = p_neg(p_mulr({sh.v[TV_DT][e], sh.v[TV_DT + 1][e]}, C.p(PC_LUNIT)));
         double e64[MK_MAX_NU], a64[MK_MAX_NU];
@@ -1390,12 +1390,12 @@ __device__ __noinline__ void tri_sample(TriShared &sh, int e, const mk_request *
             for (int i = 0; i < 3; i++) s64[1 + i] = t_to(x[i]);
 #pragma unroll
             for (int i = 0; i < 4; i++) s64[4 + i] = d_from(k[i].h) + d_from(k[i].l);
-            coefficients_fp64(R, snaps[R.snapshot], s64, e64, a64);
+            if (!coefficients_fp64(R, snaps[R.snapshot], s64, e64, a64)) got = PS_OUTSIDE;
         }
         const int step = __float_as_int(sh.v[TV_STEP][e]);
 #pragma unroll
         for (int ch = 0; ch < MK_MAX_NU; ch++) {
-            if (ch >= nnu) break;
+            if (ch >= nnu || got == PS_OUTSIDE) break;
             double wem, tau;
             if (got == PS_BINARY64) {
                 const double wd = d_from(w.h) + d_from(w.l);

@@ -122,27 +122,51 @@ __device__ __forceinline__ void pair_consts_sample(const mk_request &R, const mk
 // The snapshot's fields a sample reads.
 struct SampleView {
     const float *blocks;
-    const double *geom;
+    const double *geom, *faces;
     const int32_t *table, *block64;  // block64: null if no block is kept in binary64
     int nb[3], n;
 };
 __device__ __forceinline__ SampleView sample_view(const mk_snapshot_view &sv) {
-    return {sv.blocks, sv.geom, sv.table, sv.blocks64 ? sv.block64 : nullptr, {sv.nb[0], sv.nb[1], sv.nb[2]}, sv.n};
+    return {sv.blocks, sv.geom, sv.faces, sv.table, sv.blocks64 ? sv.block64 : nullptr, {sv.nb[0], sv.nb[1], sv.nb[2]}, sv.n};
 }
 
-// The cell of x: the block whose faces enclose it (left < x <= right, to 48
-// bits) and the ghost-shifted index and offset in it (locate_fast).  The
-// candidate comes from the float coordinate; its own cell coordinate t, faces
-// at 1/2 and n + 1/2, decides and moves it across a face it lies beyond.
+// On which side of a block's faces at f[0] and f[1] x lies (left < x <= right):
+// 0 between them.  The difference of triples has its sign to the state's 72
+// bits.
+static __device__ __noinline__ int face_side(const double *f, tri x) {
+    if (t_sub(x, t_from(__ldg(f))).h <= 0.0f) return -1;
+    return t_sub(x, t_from(__ldg(f + 1))).h > 0.0f ? 1 : 0;
+}
+// Whether block mb and its neighbour across the left (sides bit 2a) or right
+// (bit 2a + 1) face of each axis share that face to the bit; where they do
+// not, both or neither may hold a point next to it.
+static __device__ __noinline__ bool faces_shared(const SampleView &sv, int mb, int c0, int c1, int c2, unsigned sides) {
+    for (int i = 0; i < 6; i++) {
+        if (!((sides >> i) & 1u)) continue;
+        const int step = (i & 1) ? 1 : -1;
+        const int o[3] = {c0 + (i / 2 == 0 ? step : 0), c1 + (i / 2 == 1 ? step : 0), c2 + (i / 2 == 2 ? step : 0)};
+        const int nb = table_at(sv, o);
+        if (nb >= 0 && __ldg(sv.faces + 6 * (int64_t)mb + i) != __ldg(sv.faces + 6 * (int64_t)nb + (i ^ 1))) return false;
+    }
+    return true;
+}
+
+// The cell of x: the block whose faces enclose it (left < x <= right) and the
+// ghost-shifted index and offset in it (locate_fast).  The candidate comes
+// from the float coordinate; its own cell coordinate t, faces at -1/2 and n -
+// 1/2, decides and moves it across a face it lies beyond, or next to one
+// (|e| < 1e-9 of a cell; t is good to 1e-11) the face itself.  -1: outside
+// the snapshot; -2: left to the binary64 lookup (at a face that two blocks do
+// not share to the bit).
 template <int STRIDE>
 __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConsts<STRIDE> &C, const tri x[3],
                                            int idx[3], pr del[3]) {
     int c[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float lo = C.f(PC_BOX + a);
-        if (!(x[a].h >= lo && x[a].h <= C.f(PC_BOX + 3 + a))) return -1;
-        c[a] = max(0, min((int)((x[a].h - lo) * C.f(PC_INVW + a)), sv.nb[a] - 1));
+        const float lo = C.f(PC_BOX + a), hi = C.f(PC_BOX + 3 + a), iw = C.f(PC_INVW + a), u = (x[a].h - lo) * iw;
+        if (!(x[a].h >= lo && x[a].h <= hi)) return -1;
+        c[a] = max(0, min((int)u, sv.nb[a] - 1));
     }
     const float n = (float)sv.n;
     for (int it = 0; it < 4; ++it) {
@@ -150,14 +174,20 @@ __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConst
         if (mb < 0) return -1;
         const double *g = sv.geom + 6 * (int64_t)mb;
         bool moved = false;
+        unsigned sides = 0;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             const tri left = t_from(__ldg(g + a)), d = t_near(__ldg(g + 3 + a));
             const tri s = t_add(x[a], t_neg(left));
             const pr w = {d.h, d.m}, iw = p_rcp(w), t = p_mulr({s.h, s.m}, iw);
-            // t + 1 in (1/2, n + 1/2]
-            if (t.h < -0.5f || (t.h == -0.5f && t.l <= 0.0f)) { --c[a]; moved = true; }
-            else if (t.h > n - 0.5f || (t.h == n - 0.5f && t.l > 0.0f)) { ++c[a]; moved = true; }
+            const float e0 = f_add(f_add(t.h, 0.5f), t.l), e1 = f_add(f_sub(t.h, n - 0.5f), t.l);
+            int side = e0 < 0.0f ? -1 : (e1 > 0.0f ? 1 : 0);
+            if (fminf(fabsf(e0), fabsf(e1)) < 1e-9f) {
+                side = face_side(sv.faces + 6 * (int64_t)mb + 2 * a, x[a]);
+                sides |= (fabsf(e0) < fabsf(e1) ? 1u : 2u) << (2 * a);
+            }
+            c[a] += side;
+            if (side) moved = true;
             float fl = floorf(t.h);
             if (fl == t.h && t.l < 0.0f) fl -= 1.0f;
             fl = fminf(fmaxf(fl, -1.0f), n - 1.0f);
@@ -169,9 +199,9 @@ __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConst
             const pr u = p_norm({uh, f_add(f_add(ul, fmaf(-fl, d.m, s.m)), -e)});
             del[a] = p_mulr(u, iw);
         }
-        if (!moved) return mb;
+        if (!moved) return sides && !faces_shared(sv, mb, c[0], c[1], c[2], sides) ? -2 : mb;
     }
-    return -1;
+    return -2;
 }
 
 // exp(-x) for x >= 0 as m 2^-e, m in [1/2, 1]: x = (32 e + j) ln2/32 - r, the
@@ -216,7 +246,8 @@ enum { PS_OUTSIDE = 0, PS_SAMPLED = 1, PS_BINARY64 = 2 };
 // 1/(r^2 + a^2) there.  PS_SAMPLED: co holds the
 // invariant coefficients of every frequency; PS_BINARY64: the point lies in
 // the snapshot, in a block kept in binary64 or at primitives outside the
-// pairs' range, and the caller samples it in binary64.
+// pairs' range, or where only the binary64 lookup tells (locate_pair); the
+// caller samples it in binary64.
 template <int STRIDE>
 __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConsts<STRIDE> &C, int nnu,
                                            const tri x[3], const pr k[4], pr a, const pr m[4], const float2 *tab,
@@ -224,7 +255,7 @@ __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConst
     int idx[3];
     pr del[3];
     const int mb = locate_pair(sv, C, x, idx, del);
-    if (mb < 0) return PS_OUTSIDE;
+    if (mb < 0) return mb == -2 ? PS_BINARY64 : PS_OUTSIDE;
     if (sv.block64 && __ldg(sv.block64 + mb) >= 0) return PS_BINARY64;
     // Each primitive as the sum of eight weights times cells; one copy of the
     // code for the four (z, y) neighbours (see tri_step), a neighbour's cells

@@ -165,3 +165,30 @@ def test_fluid_beside_a_missing_block(cuda, orc):
     g = _model(arrs).get_fluid_scalars_from_geodesics(S)
     for k in ("dens", "u", "b"):
         assert np.nanmax(rel_err(_np(g[k]), ref[k])) < 1e-12, k
+
+
+@pytest.mark.parametrize("extent", [20.0, 21.7, 30.1, 47.3])
+def test_fp64_image_along_a_refinement_face(cuda, orc, extent):
+    """A column of rays that run in the plane of a face between coarse and
+    refined blocks: the point belongs to the block below (left < x <= right)."""
+    from mahakala_gb300.grmhd.synthetic import make_multilevel_snapshot
+    arrs = make_multilevel_snapshot(nblocks=2, cells_per_block=8, extent=extent, bhspin=0.0,
+                                    refine=[(0, i, 1, k) for i in (0, 1) for k in (0, 1)])
+    s0 = orc.initialize_geodesics_at_camera(0.0, 60.0, 1000, -10.0, 10.0, 5)
+    # (the centre has no direction)
+    assert (s0[10:15, 2] == 0).all() and (np.nan_to_num(s0[10:15, 6]) == 0).all()
+    p = _image_parity(orc, arrs, 20.0, 5, 0.0)
+    assert p["steps_equal"] and p["max_pixel_rel_err"] <= 1e-8, p
+
+
+def _image_parity(orc, arrs, fov, res, spin, nu=230e9, **kw):
+    from mahakala_gb300.images import RenderRequest, render_requests
+    req = RenderRequest(_model(arrs), camera_inclination=60.0, fov=fov, resolution=res, bhspin=spin,
+                        observing_frequency=nu, **dict(KW, **kw))
+    img = _np(render_requests([req], with_steps=True)[0]).reshape(1, -1)
+    s0 = orc.initialize_geodesics_at_camera(spin, 60.0, 1000, -fov / 2, fov / 2, res)
+    osnap = orc.OracleSnapshot(arrs, bhspin=spin)
+    with np.errstate(all="ignore"):
+        ref, rsteps = orc.render_rays(osnap, s0, observing_frequency=nu, **dict(KW, **kw))
+        pert, psteps = orc.render_rays(osnap, orc.perturbed(s0), observing_frequency=nu, **dict(KW, **kw))
+    return orc.image_parity(img, _np(req.out["nsteps"]), ref, rsteps, pert, psteps)
