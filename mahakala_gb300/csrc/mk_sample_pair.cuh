@@ -156,22 +156,25 @@ static __device__ __noinline__ bool faces_shared(const SampleView &sv, int mb, i
 // from the float coordinate; its own cell coordinate t, faces at -1/2 and n -
 // 1/2, decides and moves it across a face it lies beyond, or next to one
 // (|e| < 1e-9 of a cell; t is good to 1e-11) the face itself.  -1: outside
-// the snapshot; -2: left to the binary64 lookup (at a face that two blocks do
-// not share to the bit).
+// the snapshot; -2: left to the binary64 lookup (beside a place without a
+// block, or at a face that two blocks do not share to the bit).
 template <int STRIDE>
 __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConsts<STRIDE> &C, const tri x[3],
                                            int idx[3], pr del[3]) {
     int c[3];
+    bool beside = false;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         const float lo = C.f(PC_BOX + a), hi = C.f(PC_BOX + 3 + a), iw = C.f(PC_INVW + a), u = (x[a].h - lo) * iw;
         if (!(x[a].h >= lo && x[a].h <= hi)) return -1;
+        // within the box's margin (1e-5 of its coordinates) and a rounding of a face
+        if (fabsf(u - rintf(u)) <= 2e-5f * (fabsf(lo) + fabsf(hi)) * iw) beside = true;
         c[a] = max(0, min((int)u, sv.nb[a] - 1));
     }
     const float n = (float)sv.n;
     for (int it = 0; it < 4; ++it) {
         const int mb = table_at(sv, c);
-        if (mb < 0) return -1;
+        if (mb < 0) return it == 0 && beside ? -2 : -1;
         const double *g = sv.geom + 6 * (int64_t)mb;
         bool moved = false;
         unsigned sides = 0;

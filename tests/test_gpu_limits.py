@@ -192,3 +192,19 @@ def _image_parity(orc, arrs, fov, res, spin, nu=230e9, **kw):
         ref, rsteps = orc.render_rays(osnap, s0, observing_frequency=nu, **dict(KW, **kw))
         pert, psteps = orc.render_rays(osnap, orc.perturbed(s0), observing_frequency=nu, **dict(KW, **kw))
     return orc.image_parity(img, _np(req.out["nsteps"]), ref, rsteps, pert, psteps)
+
+
+@pytest.mark.parametrize("missing,off", [("y > 0", 1e-8), ("y < 0", -1e-8), ("y > 0", 3e-7)])
+def test_fp64_image_beside_missing_blocks(cuda, orc, missing, off):
+    """A column of rays in a plane beside the face where a snapshot ends."""
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    arrs = make_synthetic_snapshot(nblocks=4, cells_per_block=8, extent=20., bhspin=0.0)
+    arrs.x2f, arrs.x2v = arrs.x2f + off, arrs.x2v + off
+    # one far block of the missing side keeps the table's extent
+    loc = np.asarray(arrs.LogicalLocations)
+    gone = (loc[:, 1] >= 2) if missing == "y > 0" else (loc[:, 1] < 2)
+    gone &= ~(loc == ((3, 3, 0) if missing == "y > 0" else (3, 0, 0))).all(axis=1)
+    for m in np.flatnonzero(gone)[::-1]:
+        arrs = _without_block(arrs, m)
+    p = _image_parity(orc, arrs, 20.0, 5, 0.0, nu=1e9, mass_scale=1e25)
+    assert p["steps_equal"] and p["max_pixel_rel_err"] <= 1e-8, p
