@@ -1656,7 +1656,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                 if (w < warp) rank += sh.alive[w];
                 rays += sh.alive[w];
             }
-            const int need = 4 * ((rays + 127) / 128);
+            const int need = warps_for(rays, warps);
             if (need < warps) {
                 warps = need;
                 float *mv = &sh.v[0][0];

@@ -119,6 +119,14 @@ __device__ __forceinline__ void pair_consts_sample(const mk_request &R, const mk
         }
 }
 
+// The warps, of `warps`, that a block's last rays move into: one a
+// sub-partition as long as they fit.  With no ray left there is nothing to
+// move, and the block's loop still divides by what it has.
+__host__ __device__ constexpr int warps_for(int rays, int warps) {
+    const int need = 4 * ((rays + 127) / 128);
+    return rays > 0 && need < warps ? need : warps;
+}
+
 // The snapshot's fields a sample reads.
 struct SampleView {
     const float *blocks;
