@@ -1340,7 +1340,7 @@ __device__ __noinline__ int tri_acquire(TriShared &sh, int rq, const mk_request 
         if (was == -1) {
             const mk_request &R = reqs[rq];
             const PairConsts<TRI_REQS> C = {&sh.c[0][i]};
-            sh.nnu[i] = R.nnu;
+            sh.nnu[i] = min(R.nnu, MK_MAX_NU);  // the rows of the block's sums
             sh.nmax[i] = R.policy.nmax;
             sh.rows[i] = R.rows_dt ? (int)min((long long)R.rows, 0x7fffffffll) : 0;
             sh.view[i] = sample_view(snaps[R.snapshot]);

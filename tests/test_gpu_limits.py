@@ -208,3 +208,23 @@ def test_fp64_image_beside_missing_blocks(cuda, orc, missing, off):
         arrs = _without_block(arrs, m)
     p = _image_parity(orc, arrs, 20.0, 5, 0.0, nu=1e9, mass_scale=1e25)
     assert p["steps_equal"] and p["max_pixel_rel_err"] <= 1e-8, p
+
+
+def test_request_of_too_many_frequencies(cuda):
+    """A request in device memory that names more than MK_MAX_NU frequencies
+    (the Python layer refuses one) is rendered in the first MK_MAX_NU."""
+    import ctypes
+    from mahakala_gb300 import _lib
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    from mahakala_gb300.images import PreparedRender, RenderRequest
+    arrs = make_synthetic_snapshot(nblocks=4, cells_per_block=8, extent=20., bhspin=0.94)
+    nus = [86e9, 150e9, 230e9, 345e9]
+    prep = PreparedRender([RenderRequest(_model(arrs), observing_frequency=nus, resolution=9, fov=20.0, **KW)])
+    want = prep.launch()[0].clone()
+    table = _lib.Request.from_buffer_copy(prep.table_bytes)
+    for nnu in (_lib.MK_MAX_NU + 1, 1000):
+        table.nnu = nnu
+        prep.images[0].zero_()
+        prep.reqs_dev.copy_(torch.frombuffer(bytearray(ctypes.string_at(ctypes.addressof(table), ctypes.sizeof(table))),
+                                             dtype=torch.uint8))
+        assert torch.equal(torch.nan_to_num(prep.launch()[0], nan=-1.0), torch.nan_to_num(want, nan=-1.0))
