@@ -31,10 +31,6 @@ __global__ void camera_points_kernel(const double *__restrict__ xs, const double
     for (int i = 0; i < 8; i++) s0[8 * p + i] = s[i];
 }
 
-// Ranges in which the triples (mk_tri.cuh) hold every intermediate with all
-// its words inside the float range; a ray outside them is integrated in
-// binary64 from its start (integrate_*_f64).
-constexpr float TRI_MAX_R = 1e6f, TRI_MAX_K = 1e12f, TRI_MIN_K = 1e-6f;
 // distance to the horizon below which a step's accelerations are binary64
 // (see mk_tri.cuh)
 constexpr float TRI_NEAR = 0.1f;
@@ -44,13 +40,6 @@ __device__ __forceinline__ bool tri_range(const double s[8]) {
     const double x = fmax(fmax(fabs(s[1]), fabs(s[2])), fabs(s[3]));
     return fabs(s[0]) <= TRI_MAX_R && x <= TRI_MAX_R && k <= TRI_MAX_K && k >= TRI_MIN_K;
 }
-// true out of range or at NaN: a step over the horizon toward r = 0 (the
-// fixed-fraction rule's) overflows floats before doubles
-__device__ __forceinline__ bool tri_left_range(const TriState &s, float r) {
-    const float k = (fabsf(s.K[0].h) + fabsf(s.K[1].h)) + (fabsf(s.K[2].h) + fabsf(s.K[3].h));
-    return !(r <= TRI_MAX_R && k <= TRI_MAX_K);
-}
-
 // one RK4 step of the triple state by its binary64 increment (s: the state)
 __device__ __noinline__ void rk4_step_near(TriState &st, const double s[8], double dt, double a) {
     double d1[4], sum[8];

@@ -580,9 +580,18 @@ __device__ __forceinline__ void fill_req_f32(const mk_request &R, const mk_snaps
 
 
 
+// in place of a ray's first intensity: render_tri_kernel has left the ray
+constexpr unsigned long long RAY_LEFT = 0x7ff46c6566740000ull;
+__device__ __noinline__ bool left_to_fp64(const mk_request *__restrict__ reqs, int nreq, long long ray) {
+    const mk_request &R = reqs[find_request(reqs, nreq, ray)];
+    if (!pair_request(R)) return true;
+    const double I = R.image[fetch_pixel(R.camera, ray - R.ray_offset)];
+    return (unsigned long long)__double_as_longlong(I) == RAY_LEFT;
+}
+
 // Binary64 render.  SRC_CAMERA: the rays, start to end, of MK_FP64 requests
 // outside the triples' range (pair_request; render_tri_kernel takes the
-// others).  SRC_QUEUE: mixed-form phase B over the FP64 queue; rays leaving R_TURN
+// others), and rays that it marked.  SRC_QUEUE: mixed-form phase B over the FP64 queue; rays leaving R_TURN
 // outward go to the FP32 queue.  T is the geodesic arithmetic: double, or
 // dd (double-float pairs) for the MK_MIXED_DF variant of phase B.
 template <int SRC, typename T = double>
@@ -615,8 +624,7 @@ render_fp64_kernel(const mk_request *__restrict__ reqs, int nreq, long long tota
         const long long idx = fetch(lane_works && !active && !exhausted, counter, total);
         if (idx == -1) exhausted = true;
         if (!lane_works) exhausted = true;
-        if (idx >= 0 && (SRC != SRC_CAMERA || (ray_in_request(reqs, nreq, idx) &&
-                                               !pair_request(reqs[find_request(reqs, nreq, idx)])))) {
+        if (idx >= 0 && (SRC != SRC_CAMERA || (ray_in_request(reqs, nreq, idx) && left_to_fp64(reqs, nreq, idx)))) {
             if (SRC == SRC_CAMERA) {
                 rq = find_request(reqs, nreq, idx);
                 pix = fetch_pixel(reqs[rq].camera, idx - reqs[rq].ray_offset);
@@ -1267,6 +1275,44 @@ __device__ __noinline__ bool coefficients_fp64(const mk_request &R, const mk_sna
     return emission_fp64(R, sv, s, kerr_point(s[1], s[2], s[3], R.camera.bhspin), em, ab);
 }
 
+// The rest of a ray in binary64, from its state after `steps` steps, as
+// render_fp64_kernel takes it: for rays whose next step leaves the range of
+// the triples (over the horizon, mostly; tri_left_range).  Why it ended.
+__device__ __noinline__ int rest_fp64(const mk_request &R, const mk_snapshot_view &sv, const float start[21],
+                                      int64_t pix, int &steps, int &nsamples, double I[MK_MAX_NU],
+                                      double P[MK_MAX_NU], double &max_tau) {
+    const double a = R.camera.bhspin, reh = radius_eh(a);
+    double s[8], d1[4];
+    s[0] = 0.0;  // x^0 is not read
+#pragma unroll
+    for (int i = 0; i < 7; i++) s[1 + i] = t_to({start[3 * i], start[3 * i + 1], start[3 * i + 2]});
+    KerrPoint<double> m;
+    kerr_accel(s[1], s[2], s[3], s[4], s[5], s[6], s[7], a, d1[0], d1[1], d1[2], d1[3], m);
+    int why;
+    double dt = reference_dt(m.r, reh, R.policy.div, R.policy.tol, why);
+    if (dt == 0.0 || R.policy.nmax < 2) return why == MK_RAY_ACTIVE ? MK_RAY_MAXSTEPS : why;
+    for (;;) {
+        double nw[8], dn[4];
+        rk4_step_k1(s, d1, dt, a, nw);
+        kerr_accel(nw[1], nw[2], nw[3], nw[4], nw[5], nw[6], nw[7], a, dn[0], dn[1], dn[2], dn[3], m);
+        const double dtn = reference_dt(m.r, reh, R.policy.div, R.policy.tol, why);
+        if (dtn == 0.0) return why;  // the step is rejected
+#pragma unroll
+        for (int i = 0; i < 8; i++) s[i] = nw[i];
+#pragma unroll
+        for (int i = 0; i < 4; i++) d1[i] = dn[i];
+        ++steps;
+        int64_t row = -1;
+        if (R.rows_dt && steps < R.rows) {
+            row = steps;
+            R.rows_dt[(int64_t)(steps - 1) * request_pixels(R.camera) + pix] = dt;
+        }
+        sample_fp64(R, sv, s, m, dt, I, P, nsamples, max_tau, pix, R.rows_em ? row : -1);
+        dt = dtn;
+        if (steps >= R.policy.nmax - 1) return MK_RAY_MAXSTEPS;
+    }
+}
+
 // MK_FP64: every ray of the job, start to end, state in 72 bits, geodesic and
 // sampling in float pairs, transfer sums in binary64 (mk_tri.cuh,
 // mk_sample_pair.cuh say why and to what accuracy).
@@ -1299,6 +1345,15 @@ constexpr int TRI_MSGS = 1536;  // messages of a phase; its steps are as many as
 constexpr int TRI_STEPS = TRI_MSGS / 128;  // with the fewest warps, four
 constexpr int TRI_REQS = 32;    // requests a block has rays of at a time
 constexpr int TRI_REFILL = 4;   // idle lanes of a warp that take new rays together
+constexpr int TRI_LOST = -1;    // why: the ray ends in binary64 (rest_fp64)
+constexpr int TRI_LOST_MAX = 32;
+// a ray that left the triples' range: its state before that step, its sums
+struct LostRay {
+    float s[21];  // x^1..x^3, k^0..k^3, three words each
+    int rq, steps, samples;
+    long long ray, tau;
+    double I[MK_MAX_NU], P[MK_MAX_NU];
+};
 // message words: x^1..x^3 (h m l), k^0..k^3 (h l), r f l3 1/(r^2+a^2) (h l),
 // dt (h l), thread of the ray, its step; the sample's reply lies over the first:
 // per frequency w j and w alpha as doubles
@@ -1320,7 +1375,8 @@ struct TriShared {
     int count[TRI_WARPS], alive[TRI_WARPS];
     float2 exptab[EXP_STEPS];
     long long total, rest;  // rays, and those of them handed out by the counter
-    int chunk, drained;
+    int chunk, drained, nlost;
+    LostRay lost[TRI_LOST_MAX];
 };
 // words of a ray moved to another thread
 constexpr int TRI_MOVE = 39 + 4 * MK_MAX_NU;
@@ -1442,7 +1498,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
         const pr t = p_near(exp2(-(double)tid / EXP_STEPS));
         sh.exptab[tid] = make_float2(t.h, t.l);
     }
-    if (tid == 0) sh.drained = 0;
+    if (tid == 0) sh.drained = sh.nlost = 0;
     // The first rays, dealt over the blocks (by eights, so that a warp's rays
     // stay neighbours), since the first are the longest; the rest by the
     // counter.  A block's rays are spread over its sub-partitions before they
@@ -1467,6 +1523,11 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
 
     bool active = false, fresh = false, ended = false;
     int slot = 0, steps = 0;
+    // The state before a step within 1 M of the horizon, or of a ray thrown out
+    // from inside it (|k| > 64, elsewhere a few), in local memory: where the
+    // step leaves the triples' range the ray ends in binary64 from there, when
+    // the block has no other left.  No other step can leave it.
+    float kept[21];
     TriState s;
     TriPoint q;
     tri dt = {0.0f, 0.0f, 0.0f};
@@ -1481,6 +1542,15 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
             bool sample = false;
             if (active || fresh) {
                 const PairConsts<TRI_REQS> C = {&sh.c[0][slot]};
+                if (fresh || dt.h > C.f(PC_NINV) || tri_sum_k(s) > 64.0f) {  // dt = -(r - r_EH) / div
+#pragma unroll
+                    for (int i = 0; i < 7; i++) {
+                        const tri t = i < 3 ? s.X[1 + i] : s.K[i - 3];
+                        kept[3 * i] = t.h;
+                        kept[3 * i + 1] = t.m;
+                        kept[3 * i + 2] = t.l;
+                    }
+                }
                 // the new state, and with it the next step's first stage,
                 // which gives r and the metric there for the rule and the sample
                 tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), fresh);
@@ -1488,7 +1558,16 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                 float d;
                 int why;
                 const bool go = rule_dt(q.r, rule, dt, d, why);
-                if (fresh) {
+                const float k = tri_sum_k(s);
+                if (fresh && k != k) {  // no direction: its first step would be NaN
+                    fresh = active = false;
+                    ended = true;
+                    sh.why[tid] = !go ? why : (sh.nmax[slot] >= 2 ? MK_RAY_NAN : MK_RAY_MAXSTEPS);
+                } else if (tri_left_range(s, q.r.h)) {
+                    fresh = active = false;
+                    ended = true;
+                    sh.why[tid] = TRI_LOST;
+                } else if (fresh) {
                     fresh = false;
                     // stopped before its first step (reference K = 0), or N < 2
                     // leaves no row pair for the transfer solve
@@ -1508,7 +1587,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                                   fetch_pixel(R.camera, sh.ray[tid] - R.ray_offset)] = t_to(used);
                     }
                 }
-                if (!active) {
+                if (!active && !ended) {
                     ended = true;
                     sh.why[tid] = go ? MK_RAY_MAXSTEPS : why;
                 }
@@ -1543,7 +1622,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
         }
         if (lane == 0) sh.count[warp] = count;
         if (tid == 0) sh.chunk = 0;
-        if (!__syncthreads_or(active || fresh || ended || waiting || !exhausted)) return;
+        if (!__syncthreads_or(active || fresh || ended || waiting || !exhausted)) break;
 
         // ---- new rays for idle lanes, a few at a time (a camera ray is ~20 k
         // cycles of the warp, in binary64), while other warps sample
@@ -1620,8 +1699,28 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
             double I[MK_MAX_NU];
 #pragma unroll
             for (int ch = 0; ch < MK_MAX_NU; ch++) I[ch] = sh.I[ch][tid];
-            finish_ray(R, fetch_pixel(R.camera, sh.ray[tid] - R.ray_offset), I, steps, sh.why[tid],
-                       sh.samples[tid], __longlong_as_double(sh.tau[tid]), ws);
+            const int64_t pix = fetch_pixel(R.camera, sh.ray[tid] - R.ray_offset);
+            const int at = sh.why[tid] == TRI_LOST ? atomicAdd(&sh.nlost, 1) : -1;
+            if (at < 0) {
+                finish_ray(R, pix, I, steps, sh.why[tid], sh.samples[tid], __longlong_as_double(sh.tau[tid]), ws);
+            } else if (at < TRI_LOST_MAX) {
+                LostRay &l = sh.lost[at];
+#pragma unroll
+                for (int i = 0; i < 21; i++) l.s[i] = kept[i];
+                l.rq = sh.rq[slot];
+                l.steps = steps;
+                l.samples = sh.samples[tid];
+                l.ray = sh.ray[tid];
+                l.tau = sh.tau[tid];
+#pragma unroll
+                for (int ch = 0; ch < MK_MAX_NU; ch++) {
+                    l.I[ch] = I[ch];
+                    l.P[ch] = sh.P[ch][tid];
+                }
+            } else {  // more than the block has room for: from its start
+                R.image[pix] = __longlong_as_double((long long)RAY_LEFT);
+                atomicAdd(&ws->odd_rays, 1ull);
+            }
             tri_release(sh, slot);
         }
         if (const int nslot = sh.nslot[tid]; nslot >= 0) {
@@ -1709,6 +1808,17 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                 __syncthreads();
             }
         }
+    }
+
+    // the rays that left the triples' range, a lane each
+    __syncthreads();
+    if (tid < min(sh.nlost, TRI_LOST_MAX)) {
+        LostRay &l = sh.lost[tid];
+        const mk_request &R = reqs[l.rq];
+        const int64_t pix = fetch_pixel(R.camera, l.ray - R.ray_offset);
+        double tau = __longlong_as_double(l.tau);
+        const int why = rest_fp64(R, snaps[R.snapshot], l.s, pix, l.steps, l.samples, l.I, l.P, tau);
+        finish_ray(R, pix, l.I, l.steps, why, l.samples, tau, ws);
     }
 }
 

@@ -228,3 +228,22 @@ def test_request_of_too_many_frequencies(cuda):
         prep.reqs_dev.copy_(torch.frombuffer(bytearray(ctypes.string_at(ctypes.addressof(table), ctypes.sizeof(table))),
                                              dtype=torch.uint8))
         assert torch.equal(torch.nan_to_num(prep.launch()[0], nan=-1.0), torch.nan_to_num(want, nan=-1.0))
+
+
+# a step over the horizon (here the rule stops this far above it) overflows
+# floats before doubles; the last: more such rays than a block has room for
+@pytest.mark.parametrize("spin,tol,div,half,res", [(-0.9, 1e-4, 40.0, 10.0, 48), (0.5, 1e-6, 40.0, 10.0, 48),
+                                                   (0.5, 1e-8, 40.0, 10.0, 48), (0.94, 1e-8, 40.0, 10.0, 48),
+                                                   (0.5, 1e-8, 10.0, 5.0, 200)])
+def test_fp64_image_stop_reasons_at_the_horizon(cuda, orc, spin, tol, div, half, res):
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    from mahakala_gb300.images import RenderRequest, render_requests
+    arrs = make_synthetic_snapshot(nblocks=2, cells_per_block=8, extent=20., bhspin=0.94)
+    s0 = orc.initialize_geodesics_at_camera(spin, 60.0, 1000, -half, half, res)
+    o = orc.integrate(s0, 4000, div, tol, spin)
+    req = RenderRequest(_model(arrs), camera_inclination=60.0, fov=2 * half, resolution=res, bhspin=spin, tol=tol,
+                        div=div, **dict(KW, max_nsteps=4000))
+    render_requests([req], with_steps=True)
+    steps, why = _np(req.out["nsteps"]).reshape(-1), _np(req.out["status"]).reshape(-1)
+    # (which side of the horizon a last step lands on may turn on a rounding: 2 rays in 10^4)
+    assert (steps != o["K"]).sum() + (why != o["why"]).sum() <= 2e-4 * len(s0)
