@@ -415,7 +415,11 @@ __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConst
         int e;
         const pr E = p_exp_neg(x3, tab, e);
         e -= ed - shift;
-        const pr em_m = p_mulr(p_mulr(C.p(at), base_em), p_mulr(p_mulr(t, t), E));
+        // the low word of a product below 1e-28 starts to fall among the floats'
+        // last digits, before t^2 lifts it again
+        const pr e0 = p_mulr(C.p(at), base_em);
+        if (!(e0.h >= 1e-28f)) return PS_BINARY64;
+        const pr em_m = p_mulr(e0, p_mulr(p_mulr(t, t), E));
         if (!(em_m.h >= 1e-28f && em_m.h <= 1e15f)) return PS_BINARY64;
         const pr bx = p_mulr(C.p(at + 4), base_bx);
         pr den;
@@ -428,8 +432,8 @@ __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConst
             if (!(bx.h < 60.0f)) return PS_BINARY64;
             den = p_near(exp((double)bx.h + (double)bx.l) - 1.0);
         }
-        const pr ab_m = p_mulr(em_m, p_mulr(den, C.p(at + 6)));
-        if (!(ab_m.h >= 1e-30f && ab_m.h <= 1e15f)) return PS_BINARY64;
+        const pr dk = p_mulr(den, C.p(at + 6)), ab_m = p_mulr(em_m, dk);
+        if (!(bx.h >= 1e-28f && dk.h >= 1e-28f && ab_m.h >= 1e-30f && ab_m.h <= 1e15f)) return PS_BINARY64;
         co[ch] = {em_m, ab_m, e};
     }
     return PS_SAMPLED;

@@ -247,3 +247,15 @@ def test_fp64_image_stop_reasons_at_the_horizon(cuda, orc, spin, tol, div, half,
     steps, why = _np(req.out["nsteps"]).reshape(-1), _np(req.out["status"]).reshape(-1)
     # (which side of the horizon a last step lands on may turn on a rounding: 2 rays in 10^4)
     assert (steps != o["K"]).sum() + (why != o["why"]).sum() <= 2e-4 * len(s0)
+
+
+# emission factors whose product leaves the floats' range, and is lifted into
+# it again by the fit's polynomial; other images of this view differ from the
+# oracle's by at most 3e-12 of a conditioned pixel
+@pytest.mark.parametrize("u,mass", [(1e7, 1e22), (3e7, 1e22), (3e6, 1e22), (1e7, 3e21)])
+def test_fp64_image_of_faint_factors(cuda, orc, u, mass):
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    arrs = make_synthetic_snapshot(nblocks=4, cells_per_block=8, extent=20., bhspin=0.94)
+    arrs.uov[4] *= np.float32(u)
+    p = _image_parity(orc, arrs, 20.0, 16, 0.94, nu=2e8, mass_scale=mass, r_high=1.)
+    assert p["steps_equal"] and p["max_pixel_rel_err"] <= 1e-11, p
