@@ -386,14 +386,20 @@ __device__ __forceinline__ int sample_pair(const SampleView &sv, const PairConst
     // sigma cut, electron temperature
     if (p_sub(b2, p_mul(C.p(PC_SIGMA), p_two(dens, ratio))).h > 0.0f) return PS_SAMPLED;
     pr beta = p_mulr(p_mulr(p_two(ue, ratio), C.p(PC_GAM2)), p_mulr(ib, ib));
-    if (beta.h > 1e15f) beta = {1e15f, 0.0f};             // T_ratio is r_high to 2^-99
-    const pr be2 = p_mulr(beta, beta), ope = p_addr(be2, one);
+    if (fabsf(beta.h) > 1e15f) beta = {1e15f, 0.0f};      // T_ratio is r_high to 2^-99
+    // 1 and beta^2 over beta's power of two squared, where that is above one
+    // (the quotient is the same): beta^2 R_high and its reciprocal would leave
+    // the floats' range
+    const int ebe = max(0, (int)(__float_as_uint(beta.h) >> 23 & 255u) - 127);
+    const float sbe = __uint_as_float((unsigned)(127 - min(ebe, 50)) << 23), one2 = sbe * sbe;
+    beta = p_two(beta, sbe);
+    const pr be2 = p_mulr(beta, beta), ope = p_addr(be2, {one2, 0.0f});
     const pr gi = C.p(PC_GIM1), ge = C.p(PC_GEM1);
     // Theta_e = K u (1 + beta^2) / (dens (g_i (1 + beta^2) + g_e (R_high beta^2 + R_low)))
-    const pr D = p_mulr(dens, p_addr(p_mul(gi, ope), p_mul(ge, p_addr(p_mul(C.p(PC_RHIGH), be2), C.p(PC_RLOW)))));
+    const pr D = p_mulr(dens, p_addr(p_mul(gi, ope), p_mul(ge, p_addr(p_mul(C.p(PC_RHIGH), be2), p_two(C.p(PC_RLOW), one2)))));
     const pr th = p_mulr(p_mulr(C.p(PC_KTH), ue), p_mulr(ope, p_rcp(D)));
-    if (!(p_sub(th, {0.3f, (float)(0.3 - (double)0.3f)}).h >= 0.0f)) return PS_SAMPLED;
-    if (!(th.h < 1e8f)) return PS_BINARY64;
+    if (p_sub(th, {0.3f, (float)(0.3 - (double)0.3f)}).h < 0.0f) return PS_SAMPLED;
+    if (!(th.h < 1e8f)) return PS_BINARY64;               // or not a number
     const pr ith = p_rcp(th);
     const pr base_nus = p_mulr(p_mulr(p_mulr(b, sp), p_mulr(th, th)), inup);
     const pr base_em = p_mulr(p_mulr(dens, inup), p_mulr(ith, ith));

@@ -259,3 +259,14 @@ def test_fp64_image_of_faint_factors(cuda, orc, u, mass):
     arrs.uov[4] *= np.float32(u)
     p = _image_parity(orc, arrs, 20.0, 16, 0.94, nu=2e8, mass_scale=mass, r_high=1.)
     assert p["steps_equal"] and p["max_pixel_rel_err"] <= 1e-11, p
+
+
+# beta to 1e15 and beyond beside an R_high of a million (its bar as above)
+@pytest.mark.parametrize("u,B", [(1e7, 1e-4), (1e10, 1e-10), (1e9, 1e-6), (1e10, 1e-6)])
+def test_fp64_image_of_large_beta(cuda, orc, u, B):
+    from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
+    arrs = make_synthetic_snapshot(nblocks=4, cells_per_block=8, extent=20., bhspin=0.94)
+    arrs.uov[4] *= np.float32(u)
+    arrs.B *= np.float32(B)
+    p = _image_parity(orc, arrs, 20.0, 16, 0.94, r_high=1e6)
+    assert p["steps_equal"] and p["max_pixel_rel_err"] <= 1e-11, p
