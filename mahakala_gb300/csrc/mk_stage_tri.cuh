@@ -276,8 +276,15 @@ __device__ __forceinline__ bool rlow_tri(const RlowTri &k, double dens, double u
     // significands in [1, 2); the exponents go to the result
     const tri d = t_from(__hiloint2double((int)(hd - ((unsigned)ed << 20)), __double2loint(dens)));
     const tri s = t_from(__hiloint2double((int)(hu - ((unsigned)eu << 20)), __double2loint(u)));
-    const tri b = t_from(beta), b2 = t_mulr(b, b), ob = t_add({1.0f, 0.0f, 0.0f}, b2);
-    const tri D = t_add(t_mulr(k.gi, ob), t_mulr(k.ge, t_add(t_mulr(k.rh, b2), k.rl)));
+    // 1 and beta^2 over beta's power of two squared where that is above one
+    // (the quotient is the same): their products with gammas and R_high, and
+    // the reciprocal, would leave the range in which a triple keeps its words
+    const unsigned hb = (unsigned)__double2hiint(beta);
+    const int eb = max(0, (int)((hb >> 20) & 0x7ffu) - 1023);
+    const float sb = __uint_as_float((unsigned)(127 - eb) << 23), o2 = sb * sb;
+    const tri b = t_from(__hiloint2double((int)(hb - ((unsigned)eb << 20)), __double2loint(beta)));
+    const tri b2 = t_mulr(b, b), ob = t_add({o2, 0.0f, 0.0f}, b2);
+    const tri D = t_add(t_mulr(k.gi, ob), t_mulr(k.ge, t_add(t_mulr(k.rh, b2), {k.rl.h * o2, k.rl.m * o2, k.rl.l * o2})));
     const tri th = t_mulr(t_mulr(k.c, s), t_mulr(ob, t_rcp(t_mulr(d, D))));
     if (k.rh.h > 0.0f && !(th.h > 1e-30f)) return false;
     out = scaled(t_to(th), eu - ed);

@@ -270,3 +270,19 @@ def test_fp64_image_of_large_beta(cuda, orc, u, B):
     arrs.B *= np.float32(B)
     p = _image_parity(orc, arrs, 20.0, 16, 0.94, r_high=1e6)
     assert p["steps_equal"] and p["max_pixel_rel_err"] <= 1e-11, p
+
+
+@pytest.mark.parametrize("r_high,r_low,gammas", [(1e6, 1e6, (1e6, 1e6)), (1e6, 1e-4, (1e6, 2. / 3)), (40., 1., (1e6, 1e6)),
+                                                 (1e-4, 1e6, (1. / 3, 2. / 3)), (1e6, 1., (1. / 3, 2. / 3))])
+def test_electrons_at_large_beta(cuda, r_high, r_low, gammas):
+    """Against the formula in long double: 1e-15, five roundings (the binary64
+    formula's largest error here is 9e-16)."""
+    from mahakala_gb300.electrons import rlow_rhigh_model
+    rng = np.random.default_rng(5)
+    a = [10.0 ** rng.uniform(-100, 100, 20000), 10.0 ** rng.uniform(-100, 100, 20000), 10.0 ** rng.uniform(-9, 9.2, 20000)]
+    t = _np(rlow_rhigh_model(*a, r_low=r_low, r_high=r_high, electron_gamma=1 + gammas[0], ion_gamma=1 + gammas[1]))
+    dens, u, beta = (np.longdouble(x) for x in a)
+    ge, gi = (np.longdouble((1 + g) - 1.0) for g in gammas)
+    T = (r_high * beta * beta + r_low) / (1 + beta * beta)
+    exact = np.longdouble(1.6726e-24) / np.longdouble(9.1094e-28) * u * ge * gi / (dens * (gi + ge * T))
+    assert np.max(np.abs(t - exact) / exact) < 1e-15
