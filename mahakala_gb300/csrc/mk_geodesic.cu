@@ -129,9 +129,10 @@ __device__ __noinline__ void integrate_reference_f64(double s[8], int j0, int64_
 // step, and the state before a rejected step is that row.
 template <bool ROWS>
 __global__ void __launch_bounds__(GEO_THREADS)
-integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a, int N, double div, double tol,
-                           double *__restrict__ rows, double *__restrict__ dts, int32_t *__restrict__ Kout,
-                           int32_t *__restrict__ why_out, double *__restrict__ state_out, int rpw, int all_f64) {
+integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a, SpinTri sp, RuleTri R, int N,
+                           double div, double tol, double *__restrict__ rows, double *__restrict__ dts,
+                           int32_t *__restrict__ Kout, int32_t *__restrict__ why_out, double *__restrict__ state_out,
+                           int rpw, int all_f64) {
     const int lane = threadIdx.x & 31;
     const int64_t p = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * rpw + lane;
     const unsigned team = __ballot_sync(0xffffffffu, lane < rpw && p < npx);
@@ -144,8 +145,6 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
     TriState s, last;
     tri_state(s64, s);
     last = s;
-    const SpinTri sp = spin_tri(a);
-    const RuleTri R = rule_tri(a, div, tol);
     {
         TriPoint q;
         tri dt = {0.0f, 0.0f, 0.0f};
@@ -348,9 +347,9 @@ __device__ __noinline__ void shadow_ray_f64(const double start[8], int64_t p, do
 // horizon and its result decides a side of the shadow's edge.
 __global__ void __launch_bounds__(GEO_THREADS)
 shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa, const double *__restrict__ mid,
-                   int64_t n, double a, double ci, double si, double dist, int N, int32_t *__restrict__ Kout,
-                   int32_t *__restrict__ best_out, double *__restrict__ best_dt_out, double *__restrict__ r_km1,
-                   double *__restrict__ r_best, double *__restrict__ r_last, int rpw) {
+                   int64_t n, double a, SpinTri sp, RuleTri R, double ci, double si, double dist, int N,
+                   int32_t *__restrict__ Kout, int32_t *__restrict__ best_out, double *__restrict__ best_dt_out,
+                   double *__restrict__ r_km1, double *__restrict__ r_best, double *__restrict__ r_last, int rpw) {
     const int lane = threadIdx.x & 31;
     const int64_t p = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * rpw + lane;
     if (lane >= rpw || p >= n) return;
@@ -359,8 +358,6 @@ shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa,
     bool out = !tri_range(s64);
     TriState s;
     tri_state(s64, s);
-    const SpinTri sp = spin_tri(a);
-    const RuleTri R = rule_tri(a, 40.0, 1e-2);
     const tri none = {NAN, NAN, NAN};
     int K = N, best = -1;
     tri best_dt = {-INFINITY, 0.0f, 0.0f}, r_prev = none, rb = none, rk = none, rl = none;
@@ -458,8 +455,8 @@ static int integrate(const double *s0_dev, int64_t npx, double bhspin, const mk_
     if (policy->kind == MK_POLICY_REFERENCE) {
         const auto kernel = rows_dev || dt_dev ? integrate_reference_kernel<true> : integrate_reference_kernel<false>;
         kernel<<<ray_grid(npx, rpw), GEO_THREADS, 0, st>>>(
-            s0_dev, npx, bhspin, policy->nmax, policy->div, policy->tol, rows_dev, dt_dev, K_dev, why_dev, state_dev,
-            rpw, !tri_policy(*policy));
+            s0_dev, npx, bhspin, spin_tri(bhspin), rule_tri(bhspin, policy->div, policy->tol), policy->nmax,
+            policy->div, policy->tol, rows_dev, dt_dev, K_dev, why_dev, state_dev, rpw, !tri_policy(*policy));
         MK_LAUNCHED("integrate_reference_kernel");
     } else if (policy->kind == MK_POLICY_FIXED) {
         MK_REQUIRE(!rows_dev && !dt_dev, MK_ERR_UNSUPPORTED, "mk_integrate: rows only for the reference policy");
@@ -526,8 +523,8 @@ extern "C" int mk_shadow_pass(const double *cos_dev, const double *sin_dev, cons
     if (n == 0) return MK_OK;
     const int rpw = rays_per_warp(n);
     shadow_pass_kernel<<<ray_grid(n, rpw), GEO_THREADS, 0, as_stream(stream)>>>(
-        cos_dev, sin_dev, mid_dev, n, bhspin, cos_inc, sin_inc, distance, max_steps, K_dev, best_dev, best_dt_dev,
-        r_km1_dev, r_best_dev, r_last_dev, rpw);
+        cos_dev, sin_dev, mid_dev, n, bhspin, spin_tri(bhspin), rule_tri(bhspin, 40.0, 1e-2), cos_inc, sin_inc,
+        distance, max_steps, K_dev, best_dev, best_dt_dev, r_km1_dev, r_best_dev, r_last_dev, rpw);
     MK_LAUNCHED("shadow_pass_kernel");
     return MK_OK;
 }

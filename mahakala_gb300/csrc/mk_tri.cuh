@@ -203,8 +203,7 @@ MK_HD tri t_norm(tri x) {
 }
 // t_from cuts its words off; these are rounded to the nearest, as the sums
 // below leave theirs: for words that t_less compares, and for constants of
-// which a pair is kept (cut off they were up to 2^-48 too small, the spin of
-// every step among them)
+// which a pair is kept (cut off they were up to 2^-48 too small)
 MK_HD tri t_near(double v) { return t_norm(t_from(v)); }
 MK_HD pr p_near(double v) {
     const tri t = t_near(v);
@@ -285,9 +284,10 @@ struct SpinTri {
 };
 MK_HD SpinTri spin_tri(double a) {
     SpinTri s;
-    s.a = p_near(a);
-    s.aa3 = t_near(a * a);
-    s.aa = {s.aa3.h, s.aa3.m};
+    const tri t = t_from(a);  // the last word to the pair's low one, not cut off
+    s.a = {t.h, f_add(t.m, t.l)};
+    s.aa3 = t_from(a * a);
+    s.aa = {s.aa3.h, f_add(s.aa3.m, s.aa3.l)};
     return s;
 }
 
