@@ -154,6 +154,10 @@ integrate_reference_kernel(const double *__restrict__ s0, int64_t npx, double a,
         if (moving) {
             tri_step<true>(s, q, dt, sp.a, sp.aa, sp.aa3, true);
             go = rule_dt(q.r, R, dt, d, w);
+            if (tri_left_range(s, q.r.h)) {
+                out = true;
+                moving = false;
+            }
         }
         while (__any_sync(team, moving)) {
             const bool near = go && d < TRI_NEAR;
@@ -258,7 +262,8 @@ integrate_fixed_kernel(const double *__restrict__ s0, int64_t npx, double a, int
     if (!out) {
         TriPoint q;
         tri_step<true>(s, q, {0.0f, 0.0f, 0.0f}, sp.a, sp.aa, sp.aa3, true);
-        for (j = 0; j < N; j++) {
+        out = tri_left_range(s, q.r.h);
+        for (j = 0; j < N && !out; j++) {
             tri h = t_add(t_mul(hf, q.r), {0.0f, 0.0f, 0.0f});
             h = t_less(h, h0) ? h0 : (t_less(h1, h) ? h1 : h);
             h = t_neg(h);
@@ -369,7 +374,8 @@ shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa,
         float d;
         int w;
         bool go = rule_dt(q.r, R, dt, d, w);
-        for (int j = 0; j < N; j++) {
+        out = tri_left_range(s, q.r.h);
+        for (int j = 0; j < N && !out; j++) {
             tri dtn = dt;
             if (go) {
                 tri_step<false>(s, q, dt, sp.a, sp.aa, sp.aa3, false);

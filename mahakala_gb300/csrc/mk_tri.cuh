@@ -378,14 +378,16 @@ MK_HD void tri_doubles(const TriState &o, double s[8]) {
 // Ranges in which the triples hold every intermediate with all its words
 // inside the float range; a ray that leaves them is continued in binary64 from
 // the state before, one that starts outside from its start.
-constexpr float TRI_MAX_R = 1e6f, TRI_MAX_K = 1e12f, TRI_MIN_K = 1e-6f;
+constexpr float TRI_MIN_R = 1e-2f, TRI_MAX_R = 1e6f, TRI_MAX_K = 1e12f, TRI_MIN_K = 1e-6f;
 // true out of range or at NaN: a step over the horizon toward r = 0 overflows
-// floats before doubles
+// floats before doubles; r^4 underflows them, and inside the ring, where r^2
+// is a small difference, the pairs lose the radius (1e-11 of r - r_EH at r =
+// 1e-6, spin 0.9)
 __device__ __forceinline__ float tri_sum_k(const TriState &s) {
     return (fabsf(s.K[0].h) + fabsf(s.K[1].h)) + (fabsf(s.K[2].h) + fabsf(s.K[3].h));
 }
 __device__ __forceinline__ bool tri_left_range(const TriState &s, float r) {
-    return !(r <= TRI_MAX_R && tri_sum_k(s) <= TRI_MAX_K);
+    return !(r >= TRI_MIN_R && r <= TRI_MAX_R && tri_sum_k(s) <= TRI_MAX_K);
 }
 
 // first-stage acceleration, radius and metric data at a state

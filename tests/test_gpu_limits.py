@@ -286,3 +286,20 @@ def test_electrons_at_large_beta(cuda, r_high, r_low, gammas):
     T = (r_high * beta * beta + r_low) / (1 + beta * beta)
     exact = np.longdouble(1.6726e-24) / np.longdouble(9.1094e-28) * u * ge * gi / (dens * (gi + ge * T))
     assert np.max(np.abs(t - exact) / exact) < 1e-15
+
+
+# radii at which the fourth power of r, or its parts, leave the floats' range,
+# and ones inside the ring
+@pytest.mark.parametrize("spin", [0.0, 0.9])
+def test_integrator_at_small_radii(cuda, orc, spin):
+    from mahakala_gb300.geodesics import step_policy, trace
+    x = np.array([0.3, 1e-2, 1e-4, 1e-6, 1e-9, 3e-10, 1e-11, 1e-13])
+    s0 = np.zeros((len(x), 8))
+    s0[:, 1], s0[:, 3] = x, 0.5 * x
+    s0[:, 4:6] = 1.0
+    with np.errstate(all="ignore"):
+        o = orc.integrate(s0, 3, 1e4, 1e-4, spin, full=True)
+    g = trace(s0, spin, step_policy(3, 1e4, 1e-4), rows=True)
+    assert np.array_equal(_np(g["K"]), o["K"]) and np.array_equal(_np(g["why"]), o["why"])
+    ok = o["K"] > 0
+    assert np.max(rel_err(_np(g["dt"])[0][ok], o["dt"][0][ok])) < 1e-14
