@@ -1,0 +1,68 @@
+"""Writes wide.npz: end states of captured rays in more than binary64, for the
+tests that ask how far from the exact trajectory a binary64 result is.
+
+The integrator is the oracle's C source (oracle/mk_oracle.c) with `double`
+compiled as `long double` (64 bits of significand on x86-64, 113 on aarch64)
+and its literals and library calls to match.  Each state is stored as the sum
+of two doubles.  Run from the repository's root: python tests/golden/make_wide.py
+"""
+
+import ctypes
+import os
+import re
+import subprocess
+import sys
+import tempfile
+
+import numpy as np
+
+ROOT = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+CASES = ((0.0, 1e-4), (0.5, 1e-2), (0.94, 1e-2), (0.94, 1e-4), (0.998, 1e-4))  # spin, tol
+CALLS = "sqrt cbrt exp pow sin cos acos fabs fmin fmax fmod floor copysign".split()
+
+
+def wide_library(directory):
+    src = open(os.path.join(ROOT, "oracle", "mk_oracle.c")).read()
+    head, body = src.split("#include <string.h>", 1)
+    for name in "dadd dsub dmul ddiv dsqrt dsq dscale".split():   # names the C library takes for itself
+        body = re.sub(r"\b%s\b" % name, "dual_" + name, body)
+    body = re.sub(r"(?<![\w.])(\d+\.\d*(?:e[+-]?\d+)?|\d+e[+-]?\d+)(?![\w.])", r"\1L", body)
+    defs = "#define double long double\n" + "".join("#define %s %sl\n" % (c, c) for c in CALLS)
+    c = os.path.join(directory, "wide.c")
+    with open(c, "w") as f:
+        f.write(head + "#include <string.h>\n" + defs + body)
+    lib = os.path.join(directory, "libwide.so")
+    subprocess.run(["gcc", "-O2", "-std=c11", "-D_GNU_SOURCE", "-fopenmp", "-ffp-contract=off", "-shared", "-fPIC", c,
+                    "-o", lib, "-lm"], check=True)
+    return ctypes.CDLL(lib)
+
+
+def end_states(lib, s0, N, div, tol, spin):
+    """K and the state after K steps of the reference's rule, in long double."""
+    s = np.ascontiguousarray(s0, dtype=np.longdouble)
+    n, state = len(s), np.empty(s.shape, np.longdouble)
+    K, why = np.empty(n, np.int32), np.empty(n, np.int32)
+    lib.orc_integrate(s.ctypes.data_as(ctypes.c_void_p), n, N, ctypes.c_longdouble(div), ctypes.c_longdouble(tol),
+                      ctypes.c_longdouble(spin), None, None, K.ctypes.data_as(ctypes.c_void_p),
+                      why.ctypes.data_as(ctypes.c_void_p), state.ctypes.data_as(ctypes.c_void_p))
+    return K, why, state
+
+
+def main():
+    sys.path.insert(0, ROOT)
+    import oracle
+    out = {}
+    with tempfile.TemporaryDirectory() as d:
+        lib = wide_library(d)
+        for i, (spin, tol) in enumerate(CASES):
+            s0 = oracle.initialize_geodesics_at_camera(spin, 60.0, 1000, -10, 10, 20)
+            K, why, state = end_states(lib, s0, 4000, 40.0, tol, spin)
+            keep = np.flatnonzero((why == oracle.ST_CAPTURED) & (K == oracle.integrate(s0, 4000, 40.0, tol, spin)["K"]))[:40]
+            hi = state[keep].astype(np.float64)
+            out.update({f"s0_{i}": s0[keep], f"K_{i}": K[keep], f"hi_{i}": hi,
+                        f"lo_{i}": (state[keep] - hi).astype(np.float64), f"spin_{i}": spin, f"tol_{i}": tol})
+    np.savez_compressed(os.path.join(os.path.dirname(os.path.abspath(__file__)), "wide.npz"), **out)
+
+
+if __name__ == "__main__":
+    main()

@@ -303,3 +303,25 @@ def test_integrator_at_small_radii(cuda, orc, spin):
     assert np.array_equal(_np(g["K"]), o["K"]) and np.array_equal(_np(g["why"]), o["why"])
     ok = o["K"] > 0
     assert np.max(rel_err(_np(g["dt"])[0][ok], o["dt"][0][ok])) < 1e-14
+
+
+@pytest.mark.parametrize("case", range(5))
+def test_captured_rays_as_exact_as_binary64(cuda, orc, case):
+    """Captured rays' last wavevectors against an integration in long double
+    (golden/make_wide.py): the geometric mean of 40 rays' errors at most 1.5
+    times that of the oracle's binary64 (rounding scatters each error by a
+    factor of 3 or so, a mean of 40 by 1.2)."""
+    from conftest import golden
+    from mahakala_gb300.geodesics import step_policy, trace
+    d = golden("wide")
+    s0, K, hi, lo = (d[f"{k}_{case}"] for k in ("s0", "K", "hi", "lo"))
+    spin, tol = float(d[f"spin_{case}"]), float(d[f"tol_{case}"])
+    g = trace(s0, spin, step_policy(4000, 40.0, tol))
+    assert np.array_equal(_np(g["K"]), K)
+
+    def mean_error(x):
+        e = np.linalg.norm(((x - hi) - lo)[:, 4:], axis=1) / np.linalg.norm(hi[:, 4:], axis=1)
+        return np.exp(np.mean(np.log(e)))
+
+    ours, theirs = mean_error(_np(g["state"])), mean_error(orc.integrate(s0, 4000, 40.0, tol, spin)["state"])
+    assert ours <= 1.5 * theirs, (ours, theirs)
