@@ -234,6 +234,13 @@ int mk_shadow_pass(const double *cos_dev, const double *sin_dev, const double *m
                    double bhspin, double cos_inc, double sin_inc, double distance, int32_t max_steps,
                    int32_t *K_dev, int32_t *best_dev, double *best_dt_dev, double *r_km1_dev,
                    double *r_best_dev, double *r_last_dev, void *stream);
+/* The same for a caller that asks only on which side of the shadow's edge
+   each radius lies (r < 100): the last approach to the horizon in float
+   pairs, its radii up to ten times as far off as mk_shadow_pass's. */
+int mk_shadow_sides(const double *cos_dev, const double *sin_dev, const double *mid_dev, int64_t n,
+                    double bhspin, double cos_inc, double sin_inc, double distance, int32_t max_steps,
+                    int32_t *K_dev, int32_t *best_dev, double *best_dt_dev, double *r_km1_dev,
+                    double *r_best_dev, double *r_last_dev, void *stream);
 
 /* --------------------------------------------------------- snapshots */
 /* Bytes of device storage mk_snapshot_build needs for nmb blocks of n^3. */

@@ -98,6 +98,8 @@ SIGNATURES = {
     "mk_integrate_moving": (_c.c_int, [_VP, _I64, _D, _c.POINTER(StepPolicy), _VP, _VP, _VP, _VP, _VP, _VP]),
     "mk_freeze_rows": (_c.c_int, [_VP, _VP, _I64, _I32, _VP, _VP, _VP]),
     "mk_radius_cal": (_c.c_int, [_VP, _I64, _I64, _D, _VP, _VP]),
+    "mk_shadow_sides": (_c.c_int, [_VP, _VP, _VP, _I64, _D, _D, _D, _D, _I32, _VP, _VP, _VP, _VP, _VP, _VP,
+                                   _VP]),
     "mk_shadow_pass": (_c.c_int, [_VP, _VP, _VP, _I64, _D, _D, _D, _D, _I32, _VP, _VP, _VP, _VP, _VP, _VP,
                                   _VP]),
     "mk_snapshot_bytes": (_SZ, [_I32, _I32]),

@@ -133,14 +133,14 @@ def select_photons_integrator(inc, angle, radius, bhspin, distance=1000, max_ste
     return _shadow_pass(inc, np.cos(angle), np.sin(angle), radius, bhspin, distance, max_steps)
 
 
-def _shadow_pass(inc, ca, sa, mid, bhspin, distance, max_steps):
+def _shadow_pass(inc, ca, sa, mid, bhspin, distance, max_steps, entry="mk_shadow_pass"):
     dev = device()
     n = len(mid)
     ci, si = _cos_sin(inc)
     cat, sat, midt = f64(ca, dev), f64(sa, dev), f64(mid, dev)
     ints = torch.empty((2, n), dtype=torch.int32, device=dev)
     vals = torch.empty((4, n), dtype=torch.float64, device=dev)
-    _lib.call("mk_shadow_pass", ptr(cat), ptr(sat), ptr(midt), n, float(bhspin), ci, si, float(distance),
+    _lib.call(entry, ptr(cat), ptr(sat), ptr(midt), n, float(bhspin), ci, si, float(distance),
               int(max_steps), ptr(ints[0]), ptr(ints[1]), ptr(vals[0]), ptr(vals[1]), ptr(vals[2]), ptr(vals[3]),
               stream_ptr())
     K, best = ints.cpu().numpy()
@@ -192,7 +192,7 @@ def find_shadow_bisection_angles(bhspin, inc, angles, max_steps=2000, error_allo
         flat = np.concatenate(mids).reshape(-1, angles.size)
         shape = (len(flat), angles.size)
         r = _shadow_pass(inc, np.tile(ca.reshape(-1), len(flat)), np.tile(sa.reshape(-1), len(flat)),
-                         flat.reshape(-1), bhspin, 1000, max_steps).reshape(shape)
+                         flat.reshape(-1), bhspin, 1000, max_steps, "mk_shadow_sides").reshape(shape)
         node = np.zeros(angles.size, dtype=np.int64)
         stuck = np.zeros(angles.size, dtype=bool)     # a ray with no radius moves neither end
         cols = np.arange(angles.size)

@@ -1,5 +1,6 @@
-"""Writes wide.npz: end states of captured rays in more than binary64, for the
-tests that ask how far from the exact trajectory a binary64 result is.
+"""Writes wide.npz: end states of captured rays, and the radii at which those of
+a polar camera are captured, in more than binary64, for the tests that ask how
+far from the exact trajectory a binary64 result is.
 
 The integrator is the oracle's C source (oracle/mk_oracle.c) with `double`
 compiled as `long double` (64 bits of significand on x86-64, 113 on aarch64)
@@ -48,6 +49,21 @@ def end_states(lib, s0, N, div, tol, spin):
     return K, why, state
 
 
+def polar_camera(oracle, ang, rad, spin):
+    s0 = np.empty((len(ang), 8))
+    ci, si = oracle.inclination_cos_sin(60.0)
+    c, s, r = (np.ascontiguousarray(v) for v in (np.cos(ang), np.sin(ang), rad))
+    p = lambda v: v.ctypes.data_as(ctypes.c_void_p)
+    d = ctypes.c_double
+    oracle.lib().orc_camera_polar(p(c), p(s), p(r), len(r), d(ci), d(si), d(1000.0), d(spin), p(s0))
+    return s0
+
+
+def radius(x, a):
+    R2 = x[1] ** 2 + x[2] ** 2 + x[3] ** 2 - a ** 2
+    return np.sqrt((R2 + np.sqrt(R2 ** 2 + 4 * a ** 2 * x[3] ** 2)) / 2)
+
+
 def main():
     sys.path.insert(0, ROOT)
     import oracle
@@ -61,6 +77,21 @@ def main():
             hi = state[keep].astype(np.float64)
             out.update({f"s0_{i}": s0[keep], f"K_{i}": K[keep], f"hi_{i}": hi,
                         f"lo_{i}": (state[keep] - hi).astype(np.float64), f"spin_{i}": spin, f"tol_{i}": tol})
+            if spin < 0.9 or tol != 1e-4:
+                continue
+            # radii of select_photons_integrator: row argmax(dt) - 1 = K - 1 of captured rays
+            rng = np.random.default_rng(i)
+            ang, rad = rng.uniform(0, 2 * np.pi, 300), rng.uniform(0.5, 4.5, 300)
+            s0 = polar_camera(oracle, ang, rad, spin)
+            K, why, _ = end_states(lib, s0, 2000, 40.0, 1e-2, spin)
+            keep = np.flatnonzero(why == oracle.ST_CAPTURED)
+            r = np.empty(len(keep), np.longdouble)
+            for j, p in enumerate(keep):
+                x = end_states(lib, s0[p:p + 1], int(K[p]) - 1, 40.0, 1e-2, spin)[2][0]
+                r[j] = radius(x, np.longdouble(spin))
+            hi = r.astype(np.float64)
+            out.update({f"angle_{i}": ang[keep], f"radius_{i}": rad[keep], f"r_hi_{i}": hi,
+                        f"r_lo_{i}": (r - hi).astype(np.float64)})
     np.savez_compressed(os.path.join(os.path.dirname(os.path.abspath(__file__)), "wide.npz"), **out)
 
 

@@ -325,3 +325,18 @@ def test_captured_rays_as_exact_as_binary64(cuda, orc, case):
 
     ours, theirs = mean_error(_np(g["state"])), mean_error(orc.integrate(s0, 4000, 40.0, tol, spin)["state"])
     assert ours <= 1.5 * theirs, (ours, theirs)
+
+
+@pytest.mark.parametrize("case", [3, 4])
+def test_shadow_radii_as_exact_as_binary64(cuda, orc, case):
+    """Radii at the horizon of select_photons_integrator against long double
+    (golden/make_wide.py): the median error at most twice 3e-16 + that of the
+    binary64 radii r (the spacing of doubles at r, over sqrt(12), and 7e-16 and
+    4e-15 measured of a binary64 integration at spins 0.94 and 0.998)."""
+    from conftest import golden
+    from mahakala_gb300.geodesics import select_photons_integrator
+    d = golden("wide")
+    r = select_photons_integrator(60.0, d[f"angle_{case}"], d[f"radius_{case}"], float(d[f"spin_{case}"]))
+    hi, lo = d[f"r_hi_{case}"], d[f"r_lo_{case}"]
+    assert len(r) > 100
+    assert np.median(np.abs((r - hi) - lo) / hi) <= {3: 2 * 1e-15, 4: 2 * 4.3e-15}[case]
