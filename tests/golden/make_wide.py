@@ -19,6 +19,10 @@ import numpy as np
 
 ROOT = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 CASES = ((0.0, 1e-4), (0.5, 1e-2), (0.94, 1e-2), (0.94, 1e-4), (0.998, 1e-4))  # spin, tol
+# spin, inclination, distance, then the step rule: div, or hfrac of the fixed-fraction rule
+RULES = ((0.5, 60.0, 1000.0, "div", 2.0), (0.94, 60.0, 1000.0, "div", 10.0), (0.5, 60.0, 1000.0, "hfrac", 0.05),
+         (0.94, 85.0, 1000.0, "hfrac", 0.05), (0.5, 60.0, 100.0, "hfrac", 0.1), (0.94, 90.0, 1000.0, "hfrac", 0.1),
+         (0.5, 60.0, 100.0, "hfrac", 0.5), (0.94, 60.0, 100.0, "hfrac", 0.02))
 CALLS = "sqrt cbrt exp pow sin cos acos fabs fmin fmax fmod floor copysign".split()
 
 
@@ -46,6 +50,17 @@ def end_states(lib, s0, N, div, tol, spin):
     lib.orc_integrate(s.ctypes.data_as(ctypes.c_void_p), n, N, ctypes.c_longdouble(div), ctypes.c_longdouble(tol),
                       ctypes.c_longdouble(spin), None, None, K.ctypes.data_as(ctypes.c_void_p),
                       why.ctypes.data_as(ctypes.c_void_p), state.ctypes.data_as(ctypes.c_void_p))
+    return K, why, state
+
+
+def fixed_end_states(lib, s0, N, hfrac, spin):
+    """Steps and last state of the fixed-fraction rule, in long double."""
+    s = np.ascontiguousarray(s0, dtype=np.longdouble)
+    n, state = len(s), np.empty(s.shape, np.longdouble)
+    K, why = np.empty(n, np.int32), np.empty(n, np.int32)
+    numbers = [ctypes.c_longdouble(v) for v in (spin, hfrac, 0.01, 10.0, 1.01, 1000.0)]
+    lib.orc_trace_fixed(s.ctypes.data_as(ctypes.c_void_p), n, N, *numbers, state.ctypes.data_as(ctypes.c_void_p),
+                        K.ctypes.data_as(ctypes.c_void_p), why.ctypes.data_as(ctypes.c_void_p))
     return K, why, state
 
 
@@ -92,6 +107,19 @@ def main():
             hi = r.astype(np.float64)
             out.update({f"angle_{i}": ang[keep], f"radius_{i}": rad[keep], f"r_hi_{i}": hi,
                         f"r_lo_{i}": (r - hi).astype(np.float64)})
+        for i, (spin, inc, distance, rule, value) in enumerate(RULES):
+            s0 = oracle.initialize_geodesics_at_camera(spin, inc, distance, -10, 10, 14)
+            if rule == "div":
+                K, why, state = end_states(lib, s0, 4000, value, 1e-4, spin)
+                same = K == oracle.integrate(s0, 4000, value, 1e-4, spin)["K"]
+            else:
+                K, why, state = fixed_end_states(lib, s0, 4000, value, spin)
+                same = K == oracle.trace_fixed(s0, 4000, spin, hfrac=value)["nsteps"]
+            keep = np.flatnonzero((why == oracle.ST_ESCAPED) & same)[:100]
+            hi = state[keep].astype(np.float64)
+            out.update({f"rule_s0_{i}": s0[keep], f"rule_K_{i}": K[keep], f"rule_hi_{i}": hi,
+                        f"rule_lo_{i}": (state[keep] - hi).astype(np.float64), f"rule_spin_{i}": spin,
+                        f"rule_{i}": rule, f"rule_value_{i}": value})
     np.savez_compressed(os.path.join(os.path.dirname(os.path.abspath(__file__)), "wide.npz"), **out)
 
 

@@ -340,3 +340,29 @@ def test_shadow_radii_as_exact_as_binary64(cuda, orc, case):
     hi, lo = d[f"r_hi_{case}"], d[f"r_lo_{case}"]
     assert len(r) > 100
     assert np.median(np.abs((r - hi) - lo) / hi) <= {3: 2 * 1e-15, 4: 2 * 4.3e-15}[case]
+
+
+@pytest.mark.parametrize("case", range(8))
+def test_escaped_rays_as_exact_as_binary64(cuda, orc, case):
+    """Escaped rays under step rules of long and short steps, from afar and
+    near by, against long double (golden/make_wide.py): the geometric mean of
+    up to 100 rays' errors at most 1.5 times the oracle's, as above."""
+    from conftest import golden
+    from mahakala_gb300.geodesics import step_policy, trace
+    d = golden("wide")
+    s0, K, hi, lo = (d[f"rule_{k}_{case}"] for k in ("s0", "K", "hi", "lo"))
+    spin, value = float(d[f"rule_spin_{case}"]), float(d[f"rule_value_{case}"])
+    if str(d[f"rule_{case}"]) == "div":
+        g = trace(s0, spin, step_policy(4000, value, 1e-4))
+        o = orc.integrate(s0, 4000, value, 1e-4, spin)
+    else:
+        g = trace(s0, spin, step_policy(4000, kind="fixed", hfrac=value))
+        o = orc.trace_fixed(s0, 4000, spin, hfrac=value)
+    assert len(s0) > 60 and np.array_equal(_np(g["K"]), K)
+
+    def mean_error(x):
+        x, r = ((v * (1, 1, 1, 10, 10, 10, 10)) for v in (((x - hi) - lo)[:, 1:], hi[:, 1:]))
+        return np.exp(np.mean(np.log(np.maximum(np.linalg.norm(x, axis=1) / np.linalg.norm(r, axis=1), 1e-18))))
+
+    ours, theirs = mean_error(_np(g["state"])), mean_error(o["state"])
+    assert ours <= 1.5 * theirs, (ours, theirs)
