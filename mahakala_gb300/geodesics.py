@@ -175,8 +175,9 @@ def find_shadow_bisection_angles(bhspin, inc, angles, max_steps=2000, error_allo
     error = outer - inner
     counter = 0
     while np.max(error) > error_allowed and counter < max_it:
-        left = int(min(np.ceil(np.log2(max(np.max(error) / error_allowed, 2.0))) if error_allowed > 0 else max_it,
-                       max_it - counter))
+        # bisections to come, 64 at most: by then the ends are neighbouring doubles
+        left = int(np.ceil(min(np.log2(max(np.max(error) / error_allowed, 2.0)) if error_allowed > 0 else 64,
+                               max_it - counter, 64)))
         most = max(1, int(np.log2(SHADOW_RAYS / max(angles.size, 1) + 1.0)) if angles.size < SHADOW_RAYS else 1)
         passes = -(-left // most)
         depth = -(-left // passes)

@@ -21,3 +21,26 @@ def test_render_rules(tmp_path):
     out = dict(line.split() for line in subprocess.run([str(exe)], check=True, capture_output=True,
                                                        text=True).stdout.splitlines())
     assert out and set(out.values()) == {"1"}, out
+
+
+@pytest.mark.parametrize("error_allowed,max_it", [(1e-3, 40), (1e-3, 10.5), (1e-3, 0.5), (1e-3, float("inf")), (0.0, 7),
+                                                  (-1.0, 30), (1e-12, 40), (1e-3, 0), (float("nan"), 5)])
+def test_bisections_of_any_count(monkeypatch, error_allowed, max_it):
+    """Several bisections a pass take the midpoints and the decisions of one at
+    a time, for every way to say when to stop."""
+    import numpy as np
+    from mahakala_gb300 import geodesics as g
+    edge = np.array([1.3, 2.7182818, 5.0, 9.99])
+
+    def far(inc, ca, sa, mid, *rest):   # in reality the radius each ray ends at
+        n = len(mid) // len(edge)
+        return np.where(np.asarray(mid).reshape(n, -1) < edge, 1.0, 1000.0).reshape(-1)
+
+    monkeypatch.setattr(g, "_shadow_pass", far)
+    monkeypatch.setattr(g, "SHADOW_RAYS", 600)
+    got = g.find_shadow_bisection_angles(0.5, 60.0, np.arange(4.0), error_allowed=error_allowed, max_it=max_it)
+    inner, outer, count = np.full(4, 0.5), np.full(4, 10.0), 0
+    while np.max(outer - inner) > error_allowed and count < max_it:
+        mid = (outer - inner) / 2 + inner
+        inner, outer, count = np.where(mid < edge, mid, inner), np.where(mid < edge, outer, mid), count + 1
+    assert np.array_equal(got, inner)
