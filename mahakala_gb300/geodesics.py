@@ -154,10 +154,10 @@ def _shadow_pass(inc, ca, sa, mid, bhspin, distance, max_steps, entry="mk_shadow
     return np.where(am < 1, r_last, np.where(am == K, r_km1, r_best))
 
 
-# Rays a bisection pass may take: one a lane of one warp on each of the 608 SM
-# sub-partitions, up to where a pass costs its longest ray's chain of steps
-# whatever their number.
-SHADOW_RAYS = 608 * 32
+# Rays a bisection pass may take, or None for one a lane of one warp on each of
+# the device's SM sub-partitions (four an SM): up to there a pass costs its
+# longest ray's chain of steps whatever their number.
+SHADOW_RAYS = None
 
 
 def find_shadow_bisection_angles(bhspin, inc, angles, max_steps=2000, error_allowed=0.001, max_it=40):
@@ -174,11 +174,12 @@ def find_shadow_bisection_angles(bhspin, inc, angles, max_steps=2000, error_allo
     outer = np.zeros_like(angles) + 10
     error = outer - inner
     counter = 0
+    rays = SHADOW_RAYS or 128 * _lib.load().mk_device_sm_count()
     while np.max(error) > error_allowed and counter < max_it:
         # bisections to come, 64 at most: by then the ends are neighbouring doubles
         left = int(np.ceil(min(np.log2(max(np.max(error) / error_allowed, 2.0)) if error_allowed > 0 else 64,
                                max_it - counter, 64)))
-        most = max(1, int(np.log2(SHADOW_RAYS / max(angles.size, 1) + 1.0)) if angles.size < SHADOW_RAYS else 1)
+        most = max(1, int(np.log2(rays / max(angles.size, 1) + 1.0)) if angles.size < rays else 1)
         passes = -(-left // most)
         depth = -(-left // passes)
         # node i of level l: its interval's ends; children 2i (got away: the
