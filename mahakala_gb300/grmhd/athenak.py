@@ -94,15 +94,23 @@ def mesh_tables(arrs, max_table_cells=1 << 28):
         kinds, kind = np.unique(span @ np.array([1, 1 << 20, 1 << 40]), return_inverse=True)
         sets = [np.flatnonzero(kind == s) for s in range(len(kinds))]
     for m in sets:
-        sx, sy, sz = span[m[0]]
+        sx, sy, sz = (int(n) for n in span[m[0]])
+        if sx * sy * sz >= 512:                   # a slice a block: indices would be many times the table
+            for b in m:
+                x, y, z = (int(c) for c in start[b])
+                cells = table[z:z + sz, y:y + sy, x:x + sx]
+                cells[...] = b
+                taken += cells.size
+            continue
         # the table cells of these blocks, cut at the table's edge as a slice is
-        i, j, k = (start[m, a, None, None, None] + np.arange(n).reshape(sh) for a, n, sh in
-                   ((0, sx, (1, 1, 1, -1)), (1, sy, (1, 1, -1, 1)), (2, sz, (1, -1, 1, 1))))
-        ok = (i < nb[0]) & (j < nb[1]) & (k < nb[2])
-        flat = ((k * nb[1] + j) * nb[0] + i)[ok]
-        taken += flat.size
-        table.reshape(-1)[flat] = np.broadcast_to(m[:, None, None, None], ok.shape)[ok]
-    if np.count_nonzero(table >= 0) != taken:     # a cell taken twice
+        for part in np.array_split(m, -(-len(m) * sx * sy * sz // (1 << 18))):
+            i, j, k = (start[part, a, None, None, None] + np.arange(n).reshape(sh) for a, n, sh in
+                       ((0, sx, (1, 1, 1, -1)), (1, sy, (1, 1, -1, 1)), (2, sz, (1, -1, 1, 1))))
+            ok = (i < nb[0]) & (j < nb[1]) & (k < nb[2])
+            flat = ((k * nb[1] + j) * nb[0] + i)[ok]
+            taken += flat.size
+            table.reshape(-1)[flat] = np.broadcast_to(part[:, None, None, None], ok.shape)[ok]
+    if sum(np.count_nonzero(plane >= 0) for plane in table) != taken:  # a cell taken twice
         raise ValueError("overlapping blocks")
     fine_ghosts = np.zeros(nmb, bool)
     if np.any(levels != levels[0]):

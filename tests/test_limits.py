@@ -44,3 +44,32 @@ def test_bisections_of_any_count(monkeypatch, error_allowed, max_it):
         mid = (outer - inner) / 2 + inner
         inner, outer, count = np.where(mid < edge, mid, inner), np.where(mid < edge, outer, mid), count + 1
     assert np.array_equal(got, inner)
+
+
+@pytest.mark.parametrize("nblocks,depth", [(4, 6), (2, 7), (8, 2)])
+def test_mesh_tables_of_deep_meshes(nblocks, depth):
+    """A corner refined again and again: the finest-level table, one block at a
+    time, in little more memory than the table's own (a sixth of it for a
+    plane's test, the tables of the blocks, and an indexing pass of 2^18 cells)."""
+    import tracemalloc
+    from types import SimpleNamespace
+
+    import numpy as np
+    from mahakala_gb300.grmhd.athenak import mesh_tables
+    from test_tri import _table_by_loops
+    blocks = {(0,) + t for t in np.ndindex(nblocks, nblocks, nblocks)}
+    key = (0, 0, 0, 0)
+    for _ in range(depth):
+        blocks.remove(key)
+        blocks |= {(key[0] + 1,) + tuple(2 * c + d for c, d in zip(key[1:], t)) for t in np.ndindex(2, 2, 2)}
+        key = (key[0] + 1,) + tuple(2 * c + 1 for c in key[1:])
+    order = np.array(sorted(blocks))
+    width = 16.0 / nblocks / 2.0 ** order[:, 0]
+    faces = [np.stack([-8 + width * order[:, 1 + a], -8 + width * (order[:, 1 + a] + 1)], axis=1) for a in range(3)]
+    arrs = SimpleNamespace(Levels=order[:, 0], LogicalLocations=order[:, 1:], x1f=faces[0], x2f=faces[1], x3f=faces[2])
+    tracemalloc.start()
+    table = mesh_tables(arrs)["table"]
+    peak = tracemalloc.get_traced_memory()[1]
+    tracemalloc.stop()
+    assert np.array_equal(table, _table_by_loops(arrs))
+    assert peak <= 1.2 * table.nbytes + (16 << 20), (peak, table.nbytes)
