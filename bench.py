@@ -19,7 +19,9 @@ end (``e2e_fp64``, ``fp64_vs_reference``), the standalone sampling stage
 1024x1024 stress render in both forms (``stress1024``) and the 27-image
 512x512 mixed-precision sweep (``sweep512``).  ``--workload stress1024``:
 the 512^3-cell snapshot at 1024x1024, three frequencies in one pass,
-<= 16384 steps, as the headline.  Printed on rank 0 as one JSON line.
+<= 16384 steps, as the headline.  Printed on rank 0: the headline, its
+roofline, end-to-end value and clocks as one last JSON line, every other
+record before it as a line `detail <key> <JSON>`.
 
 ``--impl reference`` times the reference algorithm on the host cores
 instead: the C restatement of Mahakala's make_image (oracle/, FP64, all
@@ -72,6 +74,22 @@ NCU_TRAFFIC_RENDER256 = {"A": 106.92e6 + 3.01e6, "B": 76.74e6 + 1.58e6, "C": 113
 # operations (FMA = 2) per point of the standalone sampling stage in a binary64
 # evaluation (64x64 camera over the 256^3-cell snapshot, 19 % of points inside it)
 SAMPLING_FLOP_PER_POINT = 399
+
+
+# keys of the last line; the other records go before it, a line each
+LINE_KEYS = ("impl", "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+             "vs_baseline", "dtype", "data", "config", "images_per_s", "roofline", "cpu_baseline", "e2e", "e2e_fp64",
+             "gpu_launches", "phase_ms", "clocks")
+
+
+def print_line(line):
+    """The records of a run on stdout: `detail <key> <JSON>` for each that only a
+    reader wants, then ONE JSON line of the rest, short enough to be read back
+    from the end of a long output."""
+    for key, value in line.items():
+        if key not in LINE_KEYS:
+            print("detail", key, json.dumps(value))
+    print(json.dumps({k: v for k, v in line.items() if k in LINE_KEYS}), flush=True)
 
 
 def parse():
@@ -964,7 +982,7 @@ def main():
         "clocks": clocks,
         "snapshot_build_s": t_gen,
     })
-    print(json.dumps(line), flush=True)
+    print_line(line)
     if world > 1:
         torch.distributed.destroy_process_group()
 

@@ -73,3 +73,19 @@ def test_mesh_tables_of_deep_meshes(nblocks, depth):
     tracemalloc.stop()
     assert np.array_equal(table, _table_by_loops(arrs))
     assert peak <= 1.2 * table.nbytes + (16 << 20), (peak, table.nbytes)
+
+
+def test_bench_line_is_short_and_last(capsys):
+    """The contract's keys end up in one last JSON line, the long records before it."""
+    import json
+    import sys
+    sys.path.insert(0, ROOT)
+    import bench
+    line = {k: 1 for k in bench.LINE_KEYS if k != "impl"}
+    line.update(sweep512=[{"max_pixel_rel_err": 1.23456789e-4, "spin": 0.94}] * 400, serving={"latency": [1.0] * 500})
+    bench.print_line(line)
+    out = capsys.readouterr().out.splitlines()
+    assert json.loads(out[-1]) == {k: 1 for k in bench.LINE_KEYS if k != "impl"}
+    assert [x for x in out if x.startswith("{")] == out[-1:] and len(out) == 3
+    key, value = out[0].split(" ", 2)[1:]
+    assert key == "sweep512" and json.loads(value) == line["sweep512"]
