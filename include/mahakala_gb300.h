@@ -49,10 +49,12 @@ typedef enum {
 
 /* MK_FP64: binary64 results.  The ray state is carried in 72 bits (three
    floats), the accelerations and the sampling in float pairs (~48 bits)
-   whose errors enter the result scaled down, the transfer sums in binary64;
-   against a 140-bit evaluation the images are no further off than binary64
-   throughout.  Requests and samples whose values the pairs cannot hold are
-   taken in binary64.
+   whose errors enter the result scaled down, the transfer sums in binary64:
+   6e-14 of a pixel against a 64-bit-significand evaluation, where binary64
+   throughout leaves 1-3e-13 at ordinary views from 1000 M.  Requests for
+   which binary64 is the more exact (equator cameras, distance |sin i cos i|
+   below 78 M, div below 10), and requests, rays and samples whose values the
+   pairs cannot hold, are taken in binary64 (a ray's chain ~6 times slower).
    MK_MIXED: FP32 arithmetic (ray state as float pairs, Kahan-compensated
    intensity); near the hole (r < 3 M, or inbound inside 6 M where
    photon-ring rays turn) the wavevector is renormalised to null on entry

@@ -274,9 +274,10 @@ __device__ __forceinline__ FluidScalars fluid_frame(const double prim[8], double
 }
 
 // rlow_rhigh_model (electrons.py:32-50)
-// the same with reciprocals in place of the three divisions (the fused
-// FP64 render: within a few ulp of rlow_rhigh, which the stage kernel
-// keeps bit-exact to the reference)
+// the same with reciprocals in place of the three divisions (the binary64
+// samples of the fused renders: within a few ulp of rlow_rhigh below, which
+// follows the reference's operations and serves the stage kernel's inputs
+// outside the triples' range)
 __device__ __forceinline__ double rlow_rhigh_fast(double dens, double u, double beta, double r_low,
                                                   double r_high, double gem1, double gim1) {
     const double b2 = beta * beta;

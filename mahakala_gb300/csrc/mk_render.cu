@@ -21,9 +21,9 @@
 // Precision forms:
 //   MK_FP64  binary64 results from the FP32 pipe (render_tri_kernel): ray
 //   states in 72 bits, geodesic and sampling in float pairs, transfer sums
-//   in binary64, at most as far from a 140-bit evaluation as binary64
-//   throughout (mk_tri.cuh, mk_sample_pair.cuh).  Requests whose constants
-//   the pairs cannot hold are left to a second launch, binary64 throughout
+//   in binary64 (mk_tri.cuh, mk_sample_pair.cuh).  Requests that binary64
+//   renders more exactly, or whose constants the pairs cannot hold
+//   (pair_request), are left to a second launch, binary64 throughout
 //   (render_fp64_kernel<camera>; it returns at once when there are none).
 //   MK_MIXED three launches, A on the caller's stream, then B on it and C
 //   on a side stream forked after A and joined back after C:
@@ -856,8 +856,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Bounded wait of a whole warp (every lane calls it and gets the same
 // answer) for the phase of parity `parity` of mbarrier b: false when
 // limit_ns ran out or the block aborted.
-template <typename Shared>
-__device__ __forceinline__ bool zone_wait(unsigned long long *b, unsigned parity, const Shared &zs,
+__device__ __forceinline__ bool zone_wait(unsigned long long *b, unsigned parity, const ZoneShared &zs,
                                           unsigned long long limit_ns) {
     const unsigned FULL = 0xffffffffu;
     // the common case, a phase already complete, reads no timer
@@ -893,8 +892,7 @@ __device__ __forceinline__ bool zone_wait_fold(const ZoneShared &zs, int j, unsi
 }
 
 // a wait ran out: stop the block's other warps and count it once per warp
-template <typename Shared>
-__device__ __forceinline__ void zone_fail(Shared &zs, RenderWorkspace *ws) {
+__device__ __forceinline__ void zone_fail(ZoneShared &zs, RenderWorkspace *ws) {
     *(volatile int *)&zs.abort = 1;
     if ((threadIdx.x & 31) == 0) atomicAdd(&ws->zone_error, 1ull);
 }

@@ -7,9 +7,9 @@
 // instructions to ~2^-47 of each quantity; the emission's exponential keeps
 // its exponent apart, so faint pixels keep their digits, and the transfer
 // sums stay binary64.  A sample's error (~1e-14, times x^(1/3) through the
-// exponential) stays below what the geodesic's rounding leaves in the image
-// (1e-13 to 1e-11): images are no further from plain 64-bit arithmetic than
-// with the binary64 sampler.
+// exponential) is as large as what the pairs' geodesic leaves in the image and
+// below what binary64's leaves at the views that pair_request admits; it says
+// which, and what was measured.
 //
 // Identities used (g = eta + f l l, l null): u_i = U_i + f (l.U) l_i, l_mu
 // u^mu = gamma alpha + l.U, b^2 = (B.B + f (l.B)^2 + (B.u)^2) / (u^t)^2, so

@@ -19,10 +19,15 @@
 // rays alike, if the last approach to the horizon is taken in binary64 (in
 // triples it took longer, ~38 k cycles a step against ~31 k):
 // there k grows as 1 / (r - r_EH), and E and L, which steer the ray, are
-// small differences of its components.  TRI_NEAR is where: 0.1 M keeps
-// captured rays at 0.09-0.33 times the binary64 form's error, 0.05 M at
-// 0.23-0.81, 0.03 M at 0.28-1.6, 0.01 M at 0.57-5.5.  The fused render needs no such switch: what
-// a ray emits there is redshifted away (its images are measured instead).
+// small differences of its components.  near_distance (mk_geodesic.cu) says
+// from where.  The fused render needs no such switch: what a ray emits there
+// is redshifted away, and its images do not change with the stopping distance
+// from tol 1e-2 to 1e-8.
+//
+// That holds where binary64's own rounding of the state is large: from afar,
+// off the axes, with many short steps.  Few long steps, or a state that
+// binary64 rounds little, turn it round, and such rays stay in binary64
+// (tri_policy, fixed_range, pair_request, with the measurements).
 //
 // Error-free steps: TwoSum (Knuth, TAOCP vol. 2, 4.2.2), FastTwoSum (Dekker
 // 1971), the product error by one fused multiply-add.  Every product and sum
