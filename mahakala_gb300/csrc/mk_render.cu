@@ -1521,10 +1521,11 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
 
     bool active = false, fresh = false, ended = false;
     int slot = 0, steps = 0;
-    // The state before a step within 1 M of the horizon, or of a ray thrown out
-    // from inside it (|k| > 64, elsewhere a few), in local memory: where the
-    // step leaves the triples' range the ray ends in binary64 from there, when
-    // the block has no other left.  No other step can leave it.
+    // A ray's state with |k| > 64 (it is a few, except within ~0.03 M of the
+    // horizon and where a ray is thrown out from inside it), in local memory:
+    // where the step from it leaves the triples' range the ray ends in binary64
+    // from there, when the block has no other left.  No other step can leave it:
+    // one changes k by a few parts in div, and a camera's rays start in range.
     float kept[21];
     TriState s;
     TriPoint q;
@@ -1540,15 +1541,6 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
             bool sample = false;
             if (active || fresh) {
                 const PairConsts<TRI_REQS> C = {&sh.c[0][slot]};
-                if (fresh || dt.h > C.f(PC_NINV) || tri_sum_k(s) > 64.0f) {  // dt = -(r - r_EH) / div
-#pragma unroll
-                    for (int i = 0; i < 7; i++) {
-                        const tri t = i < 3 ? s.X[1 + i] : s.K[i - 3];
-                        kept[3 * i] = t.h;
-                        kept[3 * i + 1] = t.m;
-                        kept[3 * i + 2] = t.l;
-                    }
-                }
                 // the new state, and with it the next step's first stage,
                 // which gives r and the metric there for the rule and the sample
                 tri_step<false>(s, q, dt, C.p(PC_A), C.p(PC_AA), C.t(PC_AA), fresh);
@@ -1561,8 +1553,8 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                     fresh = active = false;
                     ended = true;
                     sh.why[tid] = !go ? why : (sh.nmax[slot] >= 2 ? MK_RAY_NAN : MK_RAY_MAXSTEPS);
-                } else if (tri_left_range(s, q.r.h)) {
-                    fresh = active = false;
+                } else if (!fresh && tri_left_range(s, q.r.h)) {
+                    active = false;
                     ended = true;
                     sh.why[tid] = TRI_LOST;
                 } else if (fresh) {
@@ -1588,6 +1580,15 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                 if (!active && !ended) {
                     ended = true;
                     sh.why[tid] = go ? MK_RAY_MAXSTEPS : why;
+                }
+                if (k > 64.0f) {
+#pragma unroll
+                    for (int i = 0; i < 7; i++) {
+                        const tri t = i < 3 ? s.X[1 + i] : s.K[i - 3];
+                        kept[3 * i] = t.h;
+                        kept[3 * i + 1] = t.m;
+                        kept[3 * i + 2] = t.l;
+                    }
                 }
             }
             const unsigned mask = __ballot_sync(FULL, sample);
