@@ -158,25 +158,18 @@ __device__ __forceinline__ SampleView sample_view(const mk_snapshot_view &sv) {
     return {sv.blocks, sv.geom, sv.faces, sv.table, sv.blocks64 ? sv.block64 : nullptr, {sv.nb[0], sv.nb[1], sv.nb[2]}, sv.n};
 }
 
-// On which side of a block's faces at f[0] and f[1] x lies (left < x <= right):
-// 0 between them.  The difference of triples has its sign to the state's 72
-// bits.
-static __device__ __noinline__ int face_side(const double *f, tri x) {
-    if (t_sub(x, t_from(__ldg(f))).h <= 0.0f) return -1;
-    return t_sub(x, t_from(__ldg(f + 1))).h > 0.0f ? 1 : 0;
-}
-// Whether block mb and its neighbour across the left (sides bit 2a) or right
-// (bit 2a + 1) face of each axis share that face to the bit; where they do
-// not, both or neither may hold a point next to it.
-static __device__ __noinline__ bool faces_shared(const SampleView &sv, int mb, int c0, int c1, int c2, unsigned sides) {
-    for (int i = 0; i < 6; i++) {
-        if (!((sides >> i) & 1u)) continue;
-        const int step = (i & 1) ? 1 : -1;
-        const int o[3] = {c0 + (i / 2 == 0 ? step : 0), c1 + (i / 2 == 1 ? step : 0), c2 + (i / 2 == 2 ? step : 0)};
-        const int nb = table_at(sv, o);
-        if (nb >= 0 && __ldg(sv.faces + 6 * (int64_t)mb + i) != __ldg(sv.faces + 6 * (int64_t)nb + (i ^ 1))) return false;
-    }
-    return true;
+// Beside face i of block mb at table cell c (0, 1: left and right in x; ...): on
+// which side of the block x lies, 0 in it (left < x <= right; the difference of
+// triples has its sign to the state's 72 bits).  2: the neighbour there does not
+// share the face to the bit, so both or neither may hold the point.
+static __device__ __noinline__ int near_face(const SampleView &sv, int mb, int c0, int c1, int c2, int i, tri x) {
+    const double face = __ldg(sv.faces + 6 * (int64_t)mb + i);
+    const int step = (i & 1) ? 1 : -1, a = i >> 1;
+    const int o[3] = {c0 + (a == 0 ? step : 0), c1 + (a == 1 ? step : 0), c2 + (a == 2 ? step : 0)};
+    const int nb = table_at(sv, o);
+    const float d = t_sub(x, t_from(face)).h;
+    if (nb >= 0 && __ldg(sv.faces + 6 * (int64_t)nb + (i ^ 1)) != face) return 2;
+    return (i & 1) ? d > 0.0f : -(d <= 0.0f);
 }
 
 // The cell of x: the block whose faces enclose it (left < x <= right) and the
@@ -193,10 +186,12 @@ __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConst
     bool beside = false;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float lo = C.f(PC_BOX + a), hi = C.f(PC_BOX + 3 + a), iw = C.f(PC_INVW + a), u = (x[a].h - lo) * iw;
+        const float lo = C.f(PC_BOX + a), hi = C.f(PC_BOX + 3 + a), iw = C.f(PC_INVW + a);
         if (!(x[a].h >= lo && x[a].h <= hi)) return -1;
-        // within the box's margin (1e-5 of its coordinates) and a rounding of a face
-        if (fabsf(u - rintf(u)) <= 2e-5f * (fabsf(lo) + fabsf(hi)) * iw) beside = true;
+        // the box's margin is 1e-5 of its coordinates; twice that off, so that a
+        // point on a face, which is in the block below, finds that block at once
+        const float tol = 2e-5f * (fabsf(lo) + fabsf(hi)) * iw, u = (x[a].h - lo) * iw - tol;
+        if (fabsf(u - rintf(u)) <= 1.5f * tol) beside = true;
         c[a] = max(0, min((int)u, sv.nb[a] - 1));
     }
     const float n = (float)sv.n;
@@ -204,8 +199,8 @@ __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConst
         const int mb = table_at(sv, c);
         if (mb < 0) return it == 0 && beside ? -2 : -1;
         const double *g = sv.geom + 6 * (int64_t)mb;
+        const int at[3] = {c[0], c[1], c[2]};
         bool moved = false;
-        unsigned sides = 0;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             const tri left = t_from(__ldg(g + a)), d = t_near(__ldg(g + 3 + a));
@@ -214,8 +209,8 @@ __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConst
             const float e0 = f_add(f_add(t.h, 0.5f), t.l), e1 = f_add(f_sub(t.h, n - 0.5f), t.l);
             int side = e0 < 0.0f ? -1 : (e1 > 0.0f ? 1 : 0);
             if (fminf(fabsf(e0), fabsf(e1)) < 1e-9f) {
-                side = face_side(sv.faces + 6 * (int64_t)mb + 2 * a, x[a]);
-                sides |= (fabsf(e0) < fabsf(e1) ? 1u : 2u) << (2 * a);
+                side = near_face(sv, mb, at[0], at[1], at[2], 2 * a + (fabsf(e1) < fabsf(e0)), x[a]);
+                if (side == 2) return -2;
             }
             c[a] += side;
             if (side) moved = true;
@@ -230,7 +225,7 @@ __device__ __forceinline__ int locate_pair(const SampleView &sv, const PairConst
             const pr u = p_norm({uh, f_add(f_add(ul, fmaf(-fl, d.m, s.m)), -e)});
             del[a] = p_mulr(u, iw);
         }
-        if (!moved) return sides && !faces_shared(sv, mb, c[0], c[1], c[2], sides) ? -2 : mb;
+        if (!moved) return mb;
     }
     return -2;
 }
