@@ -32,19 +32,18 @@ __global__ void camera_points_kernel(const double *__restrict__ xs, const double
 }
 
 // Distance to the horizon below which a step's accelerations are binary64 (see
-// mk_tri.cuh).  A fast hole's rays linger near its horizon, and a ray stopped
-// farther out has fewer binary64 steps behind it.  End states of captured rays,
-// times as far from a 64-bit-significand integration as binary64's (geometric
-// mean of 40 to 80 rays) with 0.1, 0.3 and 1 M: spin 0.94 0.7-1.4, 0.3-0.7,
-// 0.3-0.6; spin 0.998 3.5-4.6, 1.6-1.8, 0.8-1.3; tol 1e-2 at spins 0 to 0.94
-// 1.6-3.1, 0.8-1.0, 0.3-0.5.  Slower holes at tol <= 1e-4: 0.06-0.7 with 0.1 M.
-// A step costs ~31 k cycles instead of ~7.5 k: 40^2 rays 10.6, 11.7 and 14.0 ms.
+// mk_tri.cuh): a ray stopped farther out has fewer binary64 steps behind it.
+// End states of captured rays, times as far from a 64-bit-significand
+// integration as binary64's (geometric mean of 40 to 80 rays) with 0.1 and 0.3
+// M: tol 1e-2 at spins 0 to 0.94 1.6-3.1 and 0.8-1.0; tol <= 1e-4 0.06-0.7 up to
+// spin 0.5 and 0.7-1.4 at 0.94 with 0.1 M.
 constexpr float TRI_NEAR = 0.1f;
-static float near_distance(double a, double tol) {
-    const double s = fabs(a);
-    const float d = s <= 0.8 ? TRI_NEAR : (s <= 0.97 ? 0.3f : 1.0f);
-    return tol > 2e-4 ? fmaxf(d, 0.3f) : d;
-}
+static float near_distance(double tol) { return tol > 2e-4 ? 0.3f : TRI_NEAR; }
+// Above this spin the reference rule's rays linger near the horizon: at 0.998
+// their last wavevectors are 3.5-4.6, 1.6-1.8 and 0.8-1.3 times as far off with
+// 0.1, 0.3 and 1 M, and 128^2 rays take 65, 70 and 80 ms.  In binary64 from the
+// start they take 55.  Below it (spins 0.9, 0.92, 0.95) 0.1 M gives 0.2-1.2.
+constexpr double TRI_MAX_SPIN = 0.95;
 
 __device__ __forceinline__ bool tri_range(const double s[8]) {
     const double k = fmax(fmax(fabs(s[4]), fabs(s[5])), fmax(fabs(s[6]), fabs(s[7])));
@@ -377,7 +376,7 @@ __device__ __noinline__ void shadow_ray_f64(const double start[8], int64_t p, do
 // 18 ms with 0.3 M, 9.2 without); without, in pairs down to the 1e-2 M where it
 // stops, for the sides of the shadow's edge they lie on.  Radii at the horizon, in pairs and with NEAR,
 // against long double, median: spin 0.94 2.6e-15, 6e-16 (binary64 7e-16); spin
-// 0.998 4.2e-14, 1.3e-15 (4e-15).
+// 0.998 4.2e-14, 1.3e-15 with 1 M (4e-15; NEAR takes it there).
 template <bool NEAR>
 __global__ void __launch_bounds__(GEO_THREADS)
 shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa, const double *__restrict__ mid,
@@ -390,7 +389,7 @@ shadow_pass_kernel(const double *__restrict__ ca, const double *__restrict__ sa,
     if (lane >= rpw || p >= n) return;
     double s64[8];
     camera_pixel(ca[p] * mid[p], sa[p] * mid[p], ci, si, dist, a, s64);
-    bool out = !tri_range(s64);
+    bool out = !tri_range(s64) || (NEAR && fabs(a) > TRI_MAX_SPIN);
     TriState s;
     tri_state(s64, s);
     const tri none = {NAN, NAN, NAN};
@@ -477,8 +476,8 @@ static unsigned ray_grid(int64_t n, int rpw) {
 // means, spins 0.5 and 0.94, escaped and captured): div 1 29-33, 2 2.2-2.5, 4
 // 1.1-1.7, 7 0.6-0.9, 10 0.4-0.7, 40 0.1-0.7.  The fixed rule from 1000 M at 60
 // deg: hfrac 0.5 1.0-5.4, 0.2 0.7-1.1, 0.05 0.2, 0.01 0.1.
-static bool tri_policy(const mk_step_policy &p) {
-    if (p.kind == MK_POLICY_REFERENCE) return p.div >= 7.0 && p.div <= 1e6 && p.tol >= 1e-12;
+static bool tri_policy(const mk_step_policy &p, double a) {
+    if (p.kind == MK_POLICY_REFERENCE) return fabs(a) <= TRI_MAX_SPIN && p.div >= 7.0 && p.div <= 1e6 && p.tol >= 1e-12;
     return p.hfrac >= 1e-6 && p.hfrac <= 0.1 && p.hmin >= 1e-9 && p.hmax >= 1e-9 && p.hmin <= 0.2;
 }
 
@@ -519,13 +518,14 @@ static int integrate(const double *s0_dev, int64_t npx, double bhspin, const mk_
         const auto kernel = rows_dev || dt_dev ? integrate_reference_kernel<true> : integrate_reference_kernel<false>;
         kernel<<<ray_grid(npx, rpw), GEO_THREADS, 0, st>>>(
             s0_dev, npx, bhspin, spin_tri(bhspin), rule_tri(bhspin, policy->div, policy->tol),
-            near_distance(bhspin, policy->tol), policy->nmax, policy->div, policy->tol, rows_dev, dt_dev, K_dev, why_dev, state_dev, rpw, !tri_policy(*policy));
+            near_distance(policy->tol), policy->nmax, policy->div, policy->tol, rows_dev, dt_dev, K_dev, why_dev,
+            state_dev, rpw, !tri_policy(*policy, bhspin));
         MK_LAUNCHED("integrate_reference_kernel");
     } else if (policy->kind == MK_POLICY_FIXED) {
         MK_REQUIRE(!rows_dev && !dt_dev, MK_ERR_UNSUPPORTED, "mk_integrate: rows only for the reference policy");
         integrate_fixed_kernel<<<ray_grid(npx, rpw), GEO_THREADS, 0, st>>>(
             s0_dev, npx, bhspin, policy->nmax, policy->hfrac, policy->hmin, policy->hmax, policy->capture,
-            policy->r_escape, K_dev, why_dev, state_dev, rpw, !tri_policy(*policy));
+            policy->r_escape, K_dev, why_dev, state_dev, rpw, !tri_policy(*policy, bhspin));
         MK_LAUNCHED("integrate_fixed_kernel");
     } else {
         MK_REQUIRE(false, MK_ERR_ARG, "mk_integrate: unknown policy %d", (int)policy->kind);
@@ -588,7 +588,7 @@ static int shadow(const char *name, const double *cos_dev, const double *sin_dev
     const int rpw = rays_per_warp(n);
     shadow_pass_kernel<NEAR><<<ray_grid(n, rpw), GEO_THREADS, 0, as_stream(stream)>>>(
         cos_dev, sin_dev, mid_dev, n, bhspin, spin_tri(bhspin), rule_tri(bhspin, 40.0, 1e-2),
-        near_distance(bhspin, 1e-2), cos_inc, sin_inc, distance, max_steps, K_dev, best_dev, best_dt_dev, r_km1_dev,
+        near_distance(1e-2), cos_inc, sin_inc, distance, max_steps, K_dev, best_dev, best_dt_dev, r_km1_dev,
         r_best_dev, r_last_dev, rpw);
     MK_LAUNCHED("shadow_pass_kernel");
     return MK_OK;
