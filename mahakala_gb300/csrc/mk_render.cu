@@ -1524,9 +1524,10 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
     // A ray's state with |k| > 64 (it is a few, except within ~0.03 M of the
     // horizon and where a ray is thrown out from inside it), in local memory:
     // where the step from it leaves the triples' range the ray ends in binary64
-    // from there, when the block has no other left.  No other step can leave it:
-    // one changes k by a few parts in div, and a camera's rays start in range.
-    float kept[21];
+    // from there, when the block has no other left.  The last word is the steps it
+    // took: a ray lost from a state that was not kept (no step seen changes k so
+    // much) is left to render_fp64_kernel, from its start.
+    float kept[22];
     TriState s;
     TriPoint q;
     tri dt = {0.0f, 0.0f, 0.0f};
@@ -1581,7 +1582,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                     ended = true;
                     sh.why[tid] = go ? MK_RAY_MAXSTEPS : why;
                 }
-                if (k > 64.0f) {
+                if (active && k > 64.0f) {
 #pragma unroll
                     for (int i = 0; i < 7; i++) {
                         const tri t = i < 3 ? s.X[1 + i] : s.K[i - 3];
@@ -1589,6 +1590,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                         kept[3 * i + 1] = t.m;
                         kept[3 * i + 2] = t.l;
                     }
+                    kept[21] = __int_as_float(steps);
                 }
             }
             const unsigned mask = __ballot_sync(FULL, sample);
@@ -1699,7 +1701,8 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
 #pragma unroll
             for (int ch = 0; ch < MK_MAX_NU; ch++) I[ch] = sh.I[ch][tid];
             const int64_t pix = fetch_pixel(R.camera, sh.ray[tid] - R.ray_offset);
-            const int at = sh.why[tid] == TRI_LOST ? atomicAdd(&sh.nlost, 1) : -1;
+            const int at = sh.why[tid] != TRI_LOST ? -1
+                           : __float_as_int(kept[21]) == steps ? atomicAdd(&sh.nlost, 1) : TRI_LOST_MAX;
             if (at < 0) {
                 finish_ray(R, pix, I, steps, sh.why[tid], sh.samples[tid], __longlong_as_double(sh.tau[tid]), ws);
             } else if (at < TRI_LOST_MAX) {
@@ -1716,7 +1719,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                     l.I[ch] = I[ch];
                     l.P[ch] = sh.P[ch][tid];
                 }
-            } else {  // more than the block has room for: from its start
+            } else {  // not kept, or more than the block has room for: from its start
                 R.image[pix] = __longlong_as_double((long long)RAY_LEFT);
                 atomicAdd(&ws->odd_rays, 1ull);
             }
@@ -1731,6 +1734,7 @@ render_tri_kernel(const mk_request *__restrict__ reqs, int nreq, long long total
                 sh.slot[tid] = slot;
                 sh.ray[tid] = sh.nxt[tid];
                 steps = sh.samples[tid] = 0;
+                kept[21] = __int_as_float(-1);
                 sh.tau[tid] = 0;
                 fresh = true;
 #pragma unroll

@@ -231,10 +231,11 @@ def test_request_of_too_many_frequencies(cuda):
 
 
 # a step over the horizon (here the rule stops this far above it) overflows
-# floats before doubles; the last: more such rays than a block has room for
+# floats before doubles; the fifth: more such rays than a block has room for;
+# the last: its components are out of range, but finite
 @pytest.mark.parametrize("spin,tol,div,half,res", [(-0.9, 1e-4, 40.0, 10.0, 48), (0.5, 1e-6, 40.0, 10.0, 48),
                                                    (0.5, 1e-8, 40.0, 10.0, 48), (0.94, 1e-8, 40.0, 10.0, 48),
-                                                   (0.5, 1e-8, 10.0, 5.0, 200)])
+                                                   (0.5, 1e-8, 10.0, 5.0, 200), (0.1, 1e-8, 20.0, 6.0, 64)])
 def test_fp64_image_stop_reasons_at_the_horizon(cuda, orc, spin, tol, div, half, res):
     from mahakala_gb300.grmhd.synthetic import make_synthetic_snapshot
     from mahakala_gb300.images import RenderRequest, render_requests
