@@ -249,7 +249,7 @@ def cpu_baseline(spec, arrays, rays_wanted, threads):
     subset of the same image; returns (rays/s, sample description, oracle
     run).  The oracle run -- its image, steps and pixel indices, plus an
     untimed second run with each initial wavevector perturbed by 1e-12 that
-    tells well-conditioned rays from grazing ones -- is the checker the
+    tells well-conditioned rays from grazing ones -- is what the
     FP64 GPU image is compared against."""
     import oracle
     os.environ["OMP_NUM_THREADS"] = str(threads)
