@@ -103,14 +103,16 @@ def mesh_tables(arrs, max_table_cells=1 << 28):
                 taken += cells.size
             continue
         # the table cells of these blocks, cut at the table's edge as a slice is
-        for part in np.array_split(m, -(-len(m) * sx * sy * sz // (1 << 18))):
+        some = (1 << 18) // (sx * sy * sz)
+        for part in (m[b:b + some] for b in range(0, len(m), some)):
             i, j, k = (start[part, a, None, None, None] + np.arange(n).reshape(sh) for a, n, sh in
                        ((0, sx, (1, 1, 1, -1)), (1, sy, (1, 1, -1, 1)), (2, sz, (1, -1, 1, 1))))
             ok = (i < nb[0]) & (j < nb[1]) & (k < nb[2])
             flat = ((k * nb[1] + j) * nb[0] + i)[ok]
             taken += flat.size
             table.reshape(-1)[flat] = np.broadcast_to(part[:, None, None, None], ok.shape)[ok]
-    if sum(np.count_nonzero(plane >= 0) for plane in table) != taken:  # a cell taken twice
+    some = max(1, (1 << 18) // (nb[0] * nb[1]))
+    if sum(np.count_nonzero(table[k:k + some] >= 0) for k in range(0, len(table), some)) != taken:  # one taken twice
         raise ValueError("overlapping blocks")
     fine_ghosts = np.zeros(nmb, bool)
     if np.any(levels != levels[0]):
